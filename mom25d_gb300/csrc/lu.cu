@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "m25_internal.h"
+#include "m25_lu.h"
 
 namespace m25 {
 
@@ -248,324 +249,10 @@ __global__ void __launch_bounds__(256) panel_kernel(PanelArgs<T> a) {
   }
 }
 
-// ------------------------------------------------ panel on one CTA cluster
-// For trailing sizes whose panel fits in the shared memory of one cluster of
-// CL CTAs (16, the largest cluster size: about 6500 rows of
-// 64 complex64 columns), the panel is factored without global barriers. CTA q
-// of the cluster keeps rows k0 + q R .. + R - 1 in shared memory. Per column
-// j, every CTA pushes its pivot candidate (value, row index and the whole
-// row) into the shared memory of all 16 CTAs, and the owner of row j pushes
-// row j as well; one hardware cluster barrier later every CTA holds all it
-// needs locally: it picks the pivot (max |re| + |im|, first index on ties,
-// as panel_kernel), the two owners swap rows p and j in place, and every CTA
-// scales and updates its own rows, finding the next column's candidate while
-// it updates. The pushed data is double-buffered by column parity: a CTA can
-// only write column j + 2's buffers after every CTA has passed column j + 1's
-// barrier, that is, after all reads of column j's buffers.
-constexpr int kPanelCluster = 16;  // the largest cluster; smaller trailing blocks take 8 or 4 CTAs
-constexpr int kPanelLd = 65;  // padded row of the panel in shared memory
-
-template <class T>
-struct ClusterPanelArgs {
-  cx<T>* A;
-  int64_t lda;
-  int n, k0, nb, rows_per_cta;
-  int32_t* ipiv;
-  int* info;
-  int* err;  // a wait for pushed data ran out
-  float* A2; // tensor-core update: tf32 [hi | lo] planes of conj(L21) (rows of 2 P floats), or null
-  int P;
-};
-
 __device__ __forceinline__ float tf32_rna(float x) {
   uint32_t r;
   asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(r) : "f"(x));
   return __uint_as_float(r);
-}
-
-template <class T>
-struct alignas(16) PivCand {
-  T val;
-  int idx;
-};
-
-template <class T, int CL>
-constexpr size_t cluster_panel_smem(int R) {
-  // rows + candidate rows (2 x CL x 64) + row j (2 x 64)
-  return sizeof(cx<T>) * ((size_t)R * kPanelLd + 2 * CL * 64 + 2 * 64);
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-  return r;
-}
-// the address of a shared variable of this CTA in the shared memory of cluster CTA rank
-__device__ __forceinline__ uint32_t dsmem(const void* p, uint32_t rank) {
-  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-// remote store that completes its bytes on the destination CTA's mbarrier
-__device__ __forceinline__ void st_async(uint32_t a, cx<float> v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];\n" ::"r"(a),
-               "f"(v.re), "f"(v.im), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void st_async(uint32_t a, cx<double> v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];\n" ::"r"(a),
-               "d"(v.re), "d"(v.im), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void st_async(uint32_t a, PivCand<float> v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];\n" ::"r"(a),
-               "r"(__float_as_uint(v.val)), "r"(v.idx), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void st_async(uint32_t a, PivCand<double> v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];\n" ::"r"(a),
-               "l"(__double_as_longlong(v.val)), "l"((long long)v.idx), "r"(bar)
-               : "memory");
-}
-// bytes of one pushed candidate record
-template <class T>
-constexpr int cand_push_bytes() {
-  return sizeof(T) == 4 ? 8 : 16;
-}
-__device__ __forceinline__ void cl_mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(count));
-}
-__device__ __forceinline__ void cl_mbar_expect(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
-                   (uint32_t)__cvta_generic_to_shared(bar)),
-               "r"(bytes)
-               : "memory");
-}
-// bounded wait (iterations and wall clock) for the phase of the given parity
-// of a barrier completed by remote transactions; false on a timeout
-__device__ __forceinline__ bool cl_mbar_wait(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = (uint32_t)__cvta_generic_to_shared(bar);
-  unsigned long long t0;
-  asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t0));
-  for (long long it = 0; it < kBarrierSpinLimit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-    if (t - t0 > 500ull * 1000 * 1000) return false;
-  }
-  return false;
-}
-
-// better candidate: larger value, first index on ties
-template <class T>
-__device__ __forceinline__ bool piv_better(T ov, int oi, T v, int i) {
-  return oi >= 0 && (ov > v || (ov == v && (i < 0 || oi < i)));
-}
-
-constexpr int kPanelThreads = 512;
-constexpr int kPanelGroups = kPanelThreads / 64;  // row groups of the update's 2-D map
-
-template <class T, int CL>
-__global__ void __launch_bounds__(kPanelThreads, 1) panel_cluster_kernel(ClusterPanelArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int q = (int)cluster_rank(), nb = a.nb, R = a.rows_per_cta, tid = threadIdx.x;
-  const int r0 = a.k0 + q * R;
-  const int r1 = min(a.n, r0 + R);
-  const int Rq = max(0, r1 - r0);
-  cx<T>* P = reinterpret_cast<cx<T>*>(smem_raw);          // (R, kPanelLd) this CTA's rows
-  cx<T>* crow = P + (size_t)R * kPanelLd;                   // (2, 16, 64) pushed candidate rows
-  cx<T>* jrow = crow + 2 * CL * 64;              // (2, 64) pushed row k0 + j
-  __shared__ PivCand<T> cand[2][CL];             // pushed candidates
-  __shared__ T gmax_v[kPanelGroups];
-  __shared__ int gmax_i[kPanelGroups];
-  __shared__ __align__(8) uint64_t colbar[2];  // per column parity: completed by the 16 CTAs' pushes
-  if (tid == 0) {
-    cl_mbar_init(&colbar[0], 1);
-    cl_mbar_init(&colbar[1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  for (int e = tid; e < Rq * 64; e += blockDim.x) {
-    const int r = e >> 6, c = e & 63;
-    if (c < nb) P[r * kPanelLd + c] = a.A[(int64_t)(r0 + r) * a.lda + a.k0 + c];
-  }
-  // 2-D map of the update: column uc, rows ug, ug + kPanelGroups, ...
-  const int uc = tid & 63, ug = tid >> 6;
-  __syncthreads();
-  // candidate of column 0 (afterwards found during each update)
-  if (uc == 0) {
-    T bv = T(-1);
-    int bi = -1;
-    for (int r = ug; r < Rq; r += kPanelGroups) {
-      const T v = cabs1(P[r * kPanelLd]);
-      if (v > bv) {
-        bv = v;
-        bi = r0 + r;
-      }
-    }
-    gmax_v[ug] = bv;
-    gmax_i[ug] = bi;
-  }
-  __syncthreads();
-  cluster_sync_all();  // every CTA runs, with its barriers set up, before the first push
-  // bytes pushed into each CTA per column: 16 candidates, 16 rows, row j
-  const uint32_t expect = CL * (cand_push_bytes<T>() + nb * (int)sizeof(cx<T>)) + nb * sizeof(cx<T>);
-  for (int j = 0; j < nb; ++j) {
-    const int row_j = a.k0 + j, par = j & 1;
-    const int qj = j / R;
-    // this CTA's candidate for column j (rows >= row_j)
-    T bv = T(-1);
-    int bi = -1;
-#pragma unroll
-    for (int g = 0; g < kPanelGroups; ++g)
-      if (piv_better(gmax_v[g], gmax_i[g], bv, bi)) {
-        bv = gmax_v[g];
-        bi = gmax_i[g];
-      }
-    // push: candidate, candidate row (zeros without a candidate), and row j
-    // from its owner, into all 16 CTAs; each store completes its bytes on
-    // the destination's barrier of this column's parity
-    if (tid == 0) cl_mbar_expect(&colbar[par], expect);
-    if (tid < CL) st_async(dsmem(&cand[par][q], tid), PivCand<T>{bv, bi}, dsmem(&colbar[par], tid));
-    for (int e = tid; e < CL * 64; e += blockDim.x) {
-      const int dst = e >> 6, c = e & 63;
-      if (c < nb)
-        st_async(dsmem(&crow[(par * CL + q) * 64 + c], dst),
-                 bi >= 0 ? P[(bi - r0) * kPanelLd + c] : cx<T>(), dsmem(&colbar[par], dst));
-    }
-    if (q == qj)
-      for (int e = tid; e < CL * 64; e += blockDim.x) {
-        const int dst = e >> 6, c = e & 63;
-        if (c < nb)
-          st_async(dsmem(&jrow[par * 64 + c], dst), P[(row_j - r0) * kPanelLd + c], dsmem(&colbar[par], dst));
-      }
-    // wait until all of column j's pushes have landed here
-    const bool got = cl_mbar_wait(&colbar[par], (j >> 1) & 1);
-    if (__syncthreads_or(!got)) {
-      if (tid == 0) atomicExch(a.err, 1);
-      break;
-    }
-    // every thread picks the pivot from the 16 local candidates
-    T v = T(-1);
-    int p = -1, src = -1;
-#pragma unroll
-    for (int k = 0; k < CL; ++k) {
-      const PivCand<T> c = cand[par][k];
-      if (piv_better(c.val, c.idx, v, p)) {
-        v = c.val;
-        p = c.idx;
-        src = k;
-      }
-    }
-    if (p < 0 || v == T(0)) {  // zero column: no interchange, no scaling
-      if (tid == 0 && q == 0 && *a.info == 0) *a.info = row_j + 1;
-      p = row_j;
-      src = -1;
-    }
-    if (tid == 0 && q == 0) a.ipiv[row_j] = p;
-    const cx<T>* urow = src >= 0 ? crow + (par * CL + src) * 64 : jrow + par * 64;
-    if (p != row_j) {
-      if (p >= r0 && p < r1)
-        for (int c = tid; c < nb; c += blockDim.x) P[(p - r0) * kPanelLd + c] = jrow[par * 64 + c];
-      if (q == qj)
-        for (int c = tid; c < nb; c += blockDim.x) P[(row_j - r0) * kPanelLd + c] = urow[c];
-    }
-    __syncthreads();
-    // multipliers (rows below row j), by the reciprocal pivot
-    if (src >= 0) {
-      const cx<T> pv = urow[j];
-      const T m2 = pv.re * pv.re + pv.im * pv.im;
-      const cx<T> rp(pv.re / m2, -pv.im / m2);
-      for (int r = tid; r < Rq; r += blockDim.x)
-        if (r0 + r > row_j) P[r * kPanelLd + j] = P[r * kPanelLd + j] * rp;
-    }
-    __syncthreads();
-    // rank-1 update of the columns right of j, four rows at a time (loads
-    // first); the threads of column j + 1 track the next candidate
-    {
-      T gv = T(-1);
-      int gi = -1;
-      if (uc > j && uc < nb) {
-        const cx<T> u = urow[uc];
-        // first row below row j in this group
-        int r = ug;
-        const int rlo = row_j + 1 - r0;
-        if (r < rlo) r += (rlo - r + kPanelGroups - 1) / kPanelGroups * kPanelGroups;
-        for (; r + 3 * kPanelGroups < Rq; r += 4 * kPanelGroups) {
-          cx<T> x[4], m[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            x[i] = P[(r + i * kPanelGroups) * kPanelLd + uc];
-            m[i] = P[(r + i * kPanelGroups) * kPanelLd + j];
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            x[i] -= m[i] * u;
-            P[(r + i * kPanelGroups) * kPanelLd + uc] = x[i];
-          }
-          if (uc == j + 1)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const T cv = cabs1(x[i]);
-              if (cv > gv) {
-                gv = cv;
-                gi = r0 + r + i * kPanelGroups;
-              }
-            }
-        }
-        for (; r < Rq; r += kPanelGroups) {
-          const cx<T> x = P[r * kPanelLd + uc] - P[r * kPanelLd + j] * u;
-          P[r * kPanelLd + uc] = x;
-          if (uc == j + 1) {
-            const T cv = cabs1(x);
-            if (cv > gv) {
-              gv = cv;
-              gi = r0 + r;
-            }
-          }
-        }
-      }
-      if (uc == j + 1) {
-        gmax_v[ug] = gv;
-        gmax_i[ug] = gi;
-      }
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < Rq * 64; e += blockDim.x) {
-    const int r = e >> 6, c = e & 63;
-    if (c < nb) a.A[(int64_t)(r0 + r) * a.lda + a.k0 + c] = P[r * kPanelLd + c];
-  }
-  if (a.A2) {
-    // the trailing rows as the tensor-core update's A operand: real and minus
-    // imaginary parts of L21 interleaved (j = 2 t + f), split into tf32 hi
-    // and lo planes P floats apart, zero beyond the panel's 2 nb columns
-    for (int e = tid; e < Rq * a.P; e += blockDim.x) {
-      const int r = e / a.P, j = e - r * a.P, t = j >> 1;
-      const int row = r0 + r - (a.k0 + nb);
-      if (row < 0) continue;
-      float hi = 0.f, lo = 0.f;
-      if (t < nb) {
-        const cx<T> L = P[r * kPanelLd + t];
-        const float v = (j & 1) ? -(float)L.im : (float)L.re;
-        hi = tf32_rna(v);
-        lo = tf32_rna(v - hi);
-      }
-      a.A2[(int64_t)row * 2 * a.P + j] = hi;
-      a.A2[(int64_t)row * 2 * a.P + a.P + j] = lo;
-    }
-  }
-  // no CTA leaves while a peer may still store into its shared memory
-  cluster_sync_all();
 }
 
 // The panel's row interchanges applied to the columns outside it, fused with
@@ -939,96 +626,23 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
     int rc = lu_tc_prepare(ctx, n);
     if (rc) return rc;
   }
-  // the cluster panel: the smallest cluster (4, 8 or 16 CTAs) whose shared
-  // memory holds the trailing rows; the exchange per column grows with the
-  // square of the cluster size, and small clusters are easier to place next
-  // to the kernels of concurrent sweeps
-  int cl_rows[3] = {0, 0, 0};  // rows that fit in clusters of 4, 8, 16
-  {
-    int optin = 0;
-    M25_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    const size_t avail = (size_t)optin - 1024;  // static shared variables
-    auto rows_of = [&](size_t smem0) {
-      return nb > 64 ? 0 : (int)((avail - smem0) / ((size_t)kPanelLd * sizeof(cx<T>)));
-    };
-    // decided once (thread-safe initialisation: sweeps on several threads)
-    static const bool ok = [avail] {
-      bool yes = false;
-      const char* off = getenv("M25_NO_CLUSTER_PANEL");
-      if (!(off && *off == '1') &&
-          cudaFuncSetAttribute(panel_cluster_kernel<T, 16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-              cudaSuccess &&
-          cudaFuncSetAttribute(panel_cluster_kernel<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail) ==
-              cudaSuccess &&
-          cudaFuncSetAttribute(panel_cluster_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail) ==
-              cudaSuccess &&
-          cudaFuncSetAttribute(panel_cluster_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail) ==
-              cudaSuccess) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 16;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(16);
-        cfg.blockDim = dim3(kPanelThreads);
-        cfg.dynamicSmemBytes = avail;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int nclusters = 0;
-        yes = cudaOccupancyMaxActiveClusters(&nclusters, panel_cluster_kernel<T, 16>, &cfg) == cudaSuccess &&
-              nclusters > 0;
-      }
-      cudaGetLastError();  // a refused attribute only means: no cluster panel
-      return yes;
-    }();
-    // M25_PANEL_CLUSTER_MIN: the smallest cluster size used (4, 8 or 16; a tuning knob)
-    static const int cl_min_env = [] {
-      const char* e = getenv("M25_PANEL_CLUSTER_MIN");
-      const int v = e ? atoi(e) : 4;
-      return v >= 16 ? 16 : v >= 8 ? 8 : 4;
-    }();
-    // the context's setting (m25_ctx_set_tuning) over the process default
-    const int cl_min = ctx->tune_cluster_min >= 16 ? 16
-                       : ctx->tune_cluster_min >= 8 ? 8
-                       : ctx->tune_cluster_min > 0  ? 4
-                                                    : cl_min_env;
-    if (ok) {
-      cl_rows[0] = cl_min <= 4 ? 4 * rows_of(cluster_panel_smem<T, 4>(0)) : 0;
-      cl_rows[1] = cl_min <= 8 ? 8 * rows_of(cluster_panel_smem<T, 8>(0)) : 0;
-      cl_rows[2] = 16 * rows_of(cluster_panel_smem<T, 16>(0));
-    }
-  }
-  // one panel of w <= nb columns at k0 over the rows k0 .. n - 1; A2 / P2:
-  // the tensor-core operand planes of its trailing rows (cluster panel only),
-  // *packed tells whether they were written
-  auto run_panel = [&](int k0, int w, float* A2, int P2, bool* packed) -> int {
+  // blocks of up to strip_rows rows are factored by one cluster (lu_panel.cu), taller ones panel by
+  // panel on a cooperative grid
+  const int strip_rows = lu_strip_rows<T>(ctx);
+  // M25_PANEL_CLUSTER_MIN: the smallest cluster size used (4, 8 or 16; a tuning knob)
+  static const int cl_min_env = [] {
+    const char* e = getenv("M25_PANEL_CLUSTER_MIN");
+    const int v = e ? atoi(e) : 4;
+    return v >= 16 ? 16 : v >= 8 ? 8 : 4;
+  }();
+  // the context's setting (m25_ctx_set_tuning) over the process default
+  const int cl_min = ctx->tune_cluster_min >= 16 ? 16
+                     : ctx->tune_cluster_min >= 8 ? 8
+                     : ctx->tune_cluster_min > 0  ? 4
+                                                  : cl_min_env;
+  // one panel of w <= nb columns at k0 over the rows k0 .. n - 1 on a cooperative grid
+  auto run_panel = [&](int k0, int w) -> int {
     const int m = n - k0;
-    const int CL = m <= cl_rows[0] ? 4 : m <= cl_rows[1] ? 8 : m <= cl_rows[2] ? 16 : 0;
-    if (packed) *packed = CL > 0 && A2;
-    if (CL > 0) {
-      ClusterPanelArgs<T> ca{A, lda, n, k0, w, (m + CL - 1) / CL, ipiv, info, err, A2, P2};
-      const size_t smem = CL == 4    ? cluster_panel_smem<T, 4>(ca.rows_per_cta)
-                          : CL == 8 ? cluster_panel_smem<T, 8>(ca.rows_per_cta)
-                                    : cluster_panel_smem<T, 16>(ca.rows_per_cta);
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = CL;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3(CL);
-      cfg.blockDim = dim3(kPanelThreads);
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = st;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      StageTimer tm(ctx, ST_PANEL);
-      if (CL == 4) M25_CUDA(cudaLaunchKernelEx(&cfg, panel_cluster_kernel<T, 4>, ca));
-      else if (CL == 8) M25_CUDA(cudaLaunchKernelEx(&cfg, panel_cluster_kernel<T, 8>, ca));
-      else M25_CUDA(cudaLaunchKernelEx(&cfg, panel_cluster_kernel<T, 16>, ca));
-      return M25_OK;
-    }
     // grid size: as many CTAs as can be co-resident, each with >= 1 row
     int occ = 0;
     G = std::min(std::min(m, ctx->num_sms), Gmax);
@@ -1105,7 +719,9 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
     // right-looking: panel, interchanges and U12, SIMT update of the trailing matrix
     for (int k0 = 0; k0 < n; k0 += nb) {
       const int w = std::min(nb, n - k0);
-      if ((rc = run_panel(k0, w, nullptr, 0, nullptr))) return rc;
+      if (n - k0 <= strip_rows) rc = lu_strip_block<T>(ctx, A, lda, n, k0, w, ipiv, info, err, cand, cl_min);
+      else rc = run_panel(k0, w);
+      if (rc) return rc;
       if ((rc = swap_trsm(k0, w, 0, n - w, nullptr, 0))) return rc;
       if (k0 + w < n) {
         const int ncol = n - k0 - w;
@@ -1130,38 +746,43 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
     if ((rc = lu_tc_buffers(ctx, n, &A3, &B3, &Ai, &Bi))) return rc;
     constexpr int kHalf = kSwapMaxW, kBlock = 2 * kSwapMaxW, kSuper = 2 * kBlock, kPW = 2 * kSuper;
     int slot = 0;
-    // one block of W <= 128 columns at c0: both panels, the first one's U12
-    // and rank-64 update on the second one's columns, each panel's
-    // interchanges on every column left of it (none on columns right of the block)
-    auto factor_block = [&](int c0, int W) -> int {
+    // one block of W <= 128 columns at c0. By one cluster: *left false, its
+    // interchanges are still to be applied to every other column. Taller
+    // ones: both panels, the first one's U12 and rank-64 update on the second
+    // one's columns, each panel's interchanges on every column left of it
+    // (none on columns right of the block), *left true
+    auto factor_block = [&](int c0, int W, bool* left) -> int {
+      *left = n - c0 > strip_rows;
+      if (!*left) return lu_strip_block<T>(ctx, A, lda, n, c0, W, ipiv, info, err, cand, cl_min);
       const int w1 = std::min(kHalf, W), w2 = W - w1;
-      bool packed = false;
       int r;
-      if ((r = run_panel(c0, w1, w2 > 0 ? Ai : nullptr, 128, &packed))) return r;
+      if ((r = run_panel(c0, w1))) return r;
       if (w2 == 0) return swap_trsm(c0, w1, 0, c0, nullptr, 0);
       if ((r = swap_trsm(c0, w1, 0, c0 + w2, Bi, 128))) return r;
       const int m1 = n - c0 - w1;
-      if (!packed && (r = lu_tc_pack_a(ctx, A, lda, c0, w1, c0 + w1, m1, 128, 128, 0, Ai))) return r;
+      if ((r = lu_tc_pack_a(ctx, A, lda, c0, w1, c0 + w1, m1, 128, 128, 0, Ai))) return r;
       if ((r = lu_tc_update(ctx, A, lda, c0 + w1, c0 + w1, m1, w2, 128, 128, Ai, Bi, slot++))) return r;
-      if ((r = run_panel(c0 + w1, w2, nullptr, 0, nullptr))) return r;
+      if ((r = run_panel(c0 + w1, w2))) return r;
       return swap_trsm(c0 + w1, w2, 0, c0 + w1, nullptr, 0);
     };
     for (int k0 = 0; k0 < n; k0 += kSuper) {
       const int SW = std::min(kSuper, n - k0), wa = std::min(kBlock, SW), wb = SW - wa;
-      if ((rc = factor_block(k0, wa))) return rc;
+      bool left;
+      if ((rc = factor_block(k0, wa, &left))) return rc;
       const int ra = k0 + wa;  // first column (and row) right of block a
-      if (ra >= n) break;      // (then wb = 0)
-      // block a's interchanges and U_a on every column right of it
-      if ((rc = swap_trsm128(k0, wa, k0, n - wa, B3, kPW, 0, ipiv, true))) return rc;
+      // block a's interchanges (on the columns left of it too, where they are
+      // still due) and U_a on every column right of it
+      if ((rc = swap_trsm128(k0, wa, left ? k0 : 0, n - wa, B3, kPW, 0, ipiv, true))) return rc;
+      if (ra >= n) break;  // (then wb = 0)
       // block a's rank-128 update of block b's columns
       if ((rc = lu_tc_pack_a(ctx, A, lda, k0, wa, ra, n - ra, 2 * kBlock, kPW, 0, A3))) return rc;
       if ((rc = lu_tc_update(ctx, A, lda, ra, ra, n - ra, wb, 2 * kBlock, kPW, A3, B3, slot++))) return rc;
-      if ((rc = factor_block(ra, wb))) return rc;
+      if ((rc = factor_block(ra, wb, &left))) return rc;
       const int t0 = k0 + SW, nt = n - t0;  // the trailing columns
-      if (nt <= 0) continue;
       float* Bt = B3 + (size_t)2 * wb * 2 * kPW;  // B rows of the trailing columns
-      // block b's interchanges on the trailing columns
-      if ((rc = swap_trsm128(ra, wb, ra, ra + nt, nullptr, 0, 0, ipiv, false))) return rc;
+      // block b's interchanges on the other columns
+      if ((rc = swap_trsm128(ra, wb, left ? ra : 0, ra + nt, nullptr, 0, 0, ipiv, false))) return rc;
+      if (nt <= 0) continue;
       // block b's rows of the trailing columns minus L_ba U_a
       if ((rc = lu_tc_pack_a(ctx, A, lda, k0, wa, ra, wb, 2 * kBlock, kPW, 0, A3))) return rc;
       if ((rc = lu_tc_update(ctx, A, lda, ra, t0, wb, nt, 2 * kBlock, kPW, A3, Bt, slot++))) return rc;

@@ -41,6 +41,14 @@ template <class T> __host__ __device__ inline cx<T> operator*(cx<T> a, T s) { re
 template <class T> __host__ __device__ inline cx<T> operator*(T s, cx<T> a) { return {a.re * s, a.im * s}; }
 template <class T> __host__ __device__ inline cx<T>& operator+=(cx<T>& a, cx<T> b) { a.re += b.re; a.im += b.im; return a; }
 template <class T> __host__ __device__ inline cx<T>& operator-=(cx<T>& a, cx<T> b) { a.re -= b.re; a.im -= b.im; return a; }
+// a - b c as four fused multiply-adds (a -= b * c takes two multiplications, two fused ones and two
+// additions: the product is rounded on its own, and complex128 pays for each on GB300's slow fp64 pipe)
+__device__ __forceinline__ cx<double> fnma(cx<double> a, cx<double> b, cx<double> c) {
+  return {fma(b.im, c.im, fma(-b.re, c.re, a.re)), fma(-b.im, c.re, fma(-b.re, c.im, a.im))};
+}
+__device__ __forceinline__ cx<float> fnma(cx<float> a, cx<float> b, cx<float> c) {
+  return {fmaf(b.im, c.im, fmaf(-b.re, c.re, a.re)), fmaf(-b.im, c.re, fmaf(-b.re, c.im, a.im))};
+}
 template <class T> __host__ __device__ inline cx<T> conj(cx<T> a) { return {a.re, -a.im}; }
 template <class T> __host__ __device__ inline T norm2(cx<T> a) { return a.re * a.re + a.im * a.im; }
 template <class T> __host__ __device__ inline T cabs1(cx<T> a) { return fabs(a.re) + fabs(a.im); }
