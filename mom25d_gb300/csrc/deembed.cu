@@ -259,122 +259,178 @@ struct FitArgs {
   double* z0;               // (P)
 };
 
-__device__ inline double warp_sum(double v) {
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ inline zd warp_sum(zd v) { return zd(warp_sum(v.re), warp_sum(v.im)); }
-
-// Residual of the wave model at gamma for the datasets of one group (all lanes
-// of the warp return the same value); optionally stores coefficients, z0.
-__device__ double wave_objective(const FitArgs& a, int grp, zd g, double Inrm, double Vnrm, bool store) {
+// Sums of four values over the warp, returned in every lane. The lanes split
+// the values between them (two additions at distance 16, one at 8, three
+// more): six additions where four separate sums take twenty, each of which
+// holds the sub-partition's fp64 unit for 64 cycles on GB300.
+__device__ __forceinline__ void warp_sum4(double (&v)[4]) {
   const int lane = threadIdx.x & 31;
-  double res = 0.0;
-  zd UV(0.0);
-  double UU = 0.0;
-  constexpr int kPer = kMaxSamples / 32;
-  zd U[kMaxDatasets][kPer];
-  int nd = 0;
-  for (int p = 0; p < a.P; ++p) {
-    if (a.group_of[p] != grp) continue;
-    const int ns = a.ns[p], off = a.s_off[p];
-    // e^{+-g s} and the QR of [e^{gs}, e^{-gs}] depend on the port only:
-    // shared by its P excitations
-    zd ep[kPer], em[kPer], q1[kPer], q2[kPer];
-    double n11 = 0;
+  const bool hi = lane & 16, hj = lane & 8;
+  const double a = (hi ? v[2] : v[0]) + __shfl_xor_sync(~0u, hi ? v[0] : v[2], 16);
+  const double b = (hi ? v[3] : v[1]) + __shfl_xor_sync(~0u, hi ? v[1] : v[3], 16);
+  double c = (hj ? b : a) + __shfl_xor_sync(~0u, hj ? a : b, 8);
+  c += __shfl_xor_sync(~0u, c, 4);
+  c += __shfl_xor_sync(~0u, c, 2);
+  c += __shfl_xor_sync(~0u, c, 1);
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      int i = lane + 32 * u;
-      if (i < ns) {
-        double sv = a.s[off + i];
-        ep[u] = cexp(g * sv);
-        // e^{-g s} = 1 / e^{g s}: one reciprocal instead of a second exp and sincos
-        const double m2 = norm2(ep[u]);
-        em[u] = zd(ep[u].re / m2, -ep[u].im / m2);
-        n11 += m2;
+  for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(~0u, c, 8 * k);
+}
+
+// The wave fit's shared memory: the group's data, loaded once, and the
+// tables and partial sums of one objective evaluation.
+constexpr int kFitWarps = 4;
+constexpr int kFitPorts = 4;  // ports of a group: members x excitations <= kMaxDatasets, excitations >= members
+constexpr int kPer = kMaxSamples / 32;
+struct FitShared {
+  double s[kFitPorts][kMaxSamples];
+  zd I[kMaxDatasets][kMaxSamples], V[kMaxDatasets][kMaxSamples], U[kMaxDatasets][kMaxSamples];
+  double e[kFitPorts][kMaxSamples], ei[kFitPorts][kMaxSamples];    // e^{Re g s} and its reciprocal
+  double cs[kFitPorts][kMaxSamples], sn[kFitPorts][kMaxSamples];   // cos, sin of Im g s
+  double part[kFitWarps][4];                                       // per warp: sum |I - fit|^2, sum conj(U) V, sum |U|^2
+  double rv[kFitWarps];                                            // per warp: sum |V - z0 U|^2
+  int port[kFitPorts], ns[kFitPorts];
+  int nmem;
+  double inv_I, inv_V;
+};
+
+// Residual of the wave model at gamma for the datasets of one group (the
+// same value in every thread of the CTA); optionally stores coefficients, z0.
+// GB300 issues an fp64 instruction of a warp over 64 cycles whatever its active
+// lanes, on each of the four sub-partitions of an SM, so what counts is the
+// chain of fp64 instructions of the busiest warp: the exponentials and the
+// sines of the ports go to different warps, then each warp takes its share of
+// the (port, excitation) datasets, with all of a port's samples in its lanes.
+__device__ double wave_objective(const FitArgs& a, FitShared& sh, zd g, bool store) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nmem = sh.nmem, nd = nmem * a.E;
+  // tables: task = (function, port)
+  for (int t = warp; t < 2 * nmem; t += kFitWarps) {
+    const int p = t >> 1, ns = sh.ns[p];
+    for (int i = lane; i < ns; i += 32) {
+      if (t & 1) {
+        double sv, cv;
+        sincos(g.im * sh.s[p][i], &sv, &cv);
+        sh.cs[p][i] = cv;
+        sh.sn[p][i] = sv;
       } else {
-        ep[u] = em[u] = zd(0.0);
-      }
-    }
-    // two-column least squares by modified Gram-Schmidt with one re-orthogonalisation
-    const double r11 = sqrt(warp_sum(n11));
-    zd r12(0.0);
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      q1[u] = ep[u] / r11;
-      r12 += conj(q1[u]) * em[u];
-    }
-    r12 = warp_sum(r12);
-    zd r12b(0.0);
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      q2[u] = em[u] - r12 * q1[u];
-      r12b += conj(q1[u]) * q2[u];
-    }
-    r12b = warp_sum(r12b);
-    double n22 = 0;
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      q2[u] -= r12b * q1[u];
-      n22 += norm2(q2[u]);
-    }
-    r12 += r12b;
-    const double r22 = sqrt(warp_sum(n22));
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) q2[u] = q2[u] / r22;
-    for (int e = 0; e < a.E; ++e, ++nd) {
-      zd Iv[kPer];
-      zd b1(0.0), b2(0.0);
-#pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        int i = lane + 32 * u;
-        Iv[u] = i < ns ? a.I[(int64_t)(off + i) * a.E + e] : zd(0.0);
-        b1 += conj(q1[u]) * Iv[u];
-        b2 += conj(q2[u]) * Iv[u];
-      }
-      b1 = warp_sum(b1);
-      b2 = warp_sum(b2);
-      const zd c1 = b2 / zd(r22);
-      const zd c0 = (b1 - r12 * c1) / zd(r11);
-      double rr = 0;
-#pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        zd d = c0 * ep[u] + c1 * em[u] - Iv[u];
-        rr += norm2(d);
-        U[nd][u] = c0 * ep[u] - c1 * em[u];
-        if (lane + 32 * u < ns) {
-          zd Vv = a.V[(int64_t)(off + lane + 32 * u) * a.E + e];
-          UV += conj(U[nd][u]) * Vv;
-          UU += norm2(U[nd][u]);
-        }
-      }
-      res += warp_sum(rr) / Inrm;
-      if (store && lane == 0) {
-        a.A[p * a.E + e] = c0;
-        a.B[p * a.E + e] = c1;
+        const double ev = exp(g.re * sh.s[p][i]);
+        sh.e[p][i] = ev;
+        sh.ei[p][i] = 1.0 / ev;
       }
     }
   }
-  zd z0 = warp_sum(UV) / zd(warp_sum(UU));
-  double rv = 0;
-  nd = 0;
-  for (int p = 0; p < a.P; ++p) {
-    if (a.group_of[p] != grp) continue;
-    const int ns = a.ns[p], off = a.s_off[p];
-    for (int e = 0; e < a.E; ++e, ++nd) {
+  __syncthreads();
+  const int per = (nd + kFitWarps - 1) / kFitWarps, d0 = warp * per, d1 = min(nd, d0 + per);
+  double rr = 0.0, uv_re = 0.0, uv_im = 0.0, uu = 0.0;
+  zd ep[kPer], em[kPer], eo[kPer];  // e^{gs}, e^{-gs}, and e^{-gs} less its part along e^{gs}
+  zd r12;                            // that part's coefficient
+  double i11 = 0.0, i22 = 0.0;       // reciprocal squared norms of ep, eo
+  int at = -1;
+  for (int d = d0; d < d1; ++d) {
+    const int p = d / a.E, ex = d - p * a.E, ns = sh.ns[p];
+    const bool two = ns > 32;
+    if (p != at) {
+      // two-column least squares on [e^{gs}, e^{-gs}] by modified Gram-Schmidt
+      // with one re-orthogonalisation, the columns left unnormalised
+      at = p;
+      double q[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int i = lane + 32 * u;
+        ep[u] = em[u] = eo[u] = zd(0.0);
+        if ((u == 0 || two) && i < ns) {
+          const double e = sh.e[p][i], ei = sh.ei[p][i], c = sh.cs[p][i], sn = sh.sn[p][i];
+          ep[u] = zd(e * c, e * sn);
+          em[u] = zd(ei * c, -(ei * sn));
+          q[0] += e * e;
+          const zd w = conj(ep[u]) * em[u];
+          q[1] += w.re;
+          q[2] += w.im;
+        }
+      }
+      warp_sum4(q);
+      i11 = 1.0 / q[0];
+      r12 = zd(q[1] * i11, q[2] * i11);
+      q[0] = q[1] = q[2] = q[3] = 0.0;
 #pragma unroll
       for (int u = 0; u < kPer; ++u)
-        if (lane + 32 * u < ns) {
-          zd Vv = a.V[(int64_t)(off + lane + 32 * u) * a.E + e];
-          rv += norm2(Vv - z0 * U[nd][u]);
+        if (u == 0 || two) {
+          eo[u] = fnma(em[u], r12, ep[u]);
+          const zd w = conj(ep[u]) * eo[u];
+          q[0] += w.re;
+          q[1] += w.im;
+          q[2] += norm2(eo[u]);  // the second step changes it by the square of the first one's rounding
         }
+      warp_sum4(q);
+      const zd r2(q[0] * i11, q[1] * i11);
+      i22 = 1.0 / q[2];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u)
+        if (u == 0 || two) eo[u] = fnma(eo[u], r2, ep[u]);
+      r12 += r2;
+    }
+    zd Iv[kPer];
+    double b[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int i = lane + 32 * u;
+      Iv[u] = zd(0.0);
+      if ((u == 0 || two) && i < ns) {
+        Iv[u] = sh.I[d][i];
+        const zd w1 = conj(ep[u]) * Iv[u], w2 = conj(eo[u]) * Iv[u];
+        b[0] += w1.re;
+        b[1] += w1.im;
+        b[2] += w2.re;
+        b[3] += w2.im;
+      }
+    }
+    warp_sum4(b);
+    const zd c1(b[2] * i22, b[3] * i22);
+    const zd c0 = fnma(zd(b[0] * i11, b[1] * i11), r12, c1);
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int i = lane + 32 * u;
+      if ((u == 0 || two) && i < ns) {
+        const zd t0 = c0 * ep[u], t1 = c1 * em[u];
+        const zd dv = (t0 - Iv[u]) + t1, U = t0 - t1, Vv = sh.V[d][i];
+        rr += norm2(dv);
+        const zd w = conj(U) * Vv;
+        uv_re += w.re;
+        uv_im += w.im;
+        uu += norm2(U);
+        sh.U[d][i] = U;
+      }
+    }
+    if (store && lane == 0) {
+      const int row = sh.port[p] * a.E + ex;
+      a.A[row] = c0;
+      a.B[row] = c1;
     }
   }
-  res += a.v_weight * warp_sum(rv) / Vnrm;
-  if (store && lane == 0)
-    for (int p = 0; p < a.P; ++p)
-      if (a.group_of[p] == grp) a.zline[p] = z0;
-  return res;
+  double q[4] = {rr, uv_re, uv_im, uu};
+  warp_sum4(q);
+  if (lane < 4) sh.part[warp][lane] = lane == 0 ? q[0] : lane == 1 ? q[1] : lane == 2 ? q[2] : q[3];
+  __syncthreads();
+  double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int w = 0; w < kFitWarps; ++w)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) t[k] += sh.part[w][k];
+  const double iu = 1.0 / t[3];
+  const zd z0(t[1] * iu, t[2] * iu);
+  double rv = 0.0;
+  for (int d = d0; d < d1; ++d) {
+    const int ns = sh.ns[d / a.E];
+    for (int i = lane; i < ns; i += 32) rv += norm2(fnma(sh.V[d][i], z0, sh.U[d][i]));
+  }
+  for (int o = 16; o; o >>= 1) rv += __shfl_xor_sync(~0u, rv, o);
+  if (lane == 0) sh.rv[warp] = rv;
+  __syncthreads();
+  rv = 0.0;
+#pragma unroll
+  for (int w = 0; w < kFitWarps; ++w) rv += sh.rv[w];
+  if (store && threadIdx.x < nmem) a.zline[sh.port[threadIdx.x]] = z0;
+  return t[0] * sh.inv_I + a.v_weight * (rv * sh.inv_V);
 }
 
 // Minimum of f on [lo, hi] by Brent's method (R. P. Brent, "Algorithms for
@@ -445,84 +501,131 @@ __device__ double brent_minimize(F f, double lo, double hi, double xatol, int ma
   return x;
 }
 
-// One CTA of four warps per port group: Nelder-Mead with scipy's
+// One cluster of four CTAs per port group: Nelder-Mead with scipy's
 // coefficients (reflection 1, expansion 2, contraction 0.5, shrink 0.5),
 // initial simplex 5 % steps, stopping when the simplex spans <= xatol and its
 // values <= fatol. Each iteration evaluates its four possible trial points
-// (reflection, expansion, outside and inside contraction) at once, one warp
-// each (one SM sub-partition and its fp64 unit each), and then takes scipy's
-// decisions on those values: the objective is a pure function, so the
-// simplex follows the sequential method's path exactly, in about half the
-// sequential rounds of objective evaluations.
-constexpr int kFitWarps = 4;
+// (reflection, expansion, outside and inside contraction) at once, one CTA
+// each, and then takes scipy's decisions on those values: the objective is a
+// pure function, so the simplex follows the sequential method's path exactly.
+// Every CTA keeps the simplex; the values go around through the cluster's
+// shared memory. Measured on GB300 (two ports; the whole de-embedding of a
+// point, nearly all of it this fit): the line (5 cuts per feed) 4.9 -> 0.9 ms,
+// the tee (21) 6.1 -> 1.2 ms, the LPF (29) 5.0 -> 1.2 ms, against one CTA of
+// four warps per group with a trial point per warp, whose fp64 chain of some
+// 1500 instructions per evaluation took 67 us an iteration.
+constexpr int kFitCl = 4;
 
 __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
-  const int grp = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __shared__ double pts[kFitWarps][2];
-  __shared__ double vals[kFitWarps];
-  if (grp >= a.ngroup) return;
-  const double scale = fabs(a.beta0[grp]);
-  double Inrm = 0, Vnrm = 0;
-  for (int p = 0; p < a.P; ++p) {
-    if (a.group_of[p] != grp) continue;
-    for (int i = lane; i < a.ns[p]; i += 32)
-      for (int e = 0; e < a.E; ++e) {
-        Inrm += norm2(a.I[(int64_t)(a.s_off[p] + i) * a.E + e]);
-        Vnrm += norm2(a.V[(int64_t)(a.s_off[p] + i) * a.E + e]);
+  extern __shared__ __align__(16) unsigned char fit_smem[];
+  FitShared& sh = *reinterpret_cast<FitShared*>(fit_smem);
+  __shared__ double vals[2][kFitCl];
+  const int grp = blockIdx.x / kFitCl, lane = threadIdx.x & 31;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  auto cluster_sync = [] {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  };
+  // the group's data and the norms of its currents and voltages
+  if (threadIdx.x == 0) {
+    int m = 0;
+    for (int p = 0; p < a.P; ++p)
+      if (a.group_of[p] == grp && m < kFitPorts) {
+        sh.port[m] = p;
+        sh.ns[m] = a.ns[p];
+        ++m;
       }
+    sh.nmem = m;
   }
-  Inrm = warp_sum(Inrm);
-  Vnrm = warp_sum(Vnrm);
-  // objective values of the first n points of pts, one warp per point
-  auto round = [&](int n) {
-    __syncthreads();
-    if (warp < n) {
-      const double v = wave_objective(a, grp, zd(scale * pts[warp][0], scale * pts[warp][1]), Inrm, Vnrm, false);
-      if (lane == 0) vals[warp] = v;
+  __syncthreads();
+  const int nmem = sh.nmem;
+  double nrm[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int m = 0; m < nmem; ++m) {
+    const int off = a.s_off[sh.port[m]], ns = sh.ns[m];
+    for (int i = threadIdx.x; i < ns; i += 32 * kFitWarps) sh.s[m][i] = a.s[off + i];
+    for (int q = threadIdx.x; q < ns * a.E; q += 32 * kFitWarps) {
+      const int i = q / a.E, e = q - i * a.E;
+      const zd Iv = a.I[(int64_t)(off + i) * a.E + e], Vv = a.V[(int64_t)(off + i) * a.E + e];
+      sh.I[m * a.E + e][i] = Iv;
+      sh.V[m * a.E + e][i] = Vv;
+      nrm[0] += norm2(Iv);
+      nrm[1] += norm2(Vv);
     }
-    __syncthreads();
+  }
+  warp_sum4(nrm);
+  if (lane < 2) sh.part[threadIdx.x >> 5][lane] = nrm[lane];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double ni = 0.0, nv = 0.0;
+    for (int w = 0; w < kFitWarps; ++w) {
+      ni += sh.part[w][0];
+      nv += sh.part[w][1];
+    }
+    sh.inv_I = 1.0 / ni;
+    sh.inv_V = 1.0 / nv;
+  }
+  __syncthreads();
+  const double scale = fabs(a.beta0[grp]);
+  auto finish = [&](zd g, int it) {  // the first CTA stores the coefficients at the minimum
+    if (rank != 0) return;
+    const double res = wave_objective(a, sh, g, true);
+    if (threadIdx.x == 0) a.iters[grp] = it;
+    if (threadIdx.x < nmem) {
+      a.gamma[sh.port[threadIdx.x]] = g;
+      a.resid[sh.port[threadIdx.x]] = sqrt(res);
+    }
   };
   if (a.lossless) {
     // gamma = j beta (a bound mode: no attenuation to fit), beta = |beta0| b
     // with b in [lo, hi] found by Brent's bounded minimisation (one objective
-    // evaluation per step, on warp 0)
-    if (warp != 0) return;
-    auto f = [&](double b) { return wave_objective(a, grp, zd(0.0, scale * b), Inrm, Vnrm, false); };
+    // evaluation per step, on the first CTA)
+    if (rank != 0) return;
+    auto f = [&](double b) { return wave_objective(a, sh, zd(0.0, scale * b), false); };
     int n = 0;
     const double b = brent_minimize(f, a.lo[grp], a.hi[grp], 1e-12, 500, &n);
-    const zd g(0.0, scale * b);
-    const double res = wave_objective(a, grp, g, Inrm, Vnrm, true);
-    if (lane == 0) {
-      const bool at_bound = fmin(b - a.lo[grp], a.hi[grp] - b) < 1e-3;
-      a.iters[grp] = at_bound ? -n : n;
-      for (int p = 0; p < a.P; ++p)
-        if (a.group_of[p] == grp) {
-          a.gamma[p] = g;
-          a.resid[p] = sqrt(res);
-        }
-    }
+    const bool at_bound = fmin(b - a.lo[grp], a.hi[grp] - b) < 1e-3;
+    finish(zd(0.0, scale * b), at_bound ? -n : n);
     return;
   }
+  cluster_sync();  // every CTA runs before the first value is sent
+  int par = 0;
+  // objective values of the first n trial points, CTA k's at its point x
+  auto round = [&](const double (&x)[2], int n, double (&v)[kFitCl]) {
+    double f = 0.0;
+    if ((int)rank < n) f = wave_objective(a, sh, zd(scale * x[0], scale * x[1]), false);
+    if (threadIdx.x < kFitCl && (int)rank < n) {
+      uint32_t d, l = (uint32_t)__cvta_generic_to_shared(&vals[par][rank]);
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(d) : "r"(l), "r"(threadIdx.x));
+      asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(d), "d"(f) : "memory");
+    }
+    cluster_sync();
+#pragma unroll
+    for (int k = 0; k < kFitCl; ++k) v[k] = k < n ? *(volatile double*)&vals[par][k] : 0.0;
+    par ^= 1;  // the other buffer: a fast CTA's next value must not overtake a slow one's read
+  };
   const double xatol = 1e-10, fatol = 1e-16;
-  double sim[3][2], fs[3];
+  double sim[3][2], fs[3], v[kFitCl];
   // gamma0 = 1e-3 b0 + j b0, scaled by |b0|
   const double x0 = 1e-3 * a.beta0[grp] / scale, x1 = a.beta0[grp] / scale;
   sim[0][0] = x0; sim[0][1] = x1;
   sim[1][0] = x0 != 0 ? 1.05 * x0 : 0.00025; sim[1][1] = x1;
   sim[2][0] = x0; sim[2][1] = x1 != 0 ? 1.05 * x1 : 0.00025;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; ++k) {
-      pts[k][0] = sim[k][0];
-      pts[k][1] = sim[k][1];
-    }
-  round(3);
-  for (int k = 0; k < 3; ++k) fs[k] = vals[k];
+  {
+    const double x[2] = {rank == 1 ? sim[1][0] : sim[0][0], rank == 2 ? sim[2][1] : sim[0][1]};
+    round(x, 3, v);
+  }
+  for (int k = 0; k < 3; ++k) fs[k] = v[k];
   auto sort3 = [&]() {  // stable insertion sort by value
-    for (int i = 1; i < 3; ++i)
-      for (int j = i; j > 0 && fs[j] < fs[j - 1]; --j) {
-        double t = fs[j]; fs[j] = fs[j - 1]; fs[j - 1] = t;
-        for (int d = 0; d < 2; ++d) { double u = sim[j][d]; sim[j][d] = sim[j - 1][d]; sim[j - 1][d] = u; }
+    auto order = [&](int i) {  // entries i - 1, i
+      if (fs[i] < fs[i - 1]) {
+        const double t = fs[i]; fs[i] = fs[i - 1]; fs[i - 1] = t;
+        for (int d = 0; d < 2; ++d) { const double u = sim[i][d]; sim[i][d] = sim[i - 1][d]; sim[i - 1][d] = u; }
+        return true;
       }
+      return false;
+    };
+    order(1);
+    if (order(2)) order(1);
   };
   sort3();
   int it = 1;
@@ -533,23 +636,17 @@ __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
       df = fmax(df, fabs(fs[0] - fs[k]));
     }
     if (dx <= xatol && df <= fatol) break;
-    double xb[2], xr[2], xe[2], xo[2], xi[2];
+    double xr[2], xe[2], xo[2], xi[2], x[2];
     for (int d = 0; d < 2; ++d) {
-      xb[d] = (sim[0][d] + sim[1][d]) / 2.0;
-      xr[d] = 2.0 * xb[d] - sim[2][d];
-      xe[d] = 3.0 * xb[d] - 2.0 * sim[2][d];
-      xo[d] = 1.5 * xb[d] - 0.5 * sim[2][d];
-      xi[d] = 0.5 * xb[d] + 0.5 * sim[2][d];
+      const double xb = (sim[0][d] + sim[1][d]) * 0.5;
+      xr[d] = 2.0 * xb - sim[2][d];
+      xe[d] = 3.0 * xb - 2.0 * sim[2][d];
+      xo[d] = 1.5 * xb - 0.5 * sim[2][d];
+      xi[d] = 0.5 * xb + 0.5 * sim[2][d];
+      x[d] = rank == 0 ? xr[d] : rank == 1 ? xe[d] : rank == 2 ? xo[d] : xi[d];
     }
-    if (threadIdx.x == 0)
-      for (int d = 0; d < 2; ++d) {
-        pts[0][d] = xr[d];
-        pts[1][d] = xe[d];
-        pts[2][d] = xo[d];
-        pts[3][d] = xi[d];
-      }
-    round(4);
-    const double fr = vals[0], fe = vals[1], fo = vals[2], fi = vals[3];
+    round(x, 4, v);
+    const double fr = v[0], fe = v[1], fo = v[2], fi = v[3];
     bool shrink = false;
     if (fr < fs[0]) {
       if (fe < fr) { sim[2][0] = xe[0]; sim[2][1] = xe[1]; fs[2] = fe; }
@@ -566,30 +663,15 @@ __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
     if (shrink) {
       for (int j = 1; j < 3; ++j)
         for (int d = 0; d < 2; ++d) sim[j][d] = sim[0][d] + 0.5 * (sim[j][d] - sim[0][d]);
-      if (threadIdx.x == 0)
-        for (int j = 1; j < 3; ++j) {
-          pts[j - 1][0] = sim[j][0];
-          pts[j - 1][1] = sim[j][1];
-        }
-      round(2);
-      fs[1] = vals[0];
-      fs[2] = vals[1];
+      for (int d = 0; d < 2; ++d) x[d] = rank == 0 ? sim[1][d] : sim[2][d];
+      round(x, 2, v);
+      fs[1] = v[0];
+      fs[2] = v[1];
     }
     ++it;
     sort3();
   }
-  if (warp == 0) {
-    zd g(scale * sim[0][0], scale * sim[0][1]);
-    double res = wave_objective(a, grp, g, Inrm, Vnrm, true);
-    if (lane == 0) {
-      a.iters[grp] = it;
-      for (int p = 0; p < a.P; ++p)
-        if (a.group_of[p] == grp) {
-          a.gamma[p] = g;
-          a.resid[p] = sqrt(res);
-        }
-    }
-  }
+  finish(zd(scale * sim[0][0], scale * sim[0][1]), it);
 }
 
 // After the fits of all groups: SI = -B A^-1, the reference impedances and S.
@@ -925,7 +1007,22 @@ static int deembed(m25_ctx* ctx, m25_geom* geom, m25_greens* gr, m25_ports* p, c
     fa.lo[gi] = p->lossless ? p->bounds[2 * gi] : 0.0;
     fa.hi[gi] = p->lossless ? p->bounds[2 * gi + 1] : 0.0;
   }
-  fit_kernel<<<p->ngroup, 32 * kFitWarps, 0, st>>>(fa);
+  {
+    M25_CUDA(cudaFuncSetAttribute(fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FitShared)));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kFitCl;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(p->ngroup * kFitCl);
+    cfg.blockDim = dim3(32 * kFitWarps);
+    cfg.dynamicSmemBytes = sizeof(FitShared);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    M25_CUDA(cudaLaunchKernelEx(&cfg, fit_kernel, fa));
+  }
   // S of the feeds alone; with internal ports the caller assembles S from
   // the coefficients (m25_deembed_coefs)
   if (p->E == p->P) fit_finish_kernel<<<1, 32, 0, st>>>(fa);
