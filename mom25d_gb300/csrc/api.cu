@@ -248,7 +248,8 @@ extern "C" int m25_lu_factor(m25_ctx* ctx, int32_t n, int precision, void* A, in
   }
   int zinfo = 0;
   if (precision == M25_FP64)
-    rc = lu_factor<double>(ctx, static_cast<zd*>(Ad), lda, n, pd, 64, false, &zinfo);
+    rc = lu_factor<double>(ctx, static_cast<zd*>(Ad), lda, n, pd, 64,
+                           lu_tc_available() && !(flags & M25_LU_NO_TENSOR_CORES), &zinfo);
   else
     rc = lu_factor<float>(ctx, static_cast<zf*>(Ad), lda, n, pd, kPanelZ64,
                           lu_tc_available() && !(flags & M25_LU_NO_TENSOR_CORES), &zinfo);
@@ -315,7 +316,7 @@ static int dense_solve_impl(m25_ctx* ctx, int32_t n, int32_t nrhs, int precision
       Zd = ctx->Zw.as<zd>();
       M25_CUDA(cudaMemcpyAsync(Zd, Z, sizeof(zd) * nn, cudaMemcpyHostToDevice, st));
     }
-    if ((rc = lu_factor<double>(ctx, Zd, n, n, ctx->ipiv.as<int32_t>(), 64, false, &zinfo))) return rc;
+    if ((rc = lu_factor<double>(ctx, Zd, n, n, ctx->ipiv.as<int32_t>(), 64, lu_tc_available(), &zinfo))) return rc;
     if (zinfo) {
       if (info) { info[0] = 0; info[1] = zinfo; }
       set_error("m25_dense_solve: exactly singular matrix (zero pivot)");

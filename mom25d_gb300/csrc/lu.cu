@@ -2,22 +2,20 @@
 // GPU replacement of mom25d's _dense_solve (Engine/mom25d/solver.py:11-23,
 // LAPACK zgetrf / zgetrs through scipy).
 //
-// Right-looking blocked factorisation of a row-major matrix, per panel of
-// nb columns:
-//   panel_kernel   cooperative grid: each CTA keeps a slice of the panel
-//                  rows in shared memory; one bounded grid barrier per
-//                  column (pivot search |re| + |im| as izamax, swap, scale,
-//                  rank-1 update of the panel)
-//   swap_trsm_kernel  the panel's row interchanges on the other columns,
+// Right-looking blocked factorisation of a row-major matrix, per block of
+// columns (64 of complex128, 128 of complex64 with tensor cores):
+//   lu_panel.cu    the block's panel on one cluster of CTAs, in strips
+//   panel_kernel   taller panels (above 8192 rows): cooperative grid, each CTA
+//                  keeps a slice of the panel rows in shared memory; one
+//                  bounded grid barrier per column (pivot search |re| + |im|
+//                  as izamax, swap, scale, rank-1 update of the panel)
+//   swap_trsm_kernel  the block's row interchanges on the other columns,
 //                  composed into one gather, fused with U12 = L11^-1 A12
-//   gemm_kernel    A22 -= L21 U12 (SIMT)
-// The complex64 factorisation with tensor cores (lu_tc.cu) goes in blocks of
-// 128 columns, each two panels of 64: the first panel's interchanges and
-// U12 on the second panel's columns, their rank-64 update, the second panel,
-// then both panels' interchanges with U12 = L11^-1 A12 (L11 128 x 128) on
-// the trailing columns and one rank-128 update of the trailing matrix. The
-// update is bound by its read-modify-write of the trailing matrix, which
-// this does once per 128 columns.
+//   lu_oz.cu       complex128: A22 -= L21 U12 from exact integer slices
+//   lu_tc.cu       complex64: the same in 3xTF32, in super-blocks of 256
+//                  columns (the trailing matrix is read and written once per
+//                  256 columns, which bounds the update)
+//   gemm_kernel    complex64 without tensor cores (SIMT)
 // Solve: permutation, blocked forward / backward substitution. The mixed
 // path refines in fp64: r = B - Z X, X += LU32^-1 r.
 #include <algorithm>
@@ -581,6 +579,10 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
   cudaStream_t st = ctx->stream;
   // the tensor-core update reduces into C through a TMA tensor map: rows of
   // a multiple of 16 bytes and a 16-byte aligned matrix (else SIMT updates)
+  // complex128: the update by integer slices (lu_oz.cu), which needs the
+  // context's operand buffer and 16-byte aligned elements
+  const bool use_oz = use_tc && std::is_same<T, double>::value && !ctx->ext_scratch &&
+                      reinterpret_cast<uintptr_t>(A) % 16 == 0 && nb == kSwapMaxW && n > nb;
   use_tc = use_tc && std::is_same<T, float>::value && lda % 2 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
            nb == kSwapMaxW;
   // panel workspace
@@ -622,8 +624,8 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
   int* candidx = reinterpret_cast<int*>(candval + 2 * Gmax);
   cx<T>* rowj = reinterpret_cast<cx<T>*>(candidx + 2 * Gmax);
   M25_CUDA(cudaMemsetAsync(base, 0, 64, st));
-  if (use_tc) {
-    int rc = lu_tc_prepare(ctx, n);
+  if (use_tc || use_oz) {
+    int rc = use_tc ? lu_tc_prepare(ctx, n) : lu_oz_prepare(ctx, n);
     if (rc) return rc;
   }
   // blocks of up to strip_rows rows are factored by one cluster (lu_panel.cu), taller ones panel by
@@ -716,14 +718,18 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
   };
   int rc = M25_OK;
   if (!use_tc) {
-    // right-looking: panel, interchanges and U12, SIMT update of the trailing matrix
+    // right-looking: panel, interchanges and U12, update of the trailing matrix
     for (int k0 = 0; k0 < n; k0 += nb) {
       const int w = std::min(nb, n - k0);
       if (n - k0 <= strip_rows) rc = lu_strip_block<T>(ctx, A, lda, n, k0, w, ipiv, info, err, cand, cl_min);
       else rc = run_panel(k0, w);
       if (rc) return rc;
       if ((rc = swap_trsm(k0, w, 0, n - w, nullptr, 0))) return rc;
-      if (k0 + w < n) {
+      if (k0 + w >= n) break;
+      if constexpr (std::is_same<T, double>::value) {
+        // nb = 64 here: k0 + w < n
+        if ((rc = use_oz ? lu_oz_update(ctx, A, lda, n, k0) : lu_oz_update_simt(ctx, A, lda, n, k0, cand))) return rc;
+      } else {
         const int ncol = n - k0 - w;
         StageTimer tm(ctx, ST_GEMM);
         dim3 grid((ncol + 63) / 64, (ncol + 63) / 64);
@@ -800,7 +806,7 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
     set_error("dense LU: a wait of the panel factorisation ran out");
     return M25_ERR_CUDA;
   }
-  if (use_tc) {
+  if (use_tc || use_oz) {
     int tcerr = 0;
     int rc = lu_tc_error(ctx, &tcerr);
     if (rc) return rc;

@@ -43,3 +43,120 @@ def test_panel_edges(gpu, n, dtype):
     assert np.abs(L).max() <= np.sqrt(2) * (1 + 8 * u)
     if double and n <= 40:  # no ties, no empty column: LAPACK's own pivots
         assert np.array_equal(ipiv, sl.lu_factor(A)[1])
+
+
+def factor64(A, flags=0):
+    from mom25d_gb300 import engine as E
+
+    n = A.shape[0]
+    ctx = E.Context(0)
+    F, ipiv, info = np.array(A, np.complex128), np.zeros(n, np.int32), np.zeros(1, np.int32)
+    E.check(ctx.lib.m25_lu_factor(ctx.h, n, E.M25_FP64, F.ctypes.data, n, E.ptr(ipiv, C.c_int32), E.M25_ON_HOST, flags,
+                                  E.ptr(info, C.c_int32)))
+    ctx.close()
+    return F, ipiv
+
+
+@pytest.mark.parametrize("bits", [0x7F7F7F7F7F7F7C, 0x40404040404040, 0x7F80807F80807C])
+@pytest.mark.parametrize("scale", [1.0, 2.0**-340, 2.0**300])
+def test_update_slices_are_exact(gpu, bits, scale):
+    """The complex128 update by integer slices (csrc/lu_oz.cu): one entry
+    c - sum l u of 128 products whose digits are all as large as they get
+    (0x7F.. every digit 127: the accumulators' largest sums), against exact
+    rational arithmetic."""
+    from fractions import Fraction
+
+    x = bits / 2.0**55
+    A = np.zeros((65, 65), complex)
+    A[:64, :64] = 4 * np.eye(64)     # pivots, above |re| + |im| of the row below
+    A[64, :64] = x - 1j * x          # a row of A: (re, -im) = (x, x) / 4
+    A[:64, 64] = (x + 1j * x) * scale
+    F, ipiv = factor64(A)
+    assert np.array_equal(ipiv, np.arange(65))
+    want = -Fraction(x) * Fraction(x) * 32 * Fraction(scale)
+    # one rounding of the sum and of its subtraction; digit products beyond i + j = 9 are below 2^-54
+    assert abs(Fraction(F[64, 64].real) - want) <= abs(want) * Fraction(2.0**-51)
+    assert F[64, 64].imag == 0.0
+
+
+@pytest.mark.parametrize("n", [65, 129, 191, 193, 321])
+@pytest.mark.parametrize("kind", ["normal", "rows", "cols", "mixed", "wide", "signs"])
+def test_update_slices_backward_error(gpu, n, kind):
+    """P A - L U of the sliced update against the componentwise bound of an
+    fp64 factorisation, also for rows and columns of very different size."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    if kind in ("rows", "mixed"):
+        A = A * 10.0 ** rng.uniform(-8, 8, n)[:, None]
+    if kind in ("cols", "mixed"):
+        A = A * 10.0 ** rng.uniform(-8, 8, n)[None, :]
+    if kind == "wide":
+        A = A * 10.0 ** rng.uniform(-4, 4, (n, n))
+    if kind == "signs":  # +-1 with small noise: the eliminated rows mix entries of 1 and 1e-12
+        A = np.where(rng.uniform(size=(n, n)) < 0.5, 1.0, -1.0) * (1 - 1e-12 * rng.uniform(size=(n, n))) + 0j
+    F, ipiv = factor64(A)
+    L, U = np.tril(F, -1) + np.eye(n), np.triu(F)
+    P = A.copy()
+    for i, p in enumerate(ipiv):
+        P[[i, p]] = P[[p, i]]
+    # gamma_n |L| |U|, twice for complex arithmetic and twice for this product's own rounding
+    assert np.all(np.abs(P - L @ U) <= 4 * n * 2.0**-53 * (np.abs(L) @ np.abs(U)))
+    # the integer sums are exact: the CUDA cores' form gives the same bits
+    from mom25d_gb300 import engine as E
+
+    G, gpiv = factor64(A, E.M25_LU_NO_TENSOR_CORES)
+    assert np.array_equal(F, G) and np.array_equal(ipiv, gpiv)
+
+
+def test_update_slices_not_finite(gpu):
+    """An infinity or a NaN reaches the factors as it does without the slices."""
+    from mom25d_gb300 import engine as E
+
+    rng = np.random.default_rng(5)
+    A = rng.standard_normal((200, 200)) + 1j * rng.standard_normal((200, 200))
+    for bad in (np.nan, np.inf):
+        B = A.copy()
+        B[150, 10] = bad
+        F, _ = factor64(B)
+        G, _ = factor64(B, E.M25_LU_NO_TENSOR_CORES)
+        assert not np.isfinite(F).all() and not np.isfinite(G).all()
+
+
+def via_row_line(nvia):
+    """A 50 ohm line beside a pour strip tied to ground by nvia vias."""
+    import mom25d_gb300 as G
+
+    mm = 1e-3
+    W = 0.5561 * mm
+    lay = G.Layout()
+    lay.add_rect(-3 * mm, -W / 2, 3 * mm, W / 2)
+    lay.add_rect(-3 * mm, W, 3 * mm, W + 0.8 * mm)
+    for x in np.linspace(-2.5, 2.5, nvia) * mm:
+        lay.add_via(x, W + 0.4 * mm, drill=0.2 * mm, pad=0.4 * mm)
+    lay.add_port("P1", (-3 * mm, 0), "-x", W, 4 * mm)
+    lay.add_port("P2", (3 * mm, 0), "+x", W, 4 * mm)
+    return lay.mesh(max_cell=0.5 * mm, edge_cell=0.1 * mm), G.Substrate(3.66, 0.254 * mm, 0.003, 5.8e7)
+
+
+@pytest.mark.parametrize("nvia", [1, 3, 8])
+@pytest.mark.parametrize("freq", [1.5e9, 9e9])
+def test_update_slices_with_vias(gpu, nvia, freq):
+    """Via rows are 1e10 times the RWG rows of the impedance matrix: the fp64
+    solve of the sliced update is as accurate as LAPACK's (both against a
+    solve refined in extended precision; ten times for the two LUs' own
+    rounding)."""
+    from mom25d_gb300.solver import Solver, dense_solve
+
+    mesh, sub = via_row_line(nvia)
+    sol = Solver(mesh, sub, verbose=False)
+    Z, B = sol.impedance(freq), sol.port_excitations().astype(complex)
+    x = dense_solve(Z, B, precision="fp64", ctx=sol.ctx)
+    sol.close()
+    d = 1 / np.sqrt(np.abs(np.diag(Z)))
+    lu = sl.lu_factor(d[:, None] * Z * d)
+    ref = np.zeros_like(B, np.clongdouble)
+    for _ in range(4):
+        r = B - Z.astype(np.clongdouble) @ ref
+        ref = ref + d[:, None] * sl.lu_solve(lu, d[:, None] * r.astype(complex))
+    err = [float(np.linalg.norm(v - ref) / np.linalg.norm(ref)) for v in (x, np.linalg.solve(Z, B))]
+    assert err[0] <= 10 * err[1] + 1e-15
