@@ -6,7 +6,7 @@
 //                from the half-basis values of the listed fill (fill.cu,
 //                fill_listed) and symmetrised 0.5 (Z + Z^T) like the dense
 //                gather; stored row-major per leaf pair, both orders;
-//   far blocks   (aca_kernel, one CTA per block): adaptive cross
+//   far blocks   (aca_kernel, a cluster of CTAs per block): adaptive cross
 //                approximation with partial pivoting and mom25d's stopping
 //                rule on entries of the 3-point (or centroid) rule
 //                (far_entry, hmatrix.py:322-353); far_dense_kernel for the
@@ -16,7 +16,7 @@
 //                leaf's near blocks, far blocks as rows or as columns, and
 //                its via columns, in double-float on the fp32 pipes; every
 //                output entry has one writer (deterministic, no atomics);
-//   precondition (diag_kernel, ginv_kernel, psolve_kernel): restricted
+//   precondition (diag_kernel, gj_* kernels, psolve_kernel): restricted
 //                additive Schwarz over clusters of <= 256 unknowns extended
 //                by their near-coupled leaves and the vias whose pads they
 //                hold; the blocks scaled to a unit diagonal and inverted in
@@ -72,7 +72,11 @@ struct m25_hmat {
   std::vector<FarB> fb_h;
   // device: values
   m25::zd *Zn = nullptr, *pool = nullptr, *ZxbT = nullptr, *Zxx = nullptr;
-  m25::zf* D = nullptr;       // preconditioner blocks (their inverses, in place)
+  m25::zf* D = nullptr;       // preconditioner blocks, then their inverses
+  m25::zf *G = nullptr, *gj_x = nullptr;  // the blocks under elimination; a panel's pivot rows
+  float* gj_w = nullptr;
+  int32_t *gj_step = nullptr, *gj_prow = nullptr;
+  int pc_max = 0;             // unknowns of the largest block
   uint8_t* flags = nullptr;   // ACA's used rows / columns
   int64_t near_entries = 0, uv_entries = 0, dense_entries = 0, t_entries = 0, flag_bytes = 0, d_entries = 0;
   int32_t *aca_ids = nullptr, *rank = nullptr, *status = nullptr, *dense_ids = nullptr;
@@ -99,54 +103,73 @@ constexpr int kRule = 40;  // values per basis: p (12), u (12), q (6), centroid 
 struct Tabs {
   const zd* coef;
   const double* rho;
+  const float* rho32;
   int nrho, L;
   zd cA[kMaxLevSq], cV[kMaxLevSq];
   double dz[kMaxLevSq];
   zd jwmu, inv_jwe;
 };
 
-__device__ __forceinline__ int interval(const double* __restrict__ x, int n, double r) {
-  // scipy PPoly: x[i] <= r < x[i+1], clamped to the end intervals
-  if (r < x[1]) return 0;
-  if (r >= x[n - 2]) return n - 2;
-  int lo = 1, hi = n - 2;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (r < x[mid]) hi = mid; else lo = mid;
+// scipy PPoly: x[i] <= r < x[i+1], clamped to the end intervals; searched on
+// the fp32 radii and settled by one fp64 comparison (find_interval_f in fill.cu)
+__device__ __forceinline__ int interval(const double* __restrict__ x, const float* __restrict__ xf, int n, double r) {
+  const float rf = (float)r;
+  int lo;
+  if (rf < xf[1]) lo = 0;
+  else if (rf >= xf[n - 2]) lo = n - 2;
+  else {
+    lo = 1;
+    int hi = n - 2;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (rf < xf[mid]) hi = mid; else lo = mid;
+    }
   }
+  if (lo > 0 && r < x[lo]) --lo;
   return lo;
 }
 
-// Z between bases i and j (tree positions) by the 3-point rule on both sides
-// or the centroid rule: jw mu sum (u_ik . u_jl) gA + 1/(jw eps) sum q_ik q_jl gV,
-// g = c / (4 pi R) + S(rho) (Engine/mom25d/hmatrix.py:322-353, layered.py:199-206)
+// The part of Z between bases i and j (tree positions) that lane `sub` of a
+// group of SP lanes takes; their sum is Z by the 3-point rule on both sides or
+// the centroid rule: jw mu sum (u_ik . u_jl) gA + 1/(jw eps) sum q_ik q_jl gV,
+// g = c / (4 pi R) + S(rho) (Engine/mom25d/hmatrix.py:322-353, layered.py:199-206).
+// fp64 operations bound it (each holds a sub-partition's unit for 64 cycles a
+// warp): one reciprocal square root gives R and 1 / R, the cubics in Horner form,
+// the interval searched in fp32; 41 of them per pair of points, 110 before.
+template <int SP>
 __device__ zd far_entry(const Tabs& t, const double* __restrict__ rules, const int32_t* __restrict__ lev, int i,
-                        int j, int cen) {
+                        int j, int cen, int sub = 0) {
   const double* A = rules + (int64_t)i * kRule;
   const double* B = rules + (int64_t)j * kRule;
   const int pair = lev[i] * t.L + lev[j];
-  const zd cA = t.cA[pair], cV = t.cV[pair];
   const double dz = t.dz[pair];
+  const double inv4pi = 1.0 / (4.0 * kPi);
+  const zd cA = t.cA[pair] * inv4pi, cV = t.cV[pair] * inv4pi;
   const int K = cen ? 2 : 6;
   const int op = cen ? 30 : 0, ou = cen ? 34 : 12, oq = cen ? 38 : 24;
   const zd* cf = t.coef + (int64_t)pair * (t.nrho - 1) * 12;
   zd za, zv;
-  for (int k = 0; k < K; ++k) {
+  for (int k = sub; k < K; k += SP) {
     const double ax = A[op + 2 * k], ay = A[op + 2 * k + 1];
     const double uax = A[ou + 2 * k], uay = A[ou + 2 * k + 1], qa = A[oq + k];
     for (int l = 0; l < K; ++l) {
       const double dx = ax - B[op + 2 * l], dy = ay - B[op + 2 * l + 1];
-      const double rho = sqrt(dx * dx + dy * dy);
-      const double R = sqrt(rho * rho + dz * dz);
-      const int iv = interval(t.rho, t.nrho, rho);
+      const double r2 = fma(dx, dx, dy * dy);
+      double ri = rsqrt(r2);
+      const double rho = r2 > 0.0 ? r2 * ri : 0.0;
+      if (dz != 0.0) ri = rsqrt(fma(dz, dz, r2));
+      const int iv = interval(t.rho, t.rho32, t.nrho, rho);
       const double h = rho - t.rho[iv];
       const zd* c = cf + (int64_t)iv * 12;
-      const zd sa = c[9] + c[6] * h + c[3] * (h * h) + c[0] * (h * h * h);
-      const zd sv = c[10] + c[7] * h + c[4] * (h * h) + c[1] * (h * h * h);
-      const double inv = 1.0 / (4.0 * kPi * R);
-      const zd gA = cA * inv + sa, gV = cV * inv + sv;
-      za += gA * (uax * B[ou + 2 * l] + uay * B[ou + 2 * l + 1]);
-      zv += gV * (qa * B[oq + l]);
+      zd gA(fma(fma(fma(c[0].re, h, c[3].re), h, c[6].re), h, fma(cA.re, ri, c[9].re)),
+            fma(fma(fma(c[0].im, h, c[3].im), h, c[6].im), h, fma(cA.im, ri, c[9].im)));
+      zd gV(fma(fma(fma(c[1].re, h, c[4].re), h, c[7].re), h, fma(cV.re, ri, c[10].re)),
+            fma(fma(fma(c[1].im, h, c[4].im), h, c[7].im), h, fma(cV.im, ri, c[10].im)));
+      const double ua = fma(uax, B[ou + 2 * l], uay * B[ou + 2 * l + 1]), qq = qa * B[oq + l];
+      za.re = fma(gA.re, ua, za.re);
+      za.im = fma(gA.im, ua, za.im);
+      zv.re = fma(gV.re, qq, zv.re);
+      zv.im = fma(gV.im, qq, zv.im);
     }
   }
   return t.jwmu * za + t.inv_jwe * zv;
@@ -269,6 +292,10 @@ __global__ void near_kernel(const int32_t* __restrict__ near, const int64_t* __r
 }
 
 // --------------------------------------------------------------- far field
+// gridDim.y CTAs share a block's rows (the largest block alone would otherwise
+// set the time: at N = 2434 26 ms with one CTA per block, 2.9 ms so and with
+// far_entry's fewer fp64 operations)
+constexpr int kFarSplit = 16;
 __global__ void __launch_bounds__(256) far_dense_kernel(Tabs t, const double* __restrict__ rules,
                                                         const int32_t* __restrict__ lev,
                                                         const FarB* __restrict__ fb, const int32_t* __restrict__ ids,
@@ -276,13 +303,13 @@ __global__ void __launch_bounds__(256) far_dense_kernel(Tabs t, const double* __
   const FarB F = fb[ids[blockIdx.x]];
   zd* B = dpool + F.dense;
   zd* BT = B + (int64_t)F.m * F.n;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int i = wid; i < F.m; i += nw)  // one warp per row, the lanes along it
-    for (int j = lane; j < F.n; j += 32) {
-      const zd z = far_entry(t, rules, lev, F.r0 + i, F.c0 + j, F.cen);
-      B[(int64_t)i * F.n + j] = z;
-      BT[(int64_t)j * F.m + i] = z;
-    }
+  for (int64_t e = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; e < (int64_t)F.m * F.n;
+       e += (int64_t)gridDim.y * blockDim.x) {
+    const int i = (int)(e / F.n), j = (int)(e - (int64_t)i * F.n);
+    const zd z = far_entry<1>(t, rules, lev, F.r0 + i, F.c0 + j, F.cen);
+    B[e] = z;
+    BT[(int64_t)j * F.m + i] = z;
+  }
 }
 
 // Adaptive cross approximation with partial pivoting (Engine/mom25d/
@@ -290,22 +317,101 @@ __global__ void __launch_bounds__(256) far_dense_kernel(Tabs t, const double* __
 // Frobenius norm of the sum so far. rank[b] = terms, status[b] = 0 low rank,
 // 1 keep the block as it is (not low rank within kmax = min(m, n) / 3
 // iterations, or more than kcap terms).
-__global__ void __launch_bounds__(256) aca_kernel(Tabs t, const double* __restrict__ rules,
-                                                  const int32_t* __restrict__ lev, const FarB* __restrict__ fb,
-                                                  const int32_t* __restrict__ ids, zd* __restrict__ pool,
-                                                  uint8_t* __restrict__ flags, double tol, int32_t* __restrict__ rank,
-                                                  int32_t* __restrict__ status) {
-  __shared__ double sv[32];
-  __shared__ int si[32];
-  const FarB F = fb[ids[blockIdx.x]];
+// A cluster of kAcaCl CTAs per block, two lanes per entry: a term's row and
+// column are fp64 work for one SM's four units of 2200 to 4000 cycles per 32
+// entries, and the terms follow one another (one CTA per block: 33 ms at N =
+// 2434, the blocks far fewer than the SMs). Partial results go around through
+// the cluster's shared memory; the terms themselves are in global memory,
+// ordered by the cluster barriers.
+constexpr int kAcaCl = 4;  // 4 CTAs 30.5 ms a point at N = 2434, 2 35 ms, 8 34 ms, 16 47 ms (few clusters fit at once)
+
+struct AcaShared {
+  double v[2][kAcaCl][2];  // per parity: every CTA's partial result
+  int i[2][kAcaCl];
+  double sv[32];
+  int si[32];
+};
+
+__device__ __forceinline__ void aca_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// this CTA's values into slot `rank` of every CTA of the cluster
+__device__ __forceinline__ void aca_send(AcaShared& sh, int par, unsigned rank, double a, double b, int idx) {
+  if (threadIdx.x < kAcaCl) {
+    auto map = [&](const void* p) {
+      uint32_t r;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                   : "=r"(r)
+                   : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(threadIdx.x));
+      return r;
+    };
+    asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(map(&sh.v[par][rank][0])), "d"(a) : "memory");
+    asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(map(&sh.v[par][rank][1])), "d"(b) : "memory");
+    asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(map(&sh.i[par][rank])), "r"(idx) : "memory");
+  }
+}
+// largest value (ties: smallest index) over the cluster; every thread gets it
+__device__ void aca_argmax(AcaShared& sh, int& par, unsigned rank, double& v, int& idx) {
+  block_argmax(v, idx, sh.sv, sh.si);
+  aca_send(sh, par, rank, v, 0.0, idx);
+  aca_sync();
+#pragma unroll
+  for (int q = 0; q < kAcaCl; ++q) {
+    const double ov = sh.v[par][q][0];
+    const int oi = sh.i[par][q];
+    if (q == 0 || ov > v || (ov == v && oi < idx)) {
+      v = ov;
+      idx = oi;
+    }
+  }
+  par ^= 1;
+}
+// sums of two values over the cluster
+__device__ void aca_sum(AcaShared& sh, int& par, unsigned rank, double& a, double& b) {
+  a = block_sum(a, sh.sv);
+  b = block_sum(b, sh.sv);
+  aca_send(sh, par, rank, a, b, 0);
+  aca_sync();
+  a = b = 0.0;
+#pragma unroll
+  for (int q = 0; q < kAcaCl; ++q) {
+    a += sh.v[par][q][0];
+    b += sh.v[par][q][1];
+  }
+  par ^= 1;
+}
+
+__global__ void __cluster_dims__(kAcaCl, 1, 1) __launch_bounds__(256)
+    aca_kernel(Tabs t, const double* __restrict__ rules, const int32_t* __restrict__ lev, const FarB* __restrict__ fb,
+               const int32_t* __restrict__ ids, zd* pool, uint8_t* flags, double tol, int32_t* __restrict__ rank_out,
+               int32_t* __restrict__ status) {
+  __shared__ AcaShared sh;
+  unsigned rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  const int blk = blockIdx.x / kAcaCl;
+  const FarB F = fb[ids[blk]];
   const int m = F.m, n = F.n, tid = threadIdx.x;
   zd* U = pool + F.uv;
   zd* V = U + (int64_t)F.kcap * m;
   uint8_t* used_r = flags + F.flag;
   uint8_t* used_c = used_r + m;
   const int kmax = max(2, min(m, n) / 3);
-  int i = 0, k = 0, st = 1;
+  // this CTA's rows and columns; two lanes per entry
+  const int mr0 = (int)((int64_t)m * rank / kAcaCl), mr1 = (int)((int64_t)m * (rank + 1) / kAcaCl);
+  const int nc0 = (int)((int64_t)n * rank / kAcaCl), nc1 = (int)((int64_t)n * (rank + 1) / kAcaCl);
+  const int sub = tid & 1, half = tid >> 1, nh = blockDim.x >> 1;
+  int i = 0, k = 0, st = 1, par = 0;
+  // the residual's entry (r, c): the block's less sum_l a_l b_l over the k
+  // terms so far, every other term in each lane
+  auto entry = [&](int r, int c, const zd* a, int lda, const zd* b, int ldb) {
+    zd z = far_entry<2>(t, rules, lev, F.r0 + r, F.c0 + c, F.cen, sub);
+    for (int l = sub; l < k; l += 2) z = fnma(z, a[(int64_t)l * lda], b[(int64_t)l * ldb]);
+    z.re += __shfl_xor_sync(~0u, z.re, 1);
+    z.im += __shfl_xor_sync(~0u, z.im, 1);
+    return z;
+  };
   double fro2 = 0.0;
+  aca_sync();  // every CTA runs before the first value is sent
   for (int it = 0; it < kmax; ++it) {
     if (k >= F.kcap) {  // no room for another term: keep the block as it is
       st = 1;
@@ -315,28 +421,30 @@ __global__ void __launch_bounds__(256) aca_kernel(Tabs t, const double* __restri
     // the residual's row i
     double best = -1.0;
     int bj = 0x7fffffff;
-    for (int j = tid; j < n; j += blockDim.x) {
-      zd z = far_entry(t, rules, lev, F.r0 + i, F.c0 + j, F.cen);
-      for (int l = 0; l < k; ++l) z -= V[(int64_t)l * n + j] * U[(int64_t)l * m + i];
-      Vk[j] = z;
-      const double a = used_c[j] ? 0.0 : cabs(z);
-      if (a > best) {
-        best = a;
-        bj = j;
+    for (int j0 = nc0; j0 < nc1; j0 += nh) {
+      const int j = min(j0 + half, nc1 - 1);  // a whole warp evaluates
+      const zd z = entry(i, j, V + j, n, U + i, m);
+      if (sub == 0 && j0 + half < nc1) {
+        Vk[j] = z;
+        const double a = used_c[j] ? 0.0 : cabs(z);
+        if (a > best) {
+          best = a;
+          bj = j;
+        }
       }
     }
-    __syncthreads();
-    if (tid == 0) used_r[i] = 1;
-    block_argmax(best, bj, sv, si);
+    aca_argmax(sh, par, rank, best, bj);
+    if (rank == 0 && tid == 0) used_r[i] = 1;
     if (!(best > 0.0) || bj >= n) {  // a zero row (or no finite entry): take the first unused row instead
+      aca_sync();
       int fr = 0x7fffffff;
-      for (int r = tid; r < m; r += blockDim.x)
+      for (int r = mr0 + tid; r < mr1; r += blockDim.x)
         if (!used_r[r]) {
           fr = r;
           break;
         }
       double dummy = -(double)fr;
-      block_argmax(dummy, fr, sv, si);
+      aca_argmax(sh, par, rank, dummy, fr);
       if (fr == 0x7fffffff) {
         st = 0;
         break;
@@ -345,38 +453,40 @@ __global__ void __launch_bounds__(256) aca_kernel(Tabs t, const double* __restri
       continue;
     }
     const zd piv = Vk[bj];
-    __syncthreads();
-    double nv2 = 0.0;
-    for (int j = tid; j < n; j += blockDim.x) {
-      const zd v = Vk[j] / piv;
+    aca_sync();  // read before its owner scales it
+    const zd ipiv = zd(1.0) / piv;
+    double nv2 = 0.0, nu2 = 0.0;
+    for (int j = nc0 + tid; j < nc1; j += blockDim.x) {
+      const zd v = Vk[j] * ipiv;
       Vk[j] = v;
       nv2 += norm2(v);
     }
+    if (rank == 0 && tid == 0) used_c[bj] = 1;
     // the residual's column bj
     zd* Uk = U + (int64_t)k * m;
-    double nu2 = 0.0;
-    for (int r = tid; r < m; r += blockDim.x) {
-      zd z = far_entry(t, rules, lev, F.r0 + r, F.c0 + bj, F.cen);
-      for (int l = 0; l < k; ++l) z -= U[(int64_t)l * m + r] * V[(int64_t)l * n + bj];
-      Uk[r] = z;
-      nu2 += norm2(z);
+    for (int r0 = mr0; r0 < mr1; r0 += nh) {
+      const int r = min(r0 + half, mr1 - 1);
+      const zd z = entry(r, bj, U + r, m, V + bj, n);
+      if (sub == 0 && r0 + half < mr1) {
+        Uk[r] = z;
+        nu2 += norm2(z);
+      }
     }
-    nv2 = block_sum(nv2, sv);
-    nu2 = block_sum(nu2, sv);
-    if (tid == 0) used_c[bj] = 1;
+    aca_sum(sh, par, rank, nv2, nu2);
     // cross terms 2 sum_l |(u_k^H u_l)(v_k^H v_l)|, one warp per earlier term
-    double cross = 0.0;
+    double cross = 0.0, zero = 0.0;
     if (k > 0) {
-      const int lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+      const int lane = tid & 31, wid = rank * (blockDim.x >> 5) + (tid >> 5), nw = kAcaCl * (blockDim.x >> 5);
       for (int l = wid; l < k; l += nw) {
         zd d1, d2;
-        for (int r = lane; r < m; r += 32) d1 += conj(Uk[r]) * U[(int64_t)l * m + r];
-        for (int j = lane; j < n; j += 32) d2 += conj(Vk[j]) * V[(int64_t)l * n + j];
+        // d1, d2 with their signs changed: the modulus is taken
+        for (int r = lane; r < m; r += 32) d1 = fnma(d1, conj(Uk[r]), U[(int64_t)l * m + r]);
+        for (int j = lane; j < n; j += 32) d2 = fnma(d2, conj(Vk[j]), V[(int64_t)l * n + j]);
         d1 = warp_sum(d1);
         d2 = warp_sum(d2);
         if (lane == 0) cross += cabs(d1 * d2);
       }
-      cross = block_sum(cross, sv);
+      aca_sum(sh, par, rank, cross, zero);
     }
     fro2 += 2.0 * cross + nu2 * nv2;
     ++k;
@@ -387,24 +497,25 @@ __global__ void __launch_bounds__(256) aca_kernel(Tabs t, const double* __restri
     // next row: the largest entry of the new column among the unused rows
     double cb = -1.0;
     int ci = 0x7fffffff;
-    for (int r = tid; r < m; r += blockDim.x) {
+    for (int r = mr0 + tid; r < mr1; r += blockDim.x) {
       const double a = used_r[r] ? 0.0 : cabs(Uk[r]);
       if (a > cb) {
         cb = a;
         ci = r;
       }
     }
-    block_argmax(cb, ci, sv, si);
+    aca_argmax(sh, par, rank, cb, ci);
     if (!(cb > 0.0) || ci >= m) {
       st = 0;
       break;
     }
     i = ci;
   }
-  if (tid == 0) {
-    rank[blockIdx.x] = k;
-    status[blockIdx.x] = st;
+  if (rank == 0 && tid == 0) {
+    rank_out[blk] = k;
+    status[blk] = st;
   }
+  aca_sync();  // no CTA leaves while a peer may still store into its shared memory
 }
 
 // ------------------------------------------------------------------ matvec
@@ -563,7 +674,8 @@ __global__ void perm_out_kernel(int nb, int n, const int32_t* __restrict__ perm,
 
 // block k's matrix (complex64, row-major S x S): per (row leaf, column leaf)
 // pair the near block or the far block (as rows or as its transpose), then
-// the via rows / columns
+// the via rows / columns; every entry has one source. The pairs of a block are
+// shared out to gridDim.y CTAs (a few blocks alone leave the GPU idle).
 __global__ void diag_kernel(const int64_t* __restrict__ pc_off, const int32_t* __restrict__ gidx,
                             const int64_t* __restrict__ item_off, const int32_t* __restrict__ items,
                             const int64_t* __restrict__ doff, int nb, int nv, int nnear,
@@ -581,10 +693,9 @@ __global__ void diag_kernel(const int64_t* __restrict__ pc_off, const int32_t* _
   int mine = 0;
   for (int t = threadIdx.x; t < S; t += blockDim.x) mine += gidx[g0 + t] < nb;
   atomicAdd(&nr, mine);
-  for (int64_t e = threadIdx.x; e < (int64_t)S * S; e += blockDim.x) Dk[e] = zf(0.f, 0.f);
   __syncthreads();
   const int R = nr;  // RWG unknowns first, then the vias
-  for (int64_t it = item_off[k]; it < item_off[k + 1]; ++it) {
+  for (int64_t it = item_off[k] + blockIdx.y; it < item_off[k + 1]; it += gridDim.y) {
     const int src = items[5 * it], li = items[5 * it + 1], lj = items[5 * it + 2];
     const int lr0 = items[5 * it + 3], lc0 = items[5 * it + 4];
     const int a0 = leaf_lo[li], am = leaf_lo[li + 1] - a0, b0 = leaf_lo[lj], bn = leaf_lo[lj + 1] - b0;
@@ -619,6 +730,7 @@ __global__ void diag_kernel(const int64_t* __restrict__ pc_off, const int32_t* _
       Dk[(int64_t)(lr0 + ii) * S + lc0 + jj] = z;
     }
   }
+  if (blockIdx.y) return;
   const int nvk = S - R;
   for (int e = threadIdx.x; e < R * nvk; e += blockDim.x) {  // RWG x via (Z is symmetric)
     const int t = e / nvk, a = e - t * nvk;
@@ -632,89 +744,210 @@ __global__ void diag_kernel(const int64_t* __restrict__ pc_off, const int32_t* _
   }
 }
 
-// In-place inversion of each diagonal block (one CTA per block, complex64:
-// the flexible GMRES below keeps M^-1 v_j, so the preconditioner need not be
-// exact). The block is first scaled symmetrically to a unit diagonal,
-// D' = W D W with W = diag(|D_ii|^-1/2) (the via rows and the RWG rows
-// differ by many orders of magnitude), then inverted by Gauss-Jordan
-// elimination with partial pivoting (a zero pivot is replaced by 1: the
-// block then preconditions less), the row interchanges undone on the
-// columns, and D^-1 = W D'^-1 W stored in place.
+// Inversion of the diagonal blocks (complex64: the flexible GMRES below keeps
+// M^-1 v_j, so the preconditioner need not be exact). A block is first scaled
+// symmetrically to a unit diagonal, D' = W D W with W = diag(|D_ii|^-1/2) (the
+// via rows and the RWG rows differ by many orders of magnitude), then
+// inverted by Gauss-Jordan elimination with partial pivoting (a zero pivot is
+// replaced by 1: the block then preconditions less), and D^-1 = W D'^-1 W.
+// The elimination goes in panels of kGj columns, all blocks side by side:
+//   gj_panel_kernel   a CTA per block, one row per thread, the panel's columns
+//                     in registers; rows are not interchanged, a row that has
+//                     been a pivot only drops out of the search; then the pivot
+//                     rows' other columns are set aside (X)
+//   gj_update_kernel  the other columns: A_r = A_r + P_r X, or P_r X for a row
+//                     that was a pivot of this panel, tiles over the whole GPU
+// One column after the other in global memory by one CTA per block took 76 ms
+// for the 16 blocks of up to 640 unknowns at N = 2434; this takes 2.8 ms.
 __device__ __forceinline__ float fabs1(zf a) { return fabsf(a.re) + fabsf(a.im); }
 
-__global__ void __launch_bounds__(1024) ginv_kernel(const int64_t* __restrict__ pc_off, const int64_t* __restrict__ doff,
-                                                   zf* __restrict__ D) {
-  __shared__ double sv[32];
-  __shared__ int si[32];
-  __shared__ int pv[1024];
-  __shared__ float w[1024];
-  __shared__ zf fcol[1024];
-  const int k = blockIdx.x;
-  const int S = (int)(pc_off[k + 1] - pc_off[k]);
-  zf* A = D + doff[k];
-  for (int i = threadIdx.x; i < S; i += blockDim.x) {
+constexpr int kGj = 16;
+
+// D' = W D W into G, W beside it, no pivots yet
+__global__ void __launch_bounds__(256) gj_scale_kernel(const int64_t* __restrict__ pc_off,
+                                                       const int64_t* __restrict__ doff, const zf* __restrict__ D,
+                                                       zf* __restrict__ G, float* __restrict__ w,
+                                                       int32_t* __restrict__ step) {
+  const int k = blockIdx.x, S = (int)(pc_off[k + 1] - pc_off[k]);
+  const zf* A = D + doff[k];
+  zf* B = G + doff[k];
+  auto weight = [&](int i) {
     const zf a = A[(int64_t)i * S + i];
     const float m = hypotf(a.re, a.im);
-    w[i] = m > 0.f ? rsqrtf(m) : 1.f;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int r = wid; r < S; r += nw)
-    for (int j = lane; j < S; j += 32) A[(int64_t)r * S + j] = A[(int64_t)r * S + j] * (w[r] * w[j]);
-  __syncthreads();
-  for (int c = 0; c < S; ++c) {
-    double best = -1.0;
-    int bi = 0x7fffffff;
-    for (int r = c + threadIdx.x; r < S; r += blockDim.x) {
-      const double a = fabs1(A[(int64_t)r * S + c]);
-      if (a > best) {
-        best = a;
-        bi = r;
-      }
+    return m > 0.f ? rsqrtf(m) : 1.f;
+  };
+  const int lane = threadIdx.x & 31, wid = blockIdx.y * 8 + (threadIdx.x >> 5), nw = gridDim.y * 8;
+  for (int r = wid; r < S; r += nw) {
+    const float wr = weight(r);
+    if (lane == 0) {
+      w[k * 1024 + r] = wr;
+      step[k * 1024 + r] = -1;
     }
-    block_argmax(best, bi, sv, si);
-    if (bi < c || bi >= S) {
-      bi = c;
-      best = 0.0;
-    }
-    if (threadIdx.x == 0) pv[c] = bi;
-    if (bi != c)
-      for (int j = threadIdx.x; j < S; j += blockDim.x) {
-        const zf t0 = A[(int64_t)c * S + j];
-        A[(int64_t)c * S + j] = A[(int64_t)bi * S + j];
-        A[(int64_t)bi * S + j] = t0;
-      }
-    __syncthreads();
-    const zf d = best > 0.0 ? zf(1.f, 0.f) / A[(int64_t)c * S + c] : zf(1.f, 0.f);
-    __syncthreads();
-    for (int j = threadIdx.x; j < S; j += blockDim.x)
-      A[(int64_t)c * S + j] = j == c ? d : A[(int64_t)c * S + j] * d;
-    for (int r = threadIdx.x; r < S; r += blockDim.x) fcol[r] = A[(int64_t)r * S + c];
-    __syncthreads();
-    for (int r = wid; r < S; r += nw) {  // one warp per row, the lanes along it
-      if (r == c) continue;
-      const zf f = fcol[r];
-      zf* Ar = A + (int64_t)r * S;
-      const zf* Ac = A + (int64_t)c * S;
-      for (int j = lane; j < S; j += 32) Ar[j] = j == c ? -(f * d) : Ar[j] - f * Ac[j];
-    }
-    __syncthreads();
+    for (int j = lane; j < S; j += 32) B[(int64_t)r * S + j] = A[(int64_t)r * S + j] * (wr * weight(j));
   }
-  for (int c = S - 1; c >= 0; --c) {
-    const int p = pv[c];
-    if (p != c)
-      for (int r = threadIdx.x; r < S; r += blockDim.x) {
-        const zf t0 = A[(int64_t)r * S + c];
-        A[(int64_t)r * S + c] = A[(int64_t)r * S + p];
-        A[(int64_t)r * S + p] = t0;
-      }
-    __syncthreads();
-  }
-  for (int r = wid; r < S; r += nw)
-    for (int j = lane; j < S; j += 32) A[(int64_t)r * S + j] = A[(int64_t)r * S + j] * (w[r] * w[j]);
 }
 
-// out = D_k^-1 in on the unknowns block k owns (complex64 inverse, fp32 sums), one warp per row
+// columns k0 .. k0 + kGj - 1; step[r]: the panel row r was a pivot of (-1: none
+// yet); prow[c]: the pivot row of column c
+__global__ void __launch_bounds__(1024) gj_panel_kernel(const int64_t* __restrict__ pc_off,
+                                                        const int64_t* __restrict__ doff, zf* __restrict__ G,
+                                                        zf* __restrict__ X, int32_t* __restrict__ step,
+                                                        int32_t* __restrict__ prow, int k0) {
+  __shared__ unsigned wkey[2][32], wrow[2][32];
+  __shared__ float2 pr[2][kGj];
+  __shared__ int plist[kGj];
+  const int k = blockIdx.x, S = (int)(pc_off[k + 1] - pc_off[k]);
+  if (k0 >= S) return;
+  const int w = min(kGj, S - k0), r = threadIdx.x, lane = r & 31, warp = r >> 5;
+  const int nwarp = (S + 31) >> 5;  // warps with rows
+  zf* A = G + doff[k];
+  zf x[kGj];
+  const bool in = r < S;
+  if (in)
+#pragma unroll
+    for (int c = 0; c < kGj; ++c) x[c] = c < w ? A[(int64_t)r * S + k0 + c] : zf();
+  bool unused = in && step[k * 1024 + r] < 0;
+  // the current column is always x[0]: a step leaves the others one place
+  // further to the front and its own column at the end, so that after kGj
+  // steps they are in order again
+#pragma unroll 1
+  for (int j = 0; j < kGj; ++j) {
+    if (j >= w) {
+      const zf x0 = x[0];
+#pragma unroll
+      for (int c = 0; c + 1 < kGj; ++c) x[c] = x[c + 1];
+      x[kGj - 1] = x0;
+      continue;
+    }
+    const int par = j & 1;
+    // largest |re| + |im| among the unused rows, the first row on ties (or
+    // where nothing is larger than zero)
+    const float v = unused ? fabs1(x[0]) : -1.f;
+    unsigned key = unused ? (v > 0.f ? __float_as_uint(v) + 1u : 1u) : 0u;
+    unsigned row = unused ? (unsigned)r : ~0u;
+    unsigned mk = __reduce_max_sync(~0u, key);
+    row = __reduce_min_sync(~0u, key == mk ? row : ~0u);
+    if (lane == 0) {
+      wkey[par][warp] = mk;
+      wrow[par][warp] = row;
+    }
+    __syncthreads();
+    key = lane < nwarp ? wkey[par][lane] : 0u;
+    row = lane < nwarp ? wrow[par][lane] : ~0u;
+    mk = __reduce_max_sync(~0u, key);
+    const int p = (int)__reduce_min_sync(~0u, key == mk ? row : ~0u);
+    if (r == p) {
+      const zf d = mk > 1u ? zf(1.f, 0.f) / x[0] : zf(1.f, 0.f);
+#pragma unroll
+      for (int c = 0; c < kGj; ++c) {
+        x[c] = c + 1 < kGj ? x[c + 1] * d : d;
+        pr[par][c] = make_float2(x[c].re, x[c].im);
+      }
+      plist[j] = p;
+      unused = false;
+    }
+    __syncthreads();
+    if (in && r != p) {
+      const zf f = x[0];
+#pragma unroll
+      for (int c = 0; c < kGj; ++c) {
+        const float2 u = pr[par][c];
+        x[c] = fnma(c + 1 < kGj ? x[c + 1] : zf(), f, zf(u.x, u.y));
+      }
+    }
+  }
+  __syncthreads();
+  if (in)
+#pragma unroll
+    for (int c = 0; c < kGj; ++c)
+      if (c < w) A[(int64_t)r * S + k0 + c] = x[c];
+  if (r < w) {
+    prow[k * 1024 + k0 + r] = plist[r];
+    step[k * 1024 + plist[r]] = k0;
+  }
+  // the pivot rows' columns as they were before this panel
+  zf* Xk = X + (int64_t)k * kGj * 1024;
+  for (int e = r; e < kGj * S; e += blockDim.x) {
+    const int j = e / S, c = e - j * S;
+    Xk[j * 1024 + c] = j < w ? A[(int64_t)plist[j] * S + c] : zf();
+  }
+}
+
+__global__ void __launch_bounds__(256) gj_update_kernel(const int64_t* __restrict__ pc_off,
+                                                        const int64_t* __restrict__ doff, zf* __restrict__ G,
+                                                        const zf* __restrict__ X, const int32_t* __restrict__ step,
+                                                        int k0) {
+  __shared__ float2 Ps[64][kGj + 1], Xs[kGj][64];
+  const int k = blockIdx.z, S = (int)(pc_off[k + 1] - pc_off[k]);
+  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+  if (k0 >= S || r0 >= S || c0 >= S) return;
+  zf* A = G + doff[k];
+  const int w = min(kGj, S - k0), tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  for (int e = threadIdx.x; e < 64 * kGj; e += 256) {
+    const int r = e / kGj, j = e % kGj;
+    const zf v = r0 + r < S && j < w ? A[(int64_t)(r0 + r) * S + k0 + j] : zf();
+    Ps[r][j] = make_float2(v.re, v.im);
+    const int jj = e >> 6, c = e & 63;
+    const zf u = c0 + c < S ? X[((int64_t)k * kGj + jj) * 1024 + c0 + c] : zf();
+    Xs[jj][c] = make_float2(u.re, u.im);
+  }
+  zf acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = r0 + ty + 16 * i;
+    const bool keep = r < S && step[k * 1024 + r] != k0;  // a pivot row of this panel starts from zero
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + tx + 16 * j;
+      acc[i][j] = keep && c < S ? A[(int64_t)r * S + c] : zf();
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < kGj; ++t) {
+    zf a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      a[i] = zf(-Ps[ty + 16 * i][t].x, -Ps[ty + 16 * i][t].y);
+      b[i] = zf(Xs[t][tx + 16 * i].x, Xs[t][tx + 16 * i].y);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = fnma(acc[i][j], a[i], b[j]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = r0 + ty + 16 * i;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + tx + 16 * j;
+      if (r < S && c < S && (c < k0 || c >= k0 + w)) A[(int64_t)r * S + c] = acc[i][j];
+    }
+  }
+}
+
+// D^-1[c][p_j] = w_c G[p_c][j] w_{p_j}, p the columns' pivot rows
+__global__ void __launch_bounds__(256) gj_finish_kernel(const int64_t* __restrict__ pc_off,
+                                                        const int64_t* __restrict__ doff, const zf* __restrict__ G,
+                                                        const float* __restrict__ w, const int32_t* __restrict__ prow,
+                                                        zf* __restrict__ D) {
+  const int k = blockIdx.x, S = (int)(pc_off[k + 1] - pc_off[k]);
+  const zf* A = G + doff[k];
+  zf* B = D + doff[k];
+  const int lane = threadIdx.x & 31, wid = blockIdx.y * 8 + (threadIdx.x >> 5), nw = gridDim.y * 8;
+  for (int c = wid; c < S; c += nw) {
+    const zf* row = A + (int64_t)prow[k * 1024 + c] * S;
+    for (int j = lane; j < S; j += 32) {
+      const int p = prow[k * 1024 + j];
+      B[(int64_t)c * S + p] = row[j] * (w[k * 1024 + c] * w[k * 1024 + p]);
+    }
+  }
+}
+
+// out = D_k^-1 in on the unknowns block k owns (complex64 inverse, fp32 sums),
+// one warp per row, the rows shared out to gridDim.y CTAs: the 16 blocks of N =
+// 2434 hold 46 MB, read in 106 us by one CTA each, in 28 us by 16
 __global__ void __launch_bounds__(256) psolve_kernel(const int64_t* __restrict__ pc_off, const int32_t* __restrict__ gidx,
                                                      const int8_t* __restrict__ own, const int64_t* __restrict__ doff,
                                                      const zf* __restrict__ D, const zd* __restrict__ in,
@@ -727,7 +960,7 @@ __global__ void __launch_bounds__(256) psolve_kernel(const int64_t* __restrict__
   for (int i = threadIdx.x; i < S; i += blockDim.x) xs[i] = zf(in[gidx[g0 + i]]);
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int r = wid; r < S; r += nw) {
+  for (int r = blockIdx.y * nw + wid; r < S; r += gridDim.y * nw) {
     if (!own[g0 + r]) continue;
     zf acc(0.f, 0.f);
     const zf* row = A + (int64_t)r * S;
@@ -786,6 +1019,7 @@ Tabs make_tabs(m25_greens* gr) {
   Tabs t;
   t.coef = reinterpret_cast<const zd*>(gr->coef);
   t.rho = gr->rho;
+  t.rho32 = gr->rho32;
   t.nrho = gr->nrho;
   t.L = gr->nlev;
   const int L = gr->nlev;
@@ -843,7 +1077,7 @@ int apply(m25_hmat* h, const zd* x, zd* y) {
 }
 
 int precond(m25_hmat* h, const zd* in, zd* out) {
-  psolve_kernel<<<h->npc, 256, 0, h->ctx->stream>>>(h->pc_off, h->pc_gidx, h->pc_own, h->pc_doff, h->D, in, out);
+  psolve_kernel<<<dim3(h->npc, 16), 256, 0, h->ctx->stream>>>(h->pc_off, h->pc_gidx, h->pc_own, h->pc_doff, h->D, in, out);
   M25_CHECK_LAUNCH();
   return M25_OK;
 }
@@ -997,6 +1231,7 @@ extern "C" int m25_hmat_create(m25_ctx* ctx, m25_geom* geom, const m25_hmat_desc
         if (!ok) return fail((set_error("m25_hmat_create: a preconditioner item outside its source block"), M25_ERR_VALUE));
       }
       doff[k + 1] = doff[k] + S * S;
+      h->pc_max = std::max(h->pc_max, (int)S);
     }
     for (int g = 0; g < h->n; ++g)
       if (owned[g] != 1) return fail((set_error("m25_hmat_create: an unknown not owned by exactly one block"), M25_ERR_VALUE));
@@ -1042,6 +1277,11 @@ extern "C" int m25_hmat_create(m25_ctx* ctx, m25_geom* geom, const m25_hmat_desc
   TRY(dalloc(h->allocs, &h->ZxbT, (size_t)d->nb * std::max(d->nv, 1)));
   TRY(dalloc(h->allocs, &h->Zxx, (size_t)std::max(d->nv, 1) * std::max(d->nv, 1)));
   TRY(dalloc(h->allocs, &h->D, h->d_entries));
+  TRY(dalloc(h->allocs, &h->G, h->d_entries));
+  TRY(dalloc(h->allocs, &h->gj_x, (size_t)d->npc * kGj * 1024));
+  TRY(dalloc(h->allocs, &h->gj_w, (size_t)d->npc * 1024));
+  TRY(dalloc(h->allocs, &h->gj_step, (size_t)d->npc * 1024));
+  TRY(dalloc(h->allocs, &h->gj_prow, (size_t)d->npc * 1024));
   TRY(dalloc(h->allocs, &h->aca_ids, std::max(h->naca, 1)));
   TRY(dalloc(h->allocs, &h->rank, std::max(h->naca, 1)));
   TRY(dalloc(h->allocs, &h->status, std::max(h->naca, 1)));
@@ -1181,8 +1421,8 @@ extern "C" int m25_hmat_assemble(m25_hmat* h, m25_greens* gr, double zs_re, doub
       set_error("m25_hmat_assemble: copy failed");
       return done(M25_ERR_CUDA);
     }
-    aca_kernel<<<h->naca, 256, 0, st>>>(t, h->rules, h->lev, h->fb, h->aca_ids, h->pool, h->flags, h->tol, h->rank,
-                                        h->status);
+    aca_kernel<<<h->naca * kAcaCl, 256, 0, st>>>(t, h->rules, h->lev, h->fb, h->aca_ids, h->pool, h->flags, h->tol,
+                                                 h->rank, h->status);
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpyAsync(rk.data(), h->rank, sizeof(int32_t) * h->naca, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(stt.data(), h->status, sizeof(int32_t) * h->naca, cudaMemcpyDeviceToHost, st) != cudaSuccess) {
@@ -1262,7 +1502,7 @@ extern "C" int m25_hmat_assemble(m25_hmat* h, m25_greens* gr, double zs_re, doub
     return done(M25_ERR_CUDA);
   }
   if (!dense.empty())
-    far_dense_kernel<<<(unsigned)dense.size(), 256, 0, st>>>(t, h->rules, h->lev, h->fb, h->dense_ids, h->dense_pool);
+    far_dense_kernel<<<dim3((unsigned)dense.size(), kFarSplit), 256, 0, st>>>(t, h->rules, h->lev, h->fb, h->dense_ids, h->dense_pool);
   // preconditioner: the diagonal blocks and their LU
   {  // the matvec's double-float copies of the operator
     auto split = [&](const zd* src, float4* dst, int64_t n) {
@@ -1275,10 +1515,17 @@ extern "C" int m25_hmat_assemble(m25_hmat* h, m25_greens* gr, double zs_re, doub
   }
   wscale_kernel<<<(h->n + 255) / 256, 256, 0, st>>>(h->nb, h->n, h->nv, h->row_leaf, h->self_near, h->near,
                                                     h->near_off, h->Zn, h->Zxx, h->wsc);
-  diag_kernel<<<h->npc, 256, 0, st>>>(h->pc_off, h->pc_gidx, h->pc_item_off, h->pc_items, h->pc_doff, h->nb, h->nv,
+  diag_kernel<<<dim3(h->npc, 32), 256, 0, st>>>(h->pc_off, h->pc_gidx, h->pc_item_off, h->pc_items, h->pc_doff, h->nb, h->nv,
                                       h->nnear, h->leaf_lo, h->near_off, h->Zn, h->fb, h->pool, h->dense_pool, h->ZxbT,
                                       h->Zxx, h->D);
-  ginv_kernel<<<h->npc, 1024, 0, st>>>(h->pc_off, h->pc_doff, h->D);  // 32 warps: the sweeps wait on L2
+  gj_scale_kernel<<<dim3(h->npc, 16), 256, 0, st>>>(h->pc_off, h->pc_doff, h->D, h->G, h->gj_w, h->gj_step);
+  const int tiles = (h->pc_max + 63) / 64;
+  for (int k0 = 0; k0 < h->pc_max; k0 += kGj) {
+    gj_panel_kernel<<<h->npc, (h->pc_max + 31) / 32 * 32, 0, st>>>(h->pc_off, h->pc_doff, h->G, h->gj_x, h->gj_step,
+                                                                  h->gj_prow, k0);
+    gj_update_kernel<<<dim3(tiles, tiles, h->npc), 256, 0, st>>>(h->pc_off, h->pc_doff, h->G, h->gj_x, h->gj_step, k0);
+  }
+  gj_finish_kernel<<<dim3(h->npc, 16), 256, 0, st>>>(h->pc_off, h->pc_doff, h->G, h->gj_w, h->gj_prow, h->D);
   if (cudaGetLastError() != cudaSuccess) {
     set_error("m25_hmat_assemble: launch failed");
     return done(M25_ERR_CUDA);
