@@ -254,13 +254,18 @@ __device__ __forceinline__ float tf32_rna(float x) {
 }
 
 // The panel's row interchanges applied to the columns outside it, fused with
-// U12 = L11^-1 A12 on the columns to its right (L11 unit lower). A CTA owns
-// 32 columns: it gathers the rows the interchanges touch into shared memory
-// (lane = column), writes them to their final rows, and on the right-hand
-// columns runs the forward substitution with 8 lanes per column, each lane
-// holding W / 8 of the w <= W panel rows (rows l, l + 8, ...): at step t the
-// lane of row t passes x[t] to the other 7 by a shuffle. Every element
-// takes its subtractions in the order t = 0, 1, ... as in LAPACK's ztrsm.
+// U12 = L11^-1 A12 on the columns to its right (L11 unit lower). A CTA owns NC
+// columns: it gathers the rows the interchanges touch into shared memory,
+// writes them to their final rows, and on the right-hand columns runs the
+// forward substitution with LPC lanes per column, each lane holding W / LPC of
+// the w <= W panel rows (rows l, l + LPC, ...): at step t the lane of row t
+// passes x[t] to the others by a shuffle. Every element takes its
+// subtractions in the order t = 0, 1, ... as in LAPACK's ztrsm.
+// complex64: 32 columns, 8 lanes each. complex128: 8 columns, 16 lanes each, as
+// a warp's fp64 instruction holds its unit for 64 cycles: four times as many
+// CTAs share the columns and a lane has four rows (N = 546 / 1085 / 2434 / 5943,
+// all launches of a factorisation: @SWAP@ ms; 1.07 / 2.15 / 5.1 / 20.5 ms with
+// 32 columns, 8 lanes and six fp64 operations per product).
 // The interchanges are composed, not replayed: the rows touched are the w
 // panel rows and the pivot rows below the panel, and the original row that
 // ends in position x is found by applying the swaps to x in reverse order.
@@ -269,31 +274,39 @@ __device__ __forceinline__ float tf32_rna(float x) {
 // panel's (vc < k0: column vc, else column vc + w). W = 128 serves a block
 // of two 64-column panels whose interchanges and L11 are taken together.
 constexpr int kSwapMaxW = 64;
-constexpr int kSwapLd = 33;  // row stride of the gathered rows (complex elements)
-
 constexpr int kLsLd = 65;  // row stride of a 64 x 64 block of L11 in shared memory (complex elements)
+
+template <class T>
+struct SwapShape {
+  static constexpr int LPC = sizeof(T) == 4 ? 8 : 16, NC = sizeof(T) == 4 ? 32 : 8;
+  static constexpr int kThreads = LPC * NC;
+};
 
 // shared memory: W / 64 blocks of L11 (64 x 64, transposed) and the W gathered rows
 template <class T, int W = kSwapMaxW>
 __host__ __device__ constexpr size_t swap_trsm_smem() {
-  return sizeof(cx<T>) * ((size_t)(W / 64) * 64 * kLsLd + (size_t)W * kSwapLd);
+  return sizeof(cx<T>) * ((size_t)(W / 64) * 64 * kLsLd + (size_t)W * (SwapShape<T>::NC + 1));
 }
 
 // Lb[t * kLsLd + r] = L11[r0 + r][c0 + t] for r0 + r < w (strictly below the
 // diagonal on a diagonal block), zero elsewhere; rows of A read coalesced
 template <class T>
 __device__ __forceinline__ void load_l_block(cx<T>* Lb, const cx<T>* A, int64_t lda, int k0, int w, int r0, int c0) {
-  cx<T> v[16];
+  constexpr int kThreads = SwapShape<T>::kThreads;
 #pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const int e = threadIdx.x + 256 * k, t = e & 63, r = e >> 6;
-    const bool keep = r0 + r < w && (r0 != c0 || t < r);
-    v[k] = keep ? A[(int64_t)(k0 + r0 + r) * lda + k0 + c0 + t] : cx<T>();
-  }
+  for (int b = 0; b < 64 * 64 / (16 * kThreads); ++b) {
+    cx<T> v[16];
 #pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const int e = threadIdx.x + 256 * k, t = e & 63, r = e >> 6;
-    Lb[t * kLsLd + r] = v[k];
+    for (int k = 0; k < 16; ++k) {
+      const int e = threadIdx.x + kThreads * (16 * b + k), t = e & 63, r = e >> 6;
+      const bool keep = r0 + r < w && (r0 != c0 || t < r);
+      v[k] = keep ? A[(int64_t)(k0 + r0 + r) * lda + k0 + c0 + t] : cx<T>();
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const int e = threadIdx.x + kThreads * (16 * b + k), t = e & 63, r = e >> 6;
+      Lb[t * kLsLd + r] = v[k];
+    }
   }
 }
 
@@ -302,23 +315,26 @@ __device__ __forceinline__ void load_l_block(cx<T>* Lb, const cx<T>* A, int64_t 
 // ([hi | lo] planes of width P); this call writes K positions koff ..
 // koff + 2 W - 1 of each plane.
 template <class T, int W = kSwapMaxW>
-__global__ void __launch_bounds__(256) swap_trsm_kernel(cx<T>* A, int64_t lda, int n, int k0, int w,
-                                                        const int32_t* __restrict__ ipiv, float* __restrict__ B2,
-                                                        int P, int vc_begin, int vc_end, int koff = 0,
-                                                        bool solve = true) {
+__global__ void __launch_bounds__(SwapShape<T>::kThreads)
+    swap_trsm_kernel(cx<T>* A, int64_t lda, int n, int k0, int w, const int32_t* __restrict__ ipiv,
+                     float* __restrict__ B2, int P, int vc_begin, int vc_end, int koff, bool solve) {
   static_assert(W == 64 || W == 128, "panel blocks of 64 or 128 columns");
+  constexpr int LPC = SwapShape<T>::LPC, NC = SwapShape<T>::NC, kLd = NC + 1;
+  static_assert(W <= SwapShape<T>::kThreads, "a pivot per thread");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // L11 in 64 x 64 blocks, transposed: for W = 128 first [L11 of rows and
   // columns 0..63 | rows 64..127 x columns 0..63], then rows and columns 64..127
   // in the first buffer
   cx<T>* Ls = reinterpret_cast<cx<T>*>(smem_raw);
   cx<T>* Ls1 = Ls + (W / 64 - 1) * 64 * kLsLd;
-  cx<T>* V = Ls + (W / 64) * 64 * kLsLd;  // the w panel rows of the CTA's columns [W][kSwapLd]
+  cx<T>* V = Ls + (W / 64) * 64 * kLsLd;  // the w panel rows of the CTA's columns [W][kLd]
   __shared__ int piv[W], dst[2 * W], src[2 * W];
   __shared__ int nd_s;
+  grid_wait();
+  grid_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kend = k0 + w;
-  const int vc0 = vc_begin + blockIdx.x * 32;  // first column of the CTA, counted without the panel's
+  const int vc0 = vc_begin + blockIdx.x * NC;  // first column of the CTA, counted without the panel's
   // positions touched: the panel rows, then each pivot row below the panel
   // once (its first occurrence among the panel's pivots, in order); one
   // pivot per thread of the first W / 32 warps
@@ -353,8 +369,8 @@ __global__ void __launch_bounds__(256) swap_trsm_kernel(cx<T>* A, int64_t lda, i
     for (int u = 0; u < W / 32; ++u) nx += wcnt[u];
     nd_s = w + nx;
   }
-  // the CTA's columns vc0 .. vc0 + 31 map to vc (< k0) or vc + w (right of the panel)
-  const bool any_right = solve && kend < n && min(vc0 + 31, vc_end - 1) >= k0;
+  // the CTA's columns vc0 .. vc0 + NC - 1 map to vc (< k0) or vc + w (right of the panel)
+  const bool any_right = solve && kend < n && min(vc0 + NC - 1, vc_end - 1) >= k0;
   if (any_right) {
     load_l_block(Ls, A, lda, k0, w, 0, 0);
     if (W == 128) load_l_block(Ls1, A, lda, k0, w, 64, 0);
@@ -362,7 +378,7 @@ __global__ void __launch_bounds__(256) swap_trsm_kernel(cx<T>* A, int64_t lda, i
   __syncthreads();
   const int nd = nd_s;
   // the original row of each touched position: the swaps applied to it in
-  // reverse order, one position per thread (nd <= 2 W <= the CTA's threads)
+  // reverse order, one position per thread
   for (int i = threadIdx.x; i < nd; i += blockDim.x) {
     int y = dst[i];
 #pragma unroll 4
@@ -373,58 +389,59 @@ __global__ void __launch_bounds__(256) swap_trsm_kernel(cx<T>* A, int64_t lda, i
     src[i] = y;
   }
   __syncthreads();
-  const int vc = vc0 + lane;
+  const int ci = threadIdx.x % NC, ri = threadIdx.x / NC;  // rows ri, ri + LPC, ... of column ci
+  const int vc = vc0 + ci;
   const bool valid = vc < vc_end;
   const int c = vc < k0 ? vc : vc + w;
   const bool right = solve && c >= kend;
   {
-    // warp q gathers rows q, q + 8, ...; every row of the CTA's columns is
-    // read before any is written (the barrier), as rows move between warps
-    cx<T> v[2 * W / 8];
+    // every row of the CTA's columns is read before any is written (the
+    // barrier), as rows move between threads
+    cx<T> v[2 * W / LPC];
 #pragma unroll
-    for (int j = 0; j < 2 * W / 8; ++j) {
-      const int i = warp + 8 * j;
+    for (int j = 0; j < 2 * W / LPC; ++j) {
+      const int i = ri + LPC * j;
       v[j] = valid && i < nd ? A[(int64_t)src[i] * lda + c] : cx<T>();
     }
     if (any_right)
 #pragma unroll
-      for (int j = 0; j < 2 * W / 8; ++j) {
-        const int i = warp + 8 * j;
-        if (i < w) V[i * kSwapLd + lane] = v[j];
+      for (int j = 0; j < 2 * W / LPC; ++j) {
+        const int i = ri + LPC * j;
+        if (i < w) V[i * kLd + ci] = v[j];
       }
     __syncthreads();
     // rows that are not solved go straight to their final rows
 #pragma unroll
-    for (int j = 0; j < 2 * W / 8; ++j) {
-      const int i = warp + 8 * j;
+    for (int j = 0; j < 2 * W / LPC; ++j) {
+      const int i = ri + LPC * j;
       if (valid && i < nd && (i >= w || !right) && src[i] != dst[i]) A[(int64_t)dst[i] * lda + c] = v[j];
     }
   }
   if (!any_right) return;
   {
-    constexpr int R = W / 8;  // rows per lane
-    const int l8 = lane & 7, col = 4 * warp + (lane >> 3);
+    constexpr int R = W / LPC, RB = 64 / LPC;  // rows per lane, of which in the first 64
+    const int l = lane % LPC, col = threadIdx.x / LPC;
     cx<T> x[R];
 #pragma unroll
-    for (int k = 0; k < R; ++k) x[k] = l8 + 8 * k < w ? V[(l8 + 8 * k) * kSwapLd + col] : cx<T>();
+    for (int k = 0; k < R; ++k) x[k] = l + LPC * k < w ? V[(l + LPC * k) * kLd + col] : cx<T>();
     // rows 0..63 (and, for W = 128, rows 64..127 take their products with
-    // them); the loops over a lane's registers are unrolled, the 8 steps
+    // them); the loops over a lane's registers are unrolled, the LPC steps
     // within a group of rows are not (a fully unrolled substitution is
     // thousands of instructions, and the warps then wait on instruction fetch)
 #pragma unroll
-    for (int kb = 0; kb < 8; ++kb)
+    for (int kb = 0; kb < RB; ++kb)
 #pragma unroll 1
-      for (int j = 0; j < 8; ++j) {
-        const int t = 8 * kb + j;
+      for (int j = 0; j < LPC; ++j) {
+        const int t = LPC * kb + j;
         cx<T> xt;
-        xt.re = __shfl_sync(~0u, x[kb].re, (lane & ~7) | j);
-        xt.im = __shfl_sync(~0u, x[kb].im, (lane & ~7) | j);
+        xt.re = __shfl_sync(~0u, x[kb].re, (lane & ~(LPC - 1)) | j);
+        xt.im = __shfl_sync(~0u, x[kb].im, (lane & ~(LPC - 1)) | j);
         // L11 rows >= w and on / above the diagonal are zero in Ls
 #pragma unroll
-        for (int k = kb; k < 8; ++k)
-          if (k > kb || l8 > j) x[k] -= Ls[t * kLsLd + l8 + 8 * k] * xt;
+        for (int k = kb; k < RB; ++k)
+          if (k > kb || l > j) x[k] = fnma(x[k], Ls[t * kLsLd + l + LPC * k], xt);
 #pragma unroll
-        for (int k = 8; k < R; ++k) x[k] -= Ls1[t * kLsLd + l8 + 8 * (k - 8)] * xt;
+        for (int k = RB; k < R; ++k) x[k] = fnma(x[k], Ls1[t * kLsLd + l + LPC * (k - RB)], xt);
       }
     if (W == 128) {
       // rows 64..127 with their own diagonal block, loaded over the first one
@@ -432,52 +449,53 @@ __global__ void __launch_bounds__(256) swap_trsm_kernel(cx<T>* A, int64_t lda, i
       load_l_block(Ls, A, lda, k0, w, 64, 64);
       __syncthreads();
 #pragma unroll
-      for (int kb = 8; kb < R; ++kb)
+      for (int kb = RB; kb < R; ++kb)
 #pragma unroll 1
-        for (int j = 0; j < 8; ++j) {
-          const int t = 8 * (kb - 8) + j;
+        for (int j = 0; j < LPC; ++j) {
+          const int t = LPC * (kb - RB) + j;
           cx<T> xt;
-          xt.re = __shfl_sync(~0u, x[kb].re, (lane & ~7) | j);
-          xt.im = __shfl_sync(~0u, x[kb].im, (lane & ~7) | j);
+          xt.re = __shfl_sync(~0u, x[kb].re, (lane & ~(LPC - 1)) | j);
+          xt.im = __shfl_sync(~0u, x[kb].im, (lane & ~(LPC - 1)) | j);
 #pragma unroll
           for (int k = kb; k < R; ++k)
-            if (k > kb || l8 > j) x[k] -= Ls[t * kLsLd + l8 + 8 * (k - 8)] * xt;
+            if (k > kb || l > j) x[k] = fnma(x[k], Ls[t * kLsLd + l + LPC * (k - RB)], xt);
         }
     }
 #pragma unroll
     for (int k = 0; k < R; ++k)
-      if (l8 + 8 * k < w) V[(l8 + 8 * k) * kSwapLd + col] = x[k];
+      if (l + LPC * k < w) V[(l + LPC * k) * kLd + col] = x[k];
   }
   __syncthreads();
   if (valid && right)
 #pragma unroll
-    for (int j = 0; j < W / 8; ++j) {
-      const int i = warp + 8 * j;
-      if (i < w) A[(int64_t)(k0 + i) * lda + c] = V[i * kSwapLd + lane];
+    for (int j = 0; j < W / LPC; ++j) {
+      const int i = ri + LPC * j;
+      if (i < w) A[(int64_t)(k0 + i) * lda + c] = V[i * kLd + ci];
     }
-  if (B2) {
-    // U12 as the tensor-core update's B operand: for trailing column cc the
-    // rows 2 cc (re, im) and 2 cc + 1 (im, -re) of (U, -iU), K-major, split
-    // into tf32 hi and lo planes P floats apart, zero beyond 2 w
-    for (int row = warp; row < 64; row += 8) {  // row = 2 x (column of the CTA) + part
-      const int cl = row >> 1, part = row & 1;
-      const int vcl = vc0 + cl;
-      if (vcl >= vc_end || vcl < k0) continue;  // not a trailing column
-      const int cc = vcl - k0;                  // = (vcl + w) - kend
-      for (int jj = lane; jj < 2 * W; jj += 32) {
-      const int t = jj >> 1, f = jj & 1;
-      float hi = 0.f, lo = 0.f;
-      if (t < w) {
-        const cx<T> U = V[t * kSwapLd + cl];
-        const float v = part == 0 ? (f == 0 ? (float)U.re : (float)U.im) : (f == 0 ? (float)U.im : -(float)U.re);
-        hi = tf32_rna(v);
-        lo = tf32_rna(v - hi);
-      }
-      B2[(int64_t)(2 * cc + part) * 2 * P + koff + jj] = hi;
-      B2[(int64_t)(2 * cc + part) * 2 * P + P + koff + jj] = lo;
+  if constexpr (sizeof(T) == 4)
+    if (B2) {
+      // U12 as the tensor-core update's B operand: for trailing column cc the
+      // rows 2 cc (re, im) and 2 cc + 1 (im, -re) of (U, -iU), K-major, split
+      // into tf32 hi and lo planes P floats apart, zero beyond 2 w
+      for (int row = warp; row < 64; row += 8) {  // row = 2 x (column of the CTA) + part
+        const int cl = row >> 1, part = row & 1;
+        const int vcl = vc0 + cl;
+        if (vcl >= vc_end || vcl < k0) continue;  // not a trailing column
+        const int cc = vcl - k0;                  // = (vcl + w) - kend
+        for (int jj = lane; jj < 2 * W; jj += 32) {
+          const int t = jj >> 1, f = jj & 1;
+          float hi = 0.f, lo = 0.f;
+          if (t < w) {
+            const cx<T> U = V[t * kLd + cl];
+            const float v = part == 0 ? (f == 0 ? (float)U.re : (float)U.im) : (f == 0 ? (float)U.im : -(float)U.re);
+            hi = tf32_rna(v);
+            lo = tf32_rna(v - hi);
+          }
+          B2[(int64_t)(2 * cc + part) * 2 * P + koff + jj] = hi;
+          B2[(int64_t)(2 * cc + part) * 2 * P + P + koff + jj] = lo;
+        }
       }
     }
-  }
 }
 
 // C[r][c] -= sum_t Lp[r][t] Up[t][c] over rows / cols >= off, t < nb:
@@ -634,7 +652,7 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
   // M25_PANEL_CLUSTER_MIN: the smallest cluster size used (4, 8 or 16; a tuning knob)
   static const int cl_min_env = [] {
     const char* e = getenv("M25_PANEL_CLUSTER_MIN");
-    const int v = e ? atoi(e) : 4;
+    const int v = e ? atoi(e) : 8;
     return v >= 16 ? 16 : v >= 8 ? 8 : 4;
   }();
   // the context's setting (m25_ctx_set_tuning) over the process default
@@ -699,9 +717,10 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
   auto swap_trsm = [&](int k0, int w, int vc_begin, int vc_end, float* B2, int P2) -> int {
     if (vc_end <= vc_begin) return M25_OK;
     StageTimer tm(ctx, ST_TRSM);
-    swap_trsm_kernel<T><<<(vc_end - vc_begin + 31) / 32, 256, swap_trsm_smem<T>(), st>>>(A, lda, n, k0, w, ipiv, B2,
-                                                                                         P2, vc_begin, vc_end, 0, true);
-    M25_CHECK_LAUNCH();
+    using Sw = SwapShape<T>;
+    M25_CUDA(launch_chained(swap_trsm_kernel<T, kSwapMaxW>, dim3((vc_end - vc_begin + Sw::NC - 1) / Sw::NC), Sw::kThreads,
+                            swap_trsm_smem<T>(), st, A, lda, n, k0, w, (const int32_t*)ipiv, B2, P2, vc_begin, vc_end,
+                            0, true));
     return M25_OK;
   };
   // the same for a block of w <= 128 columns (two panels' interchanges and a
@@ -711,9 +730,9 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
                           bool solve) -> int {
     if (vc_end <= vc_begin) return M25_OK;
     StageTimer tm(ctx, ST_TRSM);
-    swap_trsm_kernel<T, 128><<<(vc_end - vc_begin + 31) / 32, 256, swap_trsm_smem<T, 128>(), st>>>(
-        A, lda, n, k0, w, piv, B2, P, vc_begin, vc_end, koff, solve);
-    M25_CHECK_LAUNCH();
+    using Sw = SwapShape<T>;
+    M25_CUDA(launch_chained(swap_trsm_kernel<T, 128>, dim3((vc_end - vc_begin + Sw::NC - 1) / Sw::NC), Sw::kThreads,
+                            swap_trsm_smem<T, 128>(), st, A, lda, n, k0, w, piv, B2, P, vc_begin, vc_end, koff, solve));
     return M25_OK;
   };
   int rc = M25_OK;

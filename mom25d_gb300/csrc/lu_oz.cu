@@ -173,9 +173,6 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag, n_issued, n_consumed, skip;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) skip = *(volatile int*)a.err;  // an earlier launch gave up
-  __syncthreads();
-  if (skip) return;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kOzStages; ++s) {
       bar_init(&full[s], 1);
@@ -189,6 +186,10 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(&tmA) : "memory");
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(&tmB) : "memory");
   }
+  grid_wait();
+  if (threadIdx.x == 0) skip = *(volatile int*)a.err;  // an earlier launch gave up
+  __syncthreads();
+  if (skip) return;
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(s32(&tmem_base)), "r"(512));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     }
     if (!ok) *abort_v = 1;
   }
+  grid_trigger();  // not before: CTAs of the next kernel would wait on SMs that other streams can use
   __syncthreads();
   if (threadIdx.x == 0) {
     if (abort_flag) {
@@ -384,6 +386,8 @@ __device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(~0u, v
 __global__ void __launch_bounds__(256) oz_scale_kernel(const zd* __restrict__ A, int64_t lda, int k0, int m,
                                                        int* __restrict__ gsum, int ctas_l) {
   __shared__ int red[2][64];
+  grid_wait();
+  grid_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < 128) red[threadIdx.x >> 6][threadIdx.x & 63] = 0;
   __syncthreads();
@@ -451,6 +455,8 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const zd* __restrict__ A, 
                                                       const int* __restrict__ gsum, uint2* __restrict__ Aq,
                                                       uint2* __restrict__ Bq, int* __restrict__ ea,
                                                       int* __restrict__ eb, int ctas_a) {
+  grid_wait();
+  grid_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = k0 + 64;
   const int g[2] = {oz_balance(gsum, 2 * lane), oz_balance(gsum, 2 * lane + 1)};
   double x[4];
@@ -651,9 +657,9 @@ int lu_oz_prepare(m25_ctx* ctx, int n) {
 }
 
 // the sums that balance the block at k0 (gsum: 256 ints, zero)
-static void oz_scale(m25_ctx* ctx, const zd* A, int64_t lda, int k0, int m, int* gsum) {
+static cudaError_t oz_scale(m25_ctx* ctx, const zd* A, int64_t lda, int k0, int m, int* gsum) {
   const int cl = std::min((m + 7) / 8, ctx->num_sms);
-  oz_scale_kernel<<<cl + 64, 256, 0, ctx->stream>>>(A, lda, k0, m, gsum, cl);
+  return launch_chained(oz_scale_kernel, dim3(cl + 64), 256, 0, ctx->stream, A, lda, k0, m, gsum, cl);
 }
 
 // A22 -= L21 U12 after the block of 64 columns at k0 on the CUDA cores; work: 1 KB on the device
@@ -669,7 +675,7 @@ int lu_oz_update_simt(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0, void* wor
   int* gsum = static_cast<int*>(work);
   StageTimer tm(ctx, ST_GEMM);
   M25_CUDA(cudaMemsetAsync(gsum, 0, 256 * sizeof(int), ctx->stream));
-  oz_scale(ctx, A, lda, k0, m, gsum);
+  M25_CUDA(oz_scale(ctx, A, lda, k0, m, gsum));
   oz_simt_kernel<<<dim3((m + kSimtC - 1) / kSimtC, (m + kSimtR - 1) / kSimtR), 256, kSimtSmem, ctx->stream>>>(
       A, lda, k0, m, gsum);
   M25_CHECK_LAUNCH();
@@ -703,10 +709,9 @@ int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0) {
   }
   {
     StageTimer tm(ctx, ST_PACK);
-    oz_scale(ctx, A, lda, k0, m, gsum);
+    M25_CUDA(oz_scale(ctx, A, lda, k0, m, gsum));
     const int ca = (m + 7) / 8, cb = (m + 31) / 32;
-    oz_pack_kernel<<<ca + cb, 256, 0, st>>>(A, lda, k0, m, gsum, aq, bq, ea, eb, ca);
-    M25_CHECK_LAUNCH();
+    M25_CUDA(launch_chained(oz_pack_kernel, dim3(ca + cb), 256, 0, st, A, lda, k0, m, gsum, aq, bq, ea, eb, ca));
   }
   OzArgs g;
   g.C = A + (int64_t)(k0 + 64) * lda + k0 + 64;
@@ -719,8 +724,7 @@ int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0) {
   g.eb = eb;
   g.err = reinterpret_cast<int*>(b);
   StageTimer tm(ctx, ST_GEMM);
-  oz_gemm_kernel<<<std::min(g.ntiles, ctx->num_sms), kOzThreads, kOzSmem, st>>>(ma, mb, g);
-  M25_CHECK_LAUNCH();
+  M25_CUDA(launch_chained(oz_gemm_kernel, dim3(std::min(g.ntiles, ctx->num_sms)), kOzThreads, kOzSmem, st, ma, mb, g));
   return M25_OK;
 }
 

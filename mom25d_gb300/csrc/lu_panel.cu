@@ -144,48 +144,160 @@ __device__ __forceinline__ unsigned long long val_key(double v) {
 template <class T>
 using KeyOf = decltype(val_key(T(0)));
 
+// A thread's row of the strip, from column jb on (a multiple of kGrp) at index
+// 0. complex64 columns go in pairs, real and imaginary parts apart, for the
+// packed fp32 multiply-add (two per lane and instruction). (A row that moves one
+// column to the front with every update, so that the loop over the columns
+// needs no unrolling, is half the code and 5 to 10 % slower: it spills.)
+template <class T>
+struct StripRow;
+template <>
+struct StripRow<double> {
+  static constexpr int W = strip_w<double>();
+  cx<double> x[W];
+  __device__ __forceinline__ cx<double> get(int i) const { return x[i]; }
+  __device__ __forceinline__ void set(int i, cx<double> v) { x[i] = v; }
+  // chunk k (16 bytes) of the row as it is sent
+  __device__ __forceinline__ uint4 chunk(int k) const {
+    return make_uint4((unsigned)__double2loint(x[k].re), (unsigned)__double2hiint(x[k].re),
+                      (unsigned)__double2loint(x[k].im), (unsigned)__double2hiint(x[k].im));
+  }
+  static __device__ __forceinline__ cx<double> sent(const uint4* u, int c) {
+    return *reinterpret_cast<const cx<double>*>(u + c);
+  }
+  // x_i -= l u_i for i >= i0 and jb + i < W (u: the pivot row's chunks from column jb)
+  __device__ __forceinline__ void update(int i0, int jb, cx<double> l, const uint4* u) {
+#pragma unroll
+    for (int i = 0; i < kGrp; ++i)
+      if (i >= i0) x[i] = fnma(x[i], l, *reinterpret_cast<const cx<double>*>(u + i));
+    if (jb + kGrp < W)  // no fp64 operation for nothing
+#pragma unroll
+      for (int i = kGrp; i < W; ++i) x[i] = fnma(x[i], l, *reinterpret_cast<const cx<double>*>(u + i));
+  }
+  __device__ __forceinline__ void shift() {
+#pragma unroll
+    for (int i = 0; i + kGrp < W; ++i) x[i] = x[i + kGrp];
+  }
+};
+template <>
+struct StripRow<float> {
+  static constexpr int W = strip_w<float>();
+  float4 x[W / 2];  // columns 2 k, 2 k + 1: (re, re, im, im)
+  __device__ __forceinline__ cx<float> get(int i) const {
+    return (i & 1) ? cx<float>(x[i / 2].y, x[i / 2].w) : cx<float>(x[i / 2].x, x[i / 2].z);
+  }
+  __device__ __forceinline__ void set(int i, cx<float> v) {
+    if (i & 1) {
+      x[i / 2].y = v.re;
+      x[i / 2].w = v.im;
+    } else {
+      x[i / 2].x = v.re;
+      x[i / 2].z = v.im;
+    }
+  }
+  __device__ __forceinline__ uint4 chunk(int k) const {
+    return make_uint4(__float_as_uint(x[k].x), __float_as_uint(x[k].y), __float_as_uint(x[k].z),
+                      __float_as_uint(x[k].w));
+  }
+  static __device__ __forceinline__ cx<float> sent(const uint4* u, int c) {
+    const float* f = reinterpret_cast<const float*>(u + c / 2) + (c & 1);
+    return cx<float>(f[0], f[2]);
+  }
+  static __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    union {
+      float2 f;
+      unsigned long long u;
+    } x = {a}, y = {b}, z = {c}, r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r.u) : "l"(x.u), "l"(y.u), "l"(z.u));
+    return r.f;
+  }
+  // Columns beyond the strip's end are updated too, with whatever lies behind
+  // the pivot row (within the exchange's memory): the packed multiply-adds cost
+  // less than the branches around them, which would expose the loads' latency
+  // once per group.
+  __device__ __forceinline__ void update(int i0, int jb, cx<float> l, const uint4* u) {
+    const float2 nr = make_float2(-l.re, -l.re), ni = make_float2(-l.im, -l.im), pi = make_float2(l.im, l.im);
+    auto pair = [&](int k) {
+      const float4 v = *reinterpret_cast<const float4*>(u + k);
+      const float2 ur = make_float2(v.x, v.y), ui = make_float2(v.z, v.w);
+      const float2 re = fma2(pi, ui, fma2(nr, ur, make_float2(x[k].x, x[k].y)));
+      const float2 im = fma2(ni, ur, fma2(nr, ui, make_float2(x[k].z, x[k].w)));
+      x[k] = make_float4(re.x, re.y, im.x, im.y);
+    };
+    if (i0 & 1) {  // the pair's second column alone
+      const float4 v = *reinterpret_cast<const float4*>(u + i0 / 2);
+      set(i0, fnma(get(i0), l, cx<float>(v.y, v.w)));
+    }
+#pragma unroll
+    for (int k = 0; k < W / 4; ++k)
+      if (2 * k >= i0) pair(k);
+    if (jb < W / 2)
+#pragma unroll
+      for (int k = W / 4; k < W / 2; ++k) pair(k);
+  }
+  __device__ __forceinline__ void shift() {
+#pragma unroll
+    for (int i = 0; i + kGrp / 2 < W / 2; ++i) x[i] = x[i + kGrp / 2];
+  }
+};
+
+// What the cluster's CTAs send one another, at the start of the dynamic shared
+// memory: per column parity the barrier, every CTA's candidate and its row.
+template <class T, int CL>
+struct StripShared {
+  static constexpr int kCh = strip_w<T>() * (int)sizeof(cx<T>) / 16;  // 16-byte chunks of a row
+  uint64_t colbar[2];
+  StripCand<T> cand[2][CL];
+  uint4 crow[2][CL][kCh];
+  uint4 stage[kCh];  // this CTA's candidate row; behind crow, see StripRow<float>::update
+};
+
 template <class T, int CL>
 __host__ __device__ constexpr size_t strip_smem(int R, int nother) {
   constexpr int W = strip_w<T>();
-  // the rows (padded to an even count of elements), candidate rows of both parities, the moved rows' other columns
-  return sizeof(cx<T>) * (((size_t)R * (W + 1) + 1) / 2 * 2 + 2 * CL * W + (size_t)2 * W * nother);
+  // the exchange, the rows (padded to an even count of elements), the moved rows' other columns
+  return sizeof(StripShared<T, CL>) + sizeof(cx<T>) * (((size_t)R * (W + 1) + 1) / 2 * 2 + (size_t)2 * W * nother);
 }
 
 template <class T, int CL>
 __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs<T> a) {
   constexpr int W = strip_w<T>(), LD = W + 1;
-  constexpr int kVec = 16 / (int)sizeof(cx<T>);  // elements of a 16-byte store
+  constexpr int kVec = 16 / (int)sizeof(cx<T>);  // columns of a chunk
+  using Sh = StripShared<T, CL>;
+  static_assert(Sh::kCh == 16, "half a warp sends a row");
   using Key = KeyOf<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int q = (int)cl_rank(), R = a.rows_per_cta, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarp = blockDim.x >> 5;
-  const int w = a.w, k0 = a.k0, r0 = k0 + q * R;
-  const int Rq = max(0, min(a.n, r0 + R) - r0);
+  const int w = a.w, k0 = a.k0;
+  // this CTA's rows k0 + q, k0 + q + CL, ...: dealt out one by one, so that the
+  // pivot rows (the first ones) and their columns are spread over the cluster
+  const int Rq = max(0, (a.n - k0 - q + CL - 1) / CL);
+  auto row = [&](int i) { return k0 + q + CL * i; };
   const int nother = a.blk1 - a.blk0 - w, nleft = k0 - a.blk0;
-  cx<T>* S = reinterpret_cast<cx<T>*>(smem_raw);              // (R, LD): the strip's rows
-  cx<T>* crow = S + ((size_t)R * LD + 1) / 2 * 2;              // (2, CL, W) candidate rows
-  cx<T>* mv = crow + 2 * CL * W;                               // (<= 2 W, nother) moved rows
-  __shared__ StripCand<T> cand[2][CL];
+  Sh& sh = *reinterpret_cast<Sh*>(smem_raw);
+  cx<T>* S = reinterpret_cast<cx<T>*>(smem_raw + sizeof(Sh));  // (R, LD): the strip's rows
+  cx<T>* mv = S + ((size_t)R * LD + 1) / 2 * 2;                // (<= 2 W, nother) moved rows
   __shared__ Key wkey[2][kStripThreads / 32];
   __shared__ unsigned wpos[2][kStripThreads / 32];
   __shared__ int fpos[kStripThreads];
   __shared__ int mlist[2 * W];
   __shared__ int nmoved, fail_s;
-  __shared__ __align__(8) uint64_t colbar[2];
   volatile int* fail = &fail_s;
   if (tid == 0) {
-    bar_init(&colbar[0], 1);
-    bar_init(&colbar[1], 1);
+    bar_init(&sh.colbar[0], 1);
+    bar_init(&sh.colbar[1], 1);
     nmoved = 0;
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  grid_wait();  // what the previous kernel on the stream wrote
   for (int e0 = tid; e0 < Rq * W; e0 += 8 * blockDim.x) {  // eight loads in flight per thread
     cx<T> v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int e = e0 + i * blockDim.x, r = e / W, c = e % W;
-      v[i] = r < Rq && c < w ? a.A[(int64_t)(r0 + r) * a.lda + k0 + c] : cx<T>();
+      v[i] = r < Rq && c < w ? a.A[(int64_t)row(r) * a.lda + k0 + c] : cx<T>();
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -193,12 +305,19 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
       if (r < Rq) S[r * LD + c] = v[i];
     }
   }
+  // the peers a lane sends to: its half-warp's chunks go to CTAs (lane / 16),
+  // that + 2, ...; the candidates to CTA lane
+  uint32_t peer[CL / 2];
+#pragma unroll
+  for (int i = 0; i < CL / 2; ++i) peer[i] = cl_map(&sh, (lane >> 4) + 2 * i);
+  const uint32_t cpeer = cl_map(&sh, lane < CL ? lane : 0), self = (uint32_t)__cvta_generic_to_shared(&sh);
+  auto off = [&](const void* p) { return (uint32_t)__cvta_generic_to_shared(p) - self; };
   __syncthreads();
-  cx<T> x[W];  // x[i]: column jb + i of this thread's row
+  StripRow<T> x;
   if (tid < Rq)
 #pragma unroll
-    for (int c = 0; c < W; ++c) x[c] = S[tid * LD + c];
-  unsigned pos = (unsigned)(r0 + tid);
+    for (int c = 0; c < W; ++c) x.set(c, S[tid * LD + c]);
+  unsigned pos = (unsigned)row(tid);
   bool live = tid < Rq;  // not yet a pivot row
   cl_sync();             // every CTA runs, with its barriers set up, before the first push
 #pragma unroll 1
@@ -208,67 +327,61 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
       const int j = jb + jj;
       if (j >= w) break;
       const int row_j = k0 + j, par = j & 1;
+      if (tid == 0)
+        bar_expect(&sh.colbar[par], CL * (uint32_t)(sizeof(StripCand<T>) + 16 * (Sh::kCh - j / kVec)));
       // this CTA's candidate: over the warp, then over the warps
-      Key key = live ? val_key(cabs1(x[jj])) : Key(0);
+      Key key = live ? val_key(cabs1(x.get(jj))) : Key(0);
       unsigned p = key ? pos : ~0u;
       key = warp_best(key, p);
       if (lane == 0) {
         wkey[par][warp] = key;
         wpos[par][warp] = p;
       }
-      if (tid == 0)
-        bar_expect(&colbar[par],
-                   CL * (uint32_t)(sizeof(StripCand<T>) + (W - j / kVec * kVec) * sizeof(cx<T>)));
       __syncthreads();
       key = lane < nwarp ? wkey[par][lane] : Key(0);
       p = key ? wpos[par][lane] : ~0u;
       key = warp_best(key, p);
-      // its owner puts the row's remaining columns into shared memory, and the
-      // owner's warp sends them with the candidate to all CTAs
+      // its owner stages the row's remaining columns, and the owner's warp
+      // sends them with the candidate to all CTAs
       const bool own = live && key != 0 && pos == p;
       const unsigned ob = __ballot_sync(~0u, own);
       if (key ? ob != 0 : warp == 0) {
-        const int ro = key ? (warp * 32 + __ffs(ob) - 1) : 0;
         if (own)
 #pragma unroll
-          for (int i = 0; i < W; ++i)
-            if (i >= jj && jb + i < W) S[ro * LD + jb + i] = x[i];
+          for (int k = 0; k < Sh::kCh; ++k)
+            if (k >= jj / kVec && jb / kVec + k < Sh::kCh) sh.stage[jb / kVec + k] = x.chunk(k);
+        // the reciprocal pivot, both parts in one division: the even lanes the real, the odd ones the imaginary part
+        const int lo = key ? __ffs(ob) - 1 : 0;
+        const cx<T> xj = x.get(jj);
+        const cx<T> pv(__shfl_sync(~0u, xj.re, lo), __shfl_sync(~0u, xj.im, lo));
         __syncwarp();
-        constexpr int kCh = W / kVec;
-        for (int e = lane; e < CL * kCh; e += 32) {
-          const int dst = e / kCh, c = (e % kCh) * kVec;
-          if (c + kVec > j) {
-            union {
-              uint4 v;
-              cx<T> z[kVec];
-            } u = {make_uint4(0, 0, 0, 0)};
+        const int c = lane & 15;
+        if (c >= j / kVec) {
+          const uint4 v = sh.stage[c];
+          const uint32_t oc = off(&sh.crow[par][q][c]), ob2 = off(&sh.colbar[par]);
 #pragma unroll
-            for (int i = 0; i < kVec; ++i) u.z[i] = S[ro * LD + c + i];
-            cl_put(cl_map(&crow[(par * CL + q) * W + c], dst), u.v, cl_map(&colbar[par], dst));
-          }
+          for (int i = 0; i < CL / 2; ++i) cl_put(peer[i] + oc, v, peer[i] + ob2);
         }
-        const cx<T> pv = S[ro * LD + j];
         const T m2 = pv.re * pv.re + pv.im * pv.im;
+        const T half = ((lane & 1) ? -pv.im : pv.re) / m2;
         union {
           uint4 v[sizeof(StripCand<T>) / 16];
           StripCand<T> c;
         } u;
         u.c.key = key;
         u.c.pos = (int)p;
-        // both parts of the reciprocal in one division: the even lanes the real, the odd ones the imaginary part
-        const T half = ((lane & 1) ? -pv.im : pv.re) / m2;
         u.c.rre = __shfl_sync(~0u, half, 0);
         u.c.rim = __shfl_sync(~0u, half, 1);
         if (lane < CL) {
-          const uint32_t b = cl_map(&colbar[par], lane), d = cl_map(&cand[par][q], lane);
+          const uint32_t b = cpeer + off(&sh.colbar[par]), d = cpeer + off(&sh.cand[par][q]);
 #pragma unroll
           for (int i = 0; i < (int)sizeof(StripCand<T>) / 16; ++i) cl_put(d + 16 * i, u.v[i], b);
         }
       }
-      bar_wait(&colbar[par], (j >> 1) & 1, fail);
+      bar_wait(&sh.colbar[par], (j >> 1) & 1, fail);
       // the pivot among the CTAs' candidates (each warp for itself)
-      key = lane < CL ? cand[par][lane < CL ? lane : 0].key : Key(0);
-      p = key ? (unsigned)cand[par][lane < CL ? lane : 0].pos : ~0u;
+      key = lane < CL ? sh.cand[par][lane < CL ? lane : 0].key : Key(0);
+      p = key ? (unsigned)sh.cand[par][lane < CL ? lane : 0].pos : ~0u;
       const unsigned mine = p;
       key = warp_best(key, p);
       if (key <= 1) {  // zero (or not a number) column: no interchange, no scaling
@@ -280,10 +393,10 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
           if (pos == (unsigned)row_j) {
 #pragma unroll
             for (int i = 0; i < W; ++i)
-              if (i >= jj && jb + i < W) S[tid * LD + jb + i] = x[i];
+              if (i >= jj && jb + i < W) S[tid * LD + jb + i] = x.get(i);
             live = false;
           } else {
-            S[tid * LD + j] = x[jj];
+            S[tid * LD + j] = x.get(jj);
           }
         }
         continue;
@@ -296,60 +409,63 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
           live = false;
         } else {
           if (pos == (unsigned)row_j) pos = p;
-          const cx<T> rp(cand[par][src].rre, cand[par][src].rim);
-          const cx<T> l = x[jj] * rp;
+          const cx<T> rp(sh.cand[par][src].rre, sh.cand[par][src].rim);
+          const cx<T> l = x.get(jj) * rp;
           S[tid * LD + j] = l;
-          const cx<T>* u = crow + (par * CL + src) * W + jb;
-#pragma unroll
-          for (int i = jj + 1; i < kGrp; ++i) x[i] = fnma(x[i], l, u[i]);
-#pragma unroll
-          for (int g = 1; g < W / kGrp; ++g)
-            if (jb + g * kGrp < W)
-#pragma unroll
-              for (int i = 0; i < kGrp; ++i) x[g * kGrp + i] = fnma(x[g * kGrp + i], l, u[g * kGrp + i]);
+          x.update(jj + 1, jb, l, &sh.crow[par][src][jb / kVec]);
         }
       }
+      // the pivot row's columns from j on, final now, from the exchange to its place (its owner's warp)
+      if (src == q && ob != 0 && lane >= j && lane < W)
+        S[(warp * 32 + __ffs(ob) - 1) * LD + lane] = StripRow<T>::sent(sh.crow[par][src], lane);
     }
-#pragma unroll
-    for (int i = 0; i + kGrp < W; ++i) x[i] = x[i + kGrp];
+    x.shift();
   }
+  grid_trigger();
   // rows to their positions; rows that moved or became pivot rows take the
   // block's other columns along
   if (tid < Rq) {
     fpos[tid] = (int)pos;
-    if (nother > 0 && (pos != (unsigned)(r0 + tid) || pos < (unsigned)(k0 + w))) {
+    if (nother > 0 && (pos != (unsigned)row(tid) || pos < (unsigned)(k0 + w))) {
       const int i = atomicAdd(&nmoved, 1);
       if (i < 2 * W) mlist[i] = tid;
     }
   }
   __syncthreads();
-  const int nm = min(nmoved, 2 * W);
+  const int nm = min(nmoved, 2 * W), ne = nm * nother;
   auto other = [&](int c) { return c < nleft ? a.blk0 + c : a.blk0 + w + c; };
-  if (nother > 0)
-    for (int i = warp; i < nm; i += nwarp) {
-      const cx<T>* row = a.A + (int64_t)(r0 + mlist[i]) * a.lda;
-#pragma unroll 4
-      for (int c = lane; c < nother; c += 32) mv[i * nother + c] = row[other(c)];
+  const bool dead = *fail != 0;
+  // all threads on all moved rows, eight loads in flight each
+  for (int e0 = tid; e0 < ne; e0 += 8 * blockDim.x) {
+    cx<T> v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int e = min(e0 + i * (int)blockDim.x, ne - 1), m = e / nother;
+      v[i] = a.A[(int64_t)row(mlist[m]) * a.lda + other(e - m * nother)];
     }
-  if (!*fail)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (e0 + i * (int)blockDim.x < ne) mv[e0 + i * blockDim.x] = v[i];
+  }
+  if (!dead)
+#pragma unroll 4
     for (int e = tid; e < Rq * W; e += blockDim.x) {
       const int r = e / W, c = e % W, fp = fpos[r];
       if (c < w && fp >= k0 && fp < a.n) a.A[(int64_t)fp * a.lda + k0 + c] = S[r * LD + c];
     }
   // every moved row has been read, and no CTA leaves while a peer may still store into its shared memory
   cl_sync();
-  if (*fail) {
+  if (dead) {
     if (tid == 0) atomicExch(a.err, 1);
     return;
   }
-  for (int i = warp; i < nm; i += nwarp) {
-    const int fp = fpos[mlist[i]];
+#pragma unroll 4
+  for (int e = tid; e < ne; e += blockDim.x) {
+    const int m = e / nother, c = e - m * nother, fp = fpos[mlist[m]];
     if (fp < k0 || fp >= a.n) continue;
-    for (int c = lane; c < nother; c += 32) {
-      const cx<T> v = mv[i * nother + c];
-      a.A[(int64_t)fp * a.lda + other(c)] = v;
-      if (fp < k0 + w && c >= nleft) a.Ub[(int64_t)(fp - k0) * (nother - nleft) + c - nleft] = v;
-    }
+    const cx<T> v = mv[e];
+    a.A[(int64_t)fp * a.lda + other(c)] = v;
+    if (fp < k0 + w && c >= nleft) a.Ub[(int64_t)(fp - k0) * (nother - nleft) + c - nleft] = v;
   }
 }
 
@@ -372,6 +488,8 @@ __global__ void __launch_bounds__(256) strip_update_kernel(cx<T>* __restrict__ A
   __shared__ cx<T> L[TR][W + 1];
   const int tid = threadIdx.x, c0 = k0 + W;
   const int cb = blockIdx.x * CG, rb = c0 + blockIdx.y * TR;
+  grid_wait();
+  grid_trigger();
   // outputs of this thread: column tc, rows tr + i * kRs
   constexpr int kRs = 256 / CG, kOut = TR / kRs;
   const int tc = tid % CG, tr = tid / CG;
@@ -476,17 +594,19 @@ bool strip_available(int device) {
 template <class T, int CL>
 cudaError_t launch_strip(const StripArgs<T>& a, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = CL;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(CL);
   cfg.blockDim = dim3(std::max(64, (a.rows_per_cta + 31) / 32 * 32));
   cfg.dynamicSmemBytes = strip_smem<T, CL>(a.rows_per_cta, a.blk1 - a.blk0 - a.w);
   cfg.stream = st;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, strip_panel_kernel<T, CL>, a);
 }
 
@@ -524,8 +644,7 @@ int lu_strip_block(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int b0, int bw, i
     const int nc = b0 + bw - k0 - w;
     if (nc > 0) {
       const dim3 grid((nc + StripUpd<T>::CG - 1) / StripUpd<T>::CG, (n - k0 - w + StripUpd<T>::TR - 1) / StripUpd<T>::TR);
-      strip_update_kernel<T><<<grid, 256, 0, ctx->stream>>>(A, lda, n, k0, nc, Ub);
-      M25_CHECK_LAUNCH();
+      M25_CUDA(launch_chained(strip_update_kernel<T>, grid, 256, 0, ctx->stream, A, lda, n, k0, nc, Ub));
     }
   }
   return M25_OK;

@@ -42,6 +42,7 @@
 #include <string>
 
 #include "m25_internal.h"
+#include "m25_lu.h"
 
 namespace m25 {
 
@@ -182,10 +183,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nk = a.P / kBK;  // k-blocks of one plane
   const int nch = (nk + a.chunk - 1) / a.chunk;
-  // an earlier CTA gave up: leave before taking TMEM
-  if (threadIdx.x == 0) skip = *(volatile int*)a.err;
-  __syncthreads();
-  if (skip) return;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
@@ -208,6 +205,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(&tmB) : "memory");
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(&tmC) : "memory");
   }
+  grid_wait();
+  // an earlier CTA gave up: leave before taking TMEM
+  if (threadIdx.x == 0) skip = *(volatile int*)a.err;
+  __syncthreads();
+  if (skip) return;
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base)),
                  "r"(kTmemCols));
@@ -392,6 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncwarp();
     if (!ok) *abort_v = 1;
   }
+  grid_trigger();  // not before: CTAs of the next kernel would wait on SMs that other streams can use
   __syncthreads();
   if (threadIdx.x == 0) {
     if (abort_flag) {
@@ -422,6 +425,8 @@ __device__ __forceinline__ float tf32_round(float x) {
 // real part, 1 minus imaginary part), zero for t >= w
 __global__ void pack_a_kernel(const zf* __restrict__ LU, int64_t lda, int k0, int w, int row0, int m, int P, int pw,
                               int koff, float* __restrict__ A3) {
+  grid_wait();
+  grid_trigger();
   const int K2p = 2 * P;
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (int64_t)m * K2p) return;
@@ -567,8 +572,8 @@ int lu_tc_pack_a(m25_ctx* ctx, const zf* A, int64_t lda, int k0, int w, int row0
   if (m <= 0) return M25_OK;
   StageTimer tm(ctx, ST_PACK);
   const int64_t ta = (int64_t)m * 2 * P;
-  pack_a_kernel<<<(unsigned)((ta + 255) / 256), 256, 0, ctx->stream>>>(A, lda, k0, w, row0, m, P, pw, koff, A3);
-  M25_CHECK_LAUNCH();
+  M25_CUDA(launch_chained(pack_a_kernel, dim3((unsigned)((ta + 255) / 256)), 256, 0, ctx->stream, A, lda, k0, w, row0, m,
+                          P, pw, koff, A3));
   return M25_OK;
 }
 
@@ -627,11 +632,10 @@ int lu_tc_update(m25_ctx* ctx, zf* A, int64_t lda, int r0, int c0, int m, int nc
     return M25_ERR_CUDA;
   }
   StageTimer tm(ctx, ST_GEMM);
-  if (bn == 128)
-    tc_gemm_kernel<128><<<std::min(ta.ntiles, n_sm), kThreads, smem_bytes<128>(), st>>>(ma, mb, mc, ta);
-  else
-    tc_gemm_kernel<192><<<std::min(ta.ntiles, n_sm), kThreads, smem_bytes<192>(), st>>>(ma, mb, mc, ta);
-  M25_CHECK_LAUNCH();
+  M25_CUDA(bn == 128 ? launch_chained(tc_gemm_kernel<128>, dim3(std::min(ta.ntiles, n_sm)), kThreads, smem_bytes<128>(),
+                                      st, ma, mb, mc, ta)
+                     : launch_chained(tc_gemm_kernel<192>, dim3(std::min(ta.ntiles, n_sm)), kThreads, smem_bytes<192>(),
+                                      st, ma, mb, mc, ta));
   return M25_OK;
 }
 

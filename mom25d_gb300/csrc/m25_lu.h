@@ -5,6 +5,29 @@
 
 namespace m25 {
 
+// Programmatic dependent launch: a kernel launched by launch_chained starts when
+// every CTA of the one before it on the stream has triggered (or ended), and
+// waits in grid_wait for that one's end; what comes before the wait overlaps it.
+// Every CTA of a chained kernel waits, so that the end of a kernel means the end
+// of all before it.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
+template <class... K, class... A>
+cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
 // lu_panel.cu: a block of at most 128 columns factored by one cluster (up to lu_strip_rows rows)
 template <class T> int lu_strip_rows(m25_ctx* ctx);
 template <class T> size_t lu_strip_scratch();
