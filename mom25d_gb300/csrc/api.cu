@@ -56,6 +56,11 @@ int lu_wave_reset(m25_ctx*);
 // trailing rows in the shared memory of one 16-CTA cluster
 constexpr int kPanelZ64 = 64;
 
+// A caller's complex64 array on the device may lie at any multiple of four
+// bytes; the kernels move complex64 values in one access of eight. One that is
+// not aligned to that goes by way of the workspace.
+static bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
+
 }  // namespace m25
 
 using namespace m25;
@@ -221,8 +226,17 @@ extern "C" int m25_assemble(m25_ctx* ctx, m25_geom* geom, m25_greens* gr, double
   if (precision == M25_FP64 || precision == M25_MIXED)
     return fill_driver<double>(ctx, geom, gr, zd(zs_re, zs_im), zd(zsv_re, zsv_im), Z, ldz, where,
                                precision == M25_MIXED);
-  if (precision == M25_MIXED_FILL32)
-    return fill_driver<float>(ctx, geom, gr, zd(zs_re, zs_im), zd(zsv_re, zsv_im), Z, ldz, where, false);
+  if (precision == M25_MIXED_FILL32) {
+    const zd zs(zs_re, zs_im), zsv(zsv_re, zsv_im);
+    if (where == M25_ON_HOST || aligned8(Z)) return fill_driver<float>(ctx, geom, gr, zs, zsv, Z, ldz, where, false);
+    int rc;
+    if ((rc = ctx->Zw.ensure(sizeof(zf) * (size_t)n * n)) ||
+        (rc = fill_driver<float>(ctx, geom, gr, zs, zsv, ctx->Zw.p, n, M25_ON_DEVICE, false)))
+      return rc;
+    M25_CUDA(cudaMemcpy2DAsync(Z, sizeof(zf) * ldz, ctx->Zw.p, sizeof(zf) * n, sizeof(zf) * n, n,
+                               cudaMemcpyDeviceToDevice, ctx->stream));
+    return M25_OK;
+  }
   set_error("m25_assemble: unknown precision");
   return M25_ERR_VALUE;
 }
@@ -239,12 +253,18 @@ extern "C" int m25_lu_factor(m25_ctx* ctx, int32_t n, int precision, void* A, in
   void* Ad = A;
   int32_t* pd = ipiv;
   int rc;
-  if (where == M25_ON_HOST) {
+  const bool host = where == M25_ON_HOST, staged = host || !aligned8(A);
+  if (staged) {
     if ((rc = ctx->Zw.ensure(esz * (size_t)n * lda))) return rc;
-    if ((rc = ctx->ipiv.ensure(sizeof(int32_t) * n))) return rc;
     Ad = ctx->Zw.p;
+    if (host)
+      M25_CUDA(cudaMemcpyAsync(Ad, A, esz * (size_t)n * lda, cudaMemcpyHostToDevice, st));
+    else
+      M25_CUDA(cudaMemcpy2DAsync(Ad, esz * lda, A, esz * lda, esz * n, n, cudaMemcpyDeviceToDevice, st));
+  }
+  if (host) {
+    if ((rc = ctx->ipiv.ensure(sizeof(int32_t) * n))) return rc;
     pd = ctx->ipiv.as<int32_t>();
-    M25_CUDA(cudaMemcpyAsync(Ad, A, esz * (size_t)n * lda, cudaMemcpyHostToDevice, st));
   }
   int zinfo = 0;
   if (precision == M25_FP64)
@@ -254,9 +274,11 @@ extern "C" int m25_lu_factor(m25_ctx* ctx, int32_t n, int precision, void* A, in
     rc = lu_factor<float>(ctx, static_cast<zf*>(Ad), lda, n, pd, kPanelZ64,
                           lu_tc_available() && !(flags & M25_LU_NO_TENSOR_CORES), &zinfo);
   if (rc) return rc;
-  if (where == M25_ON_HOST) {
+  if (host) {
     M25_CUDA(cudaMemcpyAsync(A, Ad, esz * (size_t)n * lda, cudaMemcpyDeviceToHost, st));
     M25_CUDA(cudaMemcpyAsync(ipiv, pd, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+  } else if (staged) {
+    M25_CUDA(cudaMemcpy2DAsync(A, esz * lda, Ad, esz * lda, esz * n, n, cudaMemcpyDeviceToDevice, st));
   }
   M25_CUDA(cudaStreamSynchronize(st));
   if (info) *info = zinfo;
@@ -330,10 +352,11 @@ static int dense_solve_impl(m25_ctx* ctx, int32_t n, int32_t nrhs, int precision
     if (!presplit && (rc = ctx->Zlu.ensure(sizeof(zf) * (size_t)n * ldl))) return rc;
     zf* LU = presplit ? presplit->LU : ctx->Zlu.as<zf>();
     const void* Zres = Z;
-    if (where == M25_ON_HOST && !presplit) {
+    if (!presplit && (where == M25_ON_HOST || !aligned8(Z))) {
       size_t zb = (precision == M25_MIXED_FILL32 ? sizeof(zf) : sizeof(zd)) * nn;
       if ((rc = ctx->Zw.ensure(zb))) return rc;
-      M25_CUDA(cudaMemcpyAsync(ctx->Zw.p, Z, zb, cudaMemcpyHostToDevice, st));
+      M25_CUDA(cudaMemcpyAsync(ctx->Zw.p, Z, zb, where == M25_ON_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
+                               st));
       Zres = ctx->Zw.p;
     }
     // Z for the residuals as complex64 planes Zh + Zl (fp64-level products on

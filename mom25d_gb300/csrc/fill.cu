@@ -1235,8 +1235,6 @@ int fill_driver(m25_ctx* ctx, m25_geom* geom, m25_greens* gr, zd zs, zd zsv, voi
   }
   M25_CHECK_LAUNCH();
   if (nv) {
-    zd* lead_dev = reinterpret_cast<zd*>(imgv + 9);  // unused slot guard
-    (void)lead_dev;
     // Im gV(rho0) per level pair from the double tables
     std::vector<zd> hv(L * L);
     std::vector<double> hdz(L * L);

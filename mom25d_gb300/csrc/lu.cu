@@ -264,8 +264,8 @@ __device__ __forceinline__ float tf32_rna(float x) {
 // complex64: 32 columns, 8 lanes each. complex128: 8 columns, 16 lanes each, as
 // a warp's fp64 instruction holds its unit for 64 cycles: four times as many
 // CTAs share the columns and a lane has four rows (N = 546 / 1085 / 2434 / 5943,
-// all launches of a factorisation: @SWAP@ ms; 1.07 / 2.15 / 5.1 / 20.5 ms with
-// 32 columns, 8 lanes and six fp64 operations per product).
+// all launches of a factorisation: 0.27 / 0.55 / 1.66 / 8.34 ms; 1.07 / 2.15 /
+// 5.1 / 20.5 ms with 32 columns, 8 lanes and six fp64 operations per product).
 // The interchanges are composed, not replayed: the rows touched are the w
 // panel rows and the pivot rows below the panel, and the original row that
 // ends in position x is found by applying the swaps to x in reverse order.
@@ -439,9 +439,9 @@ __global__ void __launch_bounds__(SwapShape<T>::kThreads)
         // L11 rows >= w and on / above the diagonal are zero in Ls
 #pragma unroll
         for (int k = kb; k < RB; ++k)
-          if (k > kb || l > j) x[k] = fnma(x[k], Ls[t * kLsLd + l + LPC * k], xt);
+          if (k > kb || l > j) x[k] = fnma(x[k], ldc(Ls + t * kLsLd + l + LPC * k), xt);
 #pragma unroll
-        for (int k = RB; k < R; ++k) x[k] = fnma(x[k], Ls1[t * kLsLd + l + LPC * (k - RB)], xt);
+        for (int k = RB; k < R; ++k) x[k] = fnma(x[k], ldc(Ls1 + t * kLsLd + l + LPC * (k - RB)), xt);
       }
     if (W == 128) {
       // rows 64..127 with their own diagonal block, loaded over the first one
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(SwapShape<T>::kThreads)
           xt.im = __shfl_sync(~0u, x[kb].im, (lane & ~(LPC - 1)) | j);
 #pragma unroll
           for (int k = kb; k < R; ++k)
-            if (k > kb || l > j) x[k] = fnma(x[k], Ls[t * kLsLd + l + LPC * (k - RB)], xt);
+            if (k > kb || l > j) x[k] = fnma(x[k], ldc(Ls + t * kLsLd + l + LPC * (k - RB)), xt);
         }
     }
 #pragma unroll
@@ -904,58 +904,68 @@ __device__ __forceinline__ void fetch_diag_t(cx<TF>* DgT, const cx<TF>* A, int64
 // the block), dinv the reciprocal diagonal (zero outside the block), so the
 // rounds load factors without any test. Lower: unit diagonal, forward; upper:
 // backward. acc (rows x P) in and out, column c.
+// The rounds have no test for the owner: its own factors are zero on and
+// beyond the diagonal, so that its rows take the right subtractions too (and
+// are scaled by the reciprocal diagonal at the end); a select per round made it
+// divergent, 180 cycles a round against 83. Rounds beyond the block's rows
+// change nothing.
 template <class TF, class TV>
 __device__ __forceinline__ void diag_solve1(int lane, int w, int P, int c, int upper, const cx<TF>* DgT,
                                             const cx<TV>* dinv, cx<TV>* acc) {
   const int ra = 2 * lane, rb = ra + 1;
   cx<TV> va = ra < w ? acc[ra * P + c] : cx<TV>();
   cx<TV> vb = rb < w ? acc[rb * P + c] : cx<TV>();
-  const int npair = (w + 1) >> 1;
-  struct Fac {
-    cx<TV> aA, aB, bA, bB, da, db;  // row ra / rb at column 2k / 2k + 1; reciprocal diagonals of the pair
-  };
-  auto load = [&](int k) {
-    Fac f;
-    const cx<TF>* ca = DgT + (2 * k) * kTileLd;
-    const cx<TF>* cb = ca + kTileLd;
-    f.aA = cx<TV>(ca[ra]);
-    f.bA = cx<TV>(ca[rb]);
-    f.aB = cx<TV>(cb[ra]);
-    f.bB = cx<TV>(cb[rb]);
-    if (upper) {
-      f.da = dinv[2 * k];
-      f.db = dinv[2 * k + 1];
+  auto bcast = [](cx<TV> v, int k) { return cx<TV>(__shfl_sync(0xffffffffu, v.re, k), __shfl_sync(0xffffffffu, v.im, k)); };
+  const cx<TV> da = upper ? ldc(dinv + ra) : cx<TV>(), db = upper ? ldc(dinv + rb) : cx<TV>();
+  if constexpr (sizeof(TV) == 8) {
+    // a column per round: the fp64 operations bound it, not the shuffles (the
+    // pair's second value formed in every lane costs four of twenty)
+    if (!upper) {
+#pragma unroll 2
+      for (int k = 0; k < 32; ++k)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const cx<TF>* cc = DgT + (2 * k + h) * kTileLd;
+          const cx<TV> x = bcast(h ? vb : va, k);
+          va = fnma(va, cx<TV>(ldc(cc + ra)), x);
+          vb = fnma(vb, cx<TV>(ldc(cc + rb)), x);
+        }
+    } else {
+#pragma unroll 2
+      for (int k = 31; k >= 0; --k)
+#pragma unroll
+        for (int h = 1; h >= 0; --h) {
+          const cx<TF>* cc = DgT + (2 * k + h) * kTileLd;
+          const cx<TV> x = bcast(h ? vb * db : va * da, k);
+          va = fnma(va, cx<TV>(ldc(cc + ra)), x);
+          vb = fnma(vb, cx<TV>(ldc(cc + rb)), x);
+        }
     }
-    return f;
-  };
-  if (!upper) {
-    Fac nx = load(0);
-    for (int k = 0; k < npair; ++k) {
-      const Fac f = nx;
-      nx = load(min(k + 1, npair - 1));
-      const bool mine = lane == k;
+  } else if (!upper) {
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+      const cx<TF>*ca = DgT + (2 * k) * kTileLd, *cb = ca + kTileLd;  // columns 2 k, 2 k + 1
+      const cx<TV> aA(ca[ra]), bA(ca[rb]), aB(cb[ra]), bB(cb[rb]);
       // owner (lane k): x_2k is final, x_2k+1 = v_2k+1 - L[2k+1][2k] x_2k
-      const cx<TV> xb_own = vb - f.bA * va;
-      const cx<TV> xa(__shfl_sync(0xffffffffu, va.re, k), __shfl_sync(0xffffffffu, va.im, k));
-      const cx<TV> xb(__shfl_sync(0xffffffffu, xb_own.re, k), __shfl_sync(0xffffffffu, xb_own.im, k));
-      // rows below the pair; the owner keeps the two values it broadcast
-      va = mine ? xa : va - (f.aA * xa + f.aB * xb);
-      vb = mine ? xb : vb - (f.bA * xa + f.bB * xb);
+      const cx<TV> xa = bcast(va, k), xb = bcast(fnma(vb, bA, va), k);
+      va = fnma(fnma(va, aA, xa), aB, xb);
+      vb = fnma(fnma(vb, bA, xa), bB, xb);
     }
   } else {
-    Fac nx = load(npair - 1);
-    for (int k = npair - 1; k >= 0; --k) {
-      const Fac f = nx;
-      nx = load(max(k - 1, 0));
-      const bool mine = lane == k;
+#pragma unroll 4
+    for (int k = 31; k >= 0; --k) {
+      const cx<TF>*ca = DgT + (2 * k) * kTileLd, *cb = ca + kTileLd;
+      const cx<TV> aA(ca[ra]), bA(ca[rb]), aB(cb[ra]), bB(cb[rb]);
       // owner: x_2k+1 = v_2k+1 / d, then x_2k = (v_2k - U[2k][2k+1] x_2k+1) / d
-      const cx<TV> xb_own = vb * f.db;
-      const cx<TV> xa_own = (va - f.aB * xb_own) * f.da;
-      const cx<TV> xa(__shfl_sync(0xffffffffu, xa_own.re, k), __shfl_sync(0xffffffffu, xa_own.im, k));
-      const cx<TV> xb(__shfl_sync(0xffffffffu, xb_own.re, k), __shfl_sync(0xffffffffu, xb_own.im, k));
-      va = mine ? xa : va - (f.aA * xa + f.aB * xb);
-      vb = mine ? xb : vb - (f.bA * xa + f.bB * xb);
+      const cx<TV> ob = vb * db, oa = fnma(va, aB, ob) * da;
+      const cx<TV> xa = bcast(oa, k), xb = bcast(ob, k);
+      va = fnma(fnma(va, aB, xb), aA, xa);
+      vb = fnma(fnma(vb, bB, xb), bA, xa);
     }
+  }
+  if (upper) {
+    va = va * da;
+    vb = vb * db;
   }
   if (ra < w) acc[ra * P + c] = va;
   if (rb < w) acc[rb * P + c] = vb;
@@ -982,8 +992,13 @@ constexpr size_t wave_smem() {
 // stream through a ring of cp.async stages so that a CTA's backlog of tiles
 // never holds up the chain; the chain step itself is the flag round trip,
 // one 64 x 64 tile product and the substitution, which one warp runs in
-// registers (lane l owns rows l and l + 32; each solved row is broadcast with
-// shuffles; the upper sweep multiplies by the reciprocal diagonal). Every
+// registers (lane l owns rows 2l and 2l + 1; each solved pair is broadcast with
+// shuffles; the upper sweep multiplies by the reciprocal diagonal). It is
+// bound by that chain, not by the factors' bytes: all sweeps of a solve, two
+// right-hand sides, N = 1085 / 3789 / 5943 in complex64 0.35 / 1.85 / 1.69 ms
+// (0.46 / 2.51 / 2.33 ms with a select per round and one lane per row of the
+// tile product), N = 546 / 2434 / 5943 in complex128 0.65 / 2.80 / 6.65 ms (0.90 /
+// 3.96 / 9.6 ms). Every
 // wait is bounded; blocks only wait on blocks solved earlier, and the
 // cooperative launch keeps all CTAs resident, so the order cannot deadlock.
 template <class TF, class TV>
@@ -1114,18 +1129,35 @@ __global__ void __launch_bounds__(256, 1) trsv_wave_kernel(WaveArgs<TF, TV> a) {
         }
         __syncthreads();
       }
-      for (int e = tid; e < w * P; e += blockDim.x) {
-        const int r = e / P, c = e % P;
-        const cx<TF>* Tr = T + r * kTileLd;
-        cx<TV> s0, s1, s2, s3;
-#pragma unroll 4
-        for (int t = 0; t < 64; t += 4) {
-          s0 += cx<TV>(Tr[t]) * y[t * P + c];
-          s1 += cx<TV>(Tr[t + 1]) * y[(t + 1) * P + c];
-          s2 += cx<TV>(Tr[t + 2]) * y[(t + 2) * P + c];
-          s3 += cx<TV>(Tr[t + 3]) * y[(t + 3) * P + c];
+      // the tile's product: four lanes per row, 16 columns each, two right-hand
+      // sides at a time. The lanes start at different columns so that a half
+      // warp's loads (4 rows x 4 lanes) fall into different banks
+      {
+        const int part = tid & 3, r = tid >> 2;
+        const cx<TF>* Tr = T + r * kTileLd + 16 * part;
+        for (int c = 0; c < P; c += 2) {
+          const bool two = c + 1 < P;
+          const cx<TV>* yc = y + 16 * part * P + c;
+          cx<TV> s[2][2];  // minus the product, in two sums per right-hand side
+#pragma unroll 8
+          for (int i = 0; i < 16; ++i) {
+            const int t = (i + 4 * part) & 15;
+            const cx<TV> tv(ldc(Tr + t));
+            s[0][i & 1] = fnma(s[0][i & 1], tv, ldc(yc + t * P));
+            if (two) s[1][i & 1] = fnma(s[1][i & 1], tv, ldc(yc + t * P + 1));
+          }
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            if (q && !two) break;
+            cx<TV> v = s[q][0] + s[q][1];
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+              v.re += __shfl_xor_sync(0xffffffffu, v.re, o);
+              v.im += __shfl_xor_sync(0xffffffffu, v.im, o);
+            }
+            if (part == 0 && r < w) acc[r * P + c + q] += v;
+          }
         }
-        acc[e] -= (s0 + s1) + (s2 + s3);
       }
       __syncthreads();  // the stage of tile d is free again
       if (d + S < ndep) fetch_dep(d + S);

@@ -483,9 +483,9 @@ template <class T>
 __global__ void __launch_bounds__(256) strip_update_kernel(cx<T>* __restrict__ A, int64_t lda, int n, int k0, int nc,
                                                            const cx<T>* __restrict__ Ub) {
   constexpr int W = StripUpd<T>::W, CG = StripUpd<T>::CG, TR = StripUpd<T>::TR;
-  __shared__ cx<T> Lt[W][W + 1];   // Lt[t][r] = L11[r][t] below the diagonal
-  __shared__ cx<T> V[W][CG + 1];
-  __shared__ cx<T> L[TR][W + 1];
+  __shared__ __align__(16) cx<T> Lt[W][W + 1];   // Lt[t][r] = L11[r][t] below the diagonal
+  __shared__ __align__(16) cx<T> V[W][CG + 1];
+  __shared__ __align__(16) cx<T> L[TR][W + 1];
   const int tid = threadIdx.x, c0 = k0 + W;
   const int cb = blockIdx.x * CG, rb = c0 + blockIdx.y * TR;
   grid_wait();
@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(256) strip_update_kernel(cx<T>* __restrict__ A
         xt.im = __shfl_sync(~0u, x[kb].im, (lane & ~7) | j);
 #pragma unroll
         for (int k = kb; k < kR; ++k)
-          if (k > kb || l8 > j) x[k] = fnma(x[k], Lt[t][l8 + 8 * k], xt);
+          if (k > kb || l8 > j) x[k] = fnma(x[k], ldc(&Lt[t][l8 + 8 * k]), xt);
       }
     __syncwarp();
 #pragma unroll
@@ -542,9 +542,9 @@ __global__ void __launch_bounds__(256) strip_update_kernel(cx<T>* __restrict__ A
     }
 #pragma unroll 8
   for (int t = 0; t < W; ++t) {
-    const cx<T> u = V[t][tc];
+    const cx<T> u = ldc(&V[t][tc]);
 #pragma unroll
-    for (int i = 0; i < kOut; ++i) c[i] = fnma(c[i], L[tr + i * kRs][t], u);
+    for (int i = 0; i < kOut; ++i) c[i] = fnma(c[i], ldc(&L[tr + i * kRs][t]), u);
   }
 #pragma unroll
   for (int i = 0; i < kOut; ++i) {

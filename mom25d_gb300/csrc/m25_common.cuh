@@ -20,8 +20,10 @@ constexpr double kMu0 = 4e-7 * kPi;
 __host__ __device__ inline double eps0() { return 1.0 / (kMu0 * kC0 * kC0); }
 
 // ------------------------------------------------------------------ complex
+// Aligned to 8 bytes, so that a complex64 value moves in one access; complex128
+// values stay at the alignment of their parts (callers' arrays may have no more).
 template <class T>
-struct cx {
+struct alignas(8) cx {
   T re, im;
   __host__ __device__ cx() : re(0), im(0) {}
   __host__ __device__ cx(T r, T i = 0) : re(r), im(i) {}
@@ -41,6 +43,13 @@ template <class T> __host__ __device__ inline cx<T> operator*(cx<T> a, T s) { re
 template <class T> __host__ __device__ inline cx<T> operator*(T s, cx<T> a) { return {a.re * s, a.im * s}; }
 template <class T> __host__ __device__ inline cx<T>& operator+=(cx<T>& a, cx<T> b) { a.re += b.re; a.im += b.im; return a; }
 template <class T> __host__ __device__ inline cx<T>& operator-=(cx<T>& a, cx<T> b) { a.re -= b.re; a.im -= b.im; return a; }
+// a complex128 value at a 16-byte boundary in one access
+__device__ __forceinline__ cx<double> ldc(const cx<double>* p) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  return {v.x, v.y};
+}
+__device__ __forceinline__ cx<float> ldc(const cx<float>* p) { return *p; }
+
 // a - b c as four fused multiply-adds (a -= b * c takes two multiplications, two fused ones and two
 // additions: the product is rounded on its own, and complex128 pays for each on GB300's slow fp64 pipe)
 __device__ __forceinline__ cx<double> fnma(cx<double> a, cx<double> b, cx<double> c) {

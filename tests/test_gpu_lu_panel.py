@@ -160,3 +160,59 @@ def test_update_slices_with_vias(gpu, nvia, freq):
         ref = ref + d[:, None] * sl.lu_solve(lu, d[:, None] * r.astype(complex))
     err = [float(np.linalg.norm(v - ref) / np.linalg.norm(ref)) for v in (x, np.linalg.solve(Z, B))]
     assert err[0] <= 10 * err[1] + 1e-15
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+def test_complex64_device_alignment(gpu, offset):
+    """Device complex64 arrays at an odd multiple of four bytes give the same
+    bits as aligned ones: the LU (rows with a gap), the fill, the solve."""
+    import torch
+
+    import mom25d_gb300 as G
+    from mom25d_gb300 import engine as E
+    from mom25d_gb300 import workloads
+    from mom25d_gb300.solver import Solver
+
+    rng = np.random.default_rng(5)
+
+    def dev(n, ld, off):
+        buf = torch.zeros(2 * n * ld + 1, dtype=torch.float32, device="cuda")
+        return buf, buf[off:off + 2 * n * ld].view(n, ld, 2), C.c_void_p(buf.data_ptr() + 4 * off)
+
+    n, ld = 97, 101
+    A = torch.from_numpy(rng.standard_normal((n, ld, 2)).astype(np.float32)).cuda()
+    B = torch.from_numpy(rng.standard_normal((n, 2, 2))).cuda()
+    _, _, mesh, freqs = workloads.build(G, "tee")
+    sol = Solver(mesh, workloads.build(G, "tee")[1], verbose=False, precision="mixed_fill32")
+    g, m = sol.greens(float(freqs[0])), mesh.n_unknowns
+    out = []
+    for off in (0, offset):
+        ctx = sol.ctx
+        buf, v, p = dev(n, ld, off)
+        v.copy_(A)
+        ipiv, info = torch.zeros(n, dtype=torch.int32, device="cuda"), np.zeros(3, np.int32)
+        torch.cuda.synchronize()
+        E.check(ctx.lib.m25_lu_factor(ctx.h, n, E.M25_MIXED, p, ld, C.cast(C.c_void_p(ipiv.data_ptr()),
+                                      C.POINTER(C.c_int32)), E.M25_ON_DEVICE, 0, E.ptr(info, C.c_int32)))
+        lu = v.cpu().numpy()
+        assert np.array_equal(lu[:, n:], A.cpu().numpy()[:, n:])  # the gap keeps its values
+        bufz, vz, pz = dev(m, m, off)
+        E.check(ctx.lib.m25_assemble(ctx.h, sol.geometry().h, g.h, 0.01, 0.01, 0.01, 0.01, E.M25_MIXED_FILL32, pz, m,
+                                     E.M25_ON_DEVICE))
+        ctx.synchronize()
+        bufs, vs, ps = dev(n, n, off)
+        vs.copy_(A[:, :n])
+        X = torch.zeros_like(B)
+        torch.cuda.synchronize()
+        E.check(ctx.lib.m25_dense_solve(ctx.h, n, 2, E.M25_MIXED_FILL32, ps, C.c_void_p(B.data_ptr()),
+                                        C.c_void_p(X.data_ptr()), E.M25_ON_DEVICE, 1e-12, 50, E.ptr(info, C.c_int32)))
+        ctx.synchronize()
+        out.append((lu, ipiv.cpu().numpy(), vz.cpu().numpy(), X.cpu().numpy()))
+    sol.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    Z = A.cpu().numpy()[:, :n].astype(float)
+    r = (Z[..., 0] + 1j * Z[..., 1]) @ (out[0][3][..., 0] + 1j * out[0][3][..., 1])
+    b = B.cpu().numpy()
+    # the refinement's own stop: the backward error (1e-12) of one column
+    assert np.linalg.norm(r - (b[..., 0] + 1j * b[..., 1])) <= 1e-11 * np.linalg.norm(Z) * np.linalg.norm(out[0][3])
