@@ -54,24 +54,39 @@ __device__ void slab_spectral(const StackDev& S, zd kr, zd& gA, zd& gV, zd& gW) 
 }
 
 // Multilayer spectral kernels via TE/TM line voltages (layered.py:238-289):
-// g[m][i][j], m = A, V, W; i observer level, j source level.
-__device__ void layered_spectral(const StackDev& S, zd kr, zd g[3][kMaxLev][kMaxLev]) {
+// g[m][i][j], m = A, V, W; i observer level, j source level. Two neighbouring
+// lanes work on one node: the layers' constants shared out between them, lane
+// `mode` the line voltages of its mode (0: h, 1: e), then the levels j in turn.
+// (One thread's chain of ~50 complex divisions, exponentials and roots was the kernel's time.)
+__device__ void layered_spectral(const StackDev& S, zd kr, int mode, zd* __restrict__ out) {
   const int N = S.nlayer, L = S.nlev;
-  zd u[kMaxLayers], T[kMaxLayers], Sh[kMaxLayers];
-  zd kr2 = kr * kr;
-  for (int n = 0; n < N; ++n) {
-    u[n] = csqrt(kr2 - S.kk[n] * S.kk[n]);
-    zd x = u[n] * S.t[n];
-    zd e = cexp(x * -2.0);
-    T[n] = (zd(1.0) - e) / (zd(1.0) + e);
-    Sh[n] = (cexp(-x) * 2.0) / (zd(1.0) + e);
+  const zd one(1.0);
+  auto other = [](zd v) { return zd(__shfl_xor_sync(0xffffffffu, v.re, 1), __shfl_xor_sync(0xffffffffu, v.im, 1)); };
+  zd u[kMaxLayers], T[kMaxLayers], Sh[kMaxLayers], iu[kMaxLayers];
+  const zd kr2 = kr * kr;
+  for (int n0 = 0; n0 < N; n0 += 2) {
+    const int n = min(n0 + mode, N - 1);
+    const zd un = csqrt(kr2 - S.kk[n] * S.kk[n]);
+    const zd x = un * S.t[n], p = cexp(-x), e = cexp(x * -2.0), d = one / (one + e);
+    const zd Tn = (one - e) * d, Sn = (p * 2.0) * d, in = one / un;
+    const zd uo = other(un), To = other(Tn), So = other(Sn), io = other(in);
+    u[n0] = mode ? uo : un;
+    T[n0] = mode ? To : Tn;
+    Sh[n0] = mode ? So : Sn;
+    iu[n0] = mode ? io : in;
+    if (n0 + 1 < N) {
+      u[n0 + 1] = mode ? un : uo;
+      T[n0 + 1] = mode ? Tn : To;
+      Sh[n0 + 1] = mode ? Sn : So;
+      iu[n0 + 1] = mode ? in : io;
+    }
   }
-  zd u0 = csqrt(kr2 - zd(S.k0 * S.k0));
-  zd Vmode[2][kMaxLev][kMaxLayers + 1];
-  for (int mode = 0; mode < 2; ++mode) {
+  const zd u0 = csqrt(kr2 - zd(S.k0 * S.k0));
+  zd Vm[kMaxLev][kMaxLayers + 1];
+  {
     zd y[kMaxLayers];
-    for (int n = 0; n < N; ++n) y[n] = mode == 0 ? u[n] : S.epsc[n] / u[n];
-    zd yair = mode == 0 ? u0 : zd(1.0) / u0;
+    for (int n = 0; n < N; ++n) y[n] = mode == 0 ? u[n] : S.epsc[n] * iu[n];
+    const zd yair = mode == 0 ? u0 : one / u0;
     zd ydn[kMaxLayers + 1], yup[kMaxLayers + 1];
     ydn[1] = y[0] / T[0];
     for (int k = 2; k <= N; ++k) {
@@ -88,40 +103,57 @@ __device__ void layered_spectral(const StackDev& S, zd kr, zd g[3][kMaxLev][kMax
         yup[k] = yk * (yl + yk * tk) / (yk + yl * tk);
       }
     }
+    // V_{k-1} / V_k below a source, V_{k+1} / V_k above it: the same for every source level
+    zd dn[kMaxLayers + 1], up[kMaxLayers + 1];
+    for (int k = 2; k <= N; ++k) dn[k] = Sh[k - 1] * y[k - 1] / (y[k - 1] + ydn[k - 1] * T[k - 1]);
+    for (int k = 1; k < N; ++k) {
+      if (S.top_pec && k + 1 == N) break;  // V_N = 0 on the cover
+      up[k] = Sh[k] * y[k] / (y[k] + yup[k + 1] * T[k]);
+    }
     for (int l = 0; l < L; ++l) {
-      zd* V = Vmode[mode][l];
+      zd* V = Vm[l];
       for (int k = 0; k <= N; ++k) V[k] = zd(0.0);
       int s = S.il[l];
-      V[s] = zd(1.0) / (ydn[s] + yup[s]);
-      for (int k = s; k >= 2; --k) V[k - 1] = V[k] * Sh[k - 1] / (zd(1.0) + ydn[k - 1] / y[k - 1] * T[k - 1]);
+      V[s] = one / (ydn[s] + yup[s]);
+      for (int k = s; k >= 2; --k) V[k - 1] = V[k] * dn[k];
       for (int k = s; k < N; ++k) {
-        if (S.top_pec && k + 1 == N) break;  // V_N = 0 on the cover
-        V[k + 1] = V[k] * Sh[k] / (zd(1.0) + yup[k + 1] / y[k] * T[k]);
+        if (S.top_pec && k + 1 == N) break;
+        V[k + 1] = V[k] * up[k];
       }
     }
   }
   const double k02 = S.k0 * S.k0;
-  for (int i = 0; i < L; ++i) {
-    const int ii = S.il[i];
-    for (int j = 0; j < L; ++j) {
-      const zd* Vh = Vmode[0][j];
-      const zd* Ve = Vmode[1][j];
-      g[0][i][j] = Vh[ii];
-      g[1][i][j] = (Ve[ii] + Vh[ii] * k02) / kr2;
-      zd cum(0.0);
-      for (int n = 0; n < ii; ++n) cum += (Ve[n + 1] - Ve[n]) / (u[n] * u[n]);
-      g[2][i][j] = cum;
+  const zd ikr2 = one / kr2;
+  for (int j = 0; j < L; ++j) {
+    zd cum(0.0);
+    int n = 0;
+    for (int i = 0; i < L; ++i) {  // levels by rising interface
+      const int ii = S.il[i];
+      const zd v = Vm[j][ii], vo = other(v);  // both modes at the level
+      if (mode == 0) {
+        out[(0 * L + i) * L + j] = v;
+        out[(1 * L + i) * L + j] = (vo + v * k02) * ikr2;
+      } else {
+        if (ii < n) {
+          cum = zd(0.0);
+          n = 0;
+        }
+        for (; n < ii; ++n) cum += (Vm[j][n + 1] - Vm[j][n]) * (iu[n] * iu[n]);
+        out[(2 * L + i) * L + j] = cum;
+      }
     }
   }
 }
 
-// Leading-term coefficients (greens.py:215-224, layered.py:292-331); gbig:
+// Leading-term coefficients (greens.py:215-224, layered.py:292-331), one warp
+// per level pair (each is a chain of fp64 latencies; one thread for all took L^2 of them); gbig:
 // the layered spectral kernels at kbig (spectral_g_kernel's last node).
 __global__ void leading_kernel(StackDev* S, double kbig, const zd* __restrict__ gbig) {
-  if (threadIdx.x || blockIdx.x) return;
+  if (threadIdx.x & 31) return;
   StackDev& s = *S;
   const int L = s.nlev, N = s.nlayer;
   if (s.single) {
+    if (threadIdx.x) return;
     zd k1 = s.kk[0], e = s.epsc[0];
     zd k02(s.k0 * s.k0);
     zd ka = csqrt((k02 + k1 * k1) * 0.5);
@@ -135,101 +167,70 @@ __global__ void leading_kernel(StackDev* S, double kbig, const zd* __restrict__ 
     s.dz[0][0] = 0.0;
     return;
   }
-  for (int i = 0; i < L; ++i)
-    for (int j = 0; j < L; ++j) {
-      s.dz[i][j] = fabs(s.zl[i] - s.zl[j]);
-      if (i == j) {
-        int n = s.il[i];
-        zd eb = s.epsc[n - 1], kb = s.kk[n - 1], ea, ka;
-        if (n == N) {
-          ea = zd(1.0);
-          ka = zd(s.k0);
-        } else {
-          ea = s.epsc[n];
-          ka = s.kk[n];
-        }
-        zd cv = zd(2.0) / (ea + eb);
-        s.lead_c[0][i][j] = zd(1.0);
-        s.lead_c[1][i][j] = cv;
-        s.lead_c[2][i][j] = cv;
-        s.kx[0][i][j] = csqrt((ka * ka + kb * kb) * 0.5);
-        s.kx[1][i][j] = csqrt((eb * (ka * ka) + ea * (kb * kb)) / (ea + eb));
-        continue;
-      }
-      zd ux = csqrt(zd(kbig * kbig - s.k0 * s.k0));
-      zd f = ux * 2.0 * cexp(ux * s.dz[i][j]);
-      zd c[3];
-      for (int m = 0; m < 3; ++m) c[m] = f * gbig[(m * L + i) * L + j];
-      if (s.zl[j] < s.zl[i]) c[2] = zd(0.0);
-      for (int m = 0; m < 3; ++m) {
-        // drop the numerical noise of static coefficients' imaginary parts
-        if (fabs(c[m].im) < 1e-9 * cabs(c[m])) c[m].im = 0.0;
-        s.lead_c[m][i][j] = c[m];
-      }
-      s.kx[0][i][j] = zd(s.k0);
-      s.kx[1][i][j] = zd(s.k0);
+  const int i = (threadIdx.x >> 5) / L, j = (threadIdx.x >> 5) % L;
+  s.dz[i][j] = fabs(s.zl[i] - s.zl[j]);
+  if (i == j) {
+    int n = s.il[i];
+    zd eb = s.epsc[n - 1], kb = s.kk[n - 1], ea, ka;
+    if (n == N) {
+      ea = zd(1.0);
+      ka = zd(s.k0);
+    } else {
+      ea = s.epsc[n];
+      ka = s.kk[n];
     }
-}
-
-// The spectral kernels g[(m*L + i)*L + j] at every path node, in one launch:
-// nodes q < nkc of the lifted arc into gc, the next nkr of the real axis into
-// gr, and (layered stacks) one more node at kbig into gbig for the leading
-// terms. Each node is one thread's fp64 chain of square roots, exponentials
-// and divisions through the layers; small CTAs spread the nodes over the SMs.
-__global__ void __launch_bounds__(64) spectral_g_kernel(const StackDev* __restrict__ Sp, int nkc,
-                                                        const double* __restrict__ kc, int nkr,
-                                                        const double* __restrict__ kr, double kbig,
-                                                        zd* __restrict__ gc, zd* __restrict__ gr,
-                                                        zd* __restrict__ gbig) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const StackDev& S = *Sp;
-  const int L = S.nlev, NC = 3 * L * L;
-  zd k;
-  zd* out;
-  if (q < nkc) {
-    k = zd(kc[2 * q], kc[2 * q + 1]);
-    out = gc + (int64_t)q * NC;
-  } else if (q < nkc + nkr) {
-    k = zd(kr[q - nkc], 0.0);
-    out = gr + (int64_t)(q - nkc) * NC;
-  } else if (q == nkc + nkr && !S.single) {
-    k = zd(kbig, 0.0);
-    out = gbig;
-  } else {
+    zd cv = zd(2.0) / (ea + eb);
+    s.lead_c[0][i][j] = zd(1.0);
+    s.lead_c[1][i][j] = cv;
+    s.lead_c[2][i][j] = cv;
+    s.kx[0][i][j] = csqrt((ka * ka + kb * kb) * 0.5);
+    s.kx[1][i][j] = csqrt((eb * (ka * ka) + ea * (kb * kb)) / (ea + eb));
     return;
   }
-  zd g[3][kMaxLev][kMaxLev];
-  if (S.single) {
-    slab_spectral(S, k, g[0][0][0], g[1][0][0], g[2][0][0]);
-  } else {
-    layered_spectral(S, k, g);
+  zd ux = csqrt(zd(kbig * kbig - s.k0 * s.k0));
+  zd f = ux * 2.0 * cexp(ux * s.dz[i][j]);
+  zd c[3];
+  for (int m = 0; m < 3; ++m) c[m] = f * gbig[(m * L + i) * L + j];
+  if (s.zl[j] < s.zl[i]) c[2] = zd(0.0);
+  for (int m = 0; m < 3; ++m) {
+    // drop the numerical noise of static coefficients' imaginary parts
+    if (fabs(c[m].im) < 1e-9 * cabs(c[m])) c[m].im = 0.0;
+    s.lead_c[m][i][j] = c[m];
   }
-  for (int m = 0; m < 3; ++m)
-    for (int i = 0; i < L; ++i)
-      for (int j = 0; j < L; ++j) out[(m * L + i) * L + j] = g[m][i][j];
+  s.kx[0][i][j] = zd(s.k0);
+  s.kx[1][i][j] = zd(s.k0);
 }
 
 // coef[q][(m*L + i)*L + j] = w k (g - leading term) / 2pi at every path node
-// (in place over the spectral kernels g), one thread per (node, column).
+// (in place over the spectral kernels g), one thread per (node, level pair):
+// V and W share their leading term's exponential, and A's too where its k is
+// the same (i != j). Pairs vary slowest, so that a warp takes one branch.
 __global__ void spectral_coef_kernel(const StackDev* __restrict__ Sp, int nkc, const double* __restrict__ kc,
                                      const double* __restrict__ wc, int nkr, const double* __restrict__ kr,
                                      const double* __restrict__ wr, zd* __restrict__ cc, zd* __restrict__ cr) {
   const StackDev& S = *Sp;
-  const int L = S.nlev, NC = 3 * L * L;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)(nkc + nkr) * NC) return;
-  const int q = (int)(t / NC), col = (int)(t % NC);
-  const int m = col / (L * L), i = (col / L) % L, j = col % L;
+  const int L = S.nlev, LL = L * L, nk = nkc + nkr;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, pair = blockIdx.y;
+  if (q >= nk) return;
+  const int i = pair / L, j = pair % L;
   const bool cpath = q < nkc;
   const int qq = cpath ? q : q - nkc;
   const zd k = cpath ? zd(kc[2 * qq], kc[2 * qq + 1]) : zd(kr[qq], 0.0);
   const zd w = cpath ? zd(wc[2 * qq], wc[2 * qq + 1]) : zd(wr[qq], 0.0);
-  zd* c = (cpath ? cc : cr) + (int64_t)qq * NC + col;
-  const zd kx = S.kx[m == 0 ? 0 : 1][i][j];
-  const zd ux = csqrt(k * k - kx * kx);
-  const zd lead = S.lead_c[m][i][j] * cexp(ux * (-S.dz[i][j])) / (ux * 2.0);
-  const zd scale = (w * k) / (2.0 * kPi);
-  *c = scale * (*c - lead);
+  zd* c = (cpath ? cc : cr) + (int64_t)qq * 3 * LL + pair;
+  const zd scale = (w * k) * (1.0 / (2.0 * kPi));
+  const double dz = S.dz[i][j];
+  // e^{-ux dz} / (2 ux)
+  auto leading = [&](zd kx) {
+    const zd ux = csqrt(k * k - kx * kx);
+    return (dz == 0.0 ? zd(1.0) : cexp(ux * (-dz))) / (ux * 2.0);
+  };
+  const zd ka = S.kx[0][i][j], kv = S.kx[1][i][j];
+  zd e = leading(ka);
+  c[0] = scale * (c[0] - S.lead_c[0][i][j] * e);
+  if (kv.re != ka.re || kv.im != ka.im) e = leading(kv);
+  c[LL] = scale * (c[LL] - S.lead_c[1][i][j] * e);
+  c[2 * LL] = scale * (c[2 * LL] - S.lead_c[2][i][j] * e);
 }
 
 // J0 of a complex argument: the trapezoidal rule on Bessel's integral
@@ -258,85 +259,349 @@ __device__ inline zd bessel_j0_complex(zd z) {
   return {(2.0 + 2.0 * cr + 4.0 * sr) / M, (2.0 * ci + 4.0 * si) / M};
 }
 
-// Path nodes per CTA of the Sommerfeld integral: each radius's sum over the
-// nk_c + nk_r path nodes is split into ceil(nk / kSomNodes) fixed ranges (at
-// most kSomMaxSplit), whatever the radii launched with it, so that a radius's
-// value does not depend on which radii share its launch.
-constexpr int kSomNodes = 1024;
-constexpr int kSomMaxSplit = 32;
-inline int som_split(int nk) { return std::min(kSomMaxSplit, std::max(1, (nk + kSomNodes - 1) / kSomNodes)); }
+// J0 at the points of the path. The integral needs it at every pair of a
+// radius and a path node, so the cost of one J0 is the cost of the tables
+// (fp64 runs at two operations per clock on an SM; CUDA's j0 with its argument
+// reduction and the trapezoidal rule above took 85 % of the tabulation). Its Taylor
+// coefficients about equidistant points are tabulated once per call instead,
+// from J0 and J1 there and the recurrence that Bessel's equation
+// x y'' + y' + x y = 0 gives them:
+//   (n+2)(n+1) x c_{n+2} = -((n+1)^2 c_{n+1} + c_{n-1} + x c_n).
+// Row i holds c_n h^n about i h, for the argument in units of h.
+//  - real axis: h = 1/8, degree 8: |J0^(9)| (h/2)^9 / 9! < 5e-17.
+//  - lifted arc: h = 1/4 and degree 19, for imaginary parts up to 1.0625 (the
+//    path's a rho <= 1): 0.4 x 1.07^20 / 20! < 1e-18. Rows below x = 2, where the
+//    expansion would reach the other solutions' singularity at 0, stay
+//    empty: the power series serves there.
+// The distance to the grid point is fma(r / h, k, -i): the product is not
+// rounded by itself, which for r k ~ 1e3 leaves J0 more accurate than j0(r * k).
+constexpr int kHankelMin = 25;  // j01_hankel from here on
+constexpr int kJ0Step = 8, kJ0Deg = 8, kJ0Row = 10;        // rows of 10 doubles: double2 loads
+constexpr int kJ0ArcStep = 4, kJ0ArcDeg = 19, kJ0ArcRow = 20;
+constexpr int kJ0ArcMin = 2 * kJ0ArcStep;                   // first row used
+constexpr double kJ0ArcIm = 1.0625 * kJ0ArcStep;            // largest |Im z| / h
+// Rows at most: arguments up to 16384 and 256, beyond which the functions themselves are called.
+constexpr int kJ0Rows = 1 << 17, kJ0ArcRows = 1 << 10;  // (j01_warp: 256)
+inline int j0_rows(double xmax, int step, int cap) {
+  return !(xmax >= 0) ? 1 : (int)std::min((double)cap, std::floor(xmax * step) + 2.0);
+}
 
-// part[s][e][c] = sum over the nodes of range s of J0(rho k) coef[k][c] at
-// radius rho[idx[e]] (idx NULL: rho[e]); complex J0 on the lifted arc, real
-// J0 on the real axis. Grid (ne, nsplit), one CTA per (radius, node range).
-// With skip set (the learned remainder was accepted) the CTAs return at once.
-template <int NC>
-__global__ void sommerfeld_kernel(int ne, const int* __restrict__ idx, const double* __restrict__ rho, int nsplit,
-                                  int nkc, const double* __restrict__ kc, const zd* __restrict__ coef_c, int nkr,
-                                  const double* __restrict__ kr, const zd* __restrict__ coef_r, zd* __restrict__ part,
-                                  const int* __restrict__ skip) {
-  if (skip && *skip) return;
-  const int e = blockIdx.x, s = blockIdx.y;
-  const double r = rho[idx ? idx[e] : e];
-  const int64_t nk = (int64_t)nkc + nkr;
-  const int q0 = (int)(nk * s / nsplit), q1 = (int)(nk * (s + 1) / nsplit);
-  double acc_re[NC], acc_im[NC];
+// CTAs of 64 threads for the arc's rows
+__host__ __device__ inline int j0_arc_ctas(int rows) { return rows > kJ0ArcMin ? (rows - kJ0ArcMin + 1) / 2 : 0; }
+// and for the axis's rows below x = 25 (by a warp each, as the arc's) and beyond
+__host__ __device__ inline int j0_near_ctas(int rows) { return (min(rows, kJ0Step * kHankelMin) + 1) / 2; }
+__host__ __device__ inline int j0_ctas(int rows_r, int rows_a) {
+  const int near = j0_near_ctas(rows_r);
+  return j0_arc_ctas(rows_a) + near + (max(rows_r - 2 * near, 0) + 63) / 64;
+}
+
+// Row i of a table (see above): `step` points per unit, coefficients to
+// degree DEG, from c0 = J0 and c1 = -J1 there.
+template <int DEG>
+__device__ __forceinline__ void j0_row(int i, int step, double c0, double c1, double* __restrict__ out) {
+  const double h = 1.0 / step, x = i * h;
+  if (i == 0) {  // c_2k = (-1/4)^k / k!^2
+    double c = 1.0;
 #pragma unroll
-  for (int c = 0; c < NC; ++c) acc_re[c] = acc_im[c] = 0.0;
-  for (int q = q0 + threadIdx.x; q < min(q1, nkc); q += blockDim.x) {
-    zd J = bessel_j0_complex(zd(r * kc[2 * q], r * kc[2 * q + 1]));
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      zd v = J * coef_c[(int64_t)q * NC + c];
-      acc_re[c] += v.re;
-      acc_im[c] += v.im;
+    for (int n = 0; n <= DEG; ++n) {
+      out[n] = (n & 1) ? 0.0 : c;
+      if (n & 1) c *= -0.25 * h * h / (((n + 1) / 2) * ((n + 1) / 2));
     }
+    return;
   }
-  for (int q = max(q0, nkc) + threadIdx.x; q < q1; q += blockDim.x) {
-    const int qr = q - nkc;
-    double J = j0(r * kr[qr]);
+  const double inv = 1.0 / x;
+  double cm = 0.0, hn = 1.0;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      zd v = coef_r[(int64_t)qr * NC + c];
-      acc_re[c] += J * v.re;
-      acc_im[c] += J * v.im;
-    }
-  }
-  __shared__ double red[32][2];
-  for (int c = 0; c < NC; ++c) {
-    double a = acc_re[c], b = acc_im[c];
-    for (int o = 16; o; o >>= 1) {
-      a += __shfl_down_sync(0xffffffffu, a, o);
-      b += __shfl_down_sync(0xffffffffu, b, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      red[threadIdx.x >> 5][0] = a;
-      red[threadIdx.x >> 5][1] = b;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double sa = 0, sb = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        sa += red[w][0];
-        sb += red[w][1];
-      }
-      part[((int64_t)s * ne + e) * NC + c] = zd(sa, sb);
-    }
-    __syncthreads();
+  for (int n = 0; n <= DEG; ++n) {
+    out[n] = c0 * hn;
+    const double c2 = -fma(fma((double)((n + 1) * (n + 1)), c1, cm), inv, c0) * (1.0 / ((n + 1) * (n + 2)));
+    cm = c0;
+    c0 = c1;
+    c1 = c2;
+    hn *= h;
   }
 }
 
-// res[idx[e]][c] = sum over the node ranges s (in order) of part[s][e][c].
-__global__ void sommerfeld_sum_kernel(int ne, int NC, const int* __restrict__ idx, int nsplit,
-                                      const zd* __restrict__ part, zd* __restrict__ res,
-                                      const int* __restrict__ skip) {
-  if (skip && *skip) return;
+// J0 and J1 at one point x <= 256 by a warp: the trapezoidal rule on Bessel's
+// integral with 512 points (a quarter period of them, four per lane). Nodes
+// share rows, so that an error of a row does not average out over them as their own
+// roundings do: many more points than the rule needs average the rounding of
+// its terms here (about 2e-17; CUDA's j0 and j1 are off by 1e-15 beyond 8 and by 1e-13 beyond 20).
+__device__ void j01_warp(double x, double& y0, double& y1) {
+  double s0 = 0.0, s1 = 0.0;
+  for (int q = 0; q < 4; ++q) {
+    int m = (threadIdx.x & 31) + 32 * q;
+    if (m == 0) m = 128;  // the quarter point in the place of the first, a constant
+    const double s = sinpi(m / 256.0), a = x * s, r = fma(x, s, -a);
+    double sa, ca;
+    sincos(a, &sa, &ca);
+    const double g = m == 128 ? 2.0 : 4.0;
+    s0 = fma(g, fma(-r, sa, ca), s0);
+    s1 = fma(g * s, fma(r, ca, sa), s1);
+  }
+  for (int o = 16; o; o >>= 1) {
+    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+  }
+  y0 = (2.0 + s0) * (1.0 / 512.0);
+  y1 = s1 * (1.0 / 512.0);
+}
+
+// J0 and J1 at x >= 25: Hankel's expansions (Abramowitz & Stegun 9.2.5 - 9.2.10),
+// J_v = (2 / pi x)^1/2 (P_v cos chi - Q_v sin chi), chi = x - (v/2 + 1/4) pi, to the
+// term of x^-17 (the next one is below 4e-17 at x = 25).
+__device__ void j01_hankel(double x, double& y0, double& y1) {
+  const double ix = 1.0 / x, amp = rsqrt(kPi * x);
+  double s, c, P[2], Q[2];
+  sincos(x, &s, &c);
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    double t = 1.0, p = 1.0, q = 0.0;
+#pragma unroll
+    for (int k = 1; k <= 17; ++k) {
+      t *= ix * ((4 * v - (2 * k - 1) * (2 * k - 1)) / (8.0 * k));
+      double& sum = (k & 1) ? q : p;
+      sum += (k & 2) ? -t : t;
+    }
+    P[v] = p;
+    Q[v] = q;
+  }
+  y0 = amp * (P[0] * (c + s) - Q[0] * (s - c));
+  y1 = amp * (P[1] * (s - c) + Q[1] * (s + c));
+}
+
+// The grid point next to r k / h for rs = r / h: its index (false: outside
+// 0 .. rows - 1, not a number) and the distance to it in units of h.
+__device__ __forceinline__ bool j0_locate(double rs, double k, int rows, int& i, double& d) {
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 x 2^52: the sum's low word is the integer next to rs k
+  const double t = fma(rs, k, kMagic);
+  i = __double2loint(t);
+  d = fma(rs, k, kMagic - t);
+  return (unsigned)i < (unsigned)rows && __double2hiint(t) == 0x43380000;
+}
+
+// J0(r k) on the real axis; rs = r kJ0Step.
+__device__ __forceinline__ double j0_real(double r, double rs, double k, const double* __restrict__ tab, int rows) {
+  int i;
+  double d;
+  if (!j0_locate(rs, k, rows, i, d)) return j0(r * k);
+  const double2* c = reinterpret_cast<const double2*>(tab + (size_t)i * kJ0Row);
+  const double2 c01 = c[0], c23 = c[1], c45 = c[2], c67 = c[3];
+  double v = tab[(size_t)i * kJ0Row + 8];
+  v = fma(v, d, c67.y);
+  v = fma(v, d, c67.x);
+  v = fma(v, d, c45.y);
+  v = fma(v, d, c45.x);
+  v = fma(v, d, c23.y);
+  v = fma(v, d, c23.x);
+  v = fma(v, d, c01.y);
+  return fma(v, d, c01.x);
+}
+
+__device__ __noinline__ zd j0_far(zd z) { return bessel_j0_complex(z); }
+
+// J0(z) for |Re z| < 2, |Im z| < 1.1: the power series in -z^2 / 4 (|.| <= 1.27: 1.27^13 / 13!^2 < 1e-18).
+__device__ __noinline__ zd j0_series(zd z) {
+  const zd w = z * z * -0.25;
+  zd v(1.0, 0.0);
+#pragma unroll
+  for (int k = 12; k >= 1; --k) {
+    const zd t = v * w;
+    v = zd(fma(t.re, 1.0 / (k * k), 1.0), t.im * (1.0 / (k * k)));
+  }
+  return v;
+}
+
+// J0(r k) on the lifted arc; rs = r kJ0ArcStep. The polynomial with real
+// coefficients at the complex distance d by division by t^2 - 2 Re d t +
+// |d|^2: two operations per coefficient.
+__device__ __forceinline__ zd j0_arc(double r, double rs, zd k, const double* __restrict__ tab, int rows) {
+  int i;
+  double dr;
+  const double di = rs * k.im;
+  const bool in = j0_locate(rs, k.re, rows, i, dr) && fabs(di) <= kJ0ArcIm;
+  if (!in) return j0_far(k * r);
+  if (i < kJ0ArcMin) return j0_series(k * r);
+  const double2* c = reinterpret_cast<const double2*>(tab + (size_t)i * kJ0ArcRow);
+  const double s = dr + dr, t = fma(dr, dr, di * di);
+  double2 a = c[kJ0ArcDeg / 2];
+  double b2 = a.y, b1 = fma(s, a.y, a.x);  // b_{n}, b_{n-1} of the quotient
+#pragma unroll
+  for (int p = kJ0ArcDeg / 2 - 1; p >= 1; --p) {
+    a = c[p];
+    b2 = fma(s, b1, fma(-t, b2, a.y));
+    b1 = fma(s, b2, fma(-t, b1, a.x));
+  }
+  a = c[0];
+  const double q1 = fma(s, b1, fma(-t, b2, a.y));
+  return {fma(q1, dr, fma(-t, b1, a.x)), q1 * di};
+}
+
+// The spectral kernels g[(m*L + i)*L + j] at every path node, in one launch:
+// nodes q < nkc of the lifted arc into gc, the next nkr of the real axis into
+// gr, and (layered stacks) one more node at kbig into gbig for the leading
+// terms. A node is a fp64 chain of square roots, exponentials and divisions
+// through the layers, on one lane (one slab) or two (layered_spectral); small
+// CTAs spread the nodes over the SMs. 7176 nodes of two layers: 48 us (one lane a
+// node and a division for every use of 1 / u^2 and 1 / k^2: 82 us).
+// The CTAs from nb on fill the J0 tables of the integral.
+__global__ void __launch_bounds__(64) spectral_g_kernel(const StackDev* __restrict__ Sp, int nkc,
+                                                        const double* __restrict__ kc, int nkr,
+                                                        const double* __restrict__ kr, double kbig,
+                                                        zd* __restrict__ gc, zd* __restrict__ gr,
+                                                        zd* __restrict__ gbig, int nb, double* __restrict__ j0r,
+                                                        int rows_r, double* __restrict__ j0a, int rows_a) {
+  if ((int)blockIdx.x >= nb) {  // the rows of the J0 tables
+    const int b = (int)blockIdx.x - nb, nba = j0_arc_ctas(rows_a), nbr = j0_near_ctas(rows_r);
+    const int w = threadIdx.x >> 5;
+    if (b < nba + nbr) {
+      const bool arc = b < nba;
+      const int i = arc ? kJ0ArcMin + 2 * b + w : 2 * (b - nba) + w;
+      double y0, y1;
+      j01_warp(arc ? (double)i / kJ0ArcStep : (double)i / kJ0Step, y0, y1);
+      if ((threadIdx.x & 31) == 0) {
+        if (arc && i < rows_a) j0_row<kJ0ArcDeg>(i, kJ0ArcStep, y0, -y1, j0a + (size_t)i * kJ0ArcRow);
+        if (!arc && i < rows_r) j0_row<kJ0Deg>(i, kJ0Step, y0, -y1, j0r + (size_t)i * kJ0Row);
+      }
+    } else {
+      const int i = 2 * nbr + (b - nba - nbr) * blockDim.x + threadIdx.x;
+      double y0, y1;
+      j01_hankel((double)i / kJ0Step, y0, y1);
+      if (i < rows_r) j0_row<kJ0Deg>(i, kJ0Step, y0, -y1, j0r + (size_t)i * kJ0Row);
+    }
+    return;
+  }
+  const StackDev& S = *Sp;
+  const int NC = 3 * S.nlev * S.nlev;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ne * NC) return;
-  const int e = t / NC, c = t % NC;
-  zd v(0.0, 0.0);
-  for (int s = 0; s < nsplit; ++s) v = v + part[((int64_t)s * ne + e) * NC + c];
-  res[(int64_t)(idx ? idx[e] : e) * NC + c] = v;
+  if (S.single) {
+    if (t >= nkc + nkr) return;
+    const zd k = t < nkc ? zd(kc[2 * t], kc[2 * t + 1]) : zd(kr[t - nkc], 0.0);
+    zd* out = t < nkc ? gc + 3 * (int64_t)t : gr + 3 * (int64_t)(t - nkc);
+    slab_spectral(S, k, out[0], out[1], out[2]);
+    return;
+  }
+  const int q = min(t >> 1, nkc + nkr);  // the lanes beyond repeat the last node (all lanes take the exchanges)
+  const zd k = q < nkc ? zd(kc[2 * q], kc[2 * q + 1]) : zd(q < nkc + nkr ? kr[q - nkc] : kbig, 0.0);
+  zd* out = q < nkc ? gc + (int64_t)q * NC : q < nkc + nkr ? gr + (int64_t)(q - nkc) * NC : gbig;
+  layered_spectral(S, k, t & 1, out);
+}
+
+// Splits of the node sum: at most kSomArcSplit ranges of the arc's nodes and
+// kSomRealSplit of the axis's, about 24 and 64 nodes in each, whatever the
+// radii launched with it, so that a radius's value does not depend on which
+// radii share its launch.
+constexpr int kSomArcSplit = 48, kSomRealSplit = 96;
+inline int som_split_arc(int nkc) { return std::min(kSomArcSplit, std::max(1, (nkc + 23) / 24)); }
+inline int som_split_real(int nkr) { return std::min(kSomRealSplit, std::max(1, (nkr + 63) / 64)); }
+
+struct SomArgs {
+  int ne;
+  const int* idx;  // radii rho[idx[e]] (NULL: rho[e])
+  const double* rho;
+  int nsa, nsr;  // ranges of arc and real nodes
+  int nkc;
+  const double* kc;
+  const zd* coef_c;
+  int nkr;
+  const double* kr;
+  const zd* coef_r;
+  const double *j0r, *j0a;  // J0 tables
+  int rows_r, rows_a;
+  double* part;
+  const int* skip;
+};
+
+// part[s][c][re / im][e] = sum over the nodes of range s of J0(rho k)
+// coef[k][c] at radius rho[idx[e]]; ranges 0 .. nsa - 1 on the lifted arc
+// (complex J0; the dearer ones, so they start first), then nsr on the real
+// axis. A CTA takes 32 radii, one per lane, and its four warps every fourth node of the
+// range: the coefficients are the same for all lanes (a thread per node had
+// to sum its 2 NC values over the CTA for every radius, more work than the
+// products), and the warps' sums meet once, in shared memory. Bound by fp64
+// operations: 11 for a real J0, about 50 for a complex one, 2 NC and 4 NC for the
+// products. 372 radii x 7176 nodes, 12 columns (the via transition's tables):
+// 270 us, 1180 us before; 233 radii, 3 columns 74 us, some 430 us before.
+// With skip set (the learned remainder was accepted) the CTAs return at once.
+template <int NC>
+__global__ void __launch_bounds__(128) sommerfeld_kernel(SomArgs a) {
+  if (a.skip && *a.skip) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int e = blockIdx.y * 32 + lane, s = blockIdx.x;
+  const int ee = min(e, a.ne - 1);
+  const double r = a.rho[a.idx ? a.idx[ee] : ee];
+  double acc_re[NC], acc_im[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc_re[c] = acc_im[c] = 0.0;
+  if (s < a.nsa) {
+    const int q0 = (int)((int64_t)a.nkc * s / a.nsa), q1 = (int)((int64_t)a.nkc * (s + 1) / a.nsa);
+    const double rs = r * kJ0ArcStep;
+    for (int q = q0 + w; q < q1; q += 4) {
+      const zd J = j0_arc(r, rs, zd(a.kc[2 * q], a.kc[2 * q + 1]), a.j0a, a.rows_a);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const zd v = ldc(a.coef_c + (int64_t)q * NC + c);
+        acc_re[c] = fma(J.re, v.re, fma(-J.im, v.im, acc_re[c]));
+        acc_im[c] = fma(J.re, v.im, fma(J.im, v.re, acc_im[c]));
+      }
+    }
+  } else {
+    const int sr = s - a.nsa;
+    const int q0 = (int)((int64_t)a.nkr * sr / a.nsr), q1 = (int)((int64_t)a.nkr * (sr + 1) / a.nsr);
+    const double rs = r * kJ0Step;
+#pragma unroll 2
+    for (int q = q0 + w; q < q1; q += 4) {
+      const double J = j0_real(r, rs, a.kr[q], a.j0r, a.rows_r);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const zd v = ldc(a.coef_r + (int64_t)q * NC + c);
+        acc_re[c] = fma(J, v.re, acc_re[c]);
+        acc_im[c] = fma(J, v.im, acc_im[c]);
+      }
+    }
+  }
+  // the warps' sums, four columns at a time: warp w adds up column c0 + w
+  __shared__ double red[4][8][32];
+#pragma unroll
+  for (int c0 = 0; c0 < NC; c0 += 4) {
+    if (c0) __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c0 + j < NC) {
+        red[w][2 * j][lane] = acc_re[c0 + j];
+        red[w][2 * j + 1][lane] = acc_im[c0 + j];
+      }
+    __syncthreads();
+    if (c0 + w < NC && e < a.ne) {
+      double* o = a.part + ((int64_t)s * NC + c0 + w) * 2 * a.ne + e;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        o[h * a.ne] = (red[0][2 * w + h][lane] + red[1][2 * w + h][lane]) +
+                      (red[2][2 * w + h][lane] + red[3][2 * w + h][lane]);
+    }
+  }
+}
+
+// res[idx[e]][c] = sum over the node ranges s of part[s][c][..][e]: eight
+// lanes per value, each every eighth range.
+__global__ void __launch_bounds__(256) sommerfeld_sum_kernel(int ne, int NC, const int* __restrict__ idx, int nsplit,
+                                                             const double* __restrict__ part, zd* __restrict__ res,
+                                                             const int* __restrict__ skip) {
+  if (skip && *skip) return;
+  const int nv = ne * NC * 2, t0 = blockIdx.x * 32, l = threadIdx.x & 31, g = threadIdx.x >> 5;
+  __shared__ double red[8][32];
+  const int t = t0 + l;
+  double v = 0.0;
+  if (t < nv)
+    for (int s = g; s < nsplit; s += 8) v += part[(int64_t)s * nv + t];
+  red[g][l] = v;
+  __syncthreads();
+  if (g == 0 && t < nv) {
+    for (int k = 1; k < 8; ++k) v += red[k][l];
+    const int e = t % ne, ch = t / ne;
+    double* o = reinterpret_cast<double*>(res + (int64_t)(idx ? idx[e] : e) * NC + (ch >> 1));
+    o[ch & 1] = v;
+  }
 }
 
 // S tables: closed-form expm1 part of the leading term, the Sommerfeld
@@ -380,44 +645,51 @@ __global__ void table_kernel(const StackDev* __restrict__ Sp, int nrho, const do
 // c_{m-1} = 0), diagonally dominant, solved by parallel cyclic reduction
 // (Hockney) with every thread of the CTA: round r combines each row with the
 // rows 2^r above and below, which removes their couplings; after ceil(log2 m)
-// rounds every row reads b_i x_i = d_i. Shared-memory arrays of m entries:
-// a, b, c, d and the copies a2, b2, c2, d2 (ping-pong); x receives the
-// solution (it may be d). The caller synchronises before the call; the call
-// ends with the CTA synchronised. A serial elimination would chain m
-// dependent fp64 divisions; here the chain is ceil(log2 m) rounds deep.
+// rounds every row reads b_i x_i = d_i. A spline's rows are dominated by their
+// diagonal two to one, so that the couplings fall below (2 - sqrt 3)^(2^r) of
+// it: the rounds end when all are below 2^-60 and adding them would change no
+// digit (six rounds instead of eight at 220 rows). Rows are kept scaled by
+// their diagonal (b = 1), which leaves one division per row and round
+// instead of two. Shared-memory arrays of m entries: a, b, c, d and the copies
+// a2, b2, c2, d2 (ping-pong); x receives the solution (it may be d). The
+// caller synchronises before the call; the call ends with the CTA synchronised. A serial
+// elimination would chain m dependent fp64 divisions; here the chain is the rounds.
 template <class T>
 __device__ void pcr_solve(int m, double* a, double* b, double* c, T* d, double* a2, double* b2, double* c2, T* d2,
                           T* x) {
+  for (int i = threadIdx.x; i < m; i += blockDim.x) {
+    const double inv = 1.0 / b[i];
+    a[i] *= inv;
+    c[i] *= inv;
+    d[i] = d[i] * inv;
+  }
+  __syncthreads();
   for (int st = 1; st < m; st <<= 1) {
+    bool coupled = false;
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
-      double na = 0.0, nc = 0.0, nb = b[i];
+      const bool lo = i - st >= 0, hi = i + st < m;
+      const double ai = lo ? a[i] : 0.0, ci = hi ? c[i] : 0.0;
+      const double al = lo ? a[i - st] : 0.0, cl = lo ? c[i - st] : 0.0;
+      const double ah = hi ? a[i + st] : 0.0, ch = hi ? c[i + st] : 0.0;
+      const double inv = 1.0 / fma(-ai, cl, fma(-ci, ah, 1.0));
       T nd = d[i];
-      if (i - st >= 0) {
-        const double k1 = a[i] / b[i - st];
-        na = -a[i - st] * k1;
-        nb -= c[i - st] * k1;
-        nd = nd - d[i - st] * k1;
-      }
-      if (i + st < m) {
-        const double k2 = c[i] / b[i + st];
-        nc = -c[i + st] * k2;
-        nb -= a[i + st] * k2;
-        nd = nd - d[i + st] * k2;
-      }
+      if (lo) nd = nd - d[i - st] * ai;
+      if (hi) nd = nd - d[i + st] * ci;
+      const double na = -ai * al * inv, nc = -ci * ch * inv;
       a2[i] = na;
-      b2[i] = nb;
       c2[i] = nc;
-      d2[i] = nd;
+      d2[i] = nd * inv;
+      coupled |= fabs(na) + fabs(nc) > 8.673617379884035e-19;  // 2^-60 of the diagonal
     }
-    __syncthreads();
+    const int more = __syncthreads_or(coupled);
     double* t;
     t = a, a = a2, a2 = t;
-    t = b, b = b2, b2 = t;
     t = c, c = c2, c2 = t;
     T* td = d;
     d = d2, d2 = td;
+    if (!more) break;
   }
-  for (int i = threadIdx.x; i < m; i += blockDim.x) x[i] = d[i] / b[i];
+  for (int i = threadIdx.x; i < m; i += blockDim.x) x[i] = d[i];
   __syncthreads();
 }
 
@@ -560,9 +832,14 @@ __global__ void __launch_bounds__(128) spline_kernel(int L, int nrho, const doub
   }
 }
 
-__global__ void to_f32_kernel(const double* __restrict__ a, float* __restrict__ b, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = float(a[i]);
+// float copies of a (na) and of b (nb)
+__global__ void to_f32_kernel(const double* __restrict__ a, float* __restrict__ oa, int64_t na,
+                              const double* __restrict__ b, float* __restrict__ ob, int nb) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < na)
+    oa[i] = float(a[i]);
+  else if (i < na + nb)
+    ob[i - na] = float(b[i - na]);
 }
 
 // ------------------------------------------------------ learned remainder
@@ -822,70 +1099,93 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
   zd *cc = nullptr, *cr = nullptr, *res = nullptr;
   std::vector<void*> tmp;
   const int n = d->nrho;
+  double rmax = 0, kcmax = 0, krmax = 0;
+  for (int i = 0; i < n; ++i) rmax = std::max(rmax, d->rho[i]);
+  for (int q = 0; q < d->nk_c; ++q) kcmax = std::max(kcmax, d->kc[2 * q]);
+  for (int q = 0; q < d->nk_r; ++q) krmax = std::max(krmax, d->kr[q]);
+  const int rows_r = j0_rows(rmax * krmax, kJ0Step, kJ0Rows), rows_a = j0_rows(rmax * kcmax, kJ0ArcStep, kJ0ArcRows);
 #define TRY(x)         \
   do {                 \
     rc = (x);          \
     if (rc) goto fail; \
   } while (0)
-  TRY(alloc_async(tmp, (void**)&Sd, sizeof(StackDev), st));
-  TRY(alloc_async(tmp, (void**)&kc, sizeof(double) * 2 * d->nk_c, st));
-  TRY(alloc_async(tmp, (void**)&wc, sizeof(double) * 2 * d->nk_c, st));
-  TRY(alloc_async(tmp, (void**)&kr, sizeof(double) * d->nk_r, st));
-  TRY(alloc_async(tmp, (void**)&wr, sizeof(double) * d->nk_r, st));
-  TRY(alloc_async(tmp, (void**)&cc, sizeof(zd) * (size_t)d->nk_c * NC, st));
-  TRY(alloc_async(tmp, (void**)&cr, sizeof(zd) * (size_t)d->nk_r * NC, st));
-  TRY(alloc_async(g->allocs, (void**)&res, sizeof(zd) * (size_t)n * NC, st));
-  g->res = res;
-  TRY(alloc_async(g->allocs, &g->sur, 16, st));
-  M25_CUDA(cudaMemsetAsync(g->sur, 0, 16, st));
-  TRY(alloc_async(g->allocs, (void**)&g->rho, sizeof(double) * n, st));
-  TRY(alloc_async(g->allocs, (void**)&g->rho32, sizeof(float) * n, st));
-  TRY(alloc_async(g->allocs, (void**)&g->S, sizeof(zd) * (size_t)NC * n, st));
-  TRY(alloc_async(g->allocs, (void**)&g->coef, sizeof(zd) * (size_t)L * L * (n - 1) * 12, st));
-  TRY(alloc_async(g->allocs, (void**)&g->coef32, sizeof(float) * 2 * (size_t)L * L * (n - 1) * 12, st));
-  TRY(alloc_async(g->allocs, (void**)&g->lead, sizeof(StackDev), st));
-  M25_CUDA(cudaMemcpyAsync(Sd, &S, sizeof(StackDev), cudaMemcpyHostToDevice, st));
-  M25_CUDA(cudaMemcpyAsync(kc, d->kc, sizeof(double) * 2 * d->nk_c, cudaMemcpyHostToDevice, st));
-  M25_CUDA(cudaMemcpyAsync(wc, d->wc, sizeof(double) * 2 * d->nk_c, cudaMemcpyHostToDevice, st));
-  M25_CUDA(cudaMemcpyAsync(kr, d->kr, sizeof(double) * d->nk_r, cudaMemcpyHostToDevice, st));
-  M25_CUDA(cudaMemcpyAsync(wr, d->wr, sizeof(double) * d->nk_r, cudaMemcpyHostToDevice, st));
-  M25_CUDA(cudaMemcpyAsync(g->rho, d->rho, sizeof(double) * n, cudaMemcpyHostToDevice, st));
+  // One block for what outlives this call and one for what does not, each
+  // carved up at multiples of 256 bytes, and the inputs in one copy.
+  size_t keep = 0, scratch = 0;
+  auto carve = [](size_t& total, size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t o_stack = carve(keep, sizeof(StackDev)), o_rho = carve(keep, sizeof(double) * n),
+               o_kc = carve(keep, sizeof(double) * 2 * d->nk_c), o_wc = carve(keep, sizeof(double) * 2 * d->nk_c),
+               o_kr = carve(keep, sizeof(double) * d->nk_r), o_wr = carve(keep, sizeof(double) * d->nk_r), n_in = keep,
+               o_res = carve(keep, sizeof(zd) * (size_t)n * NC), o_sur = carve(keep, 16),
+               o_rho32 = carve(keep, sizeof(float) * n), o_S = carve(keep, sizeof(zd) * (size_t)NC * n),
+               o_coef = carve(keep, sizeof(zd) * (size_t)L * L * (n - 1) * 12),
+               o_coef32 = carve(keep, sizeof(zf) * (size_t)L * L * (n - 1) * 12);
+  const int nsa = som_split_arc(d->nk_c), nsr = som_split_real(d->nk_r);
+  const size_t o_cc = carve(scratch, sizeof(zd) * (size_t)d->nk_c * NC),
+               o_cr = carve(scratch, sizeof(zd) * (size_t)d->nk_r * NC), o_gbig = carve(scratch, sizeof(zd) * NC),
+               o_j0r = carve(scratch, sizeof(double) * kJ0Row * (size_t)rows_r),
+               o_j0a = carve(scratch, sizeof(double) * kJ0ArcRow * (size_t)rows_a),
+               o_part = carve(scratch, sizeof(zd) * (size_t)(nsa + nsr) * n * NC);
+  std::vector<char> in(n_in);
+  memcpy(in.data() + o_stack, &S, sizeof(StackDev));
+  memcpy(in.data() + o_rho, d->rho, sizeof(double) * n);
+  memcpy(in.data() + o_kc, d->kc, sizeof(double) * 2 * d->nk_c);
+  memcpy(in.data() + o_wc, d->wc, sizeof(double) * 2 * d->nk_c);
+  memcpy(in.data() + o_kr, d->kr, sizeof(double) * d->nk_r);
+  memcpy(in.data() + o_wr, d->wr, sizeof(double) * d->nk_r);
+  char *kb = nullptr, *sb = nullptr;
+  zd* gbig = nullptr;
+  double *j0r = nullptr, *j0a = nullptr, *part = nullptr;
+  TRY(alloc_async(g->allocs, (void**)&kb, keep, st));
+  TRY(alloc_async(tmp, (void**)&sb, scratch, st));
+  Sd = reinterpret_cast<StackDev*>(kb + o_stack);
+  g->rho = reinterpret_cast<double*>(kb + o_rho);
+  kc = reinterpret_cast<double*>(kb + o_kc);
+  wc = reinterpret_cast<double*>(kb + o_wc);
+  kr = reinterpret_cast<double*>(kb + o_kr);
+  wr = reinterpret_cast<double*>(kb + o_wr);
+  g->res = res = reinterpret_cast<zd*>(kb + o_res);
+  g->sur = kb + o_sur;
+  g->rho32 = reinterpret_cast<float*>(kb + o_rho32);
+  g->S = reinterpret_cast<decltype(g->S)>(kb + o_S);
+  g->coef = reinterpret_cast<decltype(g->coef)>(kb + o_coef);
+  g->coef32 = reinterpret_cast<float*>(kb + o_coef32);
+  g->lead = reinterpret_cast<decltype(g->lead)>(Sd);
+  cc = reinterpret_cast<zd*>(sb + o_cc);
+  cr = reinterpret_cast<zd*>(sb + o_cr);
+  gbig = reinterpret_cast<zd*>(sb + o_gbig);
+  j0r = reinterpret_cast<double*>(sb + o_j0r);
+  j0a = reinterpret_cast<double*>(sb + o_j0a);
+  part = reinterpret_cast<double*>(sb + o_part);
+  M25_CUDA(cudaMemcpyAsync(kb, in.data(), n_in, cudaMemcpyHostToDevice, st));
+  if (d->surrogate) M25_CUDA(cudaMemsetAsync(g->sur, 0, 16, st));
   {
   StageTimer tm(ctx, ST_GREENS);
   {
-    zd* gbig = nullptr;
-    TRY(alloc_async(tmp, (void**)&gbig, sizeof(zd) * NC, st));
-    const int nodes = d->nk_c + d->nk_r + 1;
-    spectral_g_kernel<<<(nodes + 63) / 64, 64, 0, st>>>(Sd, d->nk_c, kc, d->nk_r, kr, d->kbig, cc, cr, gbig);
-    leading_kernel<<<1, 1, 0, st>>>(Sd, d->kbig, gbig);
-    const int64_t ncoef = (int64_t)(d->nk_c + d->nk_r) * NC;
-    spectral_coef_kernel<<<(unsigned)((ncoef + 127) / 128), 128, 0, st>>>(Sd, d->nk_c, kc, wc, d->nk_r, kr, wr, cc,
-                                                                          cr);
+    const int lanes = d->single ? d->nk_c + d->nk_r : 2 * (d->nk_c + d->nk_r + 1), nb = (lanes + 63) / 64;
+    spectral_g_kernel<<<nb + j0_ctas(rows_r, rows_a), 64, 0, st>>>(Sd, d->nk_c, kc, d->nk_r, kr, d->kbig, cc, cr,
+                                                                       gbig, nb, j0r, rows_r, j0a, rows_a);
+    leading_kernel<<<1, 32 * L * L, 0, st>>>(Sd, d->kbig, gbig);
+    spectral_coef_kernel<<<dim3((d->nk_c + d->nk_r + 63) / 64, L * L), 64, 0, st>>>(Sd, d->nk_c, kc, wc, d->nk_r, kr,
+                                                                                    wr, cc, cr);
   }
   {
     // the Sommerfeld integral at the radii rho[idx[e]], e < ne (idx NULL:
     // all n) into res; skip: see sommerfeld_kernel
-    const int nsplit = som_split(d->nk_c + d->nk_r);
-    zd* part = nullptr;
-    TRY(alloc_async(tmp, (void**)&part, sizeof(zd) * (size_t)nsplit * n * NC, st));
     auto sommerfeld = [&](int ne, const int* idx, const int* skip) {
       if (ne <= 0) return;
-      dim3 grid(ne, nsplit);
+      const dim3 grid(nsa + nsr, (ne + 31) / 32);
+      const SomArgs a{ne, idx, g->rho, nsa, nsr, d->nk_c, kc, cc, d->nk_r, kr, cr, j0r, j0a, rows_r, rows_a, part, skip};
       switch (NC) {
-        case 3:
-          sommerfeld_kernel<3><<<grid, 256, 0, st>>>(ne, idx, g->rho, nsplit, d->nk_c, kc, cc, d->nk_r, kr, cr, part,
-                                                     skip);
-          break;
-        case 12:
-          sommerfeld_kernel<12><<<grid, 256, 0, st>>>(ne, idx, g->rho, nsplit, d->nk_c, kc, cc, d->nk_r, kr, cr, part,
-                                                      skip);
-          break;
-        default:
-          sommerfeld_kernel<27><<<grid, 256, 0, st>>>(ne, idx, g->rho, nsplit, d->nk_c, kc, cc, d->nk_r, kr, cr, part,
-                                                      skip);
-          break;
+        case 3: sommerfeld_kernel<3><<<grid, 128, 0, st>>>(a); break;
+        case 12: sommerfeld_kernel<12><<<grid, 128, 0, st>>>(a); break;
+        default: sommerfeld_kernel<27><<<grid, 128, 0, st>>>(a); break;
       }
-      sommerfeld_sum_kernel<<<(ne * NC + 255) / 256, 256, 0, st>>>(ne, NC, idx, nsplit, part, res, skip);
+      sommerfeld_sum_kernel<<<(2 * ne * NC + 31) / 32, 256, 0, st>>>(ne, NC, idx, nsa + nsr, part, res, skip);
     };
     // learned remainder: which radii get the Sommerfeld integral first
     std::vector<int> ie, kpos, vpos, ir;
@@ -999,12 +1299,10 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
                                                             reinterpret_cast<zd*>(g->coef));
   }
   {
-    int64_t nc = (int64_t)L * L * (n - 1) * 12 * 2;
-    to_f32_kernel<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(g->coef, g->coef32, nc);
-    to_f32_kernel<<<(n + 255) / 256, 256, 0, st>>>(g->rho, g->rho32, n);
+    const int64_t nc = (int64_t)L * L * (n - 1) * 12 * 2;
+    to_f32_kernel<<<(unsigned)((nc + n + 255) / 256), 256, 0, st>>>(g->coef, g->coef32, nc, g->rho, g->rho32, n);
   }
   }
-  M25_CUDA(cudaMemcpyAsync(g->lead, Sd, sizeof(StackDev), cudaMemcpyDeviceToDevice, st));
   M25_CHECK_LAUNCH();
   // temporaries are released once the stream has consumed them
   free_all_async(tmp, st);
