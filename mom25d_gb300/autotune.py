@@ -55,11 +55,17 @@ class Tuning:
                 return tuple(int(r[k]) for k in KNOBS)
         return tuple(int(self.rows[-1][k]) for k in KNOBS)
 
-    def apply(self, ctx, n):
-        """Set the knobs for a point of N unknowns on an engine context."""
+    def apply(self, ctx, n, alone=False):
+        """Set the knobs for a point of N unknowns on an engine context.
+        alone: no other point runs beside it, so nothing is gained by leaving it fewer CTAs for its
+        triangular solves (the cap, measured with eight points in flight, costs a lone point of
+        N = 5943 3.5 ms of 27; it does not change a result)."""
         from . import engine as E
 
-        E.check(ctx.lib.m25_ctx_set_tuning(ctx.h, *self.knobs(n)))
+        k = dict(zip(KNOBS, self.knobs(n)))
+        if alone:
+            k["wave_ctas"] = 0
+        E.check(ctx.lib.m25_ctx_set_tuning(ctx.h, *(k[name] for name in KNOBS)))
 
     @classmethod
     def fixed(cls, **knobs):

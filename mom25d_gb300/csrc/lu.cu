@@ -544,31 +544,53 @@ __global__ void __launch_bounds__(256) gemm_kernel(cx<T>* A, int64_t lda, int n,
     }
 }
 
-// perm from the interchange list: perm[i] = the original row that ends in
-// row i after the interchanges (sequential in shared memory, one thread;
-// built once per factorisation)
-// STAGE: ipiv is first copied to shared memory, so that the serial loop of
-// swaps reads no global memory (n <= 25600)
+// perm[i] = the original row that the interchanges (0 p_0), (1 p_1), ... bring to
+// position i (p_t >= t). Undone from the last to the first, they take position
+// i to p_i and from there, at the largest s < i with p_s = p_i, to s; a row at
+// s goes on to the largest r < s with p_r = s, and so on. The second kind of step is
+// the same for every i: last[s], by an atomic maximum in shared memory. For the
+// first each thread looks through the list once. Composing the swaps forward
+// instead is one chain through shared memory (N = 5943: 235 us, here 32 us).
+// STAGE: the list in shared memory too (n <= 25600).
+constexpr int kPermThreads = 128;
 template <bool STAGE>
-__global__ void perm_kernel(int n, const int32_t* __restrict__ ipiv, int32_t* __restrict__ perm_out) {
-  extern __shared__ int perm[];
-  int* piv = perm + n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    perm[i] = i;
-    if (STAGE) piv[i] = ipiv[i];
+__global__ void __launch_bounds__(kPermThreads) perm_kernel(int n, const int32_t* __restrict__ ipiv,
+                                                            int32_t* __restrict__ perm) {
+  extern __shared__ __align__(16) int perm_smem[];
+  int* last = perm_smem;
+  int* ps = last + ((n + 3) & ~3);
+  for (int t = threadIdx.x; t < n; t += kPermThreads) last[t] = -1;
+  __syncthreads();
+  for (int t = threadIdx.x; t < n; t += kPermThreads) {
+    const int p = ipiv[t];
+    if (STAGE) ps[t] = p;
+    if (p > t && p < n) atomicMax(&last[p], t);
   }
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (int i = 0; i < n; ++i) {
-      int p = STAGE ? piv[i] : ipiv[i];
-      if (p != i && p >= 0 && p < n) {
-        int t = perm[i];
-        perm[i] = perm[p];
-        perm[p] = t;
-      }
+  const int i = blockIdx.x * kPermThreads + threadIdx.x;
+  if (i >= n) return;
+  const int* pl = STAGE ? ps : ipiv;
+  const int pi = pl[i], i0 = i & ~31;
+  int x = pi > i && pi < n ? pi : i, s = -1;
+  if (STAGE) {
+    const int4* p4 = reinterpret_cast<const int4*>(ps);
+#pragma unroll 4
+    for (int t = 0; t < i0; t += 4) {
+      const int4 v = p4[t >> 2];
+      if (v.x == x) s = t;
+      if (v.y == x) s = t + 1;
+      if (v.z == x) s = t + 2;
+      if (v.w == x) s = t + 3;
     }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) perm_out[i] = perm[i];
+  } else {
+#pragma unroll 8
+    for (int t = 0; t < i0; ++t)
+      if (ipiv[t] == x) s = t;
+  }
+  for (int t = i0; t < i; ++t)
+    if (pl[t] == x) s = t;
+  for (; s >= 0; s = last[s]) x = s;
+  perm[i] = x;
 }
 
 // Bp[i] = B[perm[i]] for every right-hand side
@@ -1202,18 +1224,20 @@ int lu_make_perm(m25_ctx* ctx, int n, const int32_t* ipiv, int32_t* perm) {
     return M25_ERR_VALUE;
   }
   static const bool attr =
-      cudaFuncSetAttribute(perm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
+      cudaFuncSetAttribute(perm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 201 * 1024) ==
           cudaSuccess &&
-      cudaFuncSetAttribute(perm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
+      cudaFuncSetAttribute(perm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 201 * 1024) ==
           cudaSuccess;
   if (!attr) {
     set_error("dense solve: the permutation kernel's shared memory could not be reserved");
     return M25_ERR_CUDA;
   }
-  if ((size_t)n * 2 * sizeof(int) <= 200 * 1024)
-    perm_kernel<true><<<1, 1024, 2 * n * sizeof(int), ctx->stream>>>(n, ipiv, perm);
+  const size_t sm = sizeof(int) * ((size_t)(n + 3) & ~(size_t)3);
+  const unsigned g = (unsigned)((n + kPermThreads - 1) / kPermThreads);
+  if (2 * sm <= 200 * 1024)
+    perm_kernel<true><<<g, kPermThreads, 2 * sm, ctx->stream>>>(n, ipiv, perm);
   else
-    perm_kernel<false><<<1, 1024, n * sizeof(int), ctx->stream>>>(n, ipiv, perm);
+    perm_kernel<false><<<g, kPermThreads, sm, ctx->stream>>>(n, ipiv, perm);
   M25_CHECK_LAUNCH();
   return M25_OK;
 }
@@ -1355,70 +1379,70 @@ __device__ __forceinline__ void dot2_acc(float& s, float& c, float ah, float al,
   c += (ep + es) + fmaf(ah, bl, al * bh);
 }
 
-// Y = Z X for ROWS rows per warp; Zl may be absent (LO false: Z is exact in complex64)
-template <int P, int ROWS, bool LO>
+// Y = Z X, a row per warp; Zl may be absent (LO false: Z is exact in complex64). Each lane has the loads of four
+// column steps (eight of eight bytes) in flight before it uses the first. Bound by the fp32 operations (some 120
+// per element and two columns), then by the matrix's bytes: N = 5943, two columns 168 us (3.4 TB/s; 183 us with one
+// step in flight; packed fp32 operations, 194 - 282 us, lose more in moves than they save).
+template <int P, bool LO>
 __global__ void __launch_bounds__(256) matvec_df_kernel(int n, const zf* __restrict__ Zh, const zf* __restrict__ Zl,
                                                         int64_t ldz, const zf* __restrict__ Xh,
                                                         const zf* __restrict__ Xl, zd* __restrict__ Y) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const int r0 = warp * ROWS;
-  if (r0 >= n) return;
-  float s[ROWS][P][2], cc[ROWS][P][2];
+  constexpr int D = 4;
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (row >= n) return;
+  float s[P][2], cc[P][2];
 #pragma unroll
-  for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-    for (int c = 0; c < P; ++c) s[r][c][0] = s[r][c][1] = cc[r][c][0] = cc[r][c][1] = 0.f;
-  for (int t = lane; t < n; t += 32) {
-    zf xh[P], xl[P];
+  for (int c = 0; c < P; ++c) s[c][0] = s[c][1] = cc[c][0] = cc[c][1] = 0.f;
+  const zf *zhp = Zh + (int64_t)row * ldz, *zlp = LO ? Zl + (int64_t)row * ldz : nullptr;
+  auto step = [&](int t, zf zh, zf zl) {
 #pragma unroll
     for (int c = 0; c < P; ++c) {
-      xh[c] = Xh[(int64_t)t * P + c];
-      xl[c] = Xl[(int64_t)t * P + c];
+      const zf xh = Xh[(int64_t)t * P + c], xl = Xl[(int64_t)t * P + c];
+      dot2_acc(s[c][0], cc[c][0], zh.re, zl.re, xh.re, xl.re);
+      dot2_acc(s[c][0], cc[c][0], zh.im, zl.im, -xh.im, -xl.im);
+      dot2_acc(s[c][1], cc[c][1], zh.re, zl.re, xh.im, xl.im);
+      dot2_acc(s[c][1], cc[c][1], zh.im, zl.im, xh.re, xl.re);
+    }
+  };
+  int t = lane;
+  for (; t + 32 * (D - 1) < n; t += 32 * D) {
+    zf zh[D], zl[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      zh[d] = zhp[t + 32 * d];
+      if (LO) zl[d] = zlp[t + 32 * d];
     }
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      if (r0 + r >= n) break;
-      const zf zh = Zh[(int64_t)(r0 + r) * ldz + t];
-      const zf zl = LO ? Zl[(int64_t)(r0 + r) * ldz + t] : zf();
-#pragma unroll
-      for (int c = 0; c < P; ++c) {
-        dot2_acc(s[r][c][0], cc[r][c][0], zh.re, zl.re, xh[c].re, xl[c].re);
-        dot2_acc(s[r][c][0], cc[r][c][0], zh.im, zl.im, -xh[c].im, -xl[c].im);
-        dot2_acc(s[r][c][1], cc[r][c][1], zh.re, zl.re, xh[c].im, xl[c].im);
-        dot2_acc(s[r][c][1], cc[r][c][1], zh.im, zl.im, xh[c].re, xl[c].re);
-      }
-    }
+    for (int d = 0; d < D; ++d) step(t + 32 * d, zh[d], zl[d]);
   }
+  for (; t < n; t += 32) step(t, zhp[t], LO ? zlp[t] : zf());
 #pragma unroll
-  for (int r = 0; r < ROWS; ++r) {
-    if (r0 + r >= n) break;
+  for (int c = 0; c < P; ++c) {
+    double v[2];
 #pragma unroll
-    for (int c = 0; c < P; ++c) {
-      double v[2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        float a = s[r][c][q], e = cc[r][c][q];
-        for (int o = 16; o; o >>= 1) {
-          const float b = __shfl_down_sync(0xffffffffu, a, o), f = __shfl_down_sync(0xffffffffu, e, o);
-          const float t = a + b, z = t - a;
-          e += f + ((a - (t - z)) + (b - z));
-          a = t;
-        }
-        v[q] = (double)a + (double)e;
+    for (int q = 0; q < 2; ++q) {
+      float a = s[c][q], e = cc[c][q];
+      for (int o = 16; o; o >>= 1) {
+        const float b = __shfl_down_sync(0xffffffffu, a, o), f = __shfl_down_sync(0xffffffffu, e, o);
+        const float u = a + b, z = u - a;
+        e += f + ((a - (u - z)) + (b - z));
+        a = u;
       }
-      if (lane == 0) Y[(int64_t)(r0 + r) * P + c] = zd(v[0], v[1]);
+      v[q] = (double)a + (double)e;
     }
+    if (lane == 0) Y[(int64_t)row * P + c] = zd(v[0], v[1]);
   }
 }
 
 // hi / lo complex64 planes of complex128 values: hi = fp32(x), lo = fp32(x - hi)
+__device__ __forceinline__ void split_z64(zd x, zf& h, zf& l) {
+  const float hr = (float)x.re, hi = (float)x.im;
+  h = zf(hr, hi);
+  l = zf((float)(x.re - (double)hr), (float)(x.im - (double)hi));
+}
 __global__ void split_z64_kernel(int64_t n, const zd* __restrict__ X, zf* __restrict__ Xh, zf* __restrict__ Xl) {
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const zd x = X[e];
-  const float hr = (float)x.re, hi = (float)x.im;
-  Xh[e] = zf(hr, hi);
-  Xl[e] = zf((float)(x.re - (double)hr), (float)(x.im - (double)hi));
+  if (e < n) split_z64(X[e], Xh[e], Xl[e]);
 }
 
 // the same for an n x m block of a matrix (leading dimensions lda / ldb),
@@ -1465,103 +1489,158 @@ __global__ void split_matrix_kernel(const zd* __restrict__ a, int64_t lda, zf* _
   l[r * ldb + c] = zf((float)(x.re - (double)hr), (float)(x.im - (double)hi));
 }
 
-// Y = (Zh + Zl) X in fp64-level accuracy; Xw holds the split X (2 n P complex64)
-void matvec_df(int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, const zd* X, zf* Xw, zd* Y, cudaStream_t st) {
-  const int64_t np = (int64_t)n * P;
-  split_z64_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(np, X, Xw, Xw + np);
-  const zf* Xh = Xw;
-  const zf* Xl = Xw + np;
-#define M25_MVDF(PP, RR)                                                                                       \
-  do {                                                                                                         \
-    const unsigned g = (unsigned)(((size_t)(n + RR - 1) / RR * 32 + 255) / 256);                               \
-    if (Zl)                                                                                                    \
-      matvec_df_kernel<PP, RR, true><<<g, 256, 0, st>>>(n, Zh, Zl, ldz, Xh, Xl, Y);                            \
-    else                                                                                                       \
-      matvec_df_kernel<PP, RR, false><<<g, 256, 0, st>>>(n, Zh, Zl, ldz, Xh, Xl, Y);                           \
-  } while (0)
-  // one row per warp: enough warps in flight to cover the HBM latency of Z
+// Y = (Zh + Zl) X in fp64-level accuracy; Xh + Xl: the split X (n P complex64 each)
+void matvec_df(int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, const zf* Xh, const zf* Xl, zd* Y,
+               cudaStream_t st) {
+  const unsigned g = (unsigned)(((size_t)n * 32 + 255) / 256);
+#define M25_MVDF(PP)                                                                \
+  case PP:                                                                          \
+    if (Zl)                                                                         \
+      matvec_df_kernel<PP, true><<<g, 256, 0, st>>>(n, Zh, Zl, ldz, Xh, Xl, Y);     \
+    else                                                                            \
+      matvec_df_kernel<PP, false><<<g, 256, 0, st>>>(n, Zh, Zl, ldz, Xh, Xl, Y);    \
+    break
   switch (P) {
-    case 1: M25_MVDF(1, 1); break;
-    case 2: M25_MVDF(2, 1); break;
-    case 3: M25_MVDF(3, 1); break;
-    case 4: M25_MVDF(4, 1); break;
-    case 5: M25_MVDF(5, 1); break;
-    case 6: M25_MVDF(6, 1); break;
-    case 7: M25_MVDF(7, 1); break;
-    case 8: M25_MVDF(8, 1); break;
+    M25_MVDF(1);
+    M25_MVDF(2);
+    M25_MVDF(3);
+    M25_MVDF(4);
+    M25_MVDF(5);
+    M25_MVDF(6);
+    M25_MVDF(7);
+    M25_MVDF(8);
     default: break;  // 1 <= P <= 8 is checked by the callers
   }
 #undef M25_MVDF
 }
 
-// h[i][c] = sum_t conj(V_i[t][c]) W[t][c] for i < nvec: one CTA per i
-__global__ void dots_kernel(int n, int P, const zd* __restrict__ V, int64_t vstride, const zd* __restrict__ W,
-                            zd* __restrict__ h) {
-  int i = blockIdx.x;
+// The vector kernels of a GMRES step. Sums over the rows are formed in a
+// fixed order: by kDotSplit CTAs (the dot products) or by the CTAs of 256 elements (the
+// norms), whose partial sums the next kernel adds up. (One CTA per dot product
+// or norm took 32 and 19 us at N = 5943 with two columns, its fp64
+// operations and latencies on one SM; the host then scaled the vector between two synchronisations.)
+constexpr int kDotSplit = 8;
+constexpr int kMaxGmres = 30;  // restart length
+
+// sum of v over the CTA (256 threads), on thread 0
+__device__ __forceinline__ double cta_sum(double v, double* red) {
+  for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < 8; ++w) s += red[w];
+  return s;
+}
+
+// hp[k][i][c] = sum over the rows of part k of conj(V_i[t][c]) W[t][c], i < nvec; grid (nvec, kDotSplit)
+__global__ void __launch_bounds__(256) dots_kernel(int n, int P, const zd* __restrict__ V, int64_t vstride,
+                                                   const zd* __restrict__ W, zd* __restrict__ hp, int hcap) {
+  const int i = blockIdx.x, k = blockIdx.y;
+  const int t0 = (int)((int64_t)n * k / kDotSplit), t1 = (int)((int64_t)n * (k + 1) / kDotSplit);
   const zd* Vi = V + (int64_t)i * vstride;
-  zd acc[8];
-  for (int t = threadIdx.x; t < n; t += blockDim.x)
-    for (int c = 0; c < P; ++c) acc[c] += conj(Vi[(int64_t)t * P + c]) * W[(int64_t)t * P + c];
-  __shared__ double red[32][2];
+  __shared__ double red[8];
   for (int c = 0; c < P; ++c) {
-    double re = acc[c].re, im = acc[c].im;
-    for (int o = 16; o; o >>= 1) {
-      re += __shfl_down_sync(0xffffffffu, re, o);
-      im += __shfl_down_sync(0xffffffffu, im, o);
+    zd acc;
+    for (int t = t0 + threadIdx.x; t < t1; t += 256) {
+      const zd v = Vi[(int64_t)t * P + c], w = W[(int64_t)t * P + c];
+      acc.re = fma(v.re, w.re, fma(v.im, w.im, acc.re));
+      acc.im = fma(v.re, w.im, fma(-v.im, w.re, acc.im));
     }
-    if ((threadIdx.x & 31) == 0) {
-      red[threadIdx.x >> 5][0] = re;
-      red[threadIdx.x >> 5][1] = im;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double a = 0, b = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        a += red[w][0];
-        b += red[w][1];
-      }
-      h[i * P + c] = zd(a, b);
-    }
-    __syncthreads();
+    const double re = cta_sum(acc.re, red), im = cta_sum(acc.im, red);
+    if (threadIdx.x == 0) hp[(size_t)k * hcap + i * P + c] = zd(re, im);
   }
 }
 
-// W[t][c] -= sum_{i < nvec} V_i[t][c] h[i][c]
-__global__ void orth_update_kernel(int n, int P, int nvec, const zd* __restrict__ V, int64_t vstride,
-                                   const zd* __restrict__ h, zd* __restrict__ W) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (int64_t)n * P) return;
-  int c = int(e % P);
-  zd s = W[e];
-  for (int i = 0; i < nvec; ++i) s -= V[(int64_t)i * vstride + e] * h[i * P + c];
-  W[e] = s;
-}
-
-// per-column squared 2-norms: out[c] (one CTA)
-__global__ void norms_kernel(int n, int P, const zd* __restrict__ W, double* __restrict__ out) {
-  double acc[8] = {};
-  for (int t = threadIdx.x; t < n; t += blockDim.x)
-    for (int c = 0; c < P; ++c) acc[c] += norm2(W[(int64_t)t * P + c]);
-  __shared__ double red[32];
+// part[b][c] = the squared 2-norm of CTA b's elements of column c (one element per thread)
+__device__ __forceinline__ void norm_parts(int64_t e, int64_t np, int P, zd v, double* red, double* part) {
+  const double q = e < np ? norm2(v) : 0.0;
+  const int col = (int)(e % P);
   for (int c = 0; c < P; ++c) {
-    double v = acc[c];
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-      out[c] = s;
-    }
-    __syncthreads();
+    const double s = cta_sum(c == col ? q : 0.0, red);
+    if (threadIdx.x == 0) part[(size_t)blockIdx.x * P + c] = s;
   }
 }
 
-// out[t][c] = in[t][c] * s[c] (s complex per column)
-__global__ void col_scale_kernel(int64_t n, int P, const zd* __restrict__ in, const zd* __restrict__ s,
-                                 zd* __restrict__ out) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < n * P) out[e] = in[e] * s[e % P];
+// W[t][c] -= sum_{i < nvec} V_i[t][c] h[i][c], h the sum of the parts hp, which CTA 0 also writes to hout; with
+// part: the partial norms of the new W, and *mx = 0 for col_scale_kernel
+__global__ void __launch_bounds__(256) orth_update_kernel(int n, int P, int nvec, const zd* __restrict__ V,
+                                                          int64_t vstride, const zd* __restrict__ hp, int hcap,
+                                                          zd* __restrict__ hout, zd* __restrict__ W,
+                                                          double* __restrict__ part,
+                                                          unsigned long long* __restrict__ mx) {
+  __shared__ zd h[kMaxGmres * 8];
+  __shared__ double red[8];
+  for (int j = threadIdx.x; j < nvec * P; j += 256) {
+    zd a;
+    for (int k = 0; k < kDotSplit; ++k) a += hp[(size_t)k * hcap + j];
+    h[j] = a;
+    if (blockIdx.x == 0) hout[j] = a;
+  }
+  if (mx && blockIdx.x == 0 && threadIdx.x == 0) *mx = 0;
+  __syncthreads();
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x, np = (int64_t)n * P;
+  zd v;
+  if (e < np) {
+    const int c = int(e % P);
+    v = W[e];
+    for (int i = 0; i < nvec; ++i) v = fnma(v, V[(int64_t)i * vstride + e], h[i * P + c]);
+    W[e] = v;
+  }
+  if (part) norm_parts(e, np, P, v, red, part);
+}
+
+// R = B - W (W = Z X), the partial norms of R, X and B, and *mx = 0
+__global__ void __launch_bounds__(256) residual_kernel(int n, int P, const zd* __restrict__ B,
+                                                       const zd* __restrict__ W, const zd* __restrict__ X,
+                                                       zd* __restrict__ R, double* __restrict__ pr,
+                                                       double* __restrict__ px, double* __restrict__ pb,
+                                                       unsigned long long* __restrict__ mx) {
+  __shared__ double red[8];
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x, np = (int64_t)n * P;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *mx = 0;
+  zd b, r, x;
+  if (e < np) {
+    b = B[e];
+    x = X[e];
+    r = b - W[e];
+    R[e] = r;
+  }
+  norm_parts(e, np, P, r, red, pr);
+  norm_parts(e, np, P, x, red, px);
+  norm_parts(e, np, P, b, red, pb);
+}
+
+// out = in / |in| per column (0 for a zero column) from the partial norms; *mx
+// = the largest |re| + |im| of out (the preconditioner's scale) and, from
+// CTA 0, norms[c] = |in|
+__global__ void __launch_bounds__(256) col_scale_kernel(int64_t np, int P, const zd* __restrict__ in, int nparts,
+                                                        const double* __restrict__ part, zd* __restrict__ out,
+                                                        double* __restrict__ norms,
+                                                        unsigned long long* __restrict__ mx) {
+  __shared__ double inv[8];
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < P; c += 8) {
+    double s = 0;
+    for (int b = lane; b < nparts; b += 32) s += part[(size_t)b * P + c];
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      const double r = sqrt(s);
+      inv[c] = r > 0 ? 1.0 / r : 0.0;
+      if (blockIdx.x == 0) norms[c] = r;
+    }
+  }
+  __syncthreads();
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  double m = 0;
+  if (e < np) {
+    const zd v = in[e] * inv[e % P];
+    out[e] = v;
+    m = cabs1(v);
+  }
+  for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) atomicMax(mx, (unsigned long long)__double_as_longlong(m));  // m >= 0: bit order = value order
 }
 
 // X[t][c] += sum_i V_i[t][c] y[i][c]
@@ -1580,11 +1659,17 @@ __global__ void combine_kernel(int n, int P, int nvec, const zd* __restrict__ V,
 __global__ void rownorm_kernel(int n, const zf* __restrict__ Z, int64_t ldz, unsigned long long* __restrict__ out) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= n) return;
+  const zf* row = Z + (int64_t)warp * ldz;
   float s = 0;
-  for (int t = lane; t < n; t += 32) {
-    const zf z = Z[(int64_t)warp * ldz + t];
-    s += sqrtf(z.re * z.re + z.im * z.im);
+  int t = lane;
+  for (; t + 7 * 32 < n; t += 8 * 32) {
+    zf z[8];
+#pragma unroll
+    for (int d = 0; d < 8; ++d) z[d] = row[t + 32 * d];
+#pragma unroll
+    for (int d = 0; d < 8; ++d) s += sqrtf(z[d].re * z[d].re + z[d].im * z[d].im);
   }
+  for (; t < n; t += 32) s += sqrtf(row[t].re * row[t].re + row[t].im * row[t].im);
   for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if (lane == 0) atomicMax(out, (unsigned long long)__double_as_longlong((double)s));  // s >= 0: bit order = value order
 }
@@ -1596,24 +1681,23 @@ __global__ void z64_to_z32_scaled(int64_t n, const zd* __restrict__ a, const dou
   const double s = *sp > 0 ? 1.0 / *sp : 1.0;
   if (e < n) o[e] = zf(float(a[e].re * s), float(a[e].im * s));
 }
+// the second with the hi / lo planes of o for the product that follows
 __global__ void z32_to_z64_scaled(int64_t n, const zf* __restrict__ a, const double* __restrict__ sp,
-                                  zd* __restrict__ o) {
+                                  zd* __restrict__ o, zf* __restrict__ oh, zf* __restrict__ ol) {
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
   const double s = *sp > 0 ? *sp : 1.0;
-  if (e < n) o[e] = zd(double(a[e].re) * s, double(a[e].im) * s);
+  const zd x(double(a[e].re) * s, double(a[e].im) * s);
+  o[e] = x;
+  split_z64(x, oh[e], ol[e]);
 }
-__global__ void maxabs_kernel(int64_t n, const zd* __restrict__ a, double* __restrict__ out) {
-  double m = 0;
-  for (int64_t e = threadIdx.x; e < n; e += blockDim.x) m = fmax(m, cabs1(a[e]));
-  __shared__ double red[32];
-  for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, red[w]);
-    *out = r;
-  }
+// *out = max |re| + |im| (*out starts at 0)
+__global__ void __launch_bounds__(256) maxabs_kernel(int64_t n, const zd* __restrict__ a,
+                                                     unsigned long long* __restrict__ out) {
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  double m = e < n ? cabs1(a[e]) : 0.0;
+  for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
 }
 
 // Restarted flexible GMRES in fp64 on Z x = B, right-preconditioned by the
@@ -1629,10 +1713,12 @@ __global__ void maxabs_kernel(int64_t n, const zd* __restrict__ a, double* __res
 int refine(m25_ctx* ctx, int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, const zf* LU, int64_t ldlu,
            const int32_t* ipiv, const zd* B, zd* X, double tol, int max_iter, int* steps) {
   cudaStream_t st = ctx->stream;
-  const int m = std::min(30, std::max(1, max_iter));
+  const int m = std::min(kMaxGmres, std::max(1, max_iter));
   const size_t np = (size_t)n * P;
-  int rc = ctx->Rw.ensure(sizeof(zd) * np * (2 * m + 3) + sizeof(zf) * np * 4 + sizeof(double) * 64 +
-                          sizeof(zd) * (size_t)(m + 2) * P * 2 + sizeof(int32_t) * n);
+  const unsigned g1 = (unsigned)((np + 255) / 256);
+  const int hcap = m * P;
+  int rc = ctx->Rw.ensure(sizeof(zd) * np * (2 * m + 3) + sizeof(zf) * np * 4 + sizeof(double) * (64 + 3 * (size_t)g1 * P) +
+                          sizeof(zd) * (size_t)hcap * (kDotSplit + 3) + sizeof(int32_t) * n);
   if (rc) return rc;
   zd* V = ctx->Rw.as<zd>();           // (m+1) Arnoldi vectors
   zd* Zp = V + np * (m + 1);          // (m) preconditioned directions
@@ -1640,31 +1726,26 @@ int refine(m25_ctx* ctx, int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, 
   zd* R = W + np;                     // residual
   zf* r32 = reinterpret_cast<zf*>(R + np);
   zf* d32 = r32 + np;
-  double* dsc = reinterpret_cast<double*>(d32 + np);  // scalars
-  zd* hdev = reinterpret_cast<zd*>(dsc + 64);
-  zd* ydev = hdev + (size_t)(m + 2) * P;
-  zf* xsplit = reinterpret_cast<zf*>(ydev + (size_t)(m + 2) * P);  // (2 n P) hi / lo planes of a vector
-  int32_t* perm = reinterpret_cast<int32_t*>(xsplit + 2 * np);       // row permutation of the LU
-  const unsigned g1 = (unsigned)((np + 255) / 256);
+  zf* xh = d32 + np;                                        // hi / lo planes of a vector
+  zf* xl = xh + np;
+  zd* hp = reinterpret_cast<zd*>(xl + np);                  // partial dot products
+  zd* ydev = hp + (size_t)hcap * kDotSplit;
+  zd* hout = ydev + hcap;                                   // the step's results for the host: two passes of dot products, norms
+  double* wnorm = reinterpret_cast<double*>(hout + 2 * (size_t)hcap);
+  double* pscale = wnorm + 48;
+  unsigned long long* mx = reinterpret_cast<unsigned long long*>(pscale);
+  double* parts = wnorm + 64;                               // partial norms: 3 x (g1, P)
+  const size_t nparts = (size_t)g1 * P;
+  int32_t* perm = reinterpret_cast<int32_t*>(parts + 3 * nparts);  // row permutation of the LU
   const unsigned gw = (unsigned)(((size_t)n * 32 + 255) / 256);
   StageTimer tm(ctx, ST_REFINE);
   // out = (LU32)^-1 in, in fp32 with the input scaled to O(1) by its
-  // largest entry (kept on the device: no host round trip)
-  double* pscale = dsc + 48;
+  // largest entry *mx (kept on the device: no host round trip), and out's planes
   auto precond = [&](const zd* in, zd* out) -> int {
-    maxabs_kernel<<<1, 1024, 0, st>>>((int64_t)np, in, pscale);
     z64_to_z32_scaled<<<g1, 256, 0, st>>>((int64_t)np, in, pscale, r32);
     int r = lu_solve_wave<float, float>(ctx, LU, ldlu, n, ipiv, r32, P, d32, perm);
     if (r) return r;
-    z32_to_z64_scaled<<<g1, 256, 0, st>>>((int64_t)np, d32, pscale, out);
-    return M25_OK;
-  };
-  auto col_norms = [&](const zd* v, std::vector<double>& out) -> int {
-    norms_kernel<<<1, 1024, 0, st>>>(n, P, v, dsc);
-    out.assign(P, 0.0);
-    M25_CUDA(cudaMemcpyAsync(out.data(), dsc, sizeof(double) * P, cudaMemcpyDeviceToHost, st));
-    M25_CUDA(cudaStreamSynchronize(st));
-    for (auto& x : out) x = sqrt(x);
+    z32_to_z64_scaled<<<g1, 256, 0, st>>>((int64_t)np, d32, pscale, out, xh, xl);
     return M25_OK;
   };
   auto set_col_scalars = [&](const std::vector<zd>& v) -> int {
@@ -1672,29 +1753,32 @@ int refine(m25_ctx* ctx, int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, 
     return M25_OK;
   };
   if ((rc = lu_make_perm(ctx, n, ipiv, perm))) return rc;
-  std::vector<double> bn, rn, xn;
-  if ((rc = col_norms(B, bn))) return rc;
-  double znorm = 0;
-  {
-    unsigned long long* zb = reinterpret_cast<unsigned long long*>(dsc + 32);
-    M25_CUDA(cudaMemsetAsync(zb, 0, sizeof(unsigned long long), st));
-    rownorm_kernel<<<gw, 256, 0, st>>>(n, Zh, ldz, zb);
-    M25_CUDA(cudaMemcpyAsync(&znorm, zb, sizeof(double), cudaMemcpyDeviceToHost, st));
-    M25_CUDA(cudaStreamSynchronize(st));
-  }
+  unsigned long long* zb = mx + 1;
+  M25_CUDA(cudaMemsetAsync(mx, 0, 2 * sizeof(unsigned long long), st));
+  rownorm_kernel<<<gw, 256, 0, st>>>(n, Zh, ldz, zb);
   // start from the fp32 solution x0 = M^-1 B
+  maxabs_kernel<<<g1, 256, 0, st>>>((int64_t)np, B, mx);
   if ((rc = precond(B, X))) return rc;
   int total = 0;
-  double prev_worst = INFINITY;
+  double prev_worst = INFINITY, znorm = 0;
+  std::vector<double> rn(P), xn(P), bn(P), hparts(64 + 3 * nparts), step(4 * (size_t)hcap + P);
   std::vector<zd> hh((size_t)(m + 2) * P), H((size_t)(m + 1) * m * P), g((size_t)(m + 1) * P), cs(m * P), sn(m * P);
   for (int outer = 0; outer < 50; ++outer) {
     // R = B - Z X
-    matvec_df(n, P, Zh, Zl, ldz, X, xsplit, W, st);
-    M25_CUDA(cudaMemcpyAsync(R, B, np * sizeof(zd), cudaMemcpyDeviceToDevice, st));
-    if ((rc = set_col_scalars(std::vector<zd>(P, zd(-1.0))))) return rc;
-    combine_kernel<<<g1, 256, 0, st>>>(n, P, 1, W, 0, ydev, R);
-    if ((rc = col_norms(R, rn))) return rc;
-    if ((rc = col_norms(X, xn))) return rc;
+    if (outer) split_z64_kernel<<<g1, 256, 0, st>>>((int64_t)np, X, xh, xl);
+    matvec_df(n, P, Zh, Zl, ldz, xh, xl, W, st);
+    residual_kernel<<<g1, 256, 0, st>>>(n, P, B, W, X, R, parts, parts + nparts, parts + 2 * nparts, mx);
+    M25_CUDA(cudaMemcpyAsync(hparts.data(), wnorm, sizeof(double) * hparts.size(), cudaMemcpyDeviceToHost, st));
+    M25_CUDA(cudaStreamSynchronize(st));
+    znorm = hparts[49];  // zb
+    for (int c = 0; c < P; ++c) {
+      double q[3] = {};
+      for (int k = 0; k < 3; ++k)
+        for (unsigned b = 0; b < g1; ++b) q[k] += hparts[64 + k * nparts + (size_t)b * P + c];
+      rn[c] = sqrt(q[0]);
+      xn[c] = sqrt(q[1]);
+      bn[c] = sqrt(q[2]);
+    }
     double worst = 0;
     std::vector<double> target(P);
     bool finite = std::isfinite(znorm);
@@ -1721,37 +1805,26 @@ int refine(m25_ctx* ctx, int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, 
     }
     prev_worst = worst;
     // V0 = R / |R|
-    {
-      std::vector<zd> inv(P);
-      for (int c = 0; c < P; ++c) inv[c] = zd(rn[c] > 0 ? 1.0 / rn[c] : 0.0);
-      if ((rc = set_col_scalars(inv))) return rc;
-      col_scale_kernel<<<g1, 256, 0, st>>>((int64_t)n, P, R, ydev, V);
-    }
+    col_scale_kernel<<<g1, 256, 0, st>>>((int64_t)np, P, R, (int)g1, parts, V, wnorm, mx);
     std::fill(g.begin(), g.end(), zd(0.0));
     for (int c = 0; c < P; ++c) g[c] = zd(rn[c]);
     int k = 0;
     for (; k < m && total < max_iter; ++k, ++total) {
       zd* zk = Zp + np * k;
       if ((rc = precond(V + np * k, zk))) return rc;
-      matvec_df(n, P, Zh, Zl, ldz, zk, xsplit, W, st);
-      // classical Gram-Schmidt, twice
-      std::fill(hh.begin(), hh.end(), zd(0.0));
+      matvec_df(n, P, Zh, Zl, ldz, xh, xl, W, st);
+      // classical Gram-Schmidt, twice; then V_{k+1} = W / |W|
       for (int pass = 0; pass < 2; ++pass) {
-        dots_kernel<<<k + 1, 256, 0, st>>>(n, P, V, (int64_t)np, W, hdev);
-        orth_update_kernel<<<g1, 256, 0, st>>>(n, P, k + 1, V, (int64_t)np, hdev, W);
-        std::vector<zd> tmp((size_t)(k + 1) * P);
-        M25_CUDA(cudaMemcpyAsync(tmp.data(), hdev, sizeof(zd) * tmp.size(), cudaMemcpyDeviceToHost, st));
-        M25_CUDA(cudaStreamSynchronize(st));
-        for (size_t i = 0; i < tmp.size(); ++i) hh[i] += tmp[i];
+        dots_kernel<<<dim3(k + 1, kDotSplit), 256, 0, st>>>(n, P, V, (int64_t)np, W, hp, hcap);
+        orth_update_kernel<<<g1, 256, 0, st>>>(n, P, k + 1, V, (int64_t)np, hp, hcap, hout + (size_t)pass * hcap, W,
+                                               pass ? parts : nullptr, pass ? mx : nullptr);
       }
-      std::vector<double> wn;
-      if ((rc = col_norms(W, wn))) return rc;
-      {
-        std::vector<zd> inv(P);
-        for (int c = 0; c < P; ++c) inv[c] = zd(wn[c] > 0 ? 1.0 / wn[c] : 0.0);
-        if ((rc = set_col_scalars(inv))) return rc;
-        col_scale_kernel<<<g1, 256, 0, st>>>((int64_t)n, P, W, ydev, V + np * (k + 1));
-      }
+      col_scale_kernel<<<g1, 256, 0, st>>>((int64_t)np, P, W, (int)g1, parts, V + np * (k + 1), wnorm, mx);
+      M25_CUDA(cudaMemcpyAsync(step.data(), hout, sizeof(double) * step.size(), cudaMemcpyDeviceToHost, st));
+      M25_CUDA(cudaStreamSynchronize(st));
+      for (int i = 0; i < (k + 1) * P; ++i)
+        hh[i] = zd(step[2 * i], step[2 * i + 1]) + zd(step[2 * (hcap + i)], step[2 * (hcap + i) + 1]);
+      const double* wn = step.data() + 4 * (size_t)hcap;
       bool done = true;
       for (int c = 0; c < P; ++c) {
         // column k of the Hessenberg matrix, rotated by the previous Givens rotations

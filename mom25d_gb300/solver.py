@@ -926,7 +926,7 @@ class Solver:
             try:  # each worker sets up its own context's device data
                 sol = self._sibling(w)
                 if tun is not None:
-                    tun.apply(sol.ctx, self.mesh.n_unknowns)
+                    tun.apply(sol.ctx, self.mesh.n_unknowns, alone=workers == 1)
                 sol.geometry()
                 sol.port_data()
             except Exception as exc:  # noqa: BLE001 - re-raised below in the caller's thread
