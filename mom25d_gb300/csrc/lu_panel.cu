@@ -15,12 +15,18 @@
 //    end, so the row at position k0 + j need not be sent around;
 //  - narrow strips: the rank-1 updates of a step cost W / 2 columns on
 //    average, and the products between strips go to the whole GPU.
+//  - complex128: two warps without rows do the division of the reciprocal
+//    pivot and send the candidate's row, while the warps with rows run the
+//    multiply-adds of the step before (kAhead below).
 // Measured on GB300 (one factorisation alone, sum over its panels):
-//   complex128, N = 546 / 1085 / 2434 / 5943: 2.2 / 4.4 / 10.4 / 32 ms (7.95 / 20.0 / 53.0 / 96.6 ms for
-//   64-column panels in shared memory, with the row k0 + j sent around and both divisions on the chain)
-//   complex64, N = 1085 / 5943: 2.0 / 11.9 ms (2.5 / 21.1 ms, and 0.2 / 2.1 ms for the products between
+//   complex128, N = 546 / 1085 / 2434 / 5943: 1.75 / 3.5 / 8.6 / 28.4 ms (1.9 / 3.9 / 9.4 / 30.6 ms with every step
+//   finished before the next one's search; 7.95 / 20.0 / 53.0 / 96.6 ms for 64-column panels in shared memory, with
+//   the row k0 + j sent around and both divisions on the chain)
+//   complex64, N = 1085 / 5943: 1.6 / 10.1 ms (2.5 / 21.1 ms, and 0.2 / 2.1 ms for the products between
 //   the two panels of a block)
-// A column step of complex64 takes 1.25 us, of which 0.45 us are the exchange's flight.
+// A column step of complex64 takes about 1 us, of which 0.45 us are the exchange's
+// flight; one of complex128 2.5 us at 64 rows per CTA: search 0.35, the candidate's staging 0.4, the multiply-adds
+// 1.0, the wait 0.2, multiplier and next column 0.5.
 #include <algorithm>
 #include <string>
 
@@ -139,7 +145,9 @@ __device__ __forceinline__ unsigned long long warp_best(unsigned long long key, 
 // bits of v + 1 (ordered as v for v >= 0), 0 for a NaN, which is never chosen
 __device__ __forceinline__ unsigned val_key(float v) { return v >= 0.f ? __float_as_uint(v) + 1u : 0u; }
 __device__ __forceinline__ unsigned long long val_key(double v) {
-  return v >= 0.0 ? (unsigned long long)__double_as_longlong(v) + 1ull : 0ull;
+  // a sum of magnitudes: not negative; the comparison as integers (a NaN's bits exceed infinity's), off the fp64 pipe
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return b <= 0x7ff0000000000000ull ? b + 1ull : 0ull;
 }
 template <class T>
 using KeyOf = decltype(val_key(T(0)));
@@ -158,10 +166,11 @@ struct StripRow<double> {
   __device__ __forceinline__ cx<double> get(int i) const { return x[i]; }
   __device__ __forceinline__ void set(int i, cx<double> v) { x[i] = v; }
   // chunk k (16 bytes) of the row as it is sent
-  __device__ __forceinline__ uint4 chunk(int k) const {
-    return make_uint4((unsigned)__double2loint(x[k].re), (unsigned)__double2hiint(x[k].re),
-                      (unsigned)__double2loint(x[k].im), (unsigned)__double2hiint(x[k].im));
+  static __device__ __forceinline__ uint4 pack(cx<double> v) {
+    return make_uint4((unsigned)__double2loint(v.re), (unsigned)__double2hiint(v.re), (unsigned)__double2loint(v.im),
+                      (unsigned)__double2hiint(v.im));
   }
+  __device__ __forceinline__ uint4 chunk(int k) const { return pack(x[k]); }
   static __device__ __forceinline__ cx<double> sent(const uint4* u, int c) {
     return *reinterpret_cast<const cx<double>*>(u + c);
   }
@@ -241,14 +250,23 @@ struct StripRow<float> {
   }
 };
 
+// complex128: a step updates only the next column before its pivot is
+// searched; the others follow while the exchange is under way (up to 3800
+// cycles of fp64 multiply-adds a step, half that on average). The candidate's
+// row, whose other columns are a step behind in its registers, is brought up
+// to date by half a warp, a column per lane, on its way out.
+template <class T>
+constexpr bool kAhead = sizeof(T) == 8;
+
 // What the cluster's CTAs send one another, at the start of the dynamic shared
 // memory: per column parity the barrier, every CTA's candidate and its row.
 template <class T, int CL>
 struct StripShared {
   static constexpr int kCh = strip_w<T>() * (int)sizeof(cx<T>) / 16;  // 16-byte chunks of a row
+  static constexpr int kBuf = kAhead<T> ? 3 : 2;  // a pivot row is read until the next one has been sent
   uint64_t colbar[2];
   StripCand<T> cand[2][CL];
-  uint4 crow[2][CL][kCh];
+  uint4 crow[kBuf][CL][kCh];
   uint4 stage[kCh];  // this CTA's candidate row; behind crow, see StripRow<float>::update
 };
 
@@ -280,9 +298,11 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
   cx<T>* mv = S + ((size_t)R * LD + 1) / 2 * 2;                // (<= 2 W, nother) moved rows
   __shared__ Key wkey[2][kStripThreads / 32];
   __shared__ unsigned wpos[2][kStripThreads / 32];
+  __shared__ cx<T> wval[2][kStripThreads / 32];
   __shared__ int fpos[kStripThreads];
   __shared__ int mlist[2 * W];
   __shared__ int nmoved, fail_s;
+  __shared__ cx<T> stage_l;
   volatile int* fail = &fail_s;
   if (tid == 0) {
     bar_init(&sh.colbar[0], 1);
@@ -320,6 +340,43 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
   unsigned pos = (unsigned)row(tid);
   bool live = tid < Rq;  // not yet a pivot row
   cl_sync();             // every CTA runs, with its barriers set up, before the first push
+  cx<T> lp;                      // kAhead: this row's multiplier of the step before,
+  const uint4* pu = nullptr;     // its pivot row,
+  bool pend = false;             // and whether the columns after the next are still to be updated with them
+  int buf = 0;
+  const int hw = kAhead<T> && blockDim.x >= (unsigned)R + 64 ? nwarp - 2 : -1;  // the first of two warps without rows
+  // the staged row to all CTAs, a half warp for half of them; l: kAhead, its multiplier of the step before
+  auto put_row = [&](int j, int par, cx<T> l) {
+    const int c = lane & 15;
+    if (c < j / kVec) return;
+    uint4 v = sh.stage[c];
+    if constexpr (kAhead<T>)
+      if (pend && c > j) v = StripRow<T>::pack(fnma(StripRow<T>::sent(sh.stage, c), l, StripRow<T>::sent(pu, c)));
+    const uint32_t oc = off(&sh.crow[buf][q][c]), ob = off(&sh.colbar[par]);
+#pragma unroll
+    for (int i = 0; i < CL / 2; ++i) cl_put(peer[i] + oc, v, peer[i] + ob);
+  };
+  // the candidate with the reciprocal pivot, both parts in one division: the even lanes the real, the odd ones the
+  // imaginary part
+  auto reciprocal = [&](cx<T> pv) {
+    const T m2 = pv.re * pv.re + pv.im * pv.im;
+    return ((lane & 1) ? -pv.im : pv.re) / m2;
+  };
+  auto put_candidate = [&](T half, Key key, unsigned p, int par) {
+    union {
+      uint4 v[sizeof(StripCand<T>) / 16];
+      StripCand<T> c;
+    } u;
+    u.c.key = key;
+    u.c.pos = (int)p;
+    u.c.rre = __shfl_sync(~0u, half, 0);
+    u.c.rim = __shfl_sync(~0u, half, 1);
+    if (lane < CL) {
+      const uint32_t b = cpeer + off(&sh.colbar[par]), d = cpeer + off(&sh.cand[par][q]);
+#pragma unroll
+      for (int i = 0; i < (int)sizeof(StripCand<T>) / 16; ++i) cl_put(d + 16 * i, u.v[i], b);
+    }
+  };
 #pragma unroll 1
   for (int jb = 0; jb < w; jb += kGrp) {
 #pragma unroll
@@ -337,47 +394,45 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
         wkey[par][warp] = key;
         wpos[par][warp] = p;
       }
+      if (hw >= 0 && live && key != 0 && pos == p) wval[par][warp] = x.get(jj);
       __syncthreads();
       key = lane < nwarp ? wkey[par][lane] : Key(0);
       p = key ? wpos[par][lane] : ~0u;
       key = warp_best(key, p);
-      // its owner stages the row's remaining columns, and the owner's warp
-      // sends them with the candidate to all CTAs
+      // its owner stages the row's remaining columns; the owner's warp, or the
+      // warps without rows, send them and the candidate to all CTAs
       const bool own = live && key != 0 && pos == p;
       const unsigned ob = __ballot_sync(~0u, own);
-      if (key ? ob != 0 : warp == 0) {
-        if (own)
+      const bool owns = key ? ob != 0 : warp == 0;  // the warp whose lane has the candidate
+      if (owns && own) {
 #pragma unroll
-          for (int k = 0; k < Sh::kCh; ++k)
-            if (k >= jj / kVec && jb / kVec + k < Sh::kCh) sh.stage[jb / kVec + k] = x.chunk(k);
-        // the reciprocal pivot, both parts in one division: the even lanes the real, the odd ones the imaginary part
-        const int lo = key ? __ffs(ob) - 1 : 0;
-        const cx<T> xj = x.get(jj);
-        const cx<T> pv(__shfl_sync(~0u, xj.re, lo), __shfl_sync(~0u, xj.im, lo));
-        __syncwarp();
-        const int c = lane & 15;
-        if (c >= j / kVec) {
-          const uint4 v = sh.stage[c];
-          const uint32_t oc = off(&sh.crow[par][q][c]), ob2 = off(&sh.colbar[par]);
-#pragma unroll
-          for (int i = 0; i < CL / 2; ++i) cl_put(peer[i] + oc, v, peer[i] + ob2);
-        }
-        const T m2 = pv.re * pv.re + pv.im * pv.im;
-        const T half = ((lane & 1) ? -pv.im : pv.re) / m2;
-        union {
-          uint4 v[sizeof(StripCand<T>) / 16];
-          StripCand<T> c;
-        } u;
-        u.c.key = key;
-        u.c.pos = (int)p;
-        u.c.rre = __shfl_sync(~0u, half, 0);
-        u.c.rim = __shfl_sync(~0u, half, 1);
-        if (lane < CL) {
-          const uint32_t b = cpeer + off(&sh.colbar[par]), d = cpeer + off(&sh.cand[par][q]);
-#pragma unroll
-          for (int i = 0; i < (int)sizeof(StripCand<T>) / 16; ++i) cl_put(d + 16 * i, u.v[i], b);
-        }
+        for (int k = 0; k < Sh::kCh; ++k)
+          if (k >= jj / kVec && jb / kVec + k < Sh::kCh) sh.stage[jb / kVec + k] = x.chunk(k);
+        if (hw >= 0) stage_l = lp;
       }
+      if (hw < 0) {
+        if (owns) {
+          const int lo = key ? __ffs(ob) - 1 : 0;
+          const cx<T> xj = x.get(jj);
+          const cx<T> pv(__shfl_sync(~0u, xj.re, lo), __shfl_sync(~0u, xj.im, lo));
+          cx<T> l;
+          if (kAhead<T>) l = cx<T>(__shfl_sync(~0u, lp.re, lo), __shfl_sync(~0u, lp.im, lo));
+          __syncwarp();
+          put_row(j, par, l);
+          put_candidate(reciprocal(pv), key, p, par);
+        }
+      } else if (warp == hw) {
+        const unsigned wb = __ballot_sync(~0u, lane < nwarp && wpos[par][lane < nwarp ? lane : 0] == p);
+        const cx<T> pv = wval[par][key ? __ffs(wb) - 1 : 0];
+        put_candidate(reciprocal(pv), key, p, par);
+      } else if (warp == hw + 1) {
+        if (key) asm volatile("bar.sync 1, 64;\n" ::: "memory");
+        put_row(j, par, stage_l);
+      } else if (key && owns) {
+        asm volatile("bar.arrive 1, 64;\n" ::: "memory");
+      }
+      if constexpr (kAhead<T>)
+        if (pend && (hw < 0 || warp < hw)) x.update(jj + 1, jb, lp, pu + jb);
       bar_wait(&sh.colbar[par], (j >> 1) & 1, fail);
       // the pivot among the CTAs' candidates (each warp for itself)
       key = lane < CL ? sh.cand[par][lane < CL ? lane : 0].key : Key(0);
@@ -399,6 +454,8 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
             S[tid * LD + j] = x.get(jj);
           }
         }
+        pend = false;
+        buf = buf + 1 == Sh::kBuf ? 0 : buf + 1;
         continue;
       }
       const int src = __ffs(__ballot_sync(~0u, mine == p)) - 1;  // positions are distinct: one CTA
@@ -412,12 +469,20 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
           const cx<T> rp(sh.cand[par][src].rre, sh.cand[par][src].rim);
           const cx<T> l = x.get(jj) * rp;
           S[tid * LD + j] = l;
-          x.update(jj + 1, jb, l, &sh.crow[par][src][jb / kVec]);
+          if constexpr (kAhead<T>) {
+            lp = l;
+            if (j + 1 < W) x.set(jj + 1, fnma(x.get(jj + 1), l, StripRow<T>::sent(sh.crow[buf][src], j + 1)));
+          } else {
+            x.update(jj + 1, jb, l, &sh.crow[buf][src][jb / kVec]);
+          }
         }
       }
       // the pivot row's columns from j on, final now, from the exchange to its place (its owner's warp)
       if (src == q && ob != 0 && lane >= j && lane < W)
-        S[(warp * 32 + __ffs(ob) - 1) * LD + lane] = StripRow<T>::sent(sh.crow[par][src], lane);
+        S[(warp * 32 + __ffs(ob) - 1) * LD + lane] = StripRow<T>::sent(sh.crow[buf][src], lane);
+      pend = true;
+      pu = sh.crow[buf][src];
+      buf = buf + 1 == Sh::kBuf ? 0 : buf + 1;
     }
     x.shift();
   }
@@ -602,7 +667,8 @@ cudaError_t launch_strip(const StripArgs<T>& a, cudaStream_t st) {
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(CL);
-  cfg.blockDim = dim3(std::max(64, (a.rows_per_cta + 31) / 32 * 32));
+  const int rows = (a.rows_per_cta + 31) / 32 * 32;
+  cfg.blockDim = dim3(kAhead<T> && rows + 64 <= kStripThreads ? rows + 64 : std::max(64, rows));
   cfg.dynamicSmemBytes = strip_smem<T, CL>(a.rows_per_cta, a.blk1 - a.blk0 - a.w);
   cfg.stream = st;
   cfg.attrs = at;
