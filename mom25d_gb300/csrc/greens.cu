@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "m25_internal.h"
+#include "m25_lu.h"
 
 namespace m25 {
 
@@ -437,6 +438,19 @@ __device__ __forceinline__ zd j0_arc(double r, double rs, zd k, const double* __
   return {fma(q1, dr, fma(-t, b1, a.x)), q1 * di};
 }
 
+// The learned remainder's network inputs of n radii at frequency f.
+struct SurFeatures {
+  int n;  // 0: none
+  const double* rho;
+  double a, rho_ref, f, fmin, fmax;
+  float* X;  // (n, 2)
+};
+__device__ void sur_features(const SurFeatures& s, int i) {
+  if (i >= s.n) return;
+  s.X[2 * i] = (float)(2.0 * log1p(s.rho[i] / s.a) / log1p(s.rho_ref / s.a) - 1.0);
+  s.X[2 * i + 1] = (float)(2.0 * (s.f - s.fmin) / (s.fmax - s.fmin) - 1.0);
+}
+
 // The spectral kernels g[(m*L + i)*L + j] at every path node, in one launch:
 // nodes q < nkc of the lifted arc into gc, the next nkr of the real axis into
 // gr, and (layered stacks) one more node at kbig into gbig for the leading
@@ -444,14 +458,21 @@ __device__ __forceinline__ zd j0_arc(double r, double rs, zd k, const double* __
 // through the layers, on one lane (one slab) or two (layered_spectral); small
 // CTAs spread the nodes over the SMs. 7176 nodes of two layers: 48 us (one lane a
 // node and a division for every use of 1 / u^2 and 1 / k^2: 82 us).
-// The CTAs from nb on fill the J0 tables of the integral.
+// The CTAs from nb on fill the J0 tables of the integral and, last, the
+// network's inputs.
 __global__ void __launch_bounds__(64) spectral_g_kernel(const StackDev* __restrict__ Sp, int nkc,
                                                         const double* __restrict__ kc, int nkr,
                                                         const double* __restrict__ kr, double kbig,
                                                         zd* __restrict__ gc, zd* __restrict__ gr,
                                                         zd* __restrict__ gbig, int nb, double* __restrict__ j0r,
-                                                        int rows_r, double* __restrict__ j0a, int rows_a) {
+                                                        int rows_r, double* __restrict__ j0a, int rows_a,
+                                                        SurFeatures sf) {
   if ((int)blockIdx.x >= nb) {  // the rows of the J0 tables
+    const int nj = j0_ctas(rows_r, rows_a);
+    if ((int)blockIdx.x >= nb + nj) {
+      sur_features(sf, ((int)blockIdx.x - nb - nj) * blockDim.x + threadIdx.x);
+      return;
+    }
     const int b = (int)blockIdx.x - nb, nba = j0_arc_ctas(rows_a), nbr = j0_near_ctas(rows_r);
     const int w = threadIdx.x >> 5;
     if (b < nba + nbr) {
@@ -523,6 +544,8 @@ struct SomArgs {
 // products. 372 radii x 7176 nodes, 12 columns (the via transition's tables):
 // 270 us, 1180 us before; 233 radii, 3 columns 74 us, some 430 us before.
 // With skip set (the learned remainder was accepted) the CTAs return at once.
+// Launched behind the network's kernel, which it does not read, it runs beside it: it waits for that one's end
+// only at its own.
 template <int NC>
 __global__ void __launch_bounds__(128) sommerfeld_kernel(SomArgs a) {
   if (a.skip && *a.skip) return;
@@ -580,6 +603,7 @@ __global__ void __launch_bounds__(128) sommerfeld_kernel(SomArgs a) {
                       (red[2][2 * w + h][lane] + red[3][2 * w + h][lane]);
     }
   }
+  grid_wait();
 }
 
 // res[idx[e]][c] = sum over the node ranges s of part[s][c][..][e]: eight
@@ -843,15 +867,6 @@ __global__ void to_f32_kernel(const double* __restrict__ a, float* __restrict__ 
 }
 
 // ------------------------------------------------------ learned remainder
-// network inputs of n radii at frequency f
-__global__ void sur_features_kernel(int n, const double* __restrict__ rho, double a, double rho_ref, double f,
-                                    double fmin, double fmax, float* __restrict__ X) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  X[2 * i] = (float)(2.0 * log1p(rho[i] / a) / log1p(rho_ref / a) - 1.0);
-  X[2 * i + 1] = (float)(2.0 * (f - fmin) / (fmax - fmin) - 1.0);
-}
-
 // Not-a-knot cubic spline through (x_j, y_j), j < K (K >= 4), with every
 // thread of the CTA: the second derivatives M_j. The end conditions (third
 // derivative continuous at x_1 and x_{K-2}) give M_0 and M_{K-1} in terms of
@@ -921,6 +936,7 @@ __global__ void __launch_bounds__(256) sur_judge_kernel(int NC, const double* __
                                                         double* __restrict__ colerr) {
   extern __shared__ double sm[];
   __shared__ double red_e[8], red_s[8];
+  grid_trigger();  // sur_fill_kernel starts beside this one
   const int ncol = 2 * NC, col = blockIdx.x;
   double* xs = sm;       // radius of integrated radius e
   double* ys = xs + ne;  // residual there
@@ -979,32 +995,18 @@ __global__ void __launch_bounds__(256) sur_judge_kernel(int NC, const double* __
 // column error <= tol x the largest |remainder| (every CTA reaches the same
 // decision; CTA 0 records it in flag / err_out). When accepted, the table's
 // other radii ir[] get network + a not-a-knot spline of the residual through
-// all ne integrated radii (a denser spline than the judged one). Shared
-// memory: 11 ne doubles.
+// all ne integrated radii (a denser spline than the judged one), which is
+// solved beside the judge's, before the wait for its verdict. Shared memory:
+// 11 ne doubles.
 __global__ void __launch_bounds__(256) sur_fill_kernel(int NC, const double* __restrict__ rho, int ne,
                                                        const int* __restrict__ ie, int nr, const int* __restrict__ ir,
                                                        const float* __restrict__ Y, const double* __restrict__ scale,
-                                                       const double* __restrict__ colerr, double tol,
+                                                       const double* colerr, double tol,
                                                        zd* __restrict__ res, int* __restrict__ flag,
                                                        double* __restrict__ err_out) {
   extern __shared__ double sm[];
   __shared__ int accepted;
   const int ncol = 2 * NC, col = blockIdx.x;
-  if (threadIdx.x == 0) {
-    double e = 0, sx = 0;
-    for (int c = 0; c < ncol; ++c) {
-      e = fmax(e, colerr[2 * c]);
-      sx = fmax(sx, colerr[2 * c + 1]);
-    }
-    const double rel = sx > 0 ? e / sx : INFINITY;
-    accepted = rel <= tol ? 1 : 0;
-    if (blockIdx.x == 0) {
-      *flag = accepted;
-      *err_out = rel;
-    }
-  }
-  __syncthreads();
-  if (!accepted) return;
   double* xs = sm;
   double* ys = xs + ne;
   double* M = ys + ne;
@@ -1018,6 +1020,22 @@ __global__ void __launch_bounds__(256) sur_fill_kernel(int NC, const double* __r
   __syncthreads();
   spline_notaknot(
       ne, [&](int e) { return xs[e]; }, [&](int e) { return ys[e]; }, M, scratch);
+  grid_wait();  // the judge's errors
+  if (threadIdx.x == 0) {
+    double e = 0, sx = 0;
+    for (int c = 0; c < ncol; ++c) {
+      e = fmax(e, __ldcg(colerr + 2 * c));  // written by the kernel before, beside which this one started
+      sx = fmax(sx, __ldcg(colerr + 2 * c + 1));
+    }
+    const double rel = sx > 0 ? e / sx : INFINITY;
+    accepted = rel <= tol ? 1 : 0;
+    if (blockIdx.x == 0) {
+      *flag = accepted;
+      *err_out = rel;
+    }
+  }
+  __syncthreads();
+  if (!accepted) return;
   for (int r = threadIdx.x; r < nr; r += blockDim.x) {
     const int i = ir[r];
     const double xv = rho[i];
@@ -1109,6 +1127,46 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
     rc = (x);          \
     if (rc) goto fail; \
   } while (0)
+  // learned remainder: which radii get the Sommerfeld integral first
+  std::vector<int> ie, kpos, vpos, ir, lists;
+  if (d->surrogate) {
+    int nin = 0, nout = 0;
+    mlp_dims(d->surrogate, &nin, &nout);
+    if (nin != 2 || nout != 2 * NC || d->sur_stride < 2 || d->sur_stride > 64 || !(d->sur_near >= 0) ||
+        !d->sur_scale || !(d->sur_fmax > d->sur_fmin) || !(d->sur_a > 0) || !(d->sur_rho_ref > 0)) {
+      set_error("m25_greens_create: surrogate does not match the stack (2 inputs, 2 NC outputs, stride 2-64)");
+      delete g;
+      return M25_ERR_VALUE;
+    }
+    std::vector<int> knots;
+    int n0 = 0;
+    while (n0 < n && d->rho[n0] < d->sur_near) knots.push_back(n0++);
+    for (int i = n0; i < n; i += d->sur_stride) knots.push_back(i);
+    if (knots.back() != n - 1) knots.push_back(n - 1);
+    std::vector<char> exact(n, 0), val(n, 0);
+    for (int i : knots) exact[i] = 1;
+    for (size_t j = 0; j + 1 < knots.size(); ++j)
+      if (knots[j + 1] - knots[j] >= 2) val[(knots[j] + knots[j + 1]) / 2] = 1;
+    for (int i = 0; i < n; ++i) {
+      if (exact[i] || val[i]) {
+        if (exact[i]) kpos.push_back((int)ie.size());
+        if (val[i]) vpos.push_back((int)ie.size());
+        ie.push_back(i);
+      } else {
+        ir.push_back(i);
+      }
+    }
+    if (kpos.size() < 4 || vpos.empty() || ir.empty() ||
+        std::max(sur_judge_smem((int)ie.size(), (int)kpos.size()), sur_fill_smem((int)ie.size())) >
+            kSurSmemMax) {  // the plain tabulation
+      ie.clear();
+      kpos.clear();
+      vpos.clear();
+      ir.clear();
+    }
+  }
+  for (const std::vector<int>* l : {&ie, &kpos, &vpos, &ir}) lists.insert(lists.end(), l->begin(), l->end());
+  const int ne = (int)ie.size();
   // One block for what outlives this call and one for what does not, each
   // carved up at multiples of 256 bytes, and the inputs in one copy.
   size_t keep = 0, scratch = 0;
@@ -1119,7 +1177,9 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
   };
   const size_t o_stack = carve(keep, sizeof(StackDev)), o_rho = carve(keep, sizeof(double) * n),
                o_kc = carve(keep, sizeof(double) * 2 * d->nk_c), o_wc = carve(keep, sizeof(double) * 2 * d->nk_c),
-               o_kr = carve(keep, sizeof(double) * d->nk_r), o_wr = carve(keep, sizeof(double) * d->nk_r), n_in = keep,
+               o_kr = carve(keep, sizeof(double) * d->nk_r), o_wr = carve(keep, sizeof(double) * d->nk_r),
+               o_lists = carve(keep, sizeof(int) * lists.size()), o_scl = carve(keep, sizeof(double) * (ne ? 2 * NC : 0)),
+               n_in = keep,
                o_res = carve(keep, sizeof(zd) * (size_t)n * NC), o_sur = carve(keep, 16),
                o_rho32 = carve(keep, sizeof(float) * n), o_S = carve(keep, sizeof(zd) * (size_t)NC * n),
                o_coef = carve(keep, sizeof(zd) * (size_t)L * L * (n - 1) * 12),
@@ -1129,7 +1189,10 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
                o_cr = carve(scratch, sizeof(zd) * (size_t)d->nk_r * NC), o_gbig = carve(scratch, sizeof(zd) * NC),
                o_j0r = carve(scratch, sizeof(double) * kJ0Row * (size_t)rows_r),
                o_j0a = carve(scratch, sizeof(double) * kJ0ArcRow * (size_t)rows_a),
-               o_part = carve(scratch, sizeof(zd) * (size_t)(nsa + nsr) * n * NC);
+               o_part = carve(scratch, sizeof(zd) * (size_t)(nsa + nsr) * n * NC),
+               o_X = carve(scratch, ne ? sizeof(float) * 2 * (size_t)n : 0),
+               o_Y = carve(scratch, ne ? sizeof(float) * 2 * NC * (size_t)n : 0),
+               o_colerr = carve(scratch, ne ? sizeof(double) * 2 * 2 * NC : 0);
   std::vector<char> in(n_in);
   memcpy(in.data() + o_stack, &S, sizeof(StackDev));
   memcpy(in.data() + o_rho, d->rho, sizeof(double) * n);
@@ -1137,6 +1200,10 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
   memcpy(in.data() + o_wc, d->wc, sizeof(double) * 2 * d->nk_c);
   memcpy(in.data() + o_kr, d->kr, sizeof(double) * d->nk_r);
   memcpy(in.data() + o_wr, d->wr, sizeof(double) * d->nk_r);
+  if (ne) {
+    memcpy(in.data() + o_lists, lists.data(), sizeof(int) * lists.size());
+    memcpy(in.data() + o_scl, d->sur_scale, sizeof(double) * 2 * NC);
+  }
   char *kb = nullptr, *sb = nullptr;
   zd* gbig = nullptr;
   double *j0r = nullptr, *j0a = nullptr, *part = nullptr;
@@ -1164,11 +1231,13 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
   M25_CUDA(cudaMemcpyAsync(kb, in.data(), n_in, cudaMemcpyHostToDevice, st));
   if (d->surrogate) M25_CUDA(cudaMemsetAsync(g->sur, 0, 16, st));
   {
+  const SurFeatures sf{ne ? n : 0,   g->rho,     d->sur_a,   d->sur_rho_ref,
+                       d->freq,      d->sur_fmin, d->sur_fmax, reinterpret_cast<float*>(sb + o_X)};
   StageTimer tm(ctx, ST_GREENS);
   {
     const int lanes = d->single ? d->nk_c + d->nk_r : 2 * (d->nk_c + d->nk_r + 1), nb = (lanes + 63) / 64;
-    spectral_g_kernel<<<nb + j0_ctas(rows_r, rows_a), 64, 0, st>>>(Sd, d->nk_c, kc, d->nk_r, kr, d->kbig, cc, cr,
-                                                                       gbig, nb, j0r, rows_r, j0a, rows_a);
+    spectral_g_kernel<<<nb + j0_ctas(rows_r, rows_a) + (sf.n + 63) / 64, 64, 0, st>>>(Sd, d->nk_c, kc, d->nk_r, kr, d->kbig, cc, cr,
+                                                                       gbig, nb, j0r, rows_r, j0a, rows_a, sf);
     leading_kernel<<<1, 32 * L * L, 0, st>>>(Sd, d->kbig, gbig);
     spectral_coef_kernel<<<dim3((d->nk_c + d->nk_r + 63) / 64, L * L), 64, 0, st>>>(Sd, d->nk_c, kc, wc, d->nk_r, kr,
                                                                                     wr, cc, cr);
@@ -1176,80 +1245,35 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
   {
     // the Sommerfeld integral at the radii rho[idx[e]], e < ne (idx NULL:
     // all n) into res; skip: see sommerfeld_kernel
-    auto sommerfeld = [&](int ne, const int* idx, const int* skip) {
+    auto sommerfeld = [&](int ne, const int* idx, const int* skip, bool chained = false) {
       if (ne <= 0) return;
+      auto launch = [&](void (*kernel)(SomArgs), dim3 grid, const SomArgs& a) {
+        if (chained)
+          launch_chained(kernel, grid, 128, 0, st, a);
+        else
+          kernel<<<grid, 128, 0, st>>>(a);
+      };
       const dim3 grid(nsa + nsr, (ne + 31) / 32);
       const SomArgs a{ne, idx, g->rho, nsa, nsr, d->nk_c, kc, cc, d->nk_r, kr, cr, j0r, j0a, rows_r, rows_a, part, skip};
       switch (NC) {
-        case 3: sommerfeld_kernel<3><<<grid, 128, 0, st>>>(a); break;
-        case 12: sommerfeld_kernel<12><<<grid, 128, 0, st>>>(a); break;
-        default: sommerfeld_kernel<27><<<grid, 128, 0, st>>>(a); break;
+        case 3: launch(sommerfeld_kernel<3>, grid, a); break;
+        case 12: launch(sommerfeld_kernel<12>, grid, a); break;
+        default: launch(sommerfeld_kernel<27>, grid, a); break;
       }
       sommerfeld_sum_kernel<<<(2 * ne * NC + 31) / 32, 256, 0, st>>>(ne, NC, idx, nsa + nsr, part, res, skip);
     };
-    // learned remainder: which radii get the Sommerfeld integral first
-    std::vector<int> ie, kpos, vpos, ir;
-    if (d->surrogate) {
-      int nin = 0, nout = 0;
-      mlp_dims(d->surrogate, &nin, &nout);
-      if (nin != 2 || nout != 2 * NC || d->sur_stride < 2 || d->sur_stride > 64 || !(d->sur_near >= 0) ||
-          !d->sur_scale || !(d->sur_fmax > d->sur_fmin) || !(d->sur_a > 0) || !(d->sur_rho_ref > 0)) {
-        set_error("m25_greens_create: surrogate does not match the stack (2 inputs, 2 NC outputs, stride 2-64)");
-        rc = M25_ERR_VALUE;
-        goto fail;
-      }
-      std::vector<int> knots;
-      int n0 = 0;
-      while (n0 < n && d->rho[n0] < d->sur_near) knots.push_back(n0++);
-      for (int i = n0; i < n; i += d->sur_stride) knots.push_back(i);
-      if (knots.back() != n - 1) knots.push_back(n - 1);
-      std::vector<char> exact(n, 0), val(n, 0);
-      for (int i : knots) exact[i] = 1;
-      for (size_t j = 0; j + 1 < knots.size(); ++j)
-        if (knots[j + 1] - knots[j] >= 2) val[(knots[j] + knots[j + 1]) / 2] = 1;
-      for (int i = 0; i < n; ++i) {
-        if (exact[i] || val[i]) {
-          if (exact[i]) kpos.push_back((int)ie.size());
-          if (val[i]) vpos.push_back((int)ie.size());
-          ie.push_back(i);
-        } else {
-          ir.push_back(i);
-        }
-      }
-      if (kpos.size() < 4 || vpos.empty() || ir.empty() ||
-          std::max(sur_judge_smem((int)ie.size(), (int)kpos.size()), sur_fill_smem((int)ie.size())) >
-              kSurSmemMax) {  // the plain tabulation
-        ie.clear();
-        kpos.clear();
-        vpos.clear();
-        ir.clear();
-      }
-    }
     if (!ie.empty()) {
       // the network at every radius, the Sommerfeld integral at the knots and
       // validation radii, the judge, then the integral at the other radii
       // unless the judge accepted
-      const int ne = (int)ie.size(), nk = (int)kpos.size(), nv = (int)vpos.size(), nr = (int)ir.size();
-      std::vector<int> lists;
-      lists.insert(lists.end(), ie.begin(), ie.end());
-      lists.insert(lists.end(), kpos.begin(), kpos.end());
-      lists.insert(lists.end(), vpos.begin(), vpos.end());
-      lists.insert(lists.end(), ir.begin(), ir.end());
-      int* dl = nullptr;
-      double *scl = nullptr, *colerr = nullptr;
-      float *X = nullptr, *Y = nullptr;
-      TRY(alloc_async(tmp, (void**)&dl, sizeof(int) * lists.size(), st));
-      TRY(alloc_async(tmp, (void**)&scl, sizeof(double) * 2 * NC, st));
-      TRY(alloc_async(tmp, (void**)&X, sizeof(float) * 2 * (size_t)n, st));
-      TRY(alloc_async(tmp, (void**)&Y, sizeof(float) * 2 * NC * (size_t)n, st));
-      TRY(alloc_async(tmp, (void**)&colerr, sizeof(double) * 2 * 2 * NC, st));
-      M25_CUDA(cudaMemcpyAsync(dl, lists.data(), sizeof(int) * lists.size(), cudaMemcpyHostToDevice, st));
-      M25_CUDA(cudaMemcpyAsync(scl, d->sur_scale, sizeof(double) * 2 * NC, cudaMemcpyHostToDevice, st));
+      const int nk = (int)kpos.size(), nv = (int)vpos.size(), nr = (int)ir.size();
+      const int* dl = reinterpret_cast<const int*>(kb + o_lists);
+      const double* scl = reinterpret_cast<const double*>(kb + o_scl);
+      double* colerr = reinterpret_cast<double*>(sb + o_colerr);
+      float* Y = reinterpret_cast<float*>(sb + o_Y);
       const int *d_ie = dl, *d_kpos = dl + ne, *d_vpos = dl + ne + nk, *d_ir = dl + ne + nk + nv;
-      sur_features_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, g->rho, d->sur_a, d->sur_rho_ref, d->freq, d->sur_fmin,
-                                                           d->sur_fmax, X);
-      TRY(mlp_forward_device(d->surrogate, n, X, Y, st));
-      sommerfeld(ne, d_ie, nullptr);
+      TRY(mlp_forward_device(d->surrogate, n, sf.X, Y, st));
+      sommerfeld(ne, d_ie, nullptr, true);
       int* flag = static_cast<int*>(g->sur);
       double* err = reinterpret_cast<double*>(static_cast<char*>(g->sur) + 8);
       static const bool smem_attr =
@@ -1264,8 +1288,8 @@ extern "C" int m25_greens_create(m25_ctx* ctx, const m25_greens_desc* d, m25_gre
       }
       sur_judge_kernel<<<2 * NC, 256, sur_judge_smem(ne, nk), st>>>(NC, g->rho, ne, d_ie, nk, d_kpos, nv, d_vpos, Y,
                                                                     scl, res, colerr);
-      sur_fill_kernel<<<2 * NC, 256, sur_fill_smem(ne), st>>>(NC, g->rho, ne, d_ie, nr, d_ir, Y, scl, colerr,
-                                                            d->sur_tol, res, flag, err);
+      launch_chained(sur_fill_kernel, dim3(2 * NC), dim3(256), sur_fill_smem(ne), st, NC, g->rho, ne, d_ie, nr, d_ir, Y, scl,
+                     colerr, d->sur_tol, res, flag, err);
       sommerfeld(nr, d_ir, flag);  // the integral at the other radii unless the judge accepted
       g->sur_planned = ne;
     } else {

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "m25_internal.h"
+#include "m25_lu.h"
 
 namespace m25 {
 
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(32 * kInferWarps) mlp_infer_kernel(MlpDims d, 
                                                                      int64_t np, int n, const float* __restrict__ X,
                                                                      float* __restrict__ Y) {
   extern __shared__ float sp[];
+  grid_trigger();  // a chained kernel behind this one that does not read Y may start (it waits for Y's end itself)
   for (int l = 0; l <= d.n_layers; ++l) {
     const int nin = mlp_in(d, l), nout = mlp_out(d, l);
     const float* W = P + d.off[l];
