@@ -48,7 +48,7 @@ void split_to_z32(m25_ctx*, const zd*, int64_t, zf*, int64_t, zf*, zf*, int64_t,
 bool lu_tc_available();
 template <class TF, class TV>
 int lu_solve_wave(m25_ctx*, const cx<TF>*, int64_t, int, const int32_t*, const cx<TV>*, int, cx<TV>*,
-                  const int32_t* perm = nullptr);
+                  const int32_t* perm = nullptr, bool wide = false);
 int lu_wave_error(m25_ctx*, int, int*);
 int lu_wave_reset(m25_ctx*);
 

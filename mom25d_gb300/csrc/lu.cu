@@ -1243,10 +1243,11 @@ int lu_make_perm(m25_ctx* ctx, int n, const int32_t* ipiv, int32_t* perm) {
 }
 
 // X = (LU)^-1 P B: the permutation (from ipiv, or the precomputed perm when
-// given), then one wavefront launch per factor.
+// given), then one wavefront launch per factor. wide: on as many CTAs as there
+// are blocks, whatever the cap.
 template <class TF, class TV>
 int lu_solve_wave(m25_ctx* ctx, const cx<TF>* A, int64_t lda, int n, const int32_t* ipiv, const cx<TV>* B, int nrhs,
-                  cx<TV>* X, const int32_t* perm) {
+                  cx<TV>* X, const int32_t* perm, bool wide) {
   cudaStream_t st = ctx->stream;
   if (nrhs > 8 || (size_t)n * sizeof(int) > 200 * 1024) {
     set_error("dense solve: at most 8 right-hand sides and n <= 51200");
@@ -1296,7 +1297,7 @@ int lu_solve_wave(m25_ctx* ctx, const cx<TF>* A, int64_t lda, int n, const int32
   }
   // M25_WAVE_CTAS: at most this many CTAs (a tuning knob; 0 or unset = one per block up to the device's fill)
   static const int wave_cap_env = getenv("M25_WAVE_CTAS") ? atoi(getenv("M25_WAVE_CTAS")) : 0;
-  const int wave_cap = ctx->tune_wave_ctas > 0 ? ctx->tune_wave_ctas : wave_cap_env;
+  const int wave_cap = wide ? 0 : ctx->tune_wave_ctas > 0 ? ctx->tune_wave_ctas : wave_cap_env;
   const int G = std::min(std::min(nblk, ctx->num_sms * occ), wave_cap > 0 ? wave_cap : nblk);
   StageTimer tm(ctx, ST_TRSV);
   if (!perm) {
@@ -1348,11 +1349,11 @@ int lu_wave_error(m25_ctx* ctx, int n, int* flag) {
 }
 
 template int lu_solve_wave<double, double>(m25_ctx*, const zd*, int64_t, int, const int32_t*, const zd*, int, zd*,
-                                           const int32_t*);
+                                           const int32_t*, bool);
 template int lu_solve_wave<float, double>(m25_ctx*, const zf*, int64_t, int, const int32_t*, const zd*, int, zd*,
-                                          const int32_t*);
+                                          const int32_t*, bool);
 template int lu_solve_wave<float, float>(m25_ctx*, const zf*, int64_t, int, const int32_t*, const zf*, int, zf*,
-                                         const int32_t*);
+                                         const int32_t*, bool);
 
 template int lu_factor<double>(m25_ctx*, zd*, int64_t, int, int32_t*, int, bool, int*);
 template int lu_factor<float>(m25_ctx*, zf*, int64_t, int, int32_t*, int, bool, int*);
@@ -1521,6 +1522,10 @@ void matvec_df(int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, const zf* 
 // operations and latencies on one SM; the host then scaled the vector between two synchronisations.)
 constexpr int kDotSplit = 8;
 constexpr int kMaxGmres = 30;  // restart length
+// A solve that takes more steps than this is the long pole of a sweep (the LPF's and the via transition's lowest
+// frequencies: 12 and 46 steps against 2 to 5): the CTA cap, which leaves room to points beside it, ends there.
+// Eight points in flight, via transition: 63 ms a sweep of eight, 72 ms with the cap throughout.
+constexpr int kCappedSteps = 4;
 
 // sum of v over the CTA (256 threads), on thread 0
 __device__ __forceinline__ double cta_sum(double v, double* red) {
@@ -1739,11 +1744,12 @@ int refine(m25_ctx* ctx, int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, 
   int32_t* perm = reinterpret_cast<int32_t*>(parts + 3 * nparts);  // row permutation of the LU
   const unsigned gw = (unsigned)(((size_t)n * 32 + 255) / 256);
   StageTimer tm(ctx, ST_REFINE);
+  int total = 0;  // GMRES steps
   // out = (LU32)^-1 in, in fp32 with the input scaled to O(1) by its
   // largest entry *mx (kept on the device: no host round trip), and out's planes
   auto precond = [&](const zd* in, zd* out) -> int {
     z64_to_z32_scaled<<<g1, 256, 0, st>>>((int64_t)np, in, pscale, r32);
-    int r = lu_solve_wave<float, float>(ctx, LU, ldlu, n, ipiv, r32, P, d32, perm);
+    int r = lu_solve_wave<float, float>(ctx, LU, ldlu, n, ipiv, r32, P, d32, perm, total >= kCappedSteps);
     if (r) return r;
     z32_to_z64_scaled<<<g1, 256, 0, st>>>((int64_t)np, d32, pscale, out, xh, xl);
     return M25_OK;
@@ -1759,7 +1765,6 @@ int refine(m25_ctx* ctx, int n, int P, const zf* Zh, const zf* Zl, int64_t ldz, 
   // start from the fp32 solution x0 = M^-1 B
   maxabs_kernel<<<g1, 256, 0, st>>>((int64_t)np, B, mx);
   if ((rc = precond(B, X))) return rc;
-  int total = 0;
   double prev_worst = INFINITY, znorm = 0;
   std::vector<double> rn(P), xn(P), bn(P), hparts(64 + 3 * nparts), step(4 * (size_t)hcap + P);
   std::vector<zd> hh((size_t)(m + 2) * P), H((size_t)(m + 1) * m * P), g((size_t)(m + 1) * P), cs(m * P), sn(m * P);
@@ -1976,7 +1981,7 @@ extern "C" int m25_dense_solve_noalloc(int32_t n, int32_t nrhs, void* Z, const v
   int32_t* perm = reinterpret_cast<int32_t*>(base + kNoAllocPermOffset);
   if ((rc = lu_make_perm(&c, n, ipiv, perm))) return rc;
   rc = lu_solve_wave<double, double>(&c, static_cast<const zd*>(Z), n, n, ipiv, static_cast<const zd*>(B), nrhs,
-                                     static_cast<zd*>(X), perm);
+                                     static_cast<zd*>(X), perm, false);
   if (rc) return rc;
   int werr = 0;
   if ((rc = lu_wave_error(&c, n, &werr))) return rc;
