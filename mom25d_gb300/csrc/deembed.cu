@@ -501,7 +501,7 @@ __device__ double brent_minimize(F f, double lo, double hi, double xatol, int ma
   return x;
 }
 
-// One cluster of four CTAs per port group: Nelder-Mead with scipy's
+// One cluster of CTAs per port group: Nelder-Mead with scipy's
 // coefficients (reflection 1, expansion 2, contraction 0.5, shrink 0.5),
 // initial simplex 5 % steps, stopping when the simplex spans <= xatol and its
 // values <= fatol. Each iteration evaluates its four possible trial points
@@ -509,18 +509,32 @@ __device__ double brent_minimize(F f, double lo, double hi, double xatol, int ma
 // each, and then takes scipy's decisions on those values: the objective is a
 // pure function, so the simplex follows the sequential method's path exactly.
 // Every CTA keeps the simplex; the values go around through the cluster's
-// shared memory. Measured on GB300 (two ports; the whole de-embedding of a
-// point, nearly all of it this fit): the line (5 cuts per feed) 4.9 -> 0.9 ms,
-// the tee (21) 6.1 -> 1.2 ms, the LPF (29) 5.0 -> 1.2 ms, against one CTA of
+// shared memory. Twelve more CTAs evaluate the four trial points of the
+// iteration after, for the three outcomes that a step has nine times in ten: the inside
+// contraction, the reflection or the outside contraction taken, and not the
+// worst of the new simplex; whichever of the two better places it takes, the
+// centroid is that of it and the old best, the worst the old middle one. On a
+// hit that iteration needs no evaluation of its own: about 0.55 rounds an
+// iteration, the tee's fit 668 us (960 us with the four CTAs alone).
+// Measured on GB300 (two ports; the whole de-embedding of a
+// point, nearly all of it this fit): the line (5 cuts per feed) 4.9 -> 0.7 ms,
+// the tee (21) 6.1 -> 0.9 ms, the LPF (29) 5.0 -> 1.0 ms, against one CTA of
 // four warps per group with a trial point per warp, whose fp64 chain of some
 // 1500 instructions per evaluation took 67 us an iteration.
-constexpr int kFitCl = 4;
+// CL: 16, or 4 (without the iteration after) where clusters of 16 cannot be launched.
 
+// trial point k of a simplex: reflection, expansion, outside, inside contraction
+__device__ __forceinline__ double fit_trial(int k, double centroid, double worst) {
+  const double al = k == 0 ? 2.0 : k == 1 ? 3.0 : k == 2 ? 1.5 : 0.5, be = k == 0 ? 1.0 : k == 1 ? 2.0 : k == 2 ? 0.5 : -0.5;
+  return fma(al, centroid, -(be * worst));
+}
+
+template <int CL>
 __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
   extern __shared__ __align__(16) unsigned char fit_smem[];
   FitShared& sh = *reinterpret_cast<FitShared*>(fit_smem);
-  __shared__ double vals[2][kFitCl];
-  const int grp = blockIdx.x / kFitCl, lane = threadIdx.x & 31;
+  __shared__ double vals[2][CL];
+  const int grp = blockIdx.x / CL, lane = threadIdx.x & 31;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
   auto cluster_sync = [] {
@@ -590,21 +604,21 @@ __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
   cluster_sync();  // every CTA runs before the first value is sent
   int par = 0;
   // objective values of the first n trial points, CTA k's at its point x
-  auto round = [&](const double (&x)[2], int n, double (&v)[kFitCl]) {
+  auto round = [&](const double (&x)[2], int n, double (&v)[CL]) {
     double f = 0.0;
     if ((int)rank < n) f = wave_objective(a, sh, zd(scale * x[0], scale * x[1]), false);
-    if (threadIdx.x < kFitCl && (int)rank < n) {
+    if (threadIdx.x < CL && (int)rank < n) {
       uint32_t d, l = (uint32_t)__cvta_generic_to_shared(&vals[par][rank]);
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(d) : "r"(l), "r"(threadIdx.x));
       asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(d), "d"(f) : "memory");
     }
     cluster_sync();
 #pragma unroll
-    for (int k = 0; k < kFitCl; ++k) v[k] = k < n ? *(volatile double*)&vals[par][k] : 0.0;
+    for (int k = 0; k < CL; ++k) v[k] = k < n ? *(volatile double*)&vals[par][k] : 0.0;
     par ^= 1;  // the other buffer: a fast CTA's next value must not overtake a slow one's read
   };
   const double xatol = 1e-10, fatol = 1e-16;
-  double sim[3][2], fs[3], v[kFitCl];
+  double sim[3][2], fs[3], v[CL];
   // gamma0 = 1e-3 b0 + j b0, scaled by |b0|
   const double x0 = 1e-3 * a.beta0[grp] / scale, x1 = a.beta0[grp] / scale;
   sim[0][0] = x0; sim[0][1] = x1;
@@ -615,7 +629,7 @@ __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
     round(x, 3, v);
   }
   for (int k = 0; k < 3; ++k) fs[k] = v[k];
-  auto sort3 = [&]() {  // stable insertion sort by value
+  auto sort3 = [&]() {  // stable insertion sort by value; where the last entry went, if the others were in order
     auto order = [&](int i) {  // entries i - 1, i
       if (fs[i] < fs[i - 1]) {
         const double t = fs[i]; fs[i] = fs[i - 1]; fs[i - 1] = t;
@@ -625,10 +639,13 @@ __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
       return false;
     };
     order(1);
-    if (order(2)) order(1);
+    if (!order(2)) return 2;
+    return order(1) ? 0 : 1;
   };
   sort3();
   int it = 1;
+  double next[4];      // values of this iteration's trial points, when the round before has them
+  bool have = false;
   while (it < 4000) {
     double dx = 0, df = 0;
     for (int k = 1; k < 3; ++k) {
@@ -637,27 +654,35 @@ __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
     }
     if (dx <= xatol && df <= fatol) break;
     double xr[2], xe[2], xo[2], xi[2], x[2];
+    const int sc = ((int)rank - 4) >> 2;  // the outcome this CTA bets on: 0 inside contraction, 1 reflection, 2 outside
     for (int d = 0; d < 2; ++d) {
       const double xb = (sim[0][d] + sim[1][d]) * 0.5;
-      xr[d] = 2.0 * xb - sim[2][d];
-      xe[d] = 3.0 * xb - 2.0 * sim[2][d];
-      xo[d] = 1.5 * xb - 0.5 * sim[2][d];
-      xi[d] = 0.5 * xb + 0.5 * sim[2][d];
-      x[d] = rank == 0 ? xr[d] : rank == 1 ? xe[d] : rank == 2 ? xo[d] : xi[d];
+      xr[d] = fit_trial(0, xb, sim[2][d]);
+      xe[d] = fit_trial(1, xb, sim[2][d]);
+      xo[d] = fit_trial(2, xb, sim[2][d]);
+      xi[d] = fit_trial(3, xb, sim[2][d]);
+      if (rank < 4)
+        x[d] = rank == 0 ? xr[d] : rank == 1 ? xe[d] : rank == 2 ? xo[d] : xi[d];
+      else
+        x[d] = fit_trial(rank & 3, ((sc == 0 ? xi[d] : sc == 1 ? xr[d] : xo[d]) + sim[0][d]) * 0.5, sim[1][d]);
     }
-    round(x, 4, v);
-    const double fr = v[0], fe = v[1], fo = v[2], fi = v[3];
+    const bool had = have;
+    if (!had) round(x, CL, v);
+    have = false;
+    const double fr = had ? next[0] : v[0], fe = had ? next[1] : v[1], fo = had ? next[2] : v[2],
+                 fi = had ? next[3] : v[3];
+    int took = -1;  // the outcome: 0 inside contraction, 1 reflection, 2 outside contraction
     bool shrink = false;
     if (fr < fs[0]) {
       if (fe < fr) { sim[2][0] = xe[0]; sim[2][1] = xe[1]; fs[2] = fe; }
-      else { sim[2][0] = xr[0]; sim[2][1] = xr[1]; fs[2] = fr; }
+      else { sim[2][0] = xr[0]; sim[2][1] = xr[1]; fs[2] = fr; took = 1; }
     } else if (fr < fs[1]) {
-      sim[2][0] = xr[0]; sim[2][1] = xr[1]; fs[2] = fr;
+      sim[2][0] = xr[0]; sim[2][1] = xr[1]; fs[2] = fr; took = 1;
     } else if (fr < fs[2]) {
-      if (fo <= fr) { sim[2][0] = xo[0]; sim[2][1] = xo[1]; fs[2] = fo; }
+      if (fo <= fr) { sim[2][0] = xo[0]; sim[2][1] = xo[1]; fs[2] = fo; took = 2; }
       else shrink = true;
     } else {
-      if (fi < fs[2]) { sim[2][0] = xi[0]; sim[2][1] = xi[1]; fs[2] = fi; }
+      if (fi < fs[2]) { sim[2][0] = xi[0]; sim[2][1] = xi[1]; fs[2] = fi; took = 0; }
       else shrink = true;
     }
     if (shrink) {
@@ -669,7 +694,13 @@ __global__ void __launch_bounds__(32 * kFitWarps) fit_kernel(FitArgs a) {
       fs[2] = v[1];
     }
     ++it;
-    sort3();
+    const int place = sort3();
+    if (CL > 4 && !had && took >= 0 && place < 2) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        next[k] = took == 0 ? v[(4 + k) % CL] : took == 1 ? v[(8 + k) % CL] : v[(12 + k) % CL];
+      have = true;
+    }
   }
   finish(zd(scale * sim[0][0], scale * sim[0][1]), it);
 }
@@ -1008,20 +1039,37 @@ static int deembed(m25_ctx* ctx, m25_geom* geom, m25_greens* gr, m25_ports* p, c
     fa.hi[gi] = p->lossless ? p->bounds[2 * gi + 1] : 0.0;
   }
   {
-    M25_CUDA(cudaFuncSetAttribute(fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FitShared)));
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kFitCl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(p->ngroup * kFitCl);
-    cfg.blockDim = dim3(32 * kFitWarps);
-    cfg.dynamicSmemBytes = sizeof(FitShared);
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    M25_CUDA(cudaLaunchKernelEx(&cfg, fit_kernel, fa));
+    const auto launch = [&](void (*kernel)(FitArgs), int cl, int* active) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = cl;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3(p->ngroup * cl);
+      cfg.blockDim = dim3(32 * kFitWarps);
+      cfg.dynamicSmemBytes = sizeof(FitShared);
+      cfg.stream = st;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      return active ? cudaOccupancyMaxActiveClusters(active, kernel, &cfg) : cudaLaunchKernelEx(&cfg, kernel, fa);
+    };
+    static const bool wide = [&] {
+      int active = 0;
+      const bool ok =
+          cudaFuncSetAttribute(fit_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FitShared)) ==
+              cudaSuccess &&
+          cudaFuncSetAttribute(fit_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+          launch(fit_kernel<16>, 16, &active) == cudaSuccess && active > 0;
+      cudaGetLastError();  // a refused attribute only means: clusters of four
+      return ok;
+    }();
+    if (wide) {
+      M25_CUDA(launch(fit_kernel<16>, 16, nullptr));
+    } else {
+      M25_CUDA(cudaFuncSetAttribute(fit_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FitShared)));
+      M25_CUDA(launch(fit_kernel<4>, 4, nullptr));
+    }
   }
   // S of the feeds alone; with internal ports the caller assembles S from
   // the coefficients (m25_deembed_coefs)
