@@ -53,20 +53,20 @@ __global__ void via_charges_kernel(int nv, int nb, int P, const int32_t* __restr
 
 __device__ inline zd spline_w(const double* __restrict__ rho, int n, const zd* __restrict__ coef, int pair, double r) {
   int i;
-  if (r < rho[1]) i = 0;
-  else if (r >= rho[n - 2]) i = n - 2;
+  if (less_nonneg(r, rho[1])) i = 0;
+  else if (!less_nonneg(r, rho[n - 2])) i = n - 2;
   else {
     int lo = 1, hi = n - 2;
     while (hi - lo > 1) {
       int mid = (lo + hi) >> 1;
-      if (r < rho[mid]) hi = mid; else lo = mid;
+      if (less_nonneg(r, rho[mid])) hi = mid; else lo = mid;
     }
     i = lo;
   }
   double dx = r - rho[i];
   const zd* c = coef + ((size_t)pair * (n - 1) + i) * 12;
-  double z = dx, z2 = dx * dx, z3 = z2 * dx;
-  return c[3 * 3 + 2] + c[2 * 3 + 2] * z + c[1 * 3 + 2] * z2 + c[0 * 3 + 2] * z3;
+  const zd c3 = c[3 * 3 + 2], c2 = c[2 * 3 + 2], c1 = c[1 * 3 + 2], c0 = c[0 * 3 + 2];
+  return {c3.re + dx * (c2.re + dx * (c1.re + dx * c0.re)), c3.im + dx * (c2.im + dx * (c1.im + dx * c0.im))};
 }
 
 // sum_k w_k S_W(|p - r_k|) + c_W I0(t, p) / 4pi of one triangle in fp64

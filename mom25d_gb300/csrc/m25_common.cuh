@@ -58,6 +58,11 @@ __device__ __forceinline__ cx<double> fnma(cx<double> a, cx<double> b, cx<double
 __device__ __forceinline__ cx<float> fnma(cx<float> a, cx<float> b, cx<float> c) {
   return {fmaf(b.im, c.im, fmaf(-b.re, c.re, a.re)), fmaf(-b.im, c.re, fmaf(-b.re, c.im, a.im))};
 }
+// a < b for a, b >= 0: complex128 paths compare the bits, off the fp64 pipe
+__device__ __forceinline__ bool less_nonneg(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ bool less_nonneg(float a, float b) { return a < b; }
 template <class T> __host__ __device__ inline cx<T> conj(cx<T> a) { return {a.re, -a.im}; }
 template <class T> __host__ __device__ inline T norm2(cx<T> a) { return a.re * a.re + a.im * a.im; }
 template <class T> __host__ __device__ inline T cabs1(cx<T> a) { return fabs(a.re) + fabs(a.im); }
