@@ -7,7 +7,7 @@
 // update), so what bounds it is the latency of a step and, in complex128, the
 // rate of fp64 multiply-adds of the SMs that hold the rows (two per clock and
 // SM). Hence:
-//  - one row per thread, its W columns in registers: a step reads only the
+//  - one row per thread (complex128 with few rows: on two or four), its W columns in registers: a step reads only the
 //    pivot row from shared memory, and has one CTA barrier and one wait for the
 //    cluster's exchange;
 //  - rows are not moved while the strip is factored: a thread follows the
@@ -19,14 +19,15 @@
 //    pivot and send the candidate's row, while the warps with rows run the
 //    multiply-adds of the step before (kAhead below).
 // Measured on GB300 (one factorisation alone, sum over its panels):
-//   complex128, N = 546 / 1085 / 2434 / 5943: 1.75 / 3.5 / 8.6 / 28.4 ms (1.9 / 3.9 / 9.4 / 30.6 ms with every step
-//   finished before the next one's search; 7.95 / 20.0 / 53.0 / 96.6 ms for 64-column panels in shared memory, with
-//   the row k0 + j sent around and both divisions on the chain)
+//   complex128, N = 546 / 1085 / 2434 / 5943: 1.4 / 3.0 / 8.0 / 27.8 ms (1.75 / 3.5 / 8.6 / 28.4 ms with one lane per
+//   row throughout; 1.9 / 3.9 / 9.4 / 30.6 ms with every step finished before the next one's search, too;
+//   7.95 / 20.0 / 53.0 / 96.6 ms for 64-column panels in shared memory, with the row k0 + j sent around and both
+//   divisions on the chain)
 //   complex64, N = 1085 / 5943: 1.6 / 10.1 ms (2.5 / 21.1 ms, and 0.2 / 2.1 ms for the products between
 //   the two panels of a block)
 // A column step of complex64 takes about 1 us, of which 0.45 us are the exchange's
-// flight; one of complex128 2.5 us at 64 rows per CTA: search 0.35, the candidate's staging 0.4, the multiply-adds
-// 1.0, the wait 0.2, multiplier and next column 0.5.
+// flight; one of complex128 with one lane per row 2.5 us: search 0.35, the candidate's staging 0.4, the
+// multiply-adds 1.0 (half with two lanes per row), the wait 0.2, multiplier and next column 0.5.
 #include <algorithm>
 #include <string>
 
@@ -157,39 +158,64 @@ using KeyOf = decltype(val_key(T(0)));
 // packed fp32 multiply-add (two per lane and instruction). (A row that moves one
 // column to the front with every update, so that the loop over the columns
 // needs no unrolling, is half the code and 5 to 10 % slower: it spills.)
-template <class T>
+// complex128 rows may lie on TPR = 2 or 4 neighbouring lanes, lane h of them
+// with the columns h, h + TPR, ...; get(i) and the update of one column are for the lane that has it.
+template <class T, int TPR>
 struct StripRow;
-template <>
-struct StripRow<double> {
-  static constexpr int W = strip_w<double>();
-  cx<double> x[W];
-  __device__ __forceinline__ cx<double> get(int i) const { return x[i]; }
-  __device__ __forceinline__ void set(int i, cx<double> v) { x[i] = v; }
-  // chunk k (16 bytes) of the row as it is sent
+template <int TPR>
+struct StripRow<double, TPR> {
+  static constexpr int W = strip_w<double>(), N = W / TPR, G = kGrp / TPR;
+  cx<double> x[N];
+  __device__ __forceinline__ cx<double> get(int i) const { return x[i / TPR]; }
+  __device__ __forceinline__ void set(int i, cx<double> v) { x[i / TPR] = v; }
+  __device__ __forceinline__ void load(const cx<double>* row, int h) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = row[TPR * i + h];
+  }
+  // the columns from i0 on to row (from column jb)
+  __device__ __forceinline__ void store(int i0, int jb, cx<double>* row, int h) const {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (TPR * i + h >= i0 && jb + TPR * i < W) row[TPR * i + h] = x[i];
+  }
   static __device__ __forceinline__ uint4 pack(cx<double> v) {
     return make_uint4((unsigned)__double2loint(v.re), (unsigned)__double2hiint(v.re), (unsigned)__double2loint(v.im),
                       (unsigned)__double2hiint(v.im));
   }
-  __device__ __forceinline__ uint4 chunk(int k) const { return pack(x[k]); }
+  // the columns from i0 on as they are sent (16 bytes each; u: from column jb)
+  __device__ __forceinline__ void stage(int i0, int jb, uint4* u, int h) const {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (TPR * i + TPR > i0 && jb + TPR * i < W) u[TPR * i + h] = pack(x[i]);
+  }
   static __device__ __forceinline__ cx<double> sent(const uint4* u, int c) {
     return *reinterpret_cast<const cx<double>*>(u + c);
   }
   // x_i -= l u_i for i >= i0 and jb + i < W (u: the pivot row's chunks from column jb)
-  __device__ __forceinline__ void update(int i0, int jb, cx<double> l, const uint4* u) {
+  __device__ __forceinline__ void update(int i0, int jb, cx<double> l, const uint4* u, int h) {
 #pragma unroll
-    for (int i = 0; i < kGrp; ++i)
-      if (i >= i0) x[i] = fnma(x[i], l, *reinterpret_cast<const cx<double>*>(u + i));
+    for (int i = 0; i < G; ++i)
+      if (TPR * i >= i0) {
+        x[i] = fnma(x[i], l, sent(u, TPR * i + h));
+      } else if (TPR * i + TPR > i0) {
+        if (TPR * i + h >= i0) x[i] = fnma(x[i], l, sent(u, TPR * i + h));
+      }
     if (jb + kGrp < W)  // no fp64 operation for nothing
 #pragma unroll
-      for (int i = kGrp; i < W; ++i) x[i] = fnma(x[i], l, *reinterpret_cast<const cx<double>*>(u + i));
+      for (int i = G; i < N; ++i)
+        if (TPR * i >= i0) {
+          x[i] = fnma(x[i], l, sent(u, TPR * i + h));
+        } else if (TPR * i + h >= i0) {
+          x[i] = fnma(x[i], l, sent(u, TPR * i + h));
+        }
   }
   __device__ __forceinline__ void shift() {
 #pragma unroll
-    for (int i = 0; i + kGrp < W; ++i) x[i] = x[i + kGrp];
+    for (int i = 0; i + G < N; ++i) x[i] = x[i + G];
   }
 };
 template <>
-struct StripRow<float> {
+struct StripRow<float, 1> {
   static constexpr int W = strip_w<float>();
   float4 x[W / 2];  // columns 2 k, 2 k + 1: (re, re, im, im)
   __device__ __forceinline__ cx<float> get(int i) const {
@@ -204,9 +230,21 @@ struct StripRow<float> {
       x[i / 2].z = v.im;
     }
   }
-  __device__ __forceinline__ uint4 chunk(int k) const {
-    return make_uint4(__float_as_uint(x[k].x), __float_as_uint(x[k].y), __float_as_uint(x[k].z),
-                      __float_as_uint(x[k].w));
+  __device__ __forceinline__ void load(const cx<float>* row, int) {
+#pragma unroll
+    for (int c = 0; c < W; ++c) set(c, row[c]);
+  }
+  __device__ __forceinline__ void store(int i0, int jb, cx<float>* row, int) const {
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+      if (i >= i0 && jb + i < W) row[i] = get(i);
+  }
+  __device__ __forceinline__ void stage(int i0, int jb, uint4* u, int) const {
+#pragma unroll
+    for (int k = 0; k < W / 2; ++k)
+      if (k >= i0 / 2 && jb / 2 + k < W / 2)
+        u[k] = make_uint4(__float_as_uint(x[k].x), __float_as_uint(x[k].y), __float_as_uint(x[k].z),
+                          __float_as_uint(x[k].w));
   }
   static __device__ __forceinline__ cx<float> sent(const uint4* u, int c) {
     const float* f = reinterpret_cast<const float*>(u + c / 2) + (c & 1);
@@ -224,7 +262,7 @@ struct StripRow<float> {
   // the pivot row (within the exchange's memory): the packed multiply-adds cost
   // less than the branches around them, which would expose the loads' latency
   // once per group.
-  __device__ __forceinline__ void update(int i0, int jb, cx<float> l, const uint4* u) {
+  __device__ __forceinline__ void update(int i0, int jb, cx<float> l, const uint4* u, int) {
     const float2 nr = make_float2(-l.re, -l.re), ni = make_float2(-l.im, -l.im), pi = make_float2(l.im, l.im);
     auto pair = [&](int k) {
       const float4 v = *reinterpret_cast<const float4*>(u + k);
@@ -277,8 +315,9 @@ __host__ __device__ constexpr size_t strip_smem(int R, int nother) {
   return sizeof(StripShared<T, CL>) + sizeof(cx<T>) * (((size_t)R * (W + 1) + 1) / 2 * 2 + (size_t)2 * W * nother);
 }
 
-template <class T, int CL>
+template <class T, int CL, int TPR>
 __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs<T> a) {
+  using Row = StripRow<T, TPR>;
   constexpr int W = strip_w<T>(), LD = W + 1;
   constexpr int kVec = 16 / (int)sizeof(cx<T>);  // columns of a chunk
   using Sh = StripShared<T, CL>;
@@ -286,6 +325,7 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
   using Key = KeyOf<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int q = (int)cl_rank(), R = a.rows_per_cta, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r = tid / TPR, h = tid % TPR;  // this thread's row and its place in it
   const int nwarp = blockDim.x >> 5;
   const int w = a.w, k0 = a.k0;
   // this CTA's rows k0 + q, k0 + q + CL, ...: dealt out one by one, so that the
@@ -333,25 +373,23 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
   const uint32_t cpeer = cl_map(&sh, lane < CL ? lane : 0), self = (uint32_t)__cvta_generic_to_shared(&sh);
   auto off = [&](const void* p) { return (uint32_t)__cvta_generic_to_shared(p) - self; };
   __syncthreads();
-  StripRow<T> x;
-  if (tid < Rq)
-#pragma unroll
-    for (int c = 0; c < W; ++c) x.set(c, S[tid * LD + c]);
-  unsigned pos = (unsigned)row(tid);
-  bool live = tid < Rq;  // not yet a pivot row
+  Row x;
+  if (r < Rq) x.load(S + r * LD, h);
+  unsigned pos = (unsigned)row(r);
+  bool live = r < Rq;  // not yet a pivot row
   cl_sync();             // every CTA runs, with its barriers set up, before the first push
   cx<T> lp;                      // kAhead: this row's multiplier of the step before,
   const uint4* pu = nullptr;     // its pivot row,
   bool pend = false;             // and whether the columns after the next are still to be updated with them
   int buf = 0;
-  const int hw = kAhead<T> && blockDim.x >= (unsigned)R + 64 ? nwarp - 2 : -1;  // the first of two warps without rows
+  const int hw = kAhead<T> && blockDim.x >= (unsigned)(TPR * R) + 64 ? nwarp - 2 : -1;  // the first of two warps without rows
   // the staged row to all CTAs, a half warp for half of them; l: kAhead, its multiplier of the step before
   auto put_row = [&](int j, int par, cx<T> l) {
     const int c = lane & 15;
     if (c < j / kVec) return;
     uint4 v = sh.stage[c];
     if constexpr (kAhead<T>)
-      if (pend && c > j) v = StripRow<T>::pack(fnma(StripRow<T>::sent(sh.stage, c), l, StripRow<T>::sent(pu, c)));
+      if (pend && c > j) v = Row::pack(fnma(Row::sent(sh.stage, c), l, Row::sent(pu, c)));
     const uint32_t oc = off(&sh.crow[buf][q][c]), ob = off(&sh.colbar[par]);
 #pragma unroll
     for (int i = 0; i < CL / 2; ++i) cl_put(peer[i] + oc, v, peer[i] + ob);
@@ -387,14 +425,15 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
       if (tid == 0)
         bar_expect(&sh.colbar[par], CL * (uint32_t)(sizeof(StripCand<T>) + 16 * (Sh::kCh - j / kVec)));
       // this CTA's candidate: over the warp, then over the warps
-      Key key = live ? val_key(cabs1(x.get(jj))) : Key(0);
+      const bool has = TPR == 1 || h == jj % TPR;  // this thread has column jj of its row
+      Key key = live && has ? val_key(cabs1(x.get(jj))) : Key(0);
       unsigned p = key ? pos : ~0u;
       key = warp_best(key, p);
       if (lane == 0) {
         wkey[par][warp] = key;
         wpos[par][warp] = p;
       }
-      if (hw >= 0 && live && key != 0 && pos == p) wval[par][warp] = x.get(jj);
+      if (hw >= 0 && live && has && key != 0 && pos == p) wval[par][warp] = x.get(jj);
       __syncthreads();
       key = lane < nwarp ? wkey[par][lane] : Key(0);
       p = key ? wpos[par][lane] : ~0u;
@@ -405,14 +444,12 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
       const unsigned ob = __ballot_sync(~0u, own);
       const bool owns = key ? ob != 0 : warp == 0;  // the warp whose lane has the candidate
       if (owns && own) {
-#pragma unroll
-        for (int k = 0; k < Sh::kCh; ++k)
-          if (k >= jj / kVec && jb / kVec + k < Sh::kCh) sh.stage[jb / kVec + k] = x.chunk(k);
-        if (hw >= 0) stage_l = lp;
+        x.stage(jj, jb, sh.stage + jb / kVec, h);
+        if (hw >= 0 && h == 0) stage_l = lp;
       }
       if (hw < 0) {
         if (owns) {
-          const int lo = key ? __ffs(ob) - 1 : 0;
+          const int lo = key ? __ffs(ob) - 1 + jj % TPR : 0;
           const cx<T> xj = x.get(jj);
           const cx<T> pv(__shfl_sync(~0u, xj.re, lo), __shfl_sync(~0u, xj.im, lo));
           cx<T> l;
@@ -432,7 +469,7 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
         asm volatile("bar.arrive 1, 64;\n" ::: "memory");
       }
       if constexpr (kAhead<T>)
-        if (pend && (hw < 0 || warp < hw)) x.update(jj + 1, jb, lp, pu + jb);
+        if (pend && (hw < 0 || warp < hw)) x.update(jj + 1, jb, lp, pu + jb, h);
       bar_wait(&sh.colbar[par], (j >> 1) & 1, fail);
       // the pivot among the CTAs' candidates (each warp for itself)
       key = lane < CL ? sh.cand[par][lane < CL ? lane : 0].key : Key(0);
@@ -446,12 +483,10 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
         }
         if (live) {
           if (pos == (unsigned)row_j) {
-#pragma unroll
-            for (int i = 0; i < W; ++i)
-              if (i >= jj && jb + i < W) S[tid * LD + jb + i] = x.get(i);
+            x.store(jj, jb, S + r * LD + jb, h);
             live = false;
-          } else {
-            S[tid * LD + j] = x.get(jj);
+          } else if (has) {
+            S[r * LD + j] = x.get(jj);
           }
         }
         pend = false;
@@ -460,6 +495,11 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
       }
       const int src = __ffs(__ballot_sync(~0u, mine == p)) - 1;  // positions are distinct: one CTA
       if (q == 0 && tid == 0) a.ipiv[row_j] = p < (unsigned)a.n ? (int)p : row_j;
+      cx<T> xj = x.get(jj);
+      if (TPR > 1) {
+        const int from = (lane & ~(TPR - 1)) | jj % TPR;
+        xj = cx<T>(__shfl_sync(~0u, xj.re, from), __shfl_sync(~0u, xj.im, from));
+      }
       if (live) {
         if (pos == p) {
           pos = (unsigned)row_j;
@@ -467,19 +507,19 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
         } else {
           if (pos == (unsigned)row_j) pos = p;
           const cx<T> rp(sh.cand[par][src].rre, sh.cand[par][src].rim);
-          const cx<T> l = x.get(jj) * rp;
-          S[tid * LD + j] = l;
+          const cx<T> l = xj * rp;
+          if (has) S[r * LD + j] = l;
           if constexpr (kAhead<T>) {
             lp = l;
-            if (j + 1 < W) x.set(jj + 1, fnma(x.get(jj + 1), l, StripRow<T>::sent(sh.crow[buf][src], j + 1)));
+            if (j + 1 < W && (TPR == 1 || h == (jj + 1) % TPR)) x.set(jj + 1, fnma(x.get(jj + 1), l, Row::sent(sh.crow[buf][src], j + 1)));
           } else {
-            x.update(jj + 1, jb, l, &sh.crow[buf][src][jb / kVec]);
+            x.update(jj + 1, jb, l, &sh.crow[buf][src][jb / kVec], h);
           }
         }
       }
       // the pivot row's columns from j on, final now, from the exchange to its place (its owner's warp)
       if (src == q && ob != 0 && lane >= j && lane < W)
-        S[(warp * 32 + __ffs(ob) - 1) * LD + lane] = StripRow<T>::sent(sh.crow[buf][src], lane);
+        S[(warp * 32 + __ffs(ob) - 1) / TPR * LD + lane] = Row::sent(sh.crow[buf][src], lane);
       pend = true;
       pu = sh.crow[buf][src];
       buf = buf + 1 == Sh::kBuf ? 0 : buf + 1;
@@ -489,11 +529,11 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
   grid_trigger();
   // rows to their positions; rows that moved or became pivot rows take the
   // block's other columns along
-  if (tid < Rq) {
-    fpos[tid] = (int)pos;
-    if (nother > 0 && (pos != (unsigned)row(tid) || pos < (unsigned)(k0 + w))) {
+  if (r < Rq && h == 0) {
+    fpos[r] = (int)pos;
+    if (nother > 0 && (pos != (unsigned)row(r) || pos < (unsigned)(k0 + w))) {
       const int i = atomicAdd(&nmoved, 1);
-      if (i < 2 * W) mlist[i] = tid;
+      if (i < 2 * W) mlist[i] = r;
     }
   }
   __syncthreads();
@@ -627,14 +667,24 @@ bool strip_available(int device) {
     const int smem = (int)strip_smem<T, 16>(kStripThreads, 128 - strip_w<T>());
     const char* off = getenv("M25_NO_CLUSTER_PANEL");
     bool yes = !(off && *off == '1') && smem + 8192 <= optin &&
-               cudaFuncSetAttribute(strip_panel_kernel<T, 16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+               cudaFuncSetAttribute(strip_panel_kernel<T, 16, 1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
                    cudaSuccess &&
-               cudaFuncSetAttribute(strip_panel_kernel<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+               cudaFuncSetAttribute(strip_panel_kernel<T, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
                    cudaSuccess &&
-               cudaFuncSetAttribute(strip_panel_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+               cudaFuncSetAttribute(strip_panel_kernel<T, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
                    cudaSuccess &&
-               cudaFuncSetAttribute(strip_panel_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+               cudaFuncSetAttribute(strip_panel_kernel<T, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
                    cudaSuccess;
+    if constexpr (sizeof(T) == 8) {
+      const auto set = [&](auto kernel, bool wide) {
+        yes = yes && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+              (!wide || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess);
+      };
+      set(strip_panel_kernel<T, 8, 2>, false);
+      set(strip_panel_kernel<T, 8, 4>, false);
+      set(strip_panel_kernel<T, 16, 2>, true);
+      set(strip_panel_kernel<T, 16, 4>, true);
+    }
     if (yes) {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1];
@@ -648,7 +698,7 @@ bool strip_available(int device) {
       cfg.attrs = at;
       cfg.numAttrs = 1;
       int nclusters = 0;
-      yes = cudaOccupancyMaxActiveClusters(&nclusters, strip_panel_kernel<T, 16>, &cfg) == cudaSuccess && nclusters > 0;
+      yes = cudaOccupancyMaxActiveClusters(&nclusters, strip_panel_kernel<T, 16, 1>, &cfg) == cudaSuccess && nclusters > 0;
     }
     cudaGetLastError();  // a refused attribute only means: no cluster panel
     return yes;
@@ -656,7 +706,7 @@ bool strip_available(int device) {
   return ok;
 }
 
-template <class T, int CL>
+template <class T, int CL, int TPR = 1>
 cudaError_t launch_strip(const StripArgs<T>& a, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
@@ -667,13 +717,25 @@ cudaError_t launch_strip(const StripArgs<T>& a, cudaStream_t st) {
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(CL);
-  const int rows = (a.rows_per_cta + 31) / 32 * 32;
+  const int rows = (TPR * a.rows_per_cta + 31) / 32 * 32;
   cfg.blockDim = dim3(kAhead<T> && rows + 64 <= kStripThreads ? rows + 64 : std::max(64, rows));
   cfg.dynamicSmemBytes = strip_smem<T, CL>(a.rows_per_cta, a.blk1 - a.blk0 - a.w);
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, strip_panel_kernel<T, CL>, a);
+  return cudaLaunchKernelEx(&cfg, strip_panel_kernel<T, CL, TPR>, a);
+}
+
+// complex128: as many lanes per row as give the four sub-partitions of the SM a warp each, as each has its own fp64
+// unit (panel of N = 546 / 1085: 1.75 / 3.52 -> 1.43 / 2.98 ms). Beyond 64 rows the warps of single lanes already share
+// them out: two lanes each would only double the warps.
+template <class T, int CL>
+cudaError_t launch_rows(const StripArgs<T>& a, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8) {
+    if (a.rows_per_cta <= 32) return launch_strip<T, CL, 4>(a, st);
+    if (a.rows_per_cta <= 64) return launch_strip<T, CL, 2>(a, st);
+  }
+  return launch_strip<T, CL>(a, st);
 }
 
 }  // namespace
@@ -705,8 +767,8 @@ int lu_strip_block(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int b0, int bw, i
     StripArgs<T> a{A, lda, n, k0, w, b0, b0 + bw, (m + CL - 1) / CL, ipiv, Ub, info, err};
     StageTimer tm(ctx, ST_PANEL);
     if (CL == 4) M25_CUDA((launch_strip<T, 4>(a, ctx->stream)));
-    else if (CL == 8) M25_CUDA((launch_strip<T, 8>(a, ctx->stream)));
-    else M25_CUDA((launch_strip<T, 16>(a, ctx->stream)));
+    else if (CL == 8) M25_CUDA((launch_rows<T, 8>(a, ctx->stream)));
+    else M25_CUDA((launch_rows<T, 16>(a, ctx->stream)));
     const int nc = b0 + bw - k0 - w;
     if (nc > 0) {
       const dim3 grid((nc + StripUpd<T>::CG - 1) / StripUpd<T>::CG, (n - k0 - w + StripUpd<T>::TR - 1) / StripUpd<T>::TR);
