@@ -894,26 +894,34 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-constexpr int kTileLd = 65;  // padded row of a 64-wide tile in shared memory
+// Rows of a block of the triangular sweeps. complex64: 64, as a step's latencies (the flag, the
+// barriers) bound the chain. complex128: 32, as the fp64 operations on the chain do - the
+// substitution and the last tile's product, both of which halve per row - and the
+// rest of a block's products runs beside it (N = 546 / 1085 / 2434 / 5943, all sweeps of a solve with
+// two right-hand sides: 0.49 / 0.91 / 2.03 / 5.1 ms, 0.63 / 1.19 / 2.71 / 6.45 ms with 64).
+template <class TV>
+__host__ __device__ constexpr int wave_b() { return sizeof(TV) == 8 ? 32 : 64; }
+template <int B>
+constexpr int kTileLd = B + 1;  // padded row of a tile in shared memory
 
-// fetch the w x 64 tile at (r0, c0) (columns >= wc zero) into a (64, 65) shared buffer; one commit group
-template <class TF>
+// fetch the w x B tile at (r0, c0) (columns >= wc zero) into a (B, B + 1) shared buffer; one commit group
+template <int B, class TF>
 __device__ __forceinline__ void fetch_tile(cx<TF>* dst, const cx<TF>* A, int64_t lda, int r0, int c0, int w, int wc) {
-  for (int e = threadIdx.x; e < w * 64; e += blockDim.x) {
-    int r = e >> 6, c = e & 63;
+  for (int e = threadIdx.x; e < w * B; e += blockDim.x) {
+    int r = e / B, c = e % B;
     const cx<TF>* src = A + (int64_t)(r0 + r) * lda + c0 + (c < wc ? c : 0);
-    cp_async_elem<sizeof(cx<TF>)>(&dst[r * kTileLd + c], src, c < wc);
+    cp_async_elem<sizeof(cx<TF>)>(&dst[r * kTileLd<B> + c], src, c < wc);
   }
   cp_async_commit();
 }
 
-// the diagonal w x w tile at (r0, r0), transposed: DgT[c * 65 + r] = A[r0 + r][r0 + c]; one commit group
-template <class TF>
+// the diagonal w x w tile at (r0, r0), transposed: DgT[c * (B + 1) + r] = A[r0 + r][r0 + c]; one commit group
+template <int B, class TF>
 __device__ __forceinline__ void fetch_diag_t(cx<TF>* DgT, const cx<TF>* A, int64_t lda, int r0, int w) {
-  for (int e = threadIdx.x; e < w * 64; e += blockDim.x) {
-    int r = e >> 6, c = e & 63;
+  for (int e = threadIdx.x; e < w * B; e += blockDim.x) {
+    int r = e / B, c = e % B;
     const cx<TF>* src = A + (int64_t)(r0 + r) * lda + r0 + (c < w ? c : 0);
-    cp_async_elem<sizeof(cx<TF>)>(&DgT[c * kTileLd + r], src, c < w);
+    cp_async_elem<sizeof(cx<TF>)>(&DgT[c * kTileLd<B> + r], src, c < w);
   }
   cp_async_commit();
 }
@@ -931,42 +939,19 @@ __device__ __forceinline__ void fetch_diag_t(cx<TF>* DgT, const cx<TF>* A, int64
 // are scaled by the reciprocal diagonal at the end); a select per round made it
 // divergent, 180 cycles a round against 83. Rounds beyond the block's rows
 // change nothing.
-template <class TF, class TV>
+template <class TF>
 __device__ __forceinline__ void diag_solve1(int lane, int w, int P, int c, int upper, const cx<TF>* DgT,
-                                            const cx<TV>* dinv, cx<TV>* acc) {
+                                            const zf* dinv, zf* acc) {
+  using TV = float;
   const int ra = 2 * lane, rb = ra + 1;
   cx<TV> va = ra < w ? acc[ra * P + c] : cx<TV>();
   cx<TV> vb = rb < w ? acc[rb * P + c] : cx<TV>();
   auto bcast = [](cx<TV> v, int k) { return cx<TV>(__shfl_sync(0xffffffffu, v.re, k), __shfl_sync(0xffffffffu, v.im, k)); };
   const cx<TV> da = upper ? ldc(dinv + ra) : cx<TV>(), db = upper ? ldc(dinv + rb) : cx<TV>();
-  if constexpr (sizeof(TV) == 8) {
-    // a column per round: the fp64 operations bound it, not the shuffles (the
-    // pair's second value formed in every lane costs four of twenty)
-    if (!upper) {
-#pragma unroll 2
-      for (int k = 0; k < 32; ++k)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const cx<TF>* cc = DgT + (2 * k + h) * kTileLd;
-          const cx<TV> x = bcast(h ? vb : va, k);
-          va = fnma(va, cx<TV>(ldc(cc + ra)), x);
-          vb = fnma(vb, cx<TV>(ldc(cc + rb)), x);
-        }
-    } else {
-#pragma unroll 2
-      for (int k = 31; k >= 0; --k)
-#pragma unroll
-        for (int h = 1; h >= 0; --h) {
-          const cx<TF>* cc = DgT + (2 * k + h) * kTileLd;
-          const cx<TV> x = bcast(h ? vb * db : va * da, k);
-          va = fnma(va, cx<TV>(ldc(cc + ra)), x);
-          vb = fnma(vb, cx<TV>(ldc(cc + rb)), x);
-        }
-    }
-  } else if (!upper) {
+  if (!upper) {
 #pragma unroll 4
     for (int k = 0; k < 32; ++k) {
-      const cx<TF>*ca = DgT + (2 * k) * kTileLd, *cb = ca + kTileLd;  // columns 2 k, 2 k + 1
+      const cx<TF>*ca = DgT + (2 * k) * kTileLd<64>, *cb = ca + kTileLd<64>;  // columns 2 k, 2 k + 1
       const cx<TV> aA(ca[ra]), bA(ca[rb]), aB(cb[ra]), bB(cb[rb]);
       // owner (lane k): x_2k is final, x_2k+1 = v_2k+1 - L[2k+1][2k] x_2k
       const cx<TV> xa = bcast(va, k), xb = bcast(fnma(vb, bA, va), k);
@@ -976,7 +961,7 @@ __device__ __forceinline__ void diag_solve1(int lane, int w, int P, int c, int u
   } else {
 #pragma unroll 4
     for (int k = 31; k >= 0; --k) {
-      const cx<TF>*ca = DgT + (2 * k) * kTileLd, *cb = ca + kTileLd;
+      const cx<TF>*ca = DgT + (2 * k) * kTileLd<64>, *cb = ca + kTileLd<64>;
       const cx<TV> aA(ca[ra]), bA(ca[rb]), aB(cb[ra]), bB(cb[rb]);
       // owner: x_2k+1 = v_2k+1 / d, then x_2k = (v_2k - U[2k][2k+1] x_2k+1) / d
       const cx<TV> ob = vb * db, oa = fnma(va, aB, ob) * da;
@@ -993,6 +978,25 @@ __device__ __forceinline__ void diag_solve1(int lane, int w, int P, int c, int u
   if (rb < w) acc[rb * P + c] = vb;
 }
 
+// complex128, 32 rows: lane l owns row l, a column per round (the fp64 operations bound it: four a round, eight
+// for the upper factor, whose solved value every lane forms).
+template <class TF>
+__device__ __forceinline__ void diag_solve1(int lane, int w, int P, int c, int upper, const cx<TF>* DgT,
+                                            const zd* dinv, zd* acc) {
+  zd v = lane < w ? acc[lane * P + c] : zd();
+  auto bcast = [](zd u, int k) { return zd(__shfl_sync(0xffffffffu, u.re, k), __shfl_sync(0xffffffffu, u.im, k)); };
+  const zd d = upper ? ldc(dinv + lane) : zd();
+  if (!upper) {
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) v = fnma(v, zd(DgT[k * kTileLd<32> + lane]), bcast(v, k));
+  } else {
+#pragma unroll 4
+    for (int k = 31; k >= 0; --k) v = fnma(v, zd(DgT[k * kTileLd<32> + lane]), bcast(v * d, k));
+    v = v * d;
+  }
+  if (lane < w) acc[lane * P + c] = v;
+}
+
 // tiles in flight per CTA: 4 complex64 or 2 complex128 tiles
 template <class TF>
 constexpr int wave_stages() {
@@ -1001,64 +1005,65 @@ constexpr int wave_stages() {
 constexpr int kYtWords = 64 * 8 * 2;  // tagged words of one block of y (64 rows, up to 8 right-hand sides)
 template <class TF, class TV>
 constexpr size_t wave_smem() {
-  return sizeof(cx<TF>) * 64 * kTileLd * (1 + wave_stages<TF>()) + sizeof(cx<TV>) * (64 * 8 * 2 + 64) +
+  constexpr int B = wave_b<TV>();
+  return sizeof(cx<TF>) * B * kTileLd<B> * (1 + wave_stages<TF>()) + sizeof(cx<TV>) * (B * 8 * 2 + B) +
          (sizeof(TV) == 4 ? sizeof(unsigned long long) * kYtWords * wave_stages<TF>() : 0);
 }
 
 // One triangular sweep as a dependency wavefront (no grid barriers): CTA g
-// owns the 64-row blocks g, g + G, ... For its block i it subtracts the
+// owns the blocks g, g + G, ... of wave_b rows. For its block i it subtracts the
 // tile products A_ij y_j of the blocks j it depends on (j < i for the unit
 // lower factor, j > i for the upper one, in the order they become final) as
 // soon as block j is flagged final, solves the diagonal block by
 // substitution, publishes y_i and raises flag i. The off-diagonal tiles
 // stream through a ring of cp.async stages so that a CTA's backlog of tiles
 // never holds up the chain; the chain step itself is the flag round trip,
-// one 64 x 64 tile product and the substitution, which one warp runs in
-// registers (lane l owns rows 2l and 2l + 1; each solved pair is broadcast with
+// one tile product and the substitution, which one warp runs in
+// registers (complex64: lane l owns rows 2l and 2l + 1; each solved pair is broadcast with
 // shuffles; the upper sweep multiplies by the reciprocal diagonal). It is
 // bound by that chain, not by the factors' bytes: all sweeps of a solve, two
 // right-hand sides, N = 1085 / 3789 / 5943 in complex64 0.35 / 1.85 / 1.69 ms
 // (0.46 / 2.51 / 2.33 ms with a select per round and one lane per row of the
-// tile product), N = 546 / 2434 / 5943 in complex128 0.65 / 2.80 / 6.65 ms (0.90 /
-// 3.96 / 9.6 ms). Every
+// tile product), N = 546 / 2434 / 5943 in complex128 0.49 / 2.03 / 5.1 ms (0.90 /
+// 3.96 / 9.6 ms, and blocks of 64 rows). Every
 // wait is bounded; blocks only wait on blocks solved earlier, and the
 // cooperative launch keeps all CTAs resident, so the order cannot deadlock.
 template <class TF, class TV>
 __global__ void __launch_bounds__(256, 1) trsv_wave_kernel(WaveArgs<TF, TV> a) {
-  constexpr int S = wave_stages<TF>();
+  constexpr int S = wave_stages<TF>(), B = wave_b<TV>(), LD = kTileLd<B>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cx<TF>* Dg = reinterpret_cast<cx<TF>*>(smem_raw);  // (64, 65) diagonal tile, transposed
-  cx<TF>* ring = Dg + 64 * kTileLd;                   // S x (64, 65) off-diagonal tiles
-  cx<TV>* acc = reinterpret_cast<cx<TV>*>(ring + S * 64 * kTileLd);  // (64, P)
-  cx<TV>* y = acc + 64 * 8;                                            // (64, P)
-  cx<TV>* dinv = y + 64 * 8;                                           // (64) reciprocal diagonal
+  cx<TF>* Dg = reinterpret_cast<cx<TF>*>(smem_raw);  // (B, B + 1) diagonal tile, transposed
+  cx<TF>* ring = Dg + B * LD;                   // S x (B, B + 1) off-diagonal tiles
+  cx<TV>* acc = reinterpret_cast<cx<TV>*>(ring + S * B * LD);  // (B, P)
+  cx<TV>* y = acc + B * 8;                                            // (B, P)
+  cx<TV>* dinv = y + B * 8;                                           // (B) reciprocal diagonal
   constexpr bool kTagged = sizeof(TV) == 4;
-  unsigned long long* yring = reinterpret_cast<unsigned long long*>(dinv + 64);  // S x kYtWords (tagged)
+  unsigned long long* yring = reinterpret_cast<unsigned long long*>(dinv + B);  // S x kYtWords (tagged)
   const unsigned tag = (unsigned)a.epoch;
   __shared__ int fail;
   const int G = gridDim.x, P = a.nrhs, tid = threadIdx.x;
-  const int nblk = (a.n + 63) / 64;
+  const int nblk = (a.n + B - 1) / B;
   if (tid == 0) fail = 0;
   __syncthreads();
   for (int q = blockIdx.x; q < nblk; q += G) {
     const int i = a.upper ? nblk - 1 - q : q;
-    const int r0 = i * 64, w = min(64, a.n - r0);
+    const int r0 = i * B, w = min(B, a.n - r0);
     // dependencies in the order they become final: j = 0 .. i-1 (lower) or nblk-1 .. i+1 (upper)
     const int ndep = a.upper ? nblk - 1 - i : i;
     auto dep = [&](int d) { return a.upper ? nblk - 1 - d : d; };
     // the tile of dependency d (and, for tagged vectors, the published y_j as
     // it stands now) into ring slot d % S; one commit group per dependency
     auto fetch_dep = [&](int d) {
-      const int j = dep(d), wj = min(64, a.n - j * 64);
+      const int j = dep(d), wj = min(B, a.n - j * B);
       if constexpr (kTagged) {
         unsigned long long* ys = yring + (d % S) * kYtWords;
         for (int e = threadIdx.x; e < wj * P; e += blockDim.x)  // 16 bytes = one complex value, L2 only
-          cp_async_elem<16>(ys + 2 * e, a.Yt + ((int64_t)j * 64 * P + e) * 2, true);
+          cp_async_elem<16>(ys + 2 * e, a.Yt + ((int64_t)j * B * P + e) * 2, true);
       }
-      fetch_tile(ring + (d % S) * 64 * kTileLd, a.A, a.lda, r0, j * 64, w, wj);
+      fetch_tile<B>(ring + (d % S) * B * LD, a.A, a.lda, r0, j * B, w, wj);
     };
     // commit groups: the diagonal tile, then one per dependency (dependency d is group d + 1)
-    fetch_diag_t(Dg, a.A, a.lda, r0, w);
+    fetch_diag_t<B>(Dg, a.A, a.lda, r0, w);
     for (int d = 0; d < S; ++d) {
       if (d < ndep) fetch_dep(d);
       else cp_async_commit();
@@ -1068,25 +1073,25 @@ __global__ void __launch_bounds__(256, 1) trsv_wave_kernel(WaveArgs<TF, TV> a) {
     // this sweep's triangle (zero elsewhere); the first step's barrier
     // separates the two, the next barrier publishes the result
     auto prep_diag = [&]() {
-      if (tid < 64) {
+      if (tid < B) {
         cx<TV> di;
         if (a.upper && tid < w) {
-          const cx<TV> dd(Dg[tid * kTileLd + tid]);
+          const cx<TV> dd(Dg[tid * LD + tid]);
           const TV m2 = dd.re * dd.re + dd.im * dd.im;
           di = cx<TV>(dd.re / m2, -dd.im / m2);
         }
         dinv[tid] = di;
       }
       __syncthreads();
-      for (int e = tid; e < 64 * 64; e += blockDim.x) {
-        const int col = e >> 6, r = e & 63;
+      for (int e = tid; e < B * B; e += blockDim.x) {
+        const int col = e / B, r = e % B;
         const bool keep = r < w && col < w && (a.upper ? r < col : r > col);
-        if (!keep) Dg[col * kTileLd + r] = cx<TF>();
+        if (!keep) Dg[col * LD + r] = cx<TF>();
       }
     };
     for (int d = 0; d < ndep; ++d) {
-      const int j = dep(d), c0 = j * 64, wj = min(64, a.n - c0);
-      const cx<TF>* T = ring + (d % S) * 64 * kTileLd;
+      const int j = dep(d), c0 = j * B, wj = min(B, a.n - c0);
+      const cx<TF>* T = ring + (d % S) * B * LD;
       if constexpr (kTagged) {
         cp_async_wait<S - 1>();  // tile d and the prefetched y_j have landed
         __syncthreads();
@@ -1094,12 +1099,12 @@ __global__ void __launch_bounds__(256, 1) trsv_wave_kernel(WaveArgs<TF, TV> a) {
         // words of y_j not yet final when prefetched are polled until they carry this sweep's tag
         const unsigned long long* ys = yring + (d % S) * kYtWords;
         bool bad = false;
-        for (int e = tid; e < 64 * P * 2; e += blockDim.x) {
+        for (int e = tid; e < B * P * 2; e += blockDim.x) {
           float f = 0.f;
           if (e < wj * P * 2) {
             unsigned long long v = ys[e];
             if ((unsigned)(v >> 32) != tag) {
-              const volatile unsigned long long* g = a.Yt + (int64_t)j * 64 * P * 2 + e;
+              const volatile unsigned long long* g = a.Yt + (int64_t)j * B * P * 2 + e;
               long long it = 0;
               while (true) {
                 v = *g;
@@ -1141,7 +1146,7 @@ __global__ void __launch_bounds__(256, 1) trsv_wave_kernel(WaveArgs<TF, TV> a) {
           cp_async_wait<0>();
           return;
         }
-        for (int e = tid; e < 64 * P; e += blockDim.x) {
+        for (int e = tid; e < B * P; e += blockDim.x) {
           if (e < wj * P) {
             volatile cx<TV>* src = &a.X[(int64_t)c0 * P + e];
             y[e] = cx<TV>(src->re, src->im);
@@ -1151,19 +1156,20 @@ __global__ void __launch_bounds__(256, 1) trsv_wave_kernel(WaveArgs<TF, TV> a) {
         }
         __syncthreads();
       }
-      // the tile's product: four lanes per row, 16 columns each, two right-hand
+      // the tile's product: kL lanes per row, kC columns each, two right-hand
       // sides at a time. The lanes start at different columns so that a half
-      // warp's loads (4 rows x 4 lanes) fall into different banks
+      // warp's loads fall into different banks
       {
-        const int part = tid & 3, r = tid >> 2;
-        const cx<TF>* Tr = T + r * kTileLd + 16 * part;
+        constexpr int kL = 256 / B, kC = B / kL;
+        const int part = tid & (kL - 1), r = (unsigned)tid / kL;
+        const cx<TF>* Tr = T + r * LD + kC * part;
         for (int c = 0; c < P; c += 2) {
           const bool two = c + 1 < P;
-          const cx<TV>* yc = y + 16 * part * P + c;
+          const cx<TV>* yc = y + kC * part * P + c;
           cx<TV> s[2][2];  // minus the product, in two sums per right-hand side
 #pragma unroll 8
-          for (int i = 0; i < 16; ++i) {
-            const int t = (i + 4 * part) & 15;
+          for (int i = 0; i < kC; ++i) {
+            const int t = (i + 4 * part) & (kC - 1);
             const cx<TV> tv(ldc(Tr + t));
             s[0][i & 1] = fnma(s[0][i & 1], tv, ldc(yc + t * P));
             if (two) s[1][i & 1] = fnma(s[1][i & 1], tv, ldc(yc + t * P + 1));
@@ -1173,7 +1179,7 @@ __global__ void __launch_bounds__(256, 1) trsv_wave_kernel(WaveArgs<TF, TV> a) {
             if (q && !two) break;
             cx<TV> v = s[q][0] + s[q][1];
 #pragma unroll
-            for (int o = 1; o < 4; o <<= 1) {
+            for (int o = 1; o < kL; o <<= 1) {
               v.re += __shfl_xor_sync(0xffffffffu, v.re, o);
               v.im += __shfl_xor_sync(0xffffffffu, v.im, o);
             }
@@ -1193,7 +1199,7 @@ __global__ void __launch_bounds__(256, 1) trsv_wave_kernel(WaveArgs<TF, TV> a) {
     }
     // diagonal block: warp c solves right-hand side c (P <= 8 warps in parallel)
     const int warp = tid >> 5, lane = tid & 31;
-    if (warp < P) diag_solve1<TF, TV>(lane, w, P, warp, a.upper, Dg, dinv, acc);
+    if (warp < P) diag_solve1(lane, w, P, warp, a.upper, Dg, dinv, acc);
     __syncthreads();
     // publish y_i (warp 0)
     if (tid < 32) {
@@ -1253,7 +1259,8 @@ int lu_solve_wave(m25_ctx* ctx, const cx<TF>* A, int64_t lda, int n, const int32
     set_error("dense solve: at most 8 right-hand sides and n <= 51200");
     return M25_ERR_VALUE;
   }
-  const int nblk = (n + 63) / 64;
+  constexpr int kB = wave_b<TV>();
+  const int nblk = (n + kB - 1) / kB;
   // layout: [0] wait error, [16 ..] ready flag per block, then the
   // permutation when it is built here; zeroed whenever the buffer is
   // (re)allocated (a caller-provided buffer comes zeroed)
@@ -1286,6 +1293,11 @@ int lu_solve_wave(m25_ctx* ctx, const cx<TF>* A, int64_t lda, int n, const int32
     // (permutations, flags) must not pass for a tag of this sweep
     M25_CUDA(cudaMemsetAsync(Yt, 0, sizeof(unsigned long long) * 2 * (size_t)n * 8, st));
     ctx->yt_off = yt_off;
+  }
+  if (!ctx->ext_flags) {
+    // what another order's permutation or tagged copy left where this one's flags lie must not pass for a flag
+    if (!tagged && ctx->flags_nblk != nblk) M25_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * nblk, st));
+    ctx->flags_nblk = tagged ? -1 : nblk;
   }
   const size_t sm = wave_smem<TF, TV>();
   M25_CUDA(cudaFuncSetAttribute(trsv_wave_kernel<TF, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -1350,8 +1362,6 @@ int lu_wave_error(m25_ctx* ctx, int n, int* flag) {
 
 template int lu_solve_wave<double, double>(m25_ctx*, const zd*, int64_t, int, const int32_t*, const zd*, int, zd*,
                                            const int32_t*, bool);
-template int lu_solve_wave<float, double>(m25_ctx*, const zf*, int64_t, int, const int32_t*, const zd*, int, zd*,
-                                          const int32_t*, bool);
 template int lu_solve_wave<float, float>(m25_ctx*, const zf*, int64_t, int, const int32_t*, const zf*, int, zf*,
                                          const int32_t*, bool);
 
@@ -1908,7 +1918,7 @@ constexpr size_t kNoAllocPanelBytes = 64 + sizeof(m25::zd) * 2 * kNoAllocGmax * 
                                       sizeof(int) * 2 * kNoAllocGmax + sizeof(m25::zd) * 2 * 64;
 constexpr size_t kNoAllocFlagsOffset = (kNoAllocPanelBytes + 255) / 256 * 256;
 constexpr size_t kNoAllocPermOffset =
-    (kNoAllocFlagsOffset + sizeof(int) * (16 + M25_NOALLOC_MAX_N / 64 + 1) + 255) / 256 * 256;
+    (kNoAllocFlagsOffset + sizeof(int) * (16 + M25_NOALLOC_MAX_N / m25::wave_b<double>() + 1) + 255) / 256 * 256;
 static_assert(kNoAllocPermOffset + sizeof(int) * M25_NOALLOC_MAX_N <= M25_NOALLOC_SCRATCH_BYTES,
               "scratch too small for the declared maximum size");
 std::mutex g_noalloc_mu;
@@ -1966,7 +1976,7 @@ extern "C" int m25_dense_solve_noalloc(int32_t n, int32_t nrhs, void* Z, const v
   c.ext_flags = reinterpret_cast<int*>(base + kNoAllocFlagsOffset);
   // the array keeps the previous call's contents: clear the barrier words
   // (lu_factor clears its header) and the ready flags
-  M25_CUDA(cudaMemsetAsync(c.ext_flags, 0, sizeof(int) * (16 + (n + 63) / 64), c.stream));
+  M25_CUDA(cudaMemsetAsync(c.ext_flags, 0, sizeof(int) * (16 + n / m25::wave_b<double>() + 1), c.stream));
   int zinfo = 0;
   int rc = lu_factor<double>(&c, static_cast<zd*>(Z), n, n, ipiv, 64, false, &zinfo);
   if (rc) return rc;

@@ -81,6 +81,7 @@ struct m25_ctx {
   // candidates + barrier words; triangular-solve flags, already zeroed)
   char* ext_scratch = nullptr;
   int ext_gmax = 0;
+  int flags_nblk = -1;  // blocks whose ready flags the flag buffer holds
   int* ext_flags = nullptr;
   std::vector<char> host_tmp;
 };

@@ -216,3 +216,26 @@ def test_complex64_device_alignment(gpu, offset):
     b = B.cpu().numpy()
     # the refinement's own stop: the backward error (1e-12) of one column
     assert np.linalg.norm(r - (b[..., 0] + 1j * b[..., 1])) <= 1e-11 * np.linalg.norm(Z) * np.linalg.norm(out[0][3])
+
+
+@pytest.mark.parametrize("orders", [(1, 31, 32, 33, 63, 64, 65), (2100, 700, 2100, 97, 1500), (300, 2500, 129, 2500)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_solves_of_changing_order(gpu, orders, precision):
+    """Solves of one context at the edges of the sweeps' blocks and one order
+    after another: what an earlier one left in the flag buffer is no flag."""
+    from mom25d_gb300 import engine as E
+    from mom25d_gb300.solver import dense_solve
+
+    ctx = E.Context(0)
+    for k, n in enumerate(orders):
+        rng = np.random.default_rng(n + k)
+        A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 2 * np.sqrt(n) * np.eye(n)
+        B = rng.standard_normal((n, 3)) + 0j
+        for p in (precision, "fp64"):
+            X = dense_solve(A, B, precision=p, ctx=ctx)
+            # the solves' backward error (Higham, theorem 9.4, with the growth of these diagonally heavy matrices
+            # near one), or the refinement's stop at 1e-12
+            bound = 1e-12 if p == "mixed" else 8 * n * 2.0**-53
+            r = np.abs(A @ X - B).max(0)
+            assert np.all(r <= 4 * bound * (np.linalg.norm(A, np.inf) * np.abs(X).max(0) + np.abs(B).max(0)))
+    ctx.close()
