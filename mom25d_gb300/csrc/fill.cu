@@ -126,10 +126,12 @@ __device__ __forceinline__ int find_interval_f(const T* __restrict__ x, const fl
 }
 
 // Smooth parts S_A, S_V at radius r from the shared-memory table of one pair:
-// sum_p c[3-p] (r - x_i)^p by Horner's rule. The fp64 fill is bound by its fp64
-// operations (some 40 for a far point): with the powers of r - x_i formed first,
-// the area in every term and the interval compared in fp64 it had 48 and
+// sum_p c[3-p] (r - x_i)^p, in fp64 by Horner's rule. The fp64 fill is bound by its
+// fp64 operations (some 40 for a far point): with the powers of r - x_i formed
+// first, the area in every term and the interval compared in fp64 it had 48 and
 // took 1.94 / 5.77 / 24.6 ms at N = 1085 / 2434 / 5943, now 1.77 / 5.25 / 22.6 ms.
+// The fp32 passes are bound by latencies and gain nothing (2.18 and 2.16 ms at N =
+// 5943): they keep the sums as they were.
 template <class T>
 __device__ __forceinline__ void spline_av(const T* __restrict__ xs, const float* __restrict__ xf,
                                           const T* __restrict__ tab, int n, T r, cx<T>& sa, cx<T>& sv,
@@ -137,10 +139,18 @@ __device__ __forceinline__ void spline_av(const T* __restrict__ xs, const float*
   int i = find_interval_f(xs, xf, n, r, bk);
   T dx = r - xs[i];
   const T* c = tab + (size_t)i * 16;  // [power 0..3][A re, A im, V re, V im], highest power first
-  sa.re = c[12] + dx * (c[8] + dx * (c[4] + dx * c[0]));
-  sa.im = c[13] + dx * (c[9] + dx * (c[5] + dx * c[1]));
-  sv.re = c[14] + dx * (c[10] + dx * (c[6] + dx * c[2]));
-  sv.im = c[15] + dx * (c[11] + dx * (c[7] + dx * c[3]));
+  if constexpr (sizeof(T) == 8) {
+    sa.re = c[12] + dx * (c[8] + dx * (c[4] + dx * c[0]));
+    sa.im = c[13] + dx * (c[9] + dx * (c[5] + dx * c[1]));
+    sv.re = c[14] + dx * (c[10] + dx * (c[6] + dx * c[2]));
+    sv.im = c[15] + dx * (c[11] + dx * (c[7] + dx * c[3]));
+  } else {
+    const T z = dx, z2 = dx * dx, z3 = z2 * dx;
+    sa.re = c[12] + c[8] * z + c[4] * z2 + c[0] * z3;
+    sa.im = c[13] + c[9] * z + c[5] * z2 + c[1] * z3;
+    sv.re = c[14] + c[10] * z + c[6] * z2 + c[2] * z3;
+    sv.im = c[15] + c[11] * z + c[7] * z2 + c[3] * z3;
+  }
 }
 
 template <class T, int NQ, bool NEAR>
@@ -150,8 +160,10 @@ __device__ __forceinline__ void source_pass(int nrho, const TriData<T>& S, T dcx
                                             cx<T> cA, cx<T> cV, T dz, const T* st, int lane, cx<T> (&Q)[3],
                                             cx<T> (&Px)[3], cx<T> (&Py)[3], cx<T>& IV, const T (&tv)[3][2],
                                             Bk bk = Bk()) {
+  constexpr bool kF64 = sizeof(T) == 8;  // fewer operations per point where they are dear
+  const T inv4pi = T(1.0 / (4.0 * kPi));
   // the 1/R parts' coefficients (not NEAR)
-  const cx<T> rA = cA * T(1.0 / (4.0 * kPi)), rV = cV * T(1.0 / (4.0 * kPi));
+  const cx<T> rA = kF64 ? cA * inv4pi : cA, rV = kF64 ? cV * inv4pi : cV;
   cx<T> S0, SX, SY, T0, T1, T2;  // sums of w_k K over the test points k, weighted by 1, x_k, y_k
   T sq[NQ][2], sw[NQ];
 #pragma unroll
@@ -194,6 +206,7 @@ __device__ __forceinline__ void source_pass(int nrho, const TriData<T>& S, T dcx
         const T ri = rsqrt(R2);
         R = R2 * ri;
         inv = dz == T(0) ? ri : rsqrt(R2 + dz * dz);
+        if (!kF64) inv = inv4pi * inv;
       }
       cx<T> sa, sv;
       spline_av(xs, xf, tab, nrho, R, sa, sv, bk);
@@ -201,7 +214,7 @@ __device__ __forceinline__ void source_pass(int nrho, const TriData<T>& S, T dcx
         sa += rA * inv;
         sv += rV * inv;
       }
-      if (NQ == 1) {  // weighted by the source's area at the end
+      if (kF64 && NQ == 1) {  // weighted by the source's area at the end
         K0A = sa;
         K0V = sv;
         break;
@@ -226,7 +239,7 @@ __device__ __forceinline__ void source_pass(int nrho, const TriData<T>& S, T dcx
       T0 += K1x * wx + K1y * wy;
     }
   }
-  if (NQ == 1) {
+  if (kF64 && NQ == 1) {
     IV = IV * sw[0];
     S0 = S0 * sw[0];
     SX = SX * sw[0];
