@@ -240,8 +240,10 @@ int m25_dense_solve(m25_ctx* ctx, int32_t n, int32_t nrhs, int precision, void* 
 /* In-place LU factorisation with partial pivoting of an n x n row-major matrix
  * (scipy.linalg.lu_factor, used by _dense_solve, Engine/mom25d/solver.py:23):
  * precision M25_FP64 factors complex128, M25_MIXED complex64; trailing
- * updates on the tensor cores (complex128: from exact integer slices, the
- * same bits either way) unless flags & M25_LU_NO_TENSOR_CORES. On return A
+ * updates on the tensor cores (complex128: from exact integer slices, and by
+ * fp64 multiply-adds where an entry is too small beside its row's and column's
+ * largest for them; the same bits either way) unless flags &
+ * M25_LU_NO_TENSOR_CORES. On return A
  * holds L (unit lower, strictly below the diagonal) and U, ipiv the
  * 0-based row interchanges (row i swapped with ipiv[i], in order). A and ipiv
  * are host or device memory (where). info = first zero pivot (1-based) or 0. */

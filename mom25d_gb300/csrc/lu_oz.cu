@@ -31,12 +31,28 @@
 //     2^-53 for one fp64 rounding), those of one i + j accumulated together:
 //     at most 8 x 128 x 2^14 = 2^24, so every sum is an exact integer in fp32;
 //   - the eight sums combined in 64-bit integers and rounded once.
-// The result is as accurate as the fp64 sums it replaces: the solution of MoM
-// systems with vias is 2e-12 to 1.3e-9 off an extended-precision one, with
-// fp64 sums 7e-12 to 1.1e-9 and LAPACK 1.7e-11 to 3.5e-9; P A - L U of random
-// matrices is 1.33e-17 of |L| |U| (norms), with fp64 sums 1.59e-17.
+// What is left out is relative to the largest entries of the row and of the
+// column, which may belong to different inner indices (two weakly coupled
+// groups of unknowns; a column of L with few large entries beside full ones):
+// then the products are small beside it and no scaling helps. So each entry of
+// C is looked at: where neither C nor the largest of its 64 products reaches
+// 2^-kSpare of the product of the row's and the column's power of two, and
+// where the row or the column has a number that is not finite or below the
+// normal range, the entry is formed with fp64 multiply-adds instead (oz_dot).
+// kSpare = 5: the error in the mean, 2^-59 of that product, is then at most
+// 2^-54 of C or of the largest product, half an ulp. Both bound
+// (|L| |U|)_ij from below (C is L U of what is left of the matrix), so that
+// the factorisation keeps the componentwise bound of an fp64 one. The largest
+// |P A - L U| / |L| |U| of any entry, in a numpy restatement, against fp64 sums: normal
+// matrices 2.5e-16 (fp64 sums 2.5e-16), three MoM lines, two of them with vias, 5.4e-16, 5.9e-16, 5.2e-16
+// (5.4e-16, 6.3e-16, 6.7e-16; without the test 2.2e-15, 5.8e-15, 1.7e-15), two groups
+// coupled by 1e-8 2.4e-16 (2.4e-16; 7.2e-11), a column of L with tiny entries beside
+// full ones 3.5e-16 (3.5e-16; 4.4e-5). Entries that take the fp64
+// path: none of normal matrices', 0.04 to 1.1 % of MoM matrices', a quarter of
+// the potentials between cells in random order, half of two groups'.
 //
 // oz_scale_kernel sums the exponents, oz_pack_kernel slices L21 and U12;
+// oz_direct_kernel does the entries that are not left to the slices;
 // oz_gemm_kernel is a persistent kernel, one
 // CTA per SM: warp 0 loads 64B-swizzled tiles by TMA (the 8 digits of 128 rows
 // of A and of 64 rows of B, 32 k's at a time, 96 KB) into a ring of two stages,
@@ -46,9 +62,10 @@
 // while the next tile's products run. Every wait is bounded, as in lu_tc.cu.
 // What bounds it: the shared-memory reads of the MMAs (4 KB of A for every 32
 // cycles of products at N = 64) and, after that, three fp64 operations per
-// element. Measured on GB300, all updates of a factorisation with their
-// slicing, N = 546 / 1085 / 2434 / 5943: 0.34 / 0.75 / 3.1 / 28 ms; 3.55 / 8.8
-// / 64 / 771 ms with fp64 multiply-adds on the CUDA cores.
+// element. Measured on GB300, all updates of a factorisation of a normal matrix with their
+// slicing and the test, N = 546 / 1085 / 2434 / 5943: 0.37 / 0.85 / 3.7 / 33.5 ms (the test 4.4 ms of
+// the last); 3.55 / 8.8 / 64 / 771 ms with fp64 multiply-adds on the CUDA cores throughout. Potentials between
+// 1543 cells in random order 5.1 ms, 3.5 of them for the fp64 entries.
 #include <cuda.h>
 
 #include <algorithm>
@@ -74,7 +91,9 @@ constexpr int kOzStage = kDig * (kDigA + kDigB);
 constexpr int kOzSmem = kOzStages * kOzStage + 1024;
 constexpr int kOzEpi = 8, kOzThreads = 64 + 32 * kOzEpi;
 constexpr int kOzHeader = 256;            // error word
-constexpr int kBadExp = 1 << 20;          // marks a row or column that is not finite
+constexpr int kBadExp = 1 << 20;          // marks a row or column with a number that is not finite or subnormal
+constexpr int kNoExp = -16000;            // exponent of a zero among the packed ones (two of them fit 16 bits)
+constexpr int kSpare = 5;                 // see above
 constexpr long long kOzWait = 1LL << 24;
 constexpr unsigned long long kOzWaitNs = 200ull * 1000 * 1000;
 
@@ -142,6 +161,7 @@ struct OzArgs {
   int tiles_m, ntiles;
   const int* ea;     // (m) exponents of the rows of A
   const int* eb;     // (n2 / 2) of the columns of B
+  const uint8_t* mask;   // (n2 / 16, m): the entries of 8 columns that are not this kernel's
   int* err;
 };
 
@@ -159,10 +179,45 @@ __device__ __forceinline__ zd oz_apply(zd c, double v0, double v1, int er, int e
     v1 *= 0x1p-512;
     e = max(e + 512, -1022);
   }
-  // a row or column that is not finite makes its products NaN, as the products themselves would be
-  const double s = er >= kBadExp || ec >= kBadExp ? __longlong_as_double(0x7FF8000000000000LL)
-                                                  : __longlong_as_double((long long)(min(e, 1024) + 1023) << 52);
+  const double s = __longlong_as_double((long long)(min(e, 1024) + 1023) << 52);
   return {fma(-v0, s, c.re), fma(-v1, s, c.im)};
+}
+
+// e with |x| < 2^e for the finite x, from the high word; kBadExp for an infinity or a NaN, a low value for what
+// is below the normal range
+__device__ __forceinline__ int exp_high(int hi) {
+  const int E = (hi >> 20) & 0x7FF;
+  return E == 0x7FF ? kBadExp : E == 0 ? -(1 << 19) : E - 1022;
+}
+// whether C is large enough for the slices (see the head of this file); re, im: its parts' high words
+__device__ __forceinline__ bool oz_c_holds(int re, int im, int er, int ec) {
+  return er < kBadExp && ec < kBadExp && max(exp_high(re), exp_high(im)) >= er + ec - kSpare;
+}
+// whether the largest product is: top, the largest sum of exponents as oz_top leaves it. No common inner index
+// (a sum with a zero's exponent): the digit products are all zero, and so is the sum
+__device__ __forceinline__ bool oz_p_holds(unsigned top, int er, int ec) {
+  const int p = max((int)(short)(top & 0xFFFF), (int)top >> 16);
+  return er < kBadExp && ec < kBadExp && (p >= er + ec - kSpare || p < -8192);
+}
+__device__ __forceinline__ unsigned oz_top(unsigned a, unsigned b, unsigned top) { return __viaddmax_s16x2(a, b, top); }
+constexpr unsigned kTopNone = 0x80008000u;
+
+// This lane's part, every eighth product from sub on, of sum_t L[t] U[t ldu], summed over its eight lanes
+__device__ __forceinline__ zd oz_dot(const zd* __restrict__ L, const zd* __restrict__ U, int64_t ldu, int sub) {
+  zd s;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int t = sub + 8 * i;
+    const zd l = L[t], u = U[t * ldu];
+    s.re = fma(l.re, u.re, fma(-l.im, u.im, s.re));
+    s.im = fma(l.re, u.im, fma(l.im, u.re, s.im));
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    s.re += __shfl_xor_sync(~0u, s.re, o);
+    s.im += __shfl_xor_sync(~0u, s.im, o);
+  }
+  return s;
 }
 
 __global__ void __launch_bounds__(kOzThreads, 1)
@@ -262,6 +317,11 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       const int m0 = (t % a.tiles_m) * kOzM, n0 = (t / a.tiles_m) * kOzN;
       const int row = m0 + q * 32 + lane, col = n0 + h * 32;
       const int er = row < a.m ? a.ea[row] : 0;
+      // the lane's entries that oz_direct_kernel has taken
+      unsigned direct = 0;
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (row < a.m && col + 16 * k < a.n2) direct |= (unsigned)a.mask[(int64_t)(col / 16 + k) * a.m + row] << 8 * k;
       ok = __all_sync(0xffffffffu, bar_wait(&tfull, nt & 1, abort_v));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -312,7 +372,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
           const bool two = col + 4 * g + 2 < a.n2;
 #pragma unroll
           for (int p = 0; p < 2; ++p)
-            if (p == 0 || two) {
+            if ((p == 0 || two) && !(direct >> (2 * g + p) & 1)) {
               double2* z = reinterpret_cast<double2*>(crow + 4 * g + 2 * p);
               const double2 c = *z;
               const int i = 4 * g + 2 * p;
@@ -346,11 +406,18 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 }
 
 // ------------------------------------------------------------------ slicing
-// e with |x| < 2^e for the finite x (kBadExp for an infinity or a NaN; a low
-// value for zero and for numbers below the normal range, which count as zero)
+// e with |x| < 2^e for the normal x; kBadExp for an infinity, a NaN or a number below the normal range, a low
+// value for zero
 __device__ __forceinline__ int exp_above(double x) {
-  const int E = (int)(__double_as_longlong(x) >> 52) & 0x7FF;
-  return E == 0x7FF ? kBadExp : E == 0 ? -(1 << 19) : E - 1022;
+  const long long b = __double_as_longlong(x) << 1;
+  const int E = (int)(b >> 53) & 0x7FF;
+  return E == 0x7FF || (E == 0 && b) ? kBadExp : E == 0 ? -(1 << 19) : E - 1022;
+}
+// the exponents of two complex entries as oz_top takes them
+__device__ __forceinline__ int oz_pair(const double (&x)[4]) {
+  const int e0 = min(max(max(exp_above(x[0]), exp_above(x[1])), kNoExp), 1100);
+  const int e1 = min(max(max(exp_above(x[2]), exp_above(x[3])), kNoExp), 1100);
+  return (e0 & 0xFFFF) | e1 << 16;
 }
 // round(x 2^(62 - e)) for |x| < 2^e
 __device__ __forceinline__ long long fixed62(double x, int e) {
@@ -445,7 +512,7 @@ __device__ __forceinline__ int oz_fixed(const double (&x)[4], const int (&g)[2],
   const bool bad = e >= kBadExp;
 #pragma unroll
   for (int i = 0; i < 4; ++i) f[i] = bad ? 0 : fixed62(x[i], e - sg * g[i >> 1]);
-  return bad ? kBadExp : e < -16384 ? 0 : e;
+  return bad ? kBadExp : max(e, -20000);  // -20000: nothing but zeros, which the slices hold whatever C is
 }
 
 // Slices of L21 (rows k0 + 64 .. n - 1 of the columns k0 .. k0 + 63; one row
@@ -454,7 +521,8 @@ __device__ __forceinline__ int oz_fixed(const double (&x)[4], const int (&g)[2],
 __global__ void __launch_bounds__(256) oz_pack_kernel(const zd* __restrict__ A, int64_t lda, int k0, int m,
                                                       const int* __restrict__ gsum, uint2* __restrict__ Aq,
                                                       uint2* __restrict__ Bq, int* __restrict__ ea,
-                                                      int* __restrict__ eb, int ctas_a) {
+                                                      int* __restrict__ eb, int* __restrict__ xa,
+                                                      int* __restrict__ xb, int ctas_a) {
   grid_wait();
   grid_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = k0 + 64;
@@ -472,6 +540,7 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const zd* __restrict__ A, 
     }
     const int e = oz_fixed(x, g, 1, f);
     if (lane == 0) ea[r] = e;
+    xa[(int64_t)r * 32 + lane] = oz_pair(x);
 #pragma unroll
     for (int d = 0; d < kDig; ++d)
       Aq[((int64_t)d * m + r) * 32 + lane] =
@@ -493,6 +562,7 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const zd* __restrict__ A, 
     for (int i = 0; i < 4; ++i) x[i] = us[2 * lane + (i >> 1)][2 * c + (i & 1)];
     const int e = oz_fixed(x, g, -1, f);
     if (lane == 0) eb[cb + c] = e;
+    xb[(int64_t)(cb + c) * 32 + lane] = oz_pair(x);
 #pragma unroll
     for (int d = 0; d < kDig; ++d) {  // rows (re, im) and (im, -re)
       const uint32_t i0 = digit16(f[1], d), i1 = digit16(f[3], d);
@@ -500,6 +570,76 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const zd* __restrict__ A, 
       Bq[row] = make_uint2(digit16(f[0], d) | i0 << 16, digit16(f[2], d) | i1 << 16);
       Bq[row + 32] = make_uint2(i0 | digit16(-f[0], d) << 16, i1 | digit16(-f[2], d) << 16);
     }
+  }
+}
+
+// The entries of C that the slices do not hold (see the head of this file). A
+// CTA takes 32 rows and 64 columns, a lane a row and a warp 8 columns: small
+// tiles, as such entries come in clusters and the last blocks are small. The
+// largest product's exponent is a maximum over sums of packed exponents, two
+// inner indices per instruction; C is read where that does not reach. The entries
+// left are listed and updated here, eight lanes each, and marked for
+// oz_gemm_kernel to leave alone. (In that kernel's own epilogue, which bounds it,
+// the test took 23 ms of a factorisation of N = 5943, here 4 ms.)
+constexpr int kDirR = 32, kDirC = 64;
+
+__global__ void __launch_bounds__(256) oz_direct_kernel(zd* A, int64_t lda, int k0, int m, const int* __restrict__ ea,
+                                                        const int* __restrict__ eb, const int* __restrict__ xa,
+                                                        const int* __restrict__ xb, uint8_t* __restrict__ mask) {
+  __shared__ uint4 xs[kDirC][8], xr[kDirR][9];  // the columns' and the rows' exponents
+  __shared__ int es[kDirC];
+  __shared__ unsigned short list[kDirR * kDirC];
+  __shared__ int nlist;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = k0 + 64;
+  const int r0 = blockIdx.y * kDirR, cb = blockIdx.x * kDirC;
+  grid_wait();
+  grid_trigger();
+  if (threadIdx.x == 0) nlist = 0;
+  for (int e = threadIdx.x; e < kDirC * 8; e += 256)
+    xs[e >> 3][e & 7] = cb + (e >> 3) < m ? reinterpret_cast<const uint4*>(xb)[(int64_t)cb * 8 + e] : uint4();
+  if (threadIdx.x < kDirC) es[threadIdx.x] = cb + (int)threadIdx.x < m ? eb[cb + threadIdx.x] : 0;
+  const int row = min(r0 + lane, m - 1), er = ea[row];
+  {
+    const int r = threadIdx.x >> 3, k = threadIdx.x & 7;
+    xr[r][k] = reinterpret_cast<const uint4*>(xa)[(int64_t)min(r0 + r, m - 1) * 8 + k];
+  }
+  __syncthreads();
+  uint4 x[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) x[k] = xr[lane][k];
+  const int cw = 8 * warp, nj = min(8, m - cb - cw);
+  unsigned bits = 0;
+  for (int c = 0; c < nj; ++c) {
+    unsigned t0 = kTopNone, t1 = kTopNone;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint4 u = xs[cw + c][k];
+      t0 = oz_top(x[k].x, u.x, oz_top(x[k].y, u.y, t0));
+      t1 = oz_top(x[k].z, u.z, oz_top(x[k].w, u.w, t1));
+    }
+    if (!oz_p_holds(__vmaxs2(t0, t1), er, es[cw + c])) bits |= 1u << c;
+  }
+  if (r0 + lane >= m) bits = 0;
+  if (bits) {
+    const int4* z = reinterpret_cast<const int4*>(A + (int64_t)(c0 + row) * lda + c0 + cb + cw);
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (bits >> c & 1) {
+        const int4 v = z[c];
+        if (oz_c_holds(v.y, v.w, er, es[cw + c])) bits &= ~(1u << c);
+      }
+  }
+  if (bits) {
+    int at = atomicAdd(&nlist, __popc(bits));
+    for (unsigned b = bits; b; b &= b - 1) list[at++] = (unsigned short)(lane * kDirC + cw + __ffs(b) - 1);
+  }
+  if (r0 + lane < m && nj > 0) mask[(int64_t)((cb + cw) / 8) * m + row] = (uint8_t)bits;
+  __syncthreads();
+  for (int e0 = 4 * warp; e0 < nlist; e0 += 32) {
+    const int e = min(e0 + (lane >> 3), nlist - 1), r = c0 + r0 + list[e] / kDirC, c = c0 + cb + list[e] % kDirC;
+    const zd s = oz_dot(A + (int64_t)r * lda + k0, A + (int64_t)k0 * lda + c, lda, lane & 7);
+    zd* z = A + (int64_t)r * lda + c;
+    if ((lane & 7) == 0 && e == e0 + (lane >> 3)) *z = *z - s;
   }
 }
 
@@ -516,6 +656,9 @@ __global__ void __launch_bounds__(256) oz_simt_kernel(zd* __restrict__ A, int64_
                                                       const int* __restrict__ gsum) {
   extern __shared__ __align__(16) int simt_smem[];
   __shared__ int ea[kSimtR], eb[kSimtC];
+  __shared__ unsigned xa[kSimtR][33], xb[kSimtC][33];    // the entries' exponents
+  __shared__ unsigned short list[kSimtR * kSimtC];        // entries for fp64 multiply-adds
+  __shared__ int nlist;
   int* As = simt_smem;                  // [row][digit][32 words of four k's]
   int* Bs = As + kSimtR * kSimtLd;      // [real column][digit][32 words]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = k0 + 64;
@@ -523,6 +666,7 @@ __global__ void __launch_bounds__(256) oz_simt_kernel(zd* __restrict__ A, int64_
   const int g[2] = {oz_balance(gsum, 2 * lane), oz_balance(gsum, 2 * lane + 1)};
   double x[4];
   long long f[4];
+  if (threadIdx.x == 0) nlist = 0;
   for (int r = warp; r < kSimtR; r += 8) {
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
@@ -532,6 +676,7 @@ __global__ void __launch_bounds__(256) oz_simt_kernel(zd* __restrict__ A, int64_
     }
     const int e = oz_fixed(x, g, 1, f);
     if (lane == 0) ea[r] = e;
+    xa[r][lane] = oz_pair(x);
 #pragma unroll
     for (int d = 0; d < kDig; ++d) As[r * kSimtLd + d * 32 + lane] = digits8(f[0], f[1], f[2], f[3], d);
   }
@@ -544,6 +689,7 @@ __global__ void __launch_bounds__(256) oz_simt_kernel(zd* __restrict__ A, int64_
     }
     const int e = oz_fixed(x, g, -1, f);
     if (lane == 0) eb[c] = e;
+    xb[c][lane] = oz_pair(x);
 #pragma unroll
     for (int d = 0; d < kDig; ++d) {
       Bs[(2 * c) * kSimtLd + d * 32 + lane] = digits8(f[0], f[1], f[2], f[3], d);
@@ -594,8 +740,24 @@ __global__ void __launch_bounds__(256) oz_simt_kernel(zd* __restrict__ A, int64_
         v[p] = oz_join(w[0], w[1]);
       }
       zd* z = A + (int64_t)(c0 + r) * lda + c0 + c;
-      *z = oz_apply(*z, v[0], v[1], ea[tr + 16 * i], eb[cl]);
+      const zd cz = *z;
+      const int rl = tr + 16 * i, er = ea[rl], ec = eb[cl];
+      bool holds = oz_c_holds(__double2hiint(cz.re), __double2hiint(cz.im), er, ec);
+      if (!holds) {
+        unsigned top = kTopNone;
+        for (int k = 0; k < 32; ++k) top = oz_top(xa[rl][k], xb[cl][k], top);
+        holds = oz_p_holds(top, er, ec);
+      }
+      if (holds) *z = oz_apply(cz, v[0], v[1], er, ec);
+      else list[atomicAdd(&nlist, 1)] = (unsigned short)(rl * kSimtC + cl);
     }
+  }
+  __syncthreads();
+  for (int e0 = 4 * warp; e0 < nlist; e0 += 32) {  // eight lanes an entry, as the tensor cores' form
+    const int e = min(e0 + (lane >> 3), nlist - 1), r = c0 + r0 + list[e] / kSimtC, c = c0 + cb + list[e] % kSimtC;
+    const zd s = oz_dot(A + (int64_t)r * lda + k0, A + (int64_t)k0 * lda + c, lda, lane & 7);
+    zd* z = A + (int64_t)r * lda + c;
+    if ((lane & 7) == 0 && e == e0 + (lane >> 3)) *z = *z - s;
   }
 }
 
@@ -629,9 +791,9 @@ int oz_map(CUtensorMap* map, const void* ptr, int rows, int box_rows) {
 }
 
 // operand buffer of an n x n factorisation: header, per block the sums and numbers of the exponents of its
-// columns, row and column exponents, the slices of L21 and U12
+// columns, row and column exponents, all entries' exponents, the marks of oz_direct_kernel, the slices of L21 and U12
 struct OzLayout {
-  size_t gsum, ea, eb, aq, bq, total;
+  size_t gsum, ea, eb, xa, xb, mask, aq, bq, total;
 };
 OzLayout oz_layout(int n) {
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -640,7 +802,10 @@ OzLayout oz_layout(int n) {
   l.gsum = kOzHeader;
   l.ea = l.gsum + up(sizeof(int) * 256 * ((m + 63) / 64));
   l.eb = l.ea + up(sizeof(int) * m);
-  l.aq = l.eb + up(sizeof(int) * m);
+  l.xa = l.eb + up(sizeof(int) * m);
+  l.xb = l.xa + up(sizeof(int) * 32 * m);
+  l.mask = l.xb + up(sizeof(int) * 32 * m);
+  l.aq = l.mask + up(m * ((m + 7) / 8));
   l.bq = l.aq + up(kDig * m * kOzK * 2);
   l.total = l.bq + up(kDig * 2 * m * kOzK * 2);
   return l;
@@ -695,6 +860,9 @@ int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0) {
   int* gsum = reinterpret_cast<int*>(b + l.gsum) + 256 * (k0 / 64);
   int* ea = reinterpret_cast<int*>(b + l.ea);
   int* eb = reinterpret_cast<int*>(b + l.eb);
+  int* xa = reinterpret_cast<int*>(b + l.xa);
+  int* xb = reinterpret_cast<int*>(b + l.xb);
+  uint8_t* mask = reinterpret_cast<uint8_t*>(b + l.mask);
   uint2* aq = reinterpret_cast<uint2*>(b + l.aq);
   uint2* bq = reinterpret_cast<uint2*>(b + l.bq);
   cudaStream_t st = ctx->stream;
@@ -711,7 +879,8 @@ int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0) {
     StageTimer tm(ctx, ST_PACK);
     M25_CUDA(oz_scale(ctx, A, lda, k0, m, gsum));
     const int ca = (m + 7) / 8, cb = (m + 31) / 32;
-    M25_CUDA(launch_chained(oz_pack_kernel, dim3(ca + cb), 256, 0, st, A, lda, k0, m, gsum, aq, bq, ea, eb, ca));
+    M25_CUDA(launch_chained(oz_pack_kernel, dim3(ca + cb), 256, 0, st, A, lda, k0, m, gsum, aq, bq, ea, eb, xa, xb,
+                            ca));
   }
   OzArgs g;
   g.C = A + (int64_t)(k0 + 64) * lda + k0 + 64;
@@ -722,8 +891,11 @@ int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0) {
   g.ntiles = g.tiles_m * ((g.n2 + kOzN - 1) / kOzN);
   g.ea = ea;
   g.eb = eb;
+  g.mask = mask;
   g.err = reinterpret_cast<int*>(b);
   StageTimer tm(ctx, ST_GEMM);
+  M25_CUDA(launch_chained(oz_direct_kernel, dim3((m + kDirC - 1) / kDirC, (m + kDirR - 1) / kDirR), 256, 0, st, A, lda, k0,
+                          m, ea, eb, xa, xb, mask));
   M25_CUDA(launch_chained(oz_gemm_kernel, dim3(std::min(g.ntiles, ctx->num_sms)), kOzThreads, kOzSmem, st, ma, mb, g));
   return M25_OK;
 }
