@@ -150,6 +150,17 @@ __device__ __forceinline__ unsigned long long val_key(double v) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   return b <= 0x7ff0000000000000ull ? b + 1ull : 0ull;
 }
+// whether a sum of two squares has neither overflowed nor lost bits below the normal range (2^-960 .. 2^1024,
+// 2^-96 .. 2^128; by the bits, off the fp64 pipe)
+__device__ __forceinline__ bool square_in_range(double m2) {
+  return (unsigned)(__double2hiint(m2) - ((1023 - 960) << 20)) < (unsigned)((2047 - (1023 - 960)) << 20);
+}
+__device__ __forceinline__ bool square_in_range(float m2) {
+  return (unsigned)(__float_as_int(m2) - ((127 - 96) << 23)) < (unsigned)((255 - (127 - 96)) << 23);
+}
+// a power of two that brings the squares of such a value into it
+__device__ __forceinline__ double pivot_scale(cx<double> v) { return cabs1(v) >= 1.0 ? 0x1p-600 : 0x1p600; }
+__device__ __forceinline__ float pivot_scale(cx<float> v) { return cabs1(v) >= 1.f ? 0x1p-70f : 0x1p70f; }
 template <class T>
 using KeyOf = decltype(val_key(T(0)));
 
@@ -397,8 +408,15 @@ __global__ void __launch_bounds__(kStripThreads, 1) strip_panel_kernel(StripArgs
   // the candidate with the reciprocal pivot, both parts in one division: the even lanes the real, the odd ones the
   // imaginary part
   auto reciprocal = [&](cx<T> pv) {
-    const T m2 = pv.re * pv.re + pv.im * pv.im;
-    return ((lane & 1) ? -pv.im : pv.re) / m2;
+    T m2 = pv.re * pv.re + pv.im * pv.im, f = T(1);
+    const bool plain = square_in_range(m2);  // the same in the whole warp
+    if (!plain) {
+      f = pivot_scale(pv);
+      pv = pv * f;
+      m2 = pv.re * pv.re + pv.im * pv.im;
+    }
+    const T half = ((lane & 1) ? -pv.im : pv.re) / m2;
+    return plain ? half : half * f;
   };
   auto put_candidate = [&](T half, Key key, unsigned p, int par) {
     union {
