@@ -674,7 +674,8 @@ __global__ void perm_out_kernel(int nb, int n, const int32_t* __restrict__ perm,
 
 // block k's matrix (complex64, row-major S x S): per (row leaf, column leaf)
 // pair the near block or the far block (as rows or as its transpose), then
-// the via rows / columns; every entry has one source. The pairs of a block are
+// the via rows / columns. Leaf pairs that no item names stay zero (cleared by
+// the caller: the kernel's CTAs are not ordered). The pairs of a block are
 // shared out to gridDim.y CTAs (a few blocks alone leave the GPU idle).
 __global__ void diag_kernel(const int64_t* __restrict__ pc_off, const int32_t* __restrict__ gidx,
                             const int64_t* __restrict__ item_off, const int32_t* __restrict__ items,
@@ -1515,6 +1516,10 @@ extern "C" int m25_hmat_assemble(m25_hmat* h, m25_greens* gr, double zs_re, doub
   }
   wscale_kernel<<<(h->n + 255) / 256, 256, 0, st>>>(h->nb, h->n, h->nv, h->row_leaf, h->self_near, h->near,
                                                     h->near_off, h->Zn, h->Zxx, h->wsc);
+  if (cudaMemsetAsync(h->D, 0, sizeof(zf) * h->d_entries, st) != cudaSuccess) {
+    set_error("m25_hmat_assemble: memset failed");
+    return done(M25_ERR_CUDA);
+  }
   diag_kernel<<<dim3(h->npc, 32), 256, 0, st>>>(h->pc_off, h->pc_gidx, h->pc_item_off, h->pc_items, h->pc_doff, h->nb, h->nv,
                                       h->nnear, h->leaf_lo, h->near_off, h->Zn, h->fb, h->pool, h->dense_pool, h->ZxbT,
                                       h->Zxx, h->D);
