@@ -73,9 +73,6 @@ struct m25_hmat {
   // device: values
   m25::zd *Zn = nullptr, *pool = nullptr, *ZxbT = nullptr, *Zxx = nullptr;
   m25::zf* D = nullptr;       // preconditioner blocks, then their inverses
-  m25::zf *G = nullptr, *gj_x = nullptr;  // the blocks under elimination; a panel's pivot rows
-  float* gj_w = nullptr;
-  int32_t *gj_step = nullptr, *gj_prow = nullptr;
   int pc_max = 0;             // unknowns of the largest block
   uint8_t* flags = nullptr;   // ACA's used rows / columns
   int64_t near_entries = 0, uv_entries = 0, dense_entries = 0, t_entries = 0, flag_bytes = 0, d_entries = 0;
@@ -1278,11 +1275,6 @@ extern "C" int m25_hmat_create(m25_ctx* ctx, m25_geom* geom, const m25_hmat_desc
   TRY(dalloc(h->allocs, &h->ZxbT, (size_t)d->nb * std::max(d->nv, 1)));
   TRY(dalloc(h->allocs, &h->Zxx, (size_t)std::max(d->nv, 1) * std::max(d->nv, 1)));
   TRY(dalloc(h->allocs, &h->D, h->d_entries));
-  TRY(dalloc(h->allocs, &h->G, h->d_entries));
-  TRY(dalloc(h->allocs, &h->gj_x, (size_t)d->npc * kGj * 1024));
-  TRY(dalloc(h->allocs, &h->gj_w, (size_t)d->npc * 1024));
-  TRY(dalloc(h->allocs, &h->gj_step, (size_t)d->npc * 1024));
-  TRY(dalloc(h->allocs, &h->gj_prow, (size_t)d->npc * 1024));
   TRY(dalloc(h->allocs, &h->aca_ids, std::max(h->naca, 1)));
   TRY(dalloc(h->allocs, &h->rank, std::max(h->naca, 1)));
   TRY(dalloc(h->allocs, &h->status, std::max(h->naca, 1)));
@@ -1441,6 +1433,21 @@ extern "C" int m25_hmat_assemble(m25_hmat* h, m25_greens* gr, double zs_re, doub
     set_error("m25_hmat_assemble: a near block needs a triangle pair the near-field list does not hold");
     return done(M25_ERR_VALUE);
   }
+  // the pairs' values make room for the elimination's buffers: the blocks under elimination, a panel's pivot rows,
+  // the scaling, the panel a row was a pivot of and the columns' pivot rows
+  free_all_async(tmp, st);
+  zf *G = nullptr, *gj_x = nullptr;
+  float* gj_w = nullptr;
+  int32_t *gj_step = nullptr, *gj_prow = nullptr;
+  {
+    const size_t rows = (size_t)h->npc * 1024;
+    if ((rc = alloc_async(tmp, reinterpret_cast<void**>(&G), sizeof(zf) * h->d_entries, st)) ||
+        (rc = alloc_async(tmp, reinterpret_cast<void**>(&gj_x), sizeof(zf) * kGj * rows, st)) ||
+        (rc = alloc_async(tmp, reinterpret_cast<void**>(&gj_w), sizeof(float) * rows, st)) ||
+        (rc = alloc_async(tmp, reinterpret_cast<void**>(&gj_step), sizeof(int32_t) * rows, st)) ||
+        (rc = alloc_async(tmp, reinterpret_cast<void**>(&gj_prow), sizeof(int32_t) * rows, st)))
+      return done(rc);
+  }
   int64_t max_rank = 0, rank_sum = 0, not_low = 0, nlow = 0, far_entries = 0;
   {
     int a = 0;
@@ -1523,14 +1530,14 @@ extern "C" int m25_hmat_assemble(m25_hmat* h, m25_greens* gr, double zs_re, doub
   diag_kernel<<<dim3(h->npc, 32), 256, 0, st>>>(h->pc_off, h->pc_gidx, h->pc_item_off, h->pc_items, h->pc_doff, h->nb, h->nv,
                                       h->nnear, h->leaf_lo, h->near_off, h->Zn, h->fb, h->pool, h->dense_pool, h->ZxbT,
                                       h->Zxx, h->D);
-  gj_scale_kernel<<<dim3(h->npc, 16), 256, 0, st>>>(h->pc_off, h->pc_doff, h->D, h->G, h->gj_w, h->gj_step);
+  gj_scale_kernel<<<dim3(h->npc, 16), 256, 0, st>>>(h->pc_off, h->pc_doff, h->D, G, gj_w, gj_step);
   const int tiles = (h->pc_max + 63) / 64;
   for (int k0 = 0; k0 < h->pc_max; k0 += kGj) {
-    gj_panel_kernel<<<h->npc, (h->pc_max + 31) / 32 * 32, 0, st>>>(h->pc_off, h->pc_doff, h->G, h->gj_x, h->gj_step,
-                                                                  h->gj_prow, k0);
-    gj_update_kernel<<<dim3(tiles, tiles, h->npc), 256, 0, st>>>(h->pc_off, h->pc_doff, h->G, h->gj_x, h->gj_step, k0);
+    gj_panel_kernel<<<h->npc, (h->pc_max + 31) / 32 * 32, 0, st>>>(h->pc_off, h->pc_doff, G, gj_x, gj_step,
+                                                                  gj_prow, k0);
+    gj_update_kernel<<<dim3(tiles, tiles, h->npc), 256, 0, st>>>(h->pc_off, h->pc_doff, G, gj_x, gj_step, k0);
   }
-  gj_finish_kernel<<<dim3(h->npc, 16), 256, 0, st>>>(h->pc_off, h->pc_doff, h->G, h->gj_w, h->gj_prow, h->D);
+  gj_finish_kernel<<<dim3(h->npc, 16), 256, 0, st>>>(h->pc_off, h->pc_doff, G, gj_w, gj_prow, h->D);
   if (cudaGetLastError() != cudaSuccess) {
     set_error("m25_hmat_assemble: launch failed");
     return done(M25_ERR_CUDA);
