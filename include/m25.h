@@ -75,8 +75,8 @@ void* m25_ctx_stream(m25_ctx* ctx); /* the cudaStream_t every call of this conte
  * point by mom25d_gb300/batch.py and Solver.sweep from the table autotune.py
  * measures), 0 keeping the process default: panel_cluster_min, the smallest
  * cluster (4, 8 or 16 CTAs) the LU panel runs on (default 8, or
- * $M25_PANEL_CLUSTER_MIN); wave_ctas, the CTA cap of the triangular solves
- * (default one per 64-row block, or
+ * $M25_PANEL_CLUSTER_MIN; complex128 panels take 8 at least); wave_ctas, the
+ * CTA cap of the triangular solves (default one per block of 64 rows, complex128 32, or
  * $M25_WAVE_CTAS; a refinement's solves beyond its fourth step take no cap); tc_chunk, the steps of
  * 32 tf32 along K (12 MMAs each) the tensor-core update accumulates in TMEM
  * before adding into its fp32 registers (1..8; default 1, or $M25_TC_CHUNK:

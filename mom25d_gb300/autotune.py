@@ -1,9 +1,9 @@
 """The engine's per-context tuning knobs, chosen by problem size N from a
 table measured on the device (mom25d has no such knobs: its LU is LAPACK's).
 
-Knobs (m25_ctx_set_tuning): the smallest cluster (4, 8 or 16 CTAs) the LU
-panel runs on, the CTA cap of the triangular solves (0: one CTA per 64-row
-block), the number of k-blocks the tensor-core update accumulates in TMEM
+Knobs (m25_ctx_set_tuning): the smallest cluster (4, 8 or 16 CTAs; 8 at
+least in complex128) the LU panel runs on, the CTA cap of the triangular
+solves (0: one CTA per block of 64 rows, complex128 32), the number of k-blocks the tensor-core update accumulates in TMEM
 before adding into fp32 registers, and the tile shape of that update (N of
 128 or 192 real columns; 0: by the update's width). The best values depend
 on N: how many rows the panel's cluster holds, how long the wavefront is,

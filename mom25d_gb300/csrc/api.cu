@@ -52,8 +52,8 @@ int lu_solve_wave(m25_ctx*, const cx<TF>*, int64_t, int, const int32_t*, const c
 int lu_wave_error(m25_ctx*, int, int*);
 int lu_wave_reset(m25_ctx*);
 
-// panel width of the complex64 LU: 64 columns keep the panel of up to ~7000
-// trailing rows in the shared memory of one 16-CTA cluster
+// panel width of the LU: the blocks that its updates take (complex64: two of them, factored in strips of 32 by one
+// cluster, or panel by panel above its 8192 rows)
 constexpr int kPanelZ64 = 64;
 
 // A caller's complex64 array on the device may lie at any multiple of four

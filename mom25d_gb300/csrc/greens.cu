@@ -675,12 +675,11 @@ __global__ void table_kernel(const StackDev* __restrict__ Sp, int nrho, const do
 // digit (six rounds instead of eight at 220 rows). Rows are kept scaled by
 // their diagonal (b = 1), which leaves one division per row and round
 // instead of two. Shared-memory arrays of m entries: a, b, c, d and the copies
-// a2, b2, c2, d2 (ping-pong); x receives the solution (it may be d). The
+// a2, c2, d2 (ping-pong); x receives the solution (it may be d). The
 // caller synchronises before the call; the call ends with the CTA synchronised. A serial
 // elimination would chain m dependent fp64 divisions; here the chain is the rounds.
 template <class T>
-__device__ void pcr_solve(int m, double* a, double* b, double* c, T* d, double* a2, double* b2, double* c2, T* d2,
-                          T* x) {
+__device__ void pcr_solve(int m, double* a, double* b, double* c, T* d, double* a2, double* c2, T* d2, T* x) {
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
     const double inv = 1.0 / b[i];
     a[i] *= inv;
@@ -720,7 +719,7 @@ __device__ void pcr_solve(int m, double* a, double* b, double* c, T* d, double* 
 __host__ __device__ inline size_t spline_smem(int n) { return (size_t)n * (2 * sizeof(double) + 4 * sizeof(zd)); }
 // with the reduced system solved by pcr_solve (n - 2 rows)
 __host__ __device__ inline size_t spline_smem_pcr(int n) {
-  return (size_t)n * (2 * sizeof(double) + 3 * sizeof(zd)) + (size_t)(n - 2) * (6 * sizeof(double) + 2 * sizeof(zd));
+  return (size_t)n * (2 * sizeof(double) + 3 * sizeof(zd)) + (size_t)(n - 2) * (5 * sizeof(double) + 2 * sizeof(zd));
 }
 
 // Not-a-knot cubic spline of one table column (scipy CubicSpline's slope
@@ -778,8 +777,7 @@ __global__ void __launch_bounds__(128) spline_kernel(int L, int nrho, const doub
     double* rb = ra + m;
     double* rc = rb + m;
     double* ra2 = rc + m;
-    double* rb2 = ra2 + m;
-    double* rc2 = rb2 + m;
+    double* rc2 = ra2 + m;
     zd* rd = reinterpret_cast<zd*>(rc2 + m);
     zd* rd2 = rd + m;
     for (int i = 1 + threadIdx.x; i <= n - 2; i += blockDim.x) {
@@ -808,7 +806,7 @@ __global__ void __launch_bounds__(128) spline_kernel(int L, int nrho, const doub
       rd[i - 1] = d;
     }
     __syncthreads();
-    pcr_solve<zd>(m, ra, rb, rc, rd, ra2, rb2, rc2, rd2, s + 1);
+    pcr_solve<zd>(m, ra, rb, rc, rd, ra2, rc2, rd2, s + 1);
     if (threadIdx.x == 0) {
       double a, b, c;
       zd d;
@@ -872,13 +870,13 @@ __global__ void to_f32_kernel(const double* __restrict__ a, float* __restrict__ 
 // derivative continuous at x_1 and x_{K-2}) give M_0 and M_{K-1} in terms of
 // their neighbours; substituted into rows 1 and K - 2 they leave a strictly
 // diagonally dominant tridiagonal system for M_1 .. M_{K-2}, solved by
-// pcr_solve. scratch: 8 (K - 2) doubles of shared memory. The caller
+// pcr_solve. scratch: 7 (K - 2) doubles of shared memory. The caller
 // synchronises before the call; the call ends synchronised.
 template <class XF, class YF>
 __device__ void spline_notaknot(int K, XF x, YF y, double* M, double* scratch) {
   const int m = K - 2;  // unknowns M_1 .. M_{K-2}
   double *a = scratch, *b = a + m, *c = b + m, *d = c + m;
-  double *a2 = d + m, *b2 = a2 + m, *c2 = b2 + m, *d2 = c2 + m;
+  double *a2 = d + m, *c2 = a2 + m, *d2 = c2 + m;
   auto h = [&](int j) { return x(j + 1) - x(j); };
   for (int k = 1 + threadIdx.x; k <= m; k += blockDim.x) {
     double ak = h(k - 1), bk = 2.0 * (h(k - 1) + h(k)), ck = h(k);
@@ -900,7 +898,7 @@ __device__ void spline_notaknot(int K, XF x, YF y, double* M, double* scratch) {
     d[k - 1] = dk;
   }
   __syncthreads();
-  pcr_solve<double>(m, a, b, c, d, a2, b2, c2, d2, M + 1);
+  pcr_solve<double>(m, a, b, c, d, a2, c2, d2, M + 1);
   if (threadIdx.x == 0) {
     M[0] = ((h(0) + h(1)) * M[1] - h(0) * M[2]) / h(1);
     M[K - 1] = ((h(K - 3) + h(K - 2)) * M[K - 2] - h(K - 2) * M[K - 3]) / h(K - 3);
@@ -927,7 +925,7 @@ __device__ inline double spline_eval(double x0, double x1, double y0, double y1,
 // spline, and the network + spline compared with the integral at the
 // validation radii. colerr[2 col] = the largest error there, colerr[2 col +
 // 1] = the largest |remainder| of the column's complex column over the ne
-// radii. Shared memory: (2 ne + 11 nk) doubles.
+// radii. Shared memory: (2 ne + 10 nk) doubles.
 __global__ void __launch_bounds__(256) sur_judge_kernel(int NC, const double* __restrict__ rho, int ne,
                                                         const int* __restrict__ ie, int nk,
                                                         const int* __restrict__ kpos, int nv,
@@ -997,7 +995,7 @@ __global__ void __launch_bounds__(256) sur_judge_kernel(int NC, const double* __
 // other radii ir[] get network + a not-a-knot spline of the residual through
 // all ne integrated radii (a denser spline than the judged one), which is
 // solved beside the judge's, before the wait for its verdict. Shared memory:
-// 11 ne doubles.
+// 10 ne doubles.
 __global__ void __launch_bounds__(256) sur_fill_kernel(int NC, const double* __restrict__ rho, int ne,
                                                        const int* __restrict__ ie, int nr, const int* __restrict__ ir,
                                                        const float* __restrict__ Y, const double* __restrict__ scale,
@@ -1052,8 +1050,8 @@ __global__ void __launch_bounds__(256) sur_fill_kernel(int NC, const double* __r
 }
 
 // shared memory of the two kernels above, and its limit
-inline size_t sur_judge_smem(int ne, int nk) { return sizeof(double) * (2 * (size_t)ne + 11 * (size_t)nk); }
-inline size_t sur_fill_smem(int ne) { return sizeof(double) * 11 * (size_t)ne; }
+inline size_t sur_judge_smem(int ne, int nk) { return sizeof(double) * (2 * (size_t)ne + 10 * (size_t)nk); }
+inline size_t sur_fill_smem(int ne) { return sizeof(double) * 10 * (size_t)ne; }
 constexpr size_t kSurSmemMax = 200 * 1024;
 
 int mlp_forward_device(const m25_mlp* m, int n, const float* X, float* Y, cudaStream_t st);  // mlp.cu

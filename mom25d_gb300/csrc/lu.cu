@@ -626,9 +626,8 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
   use_tc = use_tc && std::is_same<T, float>::value && lda % 2 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
            nb == kSwapMaxW;
   // panel workspace
-  int bps_max = 0;
   size_t panel_smem = 0;
-  int G = 0, rows = 0;
+  int G = 0;
   const size_t extra = (size_t)nb * sizeof(cx<T>);
   // pick the widest grid whose slices fit: rows_per_cta = ceil(m / G)
   auto fits = [&](int g, int m, size_t& smem) {
@@ -646,8 +645,6 @@ int lu_factor(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int32_t* ipiv, int nb,
   if constexpr (std::is_same<T, float>::value)
     M25_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<T, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)swap_trsm_smem<T, 128>()));
-  (void)bps_max;
-  (void)rows;
   int Gmax = ctx->ext_scratch ? ctx->ext_gmax : 4 * ctx->num_sms;
   char* base = ctx->ext_scratch;
   if (!base) {

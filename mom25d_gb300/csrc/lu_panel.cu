@@ -690,9 +690,10 @@ bool strip_available(int device) {
                cudaFuncSetAttribute(strip_panel_kernel<T, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
                    cudaSuccess &&
                cudaFuncSetAttribute(strip_panel_kernel<T, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
-                   cudaSuccess &&
-               cudaFuncSetAttribute(strip_panel_kernel<T, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
                    cudaSuccess;
+    if constexpr (sizeof(T) == 4)
+      yes = yes && cudaFuncSetAttribute(strip_panel_kernel<T, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        smem) == cudaSuccess;
     if constexpr (sizeof(T) == 8) {
       const auto set = [&](auto kernel, bool wide) {
         yes = yes && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
@@ -784,9 +785,13 @@ int lu_strip_block(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int b0, int bw, i
     if (sizeof(T) == 8) CL = std::max(CL, m > 256 ? 16 : 8);
     StripArgs<T> a{A, lda, n, k0, w, b0, b0 + bw, (m + CL - 1) / CL, ipiv, Ub, info, err};
     StageTimer tm(ctx, ST_PANEL);
-    if (CL == 4) M25_CUDA((launch_strip<T, 4>(a, ctx->stream)));
-    else if (CL == 8) M25_CUDA((launch_rows<T, 8>(a, ctx->stream)));
-    else M25_CUDA((launch_rows<T, 16>(a, ctx->stream)));
+    if (CL == 16) {
+      M25_CUDA((launch_rows<T, 16>(a, ctx->stream)));
+    } else if (CL == 8) {
+      M25_CUDA((launch_rows<T, 8>(a, ctx->stream)));
+    } else {
+      if constexpr (sizeof(T) == 4) M25_CUDA((launch_strip<T, 4>(a, ctx->stream)));
+    }
     const int nc = b0 + bw - k0 - w;
     if (nc > 0) {
       const dim3 grid((nc + StripUpd<T>::CG - 1) / StripUpd<T>::CG, (n - k0 - w + StripUpd<T>::TR - 1) / StripUpd<T>::TR);
