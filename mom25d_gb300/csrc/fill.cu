@@ -16,7 +16,7 @@
 // Stage 3 (via_rows_kernel, via_block_kernel): rows / columns of the via
 // segment unknowns (Engine/mom25d/solver.py:527-566).
 #include <algorithm>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -1154,8 +1154,8 @@ static void touch_pages(void* p, size_t bytes) {
   try {
     for (size_t k = 1; k < kThreads; ++k) th.emplace_back(part, k);
     part(0);
-  } catch (const std::system_error&) {
-    // no thread to be had: the copy faults the rest in
+  } catch (const std::exception&) {
+    // no thread (or no memory for one) to be had: the copy faults the rest in
   }
   for (auto& t : th) t.join();
 }
