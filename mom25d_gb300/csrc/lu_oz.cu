@@ -11,11 +11,14 @@
 //   - as in the complex64 update (lu_tc.cu) one real product on the
 //     interleaved storage, C (m x 2 nc) -= A (m x 128) B (128 x 2 nc), A the
 //     interleaved conj(L21), B rows (U, -iU) alternating;
-//   - the columns of L are divided, and the rows of U multiplied, by a power of
+//   - the real columns of L are divided, and the rows of U multiplied, by a power of
 //     two: half the difference of the mean exponents of the column and of the
-//     row. A power of two per row and per column follows below, so without
-//     this a pivot row of very different size (a via's beside RWG rows, 1e10
-//     apart) would take the bits of the others. Means, as one entry of unusual
+//     row, and besides the real and the imaginary part of a column of L are
+//     brought to the same mean (of a matrix that is nearly imaginary, or nearly
+//     real, the smaller parts of the products then have their own scale). A power
+//     of two per row and per column follows below, so without the first a pivot
+//     row of very different size (a via's beside RWG rows, 1e10 apart) would take
+//     the bits of the others. Means, as one entry of unusual
 //     size must not set the scale of all others, and of both factors, as either
 //     may be the uneven one: over MoM matrices with and without vias, entries
 //     of +-1 with 1e-12 of noise and log-normal entries, the products of a row
@@ -33,23 +36,28 @@
 //   - the eight sums combined in 64-bit integers and rounded once.
 // What is left out is relative to the largest entries of the row and of the
 // column, which may belong to different inner indices (two weakly coupled
-// groups of unknowns; a column of L with few large entries beside full ones):
-// then the products are small beside it and no scaling helps. So each entry of
-// C is looked at: where neither C nor the largest of its 64 products reaches
-// 2^-kSpare of the product of the row's and the column's power of two, and
-// where the row or the column has a number that is not finite or below the
-// normal range, the entry is formed with fp64 multiply-adds instead (oz_dot).
-// kSpare = 5: the error in the mean, 2^-59 of that product, is then at most
-// 2^-54 of C or of the largest product, half an ulp. Both bound
-// (|L| |U|)_ij from below (C is L U of what is left of the matrix), so that
-// the factorisation keeps the componentwise bound of an fp64 one. The largest
-// |P A - L U| / |L| |U| of any entry, in a numpy restatement, against fp64 sums: normal
-// matrices 2.5e-16 (fp64 sums 2.5e-16), three MoM lines, two of them with vias, 5.4e-16, 5.9e-16, 5.2e-16
-// (5.4e-16, 6.3e-16, 6.7e-16; without the test 2.2e-15, 5.8e-15, 1.7e-15), two groups
-// coupled by 1e-8 2.4e-16 (2.4e-16; 7.2e-11), a column of L with tiny entries beside
-// full ones 3.5e-16 (3.5e-16; 4.4e-5). Entries that take the fp64
-// path: none of normal matrices', 0.04 to 1.1 % of MoM matrices', a quarter of
-// the potentials between cells in random order, half of two groups'.
+// groups of unknowns; a column of L with few large entries beside full ones;
+// real and imaginary parts of different size): then the products are small beside
+// it and no scaling helps. So each real entry of C is looked at, and formed with
+// fp64 multiply-adds instead (oz_dot) unless
+//   - one of its 128 products is within 2^-7 of the product of the row's and the
+//     column's power of two (or all are zero): the error in the mean, 2^-59 of that
+//     product, is 2^-52 of the largest product at the most, where fp64 sums of 128
+//     products round 128 times by up to 2^-53 of what has been added so far; or
+//   - C is within 2^-kSpare of it: the error is then 2^-54 of C, half an ulp;
+// and always where the row or the column has a number that is not finite or below
+// the normal range. Products and C bound |Re L| |Re U| + |Im L| |Im U| (for the
+// real part; the imaginary part's accordingly) from below, as C is L U of what is left
+// of the matrix, so that the factorisation keeps the componentwise bound of an
+// fp64 one, part by part. P A - L U relative to that, root mean square and largest
+// of all real parts, in a numpy restatement, with fp64 sums in brackets: potentials between 448
+// cells in random order 1.2e-16, 1.3e-15 (1.5e-16, 1.0e-15), three MoM lines, two of them with vias, 8.5e-17,
+// 1.3e-15 (8.6e-17, 1.3e-15), 6.1e-17, 1.1e-15 (6.3e-17, 1.1e-15), 6.8e-17, 1.2e-15 (6.9e-17, 1.2e-15); log-normal
+// entries 4.9e-17, 9.3e-16 (5.1e-17, 9.3e-16). With 2^-9 for 2^-7 the potentials' are 1.4e-16 and
+// 5.4e-15; without the test 4.3e-16 and 4.4e-14, and two groups coupled by 1e-8 are off by 5.7e-11, a column of L with tiny
+// entries beside full ones by 2.5e-9. Entries that take the fp64 path: none of normal matrices' or of
+// j X + eps R, 0.05 to 1 % of MoM matrices', 45 % of the potentials between cells in random order,
+// half of two groups', all of j X + eps R with its rows turned by powers of j.
 //
 // oz_scale_kernel sums the exponents, oz_pack_kernel slices L21 and U12;
 // oz_direct_kernel does the entries that are not left to the slices;
@@ -62,10 +70,10 @@
 // while the next tile's products run. Every wait is bounded, as in lu_tc.cu.
 // What bounds it: the shared-memory reads of the MMAs (4 KB of A for every 32
 // cycles of products at N = 64) and, after that, three fp64 operations per
-// element. Measured on GB300, all updates of a factorisation of a normal matrix with their
-// slicing and the test, N = 546 / 1085 / 2434 / 5943: 0.37 / 0.85 / 3.7 / 33.5 ms (the test 4.4 ms of
-// the last); 3.55 / 8.8 / 64 / 771 ms with fp64 multiply-adds on the CUDA cores throughout. Potentials between
-// 1543 cells in random order 5.1 ms, 3.5 of them for the fp64 entries.
+// element. Measured on GB300, all updates of a factorisation of a normal
+// matrix with their slicing and the test, N = 1085 / 5943: 0.82 / 33.9 ms; 8.8 /
+// 771 ms with fp64 multiply-adds on the CUDA cores throughout. Of the LPF's matrix (N
+// = 5943) 40.3 ms, of potentials between 1543 cells in random order 7.6 ms.
 #include <cuda.h>
 
 #include <algorithm>
@@ -92,8 +100,7 @@ constexpr int kOzSmem = kOzStages * kOzStage + 1024;
 constexpr int kOzEpi = 8, kOzThreads = 64 + 32 * kOzEpi;
 constexpr int kOzHeader = 256;            // error word
 constexpr int kBadExp = 1 << 20;          // marks a row or column with a number that is not finite or subnormal
-constexpr int kNoExp = -16000;            // exponent of a zero among the packed ones (two of them fit 16 bits)
-constexpr int kSpare = 5;                 // see above
+constexpr int kSpare = 5;                 // of C, see above
 constexpr long long kOzWait = 1LL << 24;
 constexpr unsigned long long kOzWaitNs = 200ull * 1000 * 1000;
 
@@ -160,8 +167,8 @@ struct OzArgs {
   int m, n2;         // rows, real columns
   int tiles_m, ntiles;
   const int* ea;     // (m) exponents of the rows of A
-  const int* eb;     // (n2 / 2) of the columns of B
-  const uint8_t* mask;   // (n2 / 16, m): the entries of 8 columns that are not this kernel's
+  const int* eb;     // (n2) of the columns of B
+  const uint16_t* mask;  // (n2 / 16, m): the entries of 16 real columns that are not this kernel's
   int* err;
 };
 
@@ -171,52 +178,39 @@ __device__ __forceinline__ double oz_join(long long hi, long long lo) {
   return (__longlong_as_double(0x4538000000000000LL + hi) - (29014219670751100192948224.0 + 6755399441055744.0)) +
          __longlong_as_double(0x4338000000000000LL + lo);
 }
-// c - (v0 + j v1) 2^(er + ec - 68), er and ec the exponents of the row and the column
-__device__ __forceinline__ zd oz_apply(zd c, double v0, double v1, int er, int ec) {
+// c - v 2^(er + ec - 68), er and ec the exponents of the row and the column
+__device__ __forceinline__ double oz_apply(double c, double v, int er, int ec) {
   int e = er + ec - 68;
-  if (e < -1022) {  // 2^e below the normal range: in two steps
-    v0 *= 0x1p-512;
-    v1 *= 0x1p-512;
+  if (e < -1022) {  // 2^e beyond the normal range: in two steps
+    v *= 0x1p-512;
     e = max(e + 512, -1022);
+  } else if (e > 1023) {
+    v *= 0x1p512;
+    e = min(e - 512, 1023);
   }
-  const double s = __longlong_as_double((long long)(min(e, 1024) + 1023) << 52);
-  return {fma(-v0, s, c.re), fma(-v1, s, c.im)};
+  return fma(-v, __longlong_as_double((long long)(e + 1023) << 52), c);
 }
 
-// e with |x| < 2^e for the finite x, from the high word; kBadExp for an infinity or a NaN, a low value for what
-// is below the normal range
-__device__ __forceinline__ int exp_high(int hi) {
+// Whether C itself is large enough for the slices (see the head of this file); hi: its high word
+__device__ __forceinline__ bool oz_c_holds(int hi, int er, int ec) {
   const int E = (hi >> 20) & 0x7FF;
-  return E == 0x7FF ? kBadExp : E == 0 ? -(1 << 19) : E - 1022;
+  return er < kBadExp && ec < kBadExp && E != 0 && (E == 0x7FF || E - 1022 >= er + ec - kSpare);
 }
-// whether C is large enough for the slices (see the head of this file); re, im: its parts' high words
-__device__ __forceinline__ bool oz_c_holds(int re, int im, int er, int ec) {
-  return er < kBadExp && ec < kBadExp && max(exp_high(re), exp_high(im)) >= er + ec - kSpare;
-}
-// whether the largest product is: top, the largest sum of exponents as oz_top leaves it. No common inner index
-// (a sum with a zero's exponent): the digit products are all zero, and so is the sum
-__device__ __forceinline__ bool oz_p_holds(unsigned top, int er, int ec) {
-  const int p = max((int)(short)(top & 0xFFFF), (int)top >> 16);
-  return er < kBadExp && ec < kBadExp && (p >= er + ec - kSpare || p < -8192);
-}
-__device__ __forceinline__ unsigned oz_top(unsigned a, unsigned b, unsigned top) { return __viaddmax_s16x2(a, b, top); }
-constexpr unsigned kTopNone = 0x80008000u;
 
-// This lane's part, every eighth product from sub on, of sum_t L[t] U[t ldu], summed over its eight lanes
-__device__ __forceinline__ zd oz_dot(const zd* __restrict__ L, const zd* __restrict__ U, int64_t ldu, int sub) {
-  zd s;
+// One part (0: real) of sum_t L[t] U[t ldu]: this lane's share, every fourth product from sub on, summed over its
+// four lanes
+constexpr int kDot = 4, kDots = 32 / kDot;  // lanes per entry, entries of a warp at a time
+__device__ __forceinline__ double oz_dot(const zd* __restrict__ L, const zd* __restrict__ U, int64_t ldu, int sub,
+                                         int part) {
+  double s = 0.0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int t = sub + 8 * i;
+  for (int i = 0; i < 64 / kDot; ++i) {
+    const int t = sub + kDot * i;
     const zd l = L[t], u = U[t * ldu];
-    s.re = fma(l.re, u.re, fma(-l.im, u.im, s.re));
-    s.im = fma(l.re, u.im, fma(l.im, u.re, s.im));
+    s = fma(l.re, part ? u.im : u.re, fma(l.im, part ? u.re : -u.im, s));
   }
 #pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
-    s.re += __shfl_xor_sync(~0u, s.re, o);
-    s.im += __shfl_xor_sync(~0u, s.im, o);
-  }
+  for (int o = 1; o < kDot; o <<= 1) s += __shfl_xor_sync(~0u, s, o);
   return s;
 }
 
@@ -321,7 +315,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       unsigned direct = 0;
 #pragma unroll
       for (int k = 0; k < 2; ++k)
-        if (row < a.m && col + 16 * k < a.n2) direct |= (unsigned)a.mask[(int64_t)(col / 16 + k) * a.m + row] << 8 * k;
+        if (row < a.m && col + 16 * k < a.n2) direct |= (unsigned)a.mask[(int64_t)(col / 16 + k) * a.m + row] << 16 * k;
       ok = __all_sync(0xffffffffu, bar_wait(&tfull, nt & 1, abort_v));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -372,13 +366,14 @@ __global__ void __launch_bounds__(kOzThreads, 1)
           const bool two = col + 4 * g + 2 < a.n2;
 #pragma unroll
           for (int p = 0; p < 2; ++p)
-            if ((p == 0 || two) && !(direct >> (2 * g + p) & 1)) {
+            if (p == 0 || two) {
               double2* z = reinterpret_cast<double2*>(crow + 4 * g + 2 * p);
-              const double2 c = *z;
+              double2 c = *z;
               const int i = 4 * g + 2 * p;
-              const zd r = oz_apply(zd(c.x, c.y), oz_join(hi[i], lo[i]), oz_join(hi[i + 1], lo[i + 1]), er,
-                                    a.eb[(col + i) / 2]);
-              *z = make_double2(r.re, r.im);
+              const int2 ec = *reinterpret_cast<const int2*>(a.eb + col + i);
+              if (!(direct >> i & 1)) c.x = oz_apply(c.x, oz_join(hi[i], lo[i]), er, ec.x);
+              if (!(direct >> i & 2)) c.y = oz_apply(c.y, oz_join(hi[i + 1], lo[i + 1]), er, ec.y);
+              *z = c;
             }
         }
       }
@@ -413,12 +408,6 @@ __device__ __forceinline__ int exp_above(double x) {
   const int E = (int)(b >> 53) & 0x7FF;
   return E == 0x7FF || (E == 0 && b) ? kBadExp : E == 0 ? -(1 << 19) : E - 1022;
 }
-// the exponents of two complex entries as oz_top takes them
-__device__ __forceinline__ int oz_pair(const double (&x)[4]) {
-  const int e0 = min(max(max(exp_above(x[0]), exp_above(x[1])), kNoExp), 1100);
-  const int e1 = min(max(max(exp_above(x[2]), exp_above(x[3])), kNoExp), 1100);
-  return (e0 & 0xFFFF) | e1 << 16;
-}
 // round(x 2^(62 - e)) for |x| < 2^e
 __device__ __forceinline__ long long fixed62(double x, int e) {
   const long long b = __double_as_longlong(x);
@@ -446,200 +435,263 @@ __device__ __forceinline__ int digits8(long long f0, long long f1, long long f2,
 
 __device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(~0u, v); }
 
-// Sums and numbers of the exponents (entries of zero do not count) of the 64
-// columns of L21, gsum[0..63] and [64..127], and of the 64 rows of U12,
-// [128..191] and [192..255]: the first ctas_l CTAs a row of L21 per warp, two
-// columns per lane, the others a row of U12 each.
+// Sums and numbers of the exponents (entries of zero do not count) of the 128
+// real columns of L21 (real and imaginary parts alternating), gsum[0..127] and
+// [128..255], and of the 64 rows of U12 (of the larger part), [256..319] and
+// [320..383]: the first ctas_l CTAs a row of L21 per warp, two complex columns
+// per lane, the others a row of U12 each.
+constexpr int kOzSums = 384;
 __global__ void __launch_bounds__(256) oz_scale_kernel(const zd* __restrict__ A, int64_t lda, int k0, int m,
                                                        int* __restrict__ gsum, int ctas_l) {
-  __shared__ int red[2][64];
+  __shared__ int red[256];
   grid_wait();
   grid_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < 128) red[threadIdx.x >> 6][threadIdx.x & 63] = 0;
+  red[threadIdx.x] = 0;
   __syncthreads();
-  int s[2] = {0, 0}, c[2] = {0, 0};
-  auto add = [&](zd v, int p) {
-    const int e = max(exp_above(v.re), exp_above(v.im));
+  int s[4] = {}, c[4] = {};
+  auto add = [&](int e, int i) {
     if (e > -4096 && e < kBadExp) {
-      s[p] += e;
-      ++c[p];
+      s[i] += e;
+      ++c[i];
     }
   };
   if ((int)blockIdx.x < ctas_l) {
     for (int r = blockIdx.x * 8 + warp; r < m; r += ctas_l * 8)
 #pragma unroll
-      for (int p = 0; p < 2; ++p) add(A[(int64_t)(k0 + 64 + r) * lda + k0 + 2 * lane + p], p);
+      for (int p = 0; p < 2; ++p) {
+        const zd v = A[(int64_t)(k0 + 64 + r) * lda + k0 + 2 * lane + p];
+        add(exp_above(v.re), 2 * p);
+        add(exp_above(v.im), 2 * p + 1);
+      }
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      atomicAdd(&red[0][2 * lane + p], s[p]);
-      atomicAdd(&red[1][2 * lane + p], c[p]);
+    for (int i = 0; i < 4; ++i) {
+      atomicAdd(&red[4 * lane + i], s[i]);
+      atomicAdd(&red[128 + 4 * lane + i], c[i]);
     }
     __syncthreads();
-    if (threadIdx.x < 128) atomicAdd(&gsum[threadIdx.x], red[threadIdx.x >> 6][threadIdx.x & 63]);
+    atomicAdd(&gsum[threadIdx.x], red[threadIdx.x]);
   } else {
     const int t = blockIdx.x - ctas_l;
     const zd* row = A + (int64_t)(k0 + t) * lda + k0 + 64;
-    for (int i = threadIdx.x; i < m; i += 256) add(row[i], 0);
+    for (int i = threadIdx.x; i < m; i += 256) add(max(exp_above(row[i].re), exp_above(row[i].im)), 0);
     s[0] = __reduce_add_sync(~0u, s[0]);
     c[0] = __reduce_add_sync(~0u, c[0]);
     if (lane == 0) {
-      atomicAdd(&gsum[128 + t], s[0]);
-      atomicAdd(&gsum[192 + t], c[0]);
+      atomicAdd(&gsum[256 + t], s[0]);
+      atomicAdd(&gsum[320 + t], c[0]);
     }
   }
 }
 
-// the power of two that column t of L21 is multiplied and row t of U12 divided
-// by; where one of the two is empty, one that takes the other out of the way
-__device__ __forceinline__ int oz_balance(const int* __restrict__ gsum, int t) {
-  const int cl = gsum[64 + t], cu = gsum[192 + t];
-  if (!cl || !cu) return cl ? -2500 : 2500;
-  return (int)rintf(0.5f * ((float)gsum[128 + t] / (float)cu - (float)gsum[t] / (float)cl));
+// the powers of two that the real and the imaginary part of column t of L21 are
+// multiplied, and the matching parts of row t of U12 divided by; where one of
+// the two is empty, one that takes the other out of the way
+__device__ __forceinline__ void oz_balance(const int* __restrict__ gsum, int t, int& gr, int& gi) {
+  const int cr = gsum[128 + 2 * t], ci = gsum[129 + 2 * t], cu = gsum[320 + t];
+  if ((!cr && !ci) || !cu) {
+    gr = gi = cr || ci ? -2500 : 2500;
+    return;
+  }
+  // means as whole numbers and fractions, so that a matrix scaled by an even power of two takes the same digits
+  struct Mean {
+    int q;
+    float f;  // 0 <= f < 1
+  };
+  auto mean = [](int sum, int n) {
+    int q = sum / n, r = sum - q * n;
+    if (r < 0) {
+      r += n;
+      --q;
+    }
+    return Mean{q, (float)r / (float)n};
+  };
+  const Mean u = mean(gsum[256 + t], cu), ar = mean(gsum[2 * t], max(cr, 1)), ai = mean(gsum[2 * t + 1], max(ci, 1));
+  const bool re = cr && (!ci || ar.q > ai.q || (ar.q == ai.q && ar.f >= ai.f));  // the part with the larger mean
+  const Mean al = re ? ar : ai;
+  const int d = u.q - al.q, b = (d >> 1) + (int)floorf(0.5f * ((float)(d & 1) + (u.f - al.f)) + 0.5f);
+  auto above = [&](Mean a) { return al.q - a.q + (int)floorf(al.f - a.f + 0.5f); };
+  gr = cr ? b + above(ar) : b;
+  gi = ci ? b + above(ai) : b;
 }
 
-// the exponent and the biased fixed-point fractions of four values (two k's)
-// of a row of A or a column of B, each held by one warp; sg: the sign with
-// which the balance enters. Returns the exponent of the row or column.
-__device__ __forceinline__ int oz_fixed(const double (&x)[4], const int (&g)[2], int sg, long long (&f)[4]) {
+// the exponent and the biased fixed-point fractions of four values (two complex
+// inner indices) of a row of A or a column of B, each held by one warp; sg: the
+// sign with which the balance enters. Returns the exponent of the row or column.
+__device__ __forceinline__ int oz_fixed(const double (&x)[4], const int (&g)[4], int sg, long long (&f)[4]) {
   int e = -(1 << 19);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int xe = exp_above(x[i]);
-    e = max(e, xe >= kBadExp ? kBadExp + (1 << 18) : xe + sg * g[i >> 1]);
+    e = max(e, xe >= kBadExp ? kBadExp + (1 << 18) : xe + sg * g[i]);
   }
   e = warp_max(e);
   const bool bad = e >= kBadExp;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) f[i] = bad ? 0 : fixed62(x[i], e - sg * g[i >> 1]);
-  return bad ? kBadExp : max(e, -20000);  // -20000: nothing but zeros, which the slices hold whatever C is
+  for (int i = 0; i < 4; ++i) f[i] = bad ? 0 : fixed62(x[i], e - sg * g[i]);
+  return bad ? kBadExp : max(e, -20000);  // -20000: nothing but zeros
 }
 
-// Slices of L21 (rows k0 + 64 .. n - 1 of the columns k0 .. k0 + 63; one row
-// per warp, two k's per lane) and of U12 (the rows k0 .. k0 + 63 of the columns
-// right of the block; 32 columns per CTA through shared memory).
+// Sets of a row's (column's) 128 inner indices: those whose entries are within
+// 2^-D of the row's exponent e, D = 1, 3, 5, 7 (a column: 6, 4, 2, 0), and
+// those that are not zero; 20 words, word l returned in lane l. Two sets of the
+// same place share an index only if its product is within 2^-7 of both
+// exponents, and two do if it is within 2^-6.
+constexpr int kSets = 5;
+template <bool ROW>
+__device__ __forceinline__ unsigned oz_sets(const double (&x)[4], const int (&g)[4], int e) {
+  const int lane = threadIdx.x & 31;
+  unsigned w = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int d = e >= kBadExp ? 1 << 20 : e - (exp_above(x[i]) + (ROW ? g[i] : -g[i]));
+#pragma unroll
+    for (int k = 0; k < kSets; ++k) {
+      const unsigned b = __ballot_sync(~0u, k == kSets - 1 ? x[i] != 0.0 : d <= (ROW ? 2 * k + 1 : 6 - 2 * k));
+      if (lane == 4 * k + i) w = b;
+    }
+  }
+  return w;
+}
+// whether the first four sets of a row and a column meet
+__device__ __forceinline__ unsigned oz_meet(uint4 a, uint4 b) {
+  return (a.x & b.x) | (a.y & b.y) | (a.z & b.z) | (a.w & b.w);
+}
+
+// Slices and sets of L21 (rows k0 + 64 .. n - 1 of the columns k0 .. k0 + 63; a row
+// per warp at a time, two k's per lane) and of U12 (the rows k0 .. k0 + 63 of the columns
+// right of the block; kPackC columns per CTA through shared memory: two real
+// columns a warp, as a column is a long chain. All of N = 546 / 5943 with their sums: 0.10 / 1.9 ms,
+// 0.16 / 3.7 ms with 32 columns per CTA).
+constexpr int kPackC = 8;
 __global__ void __launch_bounds__(256) oz_pack_kernel(const zd* __restrict__ A, int64_t lda, int k0, int m,
                                                       const int* __restrict__ gsum, uint2* __restrict__ Aq,
                                                       uint2* __restrict__ Bq, int* __restrict__ ea,
-                                                      int* __restrict__ eb, int* __restrict__ xa,
-                                                      int* __restrict__ xb, int ctas_a) {
+                                                      int* __restrict__ eb, unsigned* __restrict__ xa,
+                                                      unsigned* __restrict__ xb, int ctas_a) {
   grid_wait();
   grid_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = k0 + 64;
-  const int g[2] = {oz_balance(gsum, 2 * lane), oz_balance(gsum, 2 * lane + 1)};
+  int g[4];
+  oz_balance(gsum, 2 * lane, g[0], g[1]);
+  oz_balance(gsum, 2 * lane + 1, g[2], g[3]);
   double x[4];
   long long f[4];
   if ((int)blockIdx.x < ctas_a) {
-    const int r = blockIdx.x * 8 + warp;
-    if (r >= m) return;
+    for (int r = blockIdx.x * 8 + warp; r < m; r += 8 * ctas_a) {
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      const zd v = A[(int64_t)(c0 + r) * lda + k0 + 2 * lane + p];
-      x[2 * p] = v.re;
-      x[2 * p + 1] = -v.im;
+      for (int p = 0; p < 2; ++p) {
+        const zd v = A[(int64_t)(c0 + r) * lda + k0 + 2 * lane + p];
+        x[2 * p] = v.re;
+        x[2 * p + 1] = -v.im;
+      }
+      const int e = oz_fixed(x, g, 1, f);
+      const unsigned w = oz_sets<true>(x, g, e);
+      if (lane == 0) ea[r] = e;
+      if (lane < 4 * kSets) xa[(int64_t)r * 4 * kSets + lane] = w;
+#pragma unroll
+      for (int d = 0; d < kDig; ++d)
+        Aq[((int64_t)d * m + r) * 32 + lane] =
+            make_uint2(digit16(f[0], d) | digit16(f[1], d) << 16, digit16(f[2], d) | digit16(f[3], d) << 16);
     }
-    const int e = oz_fixed(x, g, 1, f);
-    if (lane == 0) ea[r] = e;
-    xa[(int64_t)r * 32 + lane] = oz_pair(x);
-#pragma unroll
-    for (int d = 0; d < kDig; ++d)
-      Aq[((int64_t)d * m + r) * 32 + lane] =
-          make_uint2(digit16(f[0], d) | digit16(f[1], d) << 16, digit16(f[2], d) | digit16(f[3], d) << 16);
     return;
   }
-  __shared__ double us[64][66];  // 32 columns of U12, re / im alternating
-  const int cb = (blockIdx.x - ctas_a) * 32, nc = m;  // as many columns as rows
-  for (int e = threadIdx.x; e < 64 * 32; e += 256) {
-    const int t = e >> 5, c = e & 31;
+  __shared__ double us[64][2 * kPackC + 2];  // columns of U12, re / im alternating
+  const int cb = (blockIdx.x - ctas_a) * kPackC, nc = m;  // as many columns as rows
+  for (int e = threadIdx.x; e < 64 * kPackC; e += 256) {
+    const int t = e / kPackC, c = e % kPackC;
     const zd v = cb + c < nc ? A[(int64_t)(k0 + t) * lda + c0 + cb + c] : zd();
     us[t][2 * c] = v.re;
     us[t][2 * c + 1] = v.im;
   }
   __syncthreads();
   const int n2 = 2 * nc;
-  for (int c = warp; c < 32 && cb + c < nc; c += 8) {
+  for (int j = warp; j < 2 * kPackC && cb + (j >> 1) < nc; j += 8) {  // real columns: (re, im) and (im, -re)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = us[2 * lane + (i >> 1)][2 * c + (i & 1)];
-    const int e = oz_fixed(x, g, -1, f);
-    if (lane == 0) eb[cb + c] = e;
-    xb[(int64_t)(cb + c) * 32 + lane] = oz_pair(x);
-#pragma unroll
-    for (int d = 0; d < kDig; ++d) {  // rows (re, im) and (im, -re)
-      const uint32_t i0 = digit16(f[1], d), i1 = digit16(f[3], d);
-      const int64_t row = ((int64_t)d * n2 + 2 * (cb + c)) * 32 + lane;
-      Bq[row] = make_uint2(digit16(f[0], d) | i0 << 16, digit16(f[2], d) | i1 << 16);
-      Bq[row + 32] = make_uint2(i0 | digit16(-f[0], d) << 16, i1 | digit16(-f[2], d) << 16);
+    for (int i = 0; i < 4; ++i) {
+      const double v = us[2 * lane + (i >> 1)][(j & ~1) + ((i ^ j) & 1)];
+      x[i] = i & j & 1 ? -v : v;
     }
+    const int e = oz_fixed(x, g, -1, f);
+    const unsigned w = oz_sets<false>(x, g, e);
+    const int64_t col = 2 * cb + j;
+    if (lane == 0) eb[col] = e;
+    if (lane < 4 * kSets) xb[col * 4 * kSets + lane] = w;
+#pragma unroll
+    for (int d = 0; d < kDig; ++d)
+      Bq[((int64_t)d * n2 + col) * 32 + lane] =
+          make_uint2(digit16(f[0], d) | digit16(f[1], d) << 16, digit16(f[2], d) | digit16(f[3], d) << 16);
   }
 }
 
-// The entries of C that the slices do not hold (see the head of this file). A
-// CTA takes 32 rows and 64 columns, a lane a row and a warp 8 columns: small
-// tiles, as such entries come in clusters and the last blocks are small. The
-// largest product's exponent is a maximum over sums of packed exponents, two
-// inner indices per instruction; C is read where that does not reach. The entries
-// left are listed and updated here, eight lanes each, and marked for
-// oz_gemm_kernel to leave alone. (In that kernel's own epilogue, which bounds it,
-// the test took 23 ms of a factorisation of N = 5943, here 4 ms.)
+// The real entries of C that the slices do not hold (see the head of this file).
+// A CTA takes 32 rows and 64 complex columns, a lane a row and a warp 8 columns:
+// small tiles, as such entries come in clusters and the last blocks are small. C is
+// read where no product reaches. The entries left are listed and updated here,
+// four lanes each, and marked for oz_gemm_kernel to leave alone. The test takes 3.6 ms
+// of a factorisation of N = 5943 (4.4 ms with sums of packed exponents for both parts together, 23 ms with these
+// in oz_gemm_kernel's epilogue, which bounds that kernel), the entries of the LPF's matrix 6.4 ms. With eight
+// lanes an entry 6.9 ms, and the entries of 1543 potentials in random order 6.5 instead of 6.0 ms.
 constexpr int kDirR = 32, kDirC = 64;
 
 __global__ void __launch_bounds__(256) oz_direct_kernel(zd* A, int64_t lda, int k0, int m, const int* __restrict__ ea,
-                                                        const int* __restrict__ eb, const int* __restrict__ xa,
-                                                        const int* __restrict__ xb, uint8_t* __restrict__ mask) {
-  __shared__ uint4 xs[kDirC][8], xr[kDirR][9];  // the columns' and the rows' exponents
-  __shared__ int es[kDirC];
-  __shared__ unsigned short list[kDirR * kDirC];
+                                                        const int* __restrict__ eb, const uint4* __restrict__ xa,
+                                                        const uint4* __restrict__ xb, uint16_t* __restrict__ mask) {
+  __shared__ uint4 xs[2 * kDirC][kSets], xr[kDirR][kSets];  // the columns' and the rows' sets
+  __shared__ int es[2 * kDirC];
+  __shared__ unsigned short list[kDirR * 2 * kDirC];
   __shared__ int nlist;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = k0 + 64;
   const int r0 = blockIdx.y * kDirR, cb = blockIdx.x * kDirC;
   grid_wait();
   grid_trigger();
   if (threadIdx.x == 0) nlist = 0;
-  for (int e = threadIdx.x; e < kDirC * 8; e += 256)
-    xs[e >> 3][e & 7] = cb + (e >> 3) < m ? reinterpret_cast<const uint4*>(xb)[(int64_t)cb * 8 + e] : uint4();
-  if (threadIdx.x < kDirC) es[threadIdx.x] = cb + (int)threadIdx.x < m ? eb[cb + threadIdx.x] : 0;
-  const int row = min(r0 + lane, m - 1), er = ea[row];
-  {
-    const int r = threadIdx.x >> 3, k = threadIdx.x & 7;
-    xr[r][k] = reinterpret_cast<const uint4*>(xa)[(int64_t)min(r0 + r, m - 1) * 8 + k];
+  for (int e = threadIdx.x; e < 2 * kDirC * kSets; e += 256)
+    xs[e / kSets][e % kSets] = 2 * cb + e / kSets < 2 * m ? xb[(int64_t)cb * 2 * kSets + e] : uint4();
+  if (threadIdx.x < 2 * kDirC) es[threadIdx.x] = 2 * cb + (int)threadIdx.x < 2 * m ? eb[2 * cb + threadIdx.x] : 0;
+  if (threadIdx.x < kDirR * kSets) {
+    const int r = threadIdx.x / kSets, k = threadIdx.x % kSets;
+    xr[r][k] = xa[(int64_t)min(r0 + r, m - 1) * kSets + k];
   }
   __syncthreads();
-  uint4 x[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) x[k] = xr[lane][k];
+  const int row = min(r0 + lane, m - 1), er = ea[row];
+  const uint4 x0 = xr[lane][0], x1 = xr[lane][1], x2 = xr[lane][2], x3 = xr[lane][3];
   const int cw = 8 * warp, nj = min(8, m - cb - cw);
   unsigned bits = 0;
-  for (int c = 0; c < nj; ++c) {
-    unsigned t0 = kTopNone, t1 = kTopNone;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint4 u = xs[cw + c][k];
-      t0 = oz_top(x[k].x, u.x, oz_top(x[k].y, u.y, t0));
-      t1 = oz_top(x[k].z, u.z, oz_top(x[k].w, u.w, t1));
-    }
-    if (!oz_p_holds(__vmaxs2(t0, t1), er, es[cw + c])) bits |= 1u << c;
+#pragma unroll 4
+  for (int j = 0; j < 2 * nj; ++j) {
+    const uint4* u = xs[2 * cw + j];
+    if (!(oz_meet(x0, u[0]) | oz_meet(x1, u[1]) | oz_meet(x2, u[2]) | oz_meet(x3, u[3]))) bits |= 1u << j;
   }
   if (r0 + lane >= m) bits = 0;
   if (bits) {
+    const uint4 nz = xr[lane][kSets - 1];
     const int4* z = reinterpret_cast<const int4*>(A + (int64_t)(c0 + row) * lda + c0 + cb + cw);
 #pragma unroll
     for (int c = 0; c < 8; ++c)
-      if (bits >> c & 1) {
+      if (bits >> 2 * c & 3) {
         const int4 v = z[c];
-        if (oz_c_holds(v.y, v.w, er, es[cw + c])) bits &= ~(1u << c);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const int j = 2 * (cw + c) + p, ec = es[j];
+          // no common inner index: the digit products are all zero, and so is the sum
+          if (oz_c_holds(p ? v.w : v.y, er, ec) || (er < kBadExp && ec < kBadExp && !oz_meet(nz, xs[j][kSets - 1])))
+            bits &= ~(1u << (2 * c + p));
+        }
       }
   }
   if (bits) {
     int at = atomicAdd(&nlist, __popc(bits));
-    for (unsigned b = bits; b; b &= b - 1) list[at++] = (unsigned short)(lane * kDirC + cw + __ffs(b) - 1);
+    for (unsigned b = bits; b; b &= b - 1) list[at++] = (unsigned short)(lane * 2 * kDirC + 2 * cw + __ffs(b) - 1);
   }
-  if (r0 + lane < m && nj > 0) mask[(int64_t)((cb + cw) / 8) * m + row] = (uint8_t)bits;
+  if (r0 + lane < m && nj > 0) mask[(int64_t)((cb + cw) / 8) * m + row] = (uint16_t)bits;
   __syncthreads();
-  for (int e0 = 4 * warp; e0 < nlist; e0 += 32) {
-    const int e = min(e0 + (lane >> 3), nlist - 1), r = c0 + r0 + list[e] / kDirC, c = c0 + cb + list[e] % kDirC;
-    const zd s = oz_dot(A + (int64_t)r * lda + k0, A + (int64_t)k0 * lda + c, lda, lane & 7);
-    zd* z = A + (int64_t)r * lda + c;
-    if ((lane & 7) == 0 && e == e0 + (lane >> 3)) *z = *z - s;
+  for (int e0 = kDots * warp; e0 < nlist; e0 += 8 * kDots) {
+    const int e = min(e0 + lane / kDot, nlist - 1), r = c0 + r0 + list[e] / (2 * kDirC), j = list[e] % (2 * kDirC);
+    const int c = c0 + cb + (j >> 1);
+    const double s = oz_dot(A + (int64_t)r * lda + k0, A + (int64_t)k0 * lda + c, lda, lane % kDot, j & 1);
+    double* z = reinterpret_cast<double*>(A + (int64_t)r * lda + c) + (j & 1);
+    if (lane % kDot == 0 && e == e0 + lane / kDot) *z -= s;
   }
 }
 
@@ -655,15 +707,17 @@ constexpr size_t kSimtSmem = sizeof(int) * (kSimtR + 2 * kSimtC) * kSimtLd;
 __global__ void __launch_bounds__(256) oz_simt_kernel(zd* __restrict__ A, int64_t lda, int k0, int m,
                                                       const int* __restrict__ gsum) {
   extern __shared__ __align__(16) int simt_smem[];
-  __shared__ int ea[kSimtR], eb[kSimtC];
-  __shared__ unsigned xa[kSimtR][33], xb[kSimtC][33];    // the entries' exponents
-  __shared__ unsigned short list[kSimtR * kSimtC];        // entries for fp64 multiply-adds
+  __shared__ int ea[kSimtR], eb[2 * kSimtC];
+  __shared__ uint4 xa[kSimtR][kSets], xb[2 * kSimtC][kSets];  // the rows' and columns' sets
+  __shared__ unsigned short list[kSimtR * 2 * kSimtC];    // entries for fp64 multiply-adds
   __shared__ int nlist;
   int* As = simt_smem;                  // [row][digit][32 words of four k's]
   int* Bs = As + kSimtR * kSimtLd;      // [real column][digit][32 words]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = k0 + 64;
   const int r0 = blockIdx.y * kSimtR, cb = blockIdx.x * kSimtC;
-  const int g[2] = {oz_balance(gsum, 2 * lane), oz_balance(gsum, 2 * lane + 1)};
+  int g[4];
+  oz_balance(gsum, 2 * lane, g[0], g[1]);
+  oz_balance(gsum, 2 * lane + 1, g[2], g[3]);
   double x[4];
   long long f[4];
   if (threadIdx.x == 0) nlist = 0;
@@ -675,25 +729,29 @@ __global__ void __launch_bounds__(256) oz_simt_kernel(zd* __restrict__ A, int64_
       x[2 * p + 1] = -v.im;
     }
     const int e = oz_fixed(x, g, 1, f);
+    const unsigned w = oz_sets<true>(x, g, e);
     if (lane == 0) ea[r] = e;
-    xa[r][lane] = oz_pair(x);
+    if (lane < 4 * kSets) reinterpret_cast<unsigned*>(xa[r])[lane] = w;
 #pragma unroll
     for (int d = 0; d < kDig; ++d) As[r * kSimtLd + d * 32 + lane] = digits8(f[0], f[1], f[2], f[3], d);
   }
   for (int c = warp; c < kSimtC; c += 8) {
+    zd v[2];
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      const zd v = cb + c < m ? A[(int64_t)(k0 + 2 * lane + p) * lda + c0 + cb + c] : zd();
-      x[2 * p] = v.re;
-      x[2 * p + 1] = v.im;
-    }
-    const int e = oz_fixed(x, g, -1, f);
-    if (lane == 0) eb[c] = e;
-    xb[c][lane] = oz_pair(x);
+    for (int p = 0; p < 2; ++p) v[p] = cb + c < m ? A[(int64_t)(k0 + 2 * lane + p) * lda + c0 + cb + c] : zd();
 #pragma unroll
-    for (int d = 0; d < kDig; ++d) {
-      Bs[(2 * c) * kSimtLd + d * 32 + lane] = digits8(f[0], f[1], f[2], f[3], d);
-      Bs[(2 * c + 1) * kSimtLd + d * 32 + lane] = digits8(f[1], -f[0], f[3], -f[2], d);
+    for (int q = 0; q < 2; ++q) {  // real columns: (re, im) and (im, -re)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        x[2 * p] = q ? v[p].im : v[p].re;
+        x[2 * p + 1] = q ? -v[p].re : v[p].im;
+      }
+      const int e = oz_fixed(x, g, -1, f);
+      const unsigned w = oz_sets<false>(x, g, e);
+      if (lane == 0) eb[2 * c + q] = e;
+      if (lane < 4 * kSets) reinterpret_cast<unsigned*>(xb[2 * c + q])[lane] = w;
+#pragma unroll
+      for (int d = 0; d < kDig; ++d) Bs[(2 * c + q) * kSimtLd + d * 32 + lane] = digits8(f[0], f[1], f[2], f[3], d);
     }
   }
   __syncthreads();
@@ -739,25 +797,28 @@ __global__ void __launch_bounds__(256) oz_simt_kernel(zd* __restrict__ A, int64_
         }
         v[p] = oz_join(w[0], w[1]);
       }
-      zd* z = A + (int64_t)(c0 + r) * lda + c0 + c;
-      const zd cz = *z;
-      const int rl = tr + 16 * i, er = ea[rl], ec = eb[cl];
-      bool holds = oz_c_holds(__double2hiint(cz.re), __double2hiint(cz.im), er, ec);
-      if (!holds) {
-        unsigned top = kTopNone;
-        for (int k = 0; k < 32; ++k) top = oz_top(xa[rl][k], xb[cl][k], top);
-        holds = oz_p_holds(top, er, ec);
+      double* z = reinterpret_cast<double*>(A + (int64_t)(c0 + r) * lda + c0 + c);
+      const int rl = tr + 16 * i, er = ea[rl];
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int j = 2 * cl + p, ec = eb[j];
+        const double cz = z[p];
+        const bool holds = (oz_meet(xa[rl][0], xb[j][0]) | oz_meet(xa[rl][1], xb[j][1]) | oz_meet(xa[rl][2], xb[j][2]) |
+                            oz_meet(xa[rl][3], xb[j][3])) ||
+                           oz_c_holds(__double2hiint(cz), er, ec) ||
+                           (er < kBadExp && ec < kBadExp && !oz_meet(xa[rl][kSets - 1], xb[j][kSets - 1]));
+        if (holds) z[p] = oz_apply(cz, v[p], er, ec);
+        else list[atomicAdd(&nlist, 1)] = (unsigned short)(rl * 2 * kSimtC + j);
       }
-      if (holds) *z = oz_apply(cz, v[0], v[1], er, ec);
-      else list[atomicAdd(&nlist, 1)] = (unsigned short)(rl * kSimtC + cl);
     }
   }
   __syncthreads();
-  for (int e0 = 4 * warp; e0 < nlist; e0 += 32) {  // eight lanes an entry, as the tensor cores' form
-    const int e = min(e0 + (lane >> 3), nlist - 1), r = c0 + r0 + list[e] / kSimtC, c = c0 + cb + list[e] % kSimtC;
-    const zd s = oz_dot(A + (int64_t)r * lda + k0, A + (int64_t)k0 * lda + c, lda, lane & 7);
-    zd* z = A + (int64_t)r * lda + c;
-    if ((lane & 7) == 0 && e == e0 + (lane >> 3)) *z = *z - s;
+  for (int e0 = kDots * warp; e0 < nlist; e0 += 8 * kDots) {  // as the tensor cores' form
+    const int e = min(e0 + lane / kDot, nlist - 1), r = c0 + r0 + list[e] / (2 * kSimtC), j = list[e] % (2 * kSimtC);
+    const int c = c0 + cb + (j >> 1);
+    const double s = oz_dot(A + (int64_t)r * lda + k0, A + (int64_t)k0 * lda + c, lda, lane % kDot, j & 1);
+    double* z = reinterpret_cast<double*>(A + (int64_t)r * lda + c) + (j & 1);
+    if (lane % kDot == 0 && e == e0 + lane / kDot) *z -= s;
   }
 }
 
@@ -791,7 +852,7 @@ int oz_map(CUtensorMap* map, const void* ptr, int rows, int box_rows) {
 }
 
 // operand buffer of an n x n factorisation: header, per block the sums and numbers of the exponents of its
-// columns, row and column exponents, all entries' exponents, the marks of oz_direct_kernel, the slices of L21 and U12
+// columns, row and column exponents, rows' and columns' sets, the marks of oz_direct_kernel, the slices of L21 and U12
 struct OzLayout {
   size_t gsum, ea, eb, xa, xb, mask, aq, bq, total;
 };
@@ -800,12 +861,12 @@ OzLayout oz_layout(int n) {
   const size_t m = (size_t)std::max(n, 1);
   OzLayout l;
   l.gsum = kOzHeader;
-  l.ea = l.gsum + up(sizeof(int) * 256 * ((m + 63) / 64));
+  l.ea = l.gsum + up(sizeof(int) * kOzSums * ((m + 63) / 64));
   l.eb = l.ea + up(sizeof(int) * m);
-  l.xa = l.eb + up(sizeof(int) * m);
-  l.xb = l.xa + up(sizeof(int) * 32 * m);
-  l.mask = l.xb + up(sizeof(int) * 32 * m);
-  l.aq = l.mask + up(m * ((m + 7) / 8));
+  l.xa = l.eb + up(sizeof(int) * 2 * m);
+  l.xb = l.xa + up(16 * kSets * m);
+  l.mask = l.xb + up(16 * kSets * 2 * m);
+  l.aq = l.mask + up(sizeof(uint16_t) * m * ((m + 7) / 8));
   l.bq = l.aq + up(kDig * m * kOzK * 2);
   l.total = l.bq + up(kDig * 2 * m * kOzK * 2);
   return l;
@@ -821,13 +882,13 @@ int lu_oz_prepare(m25_ctx* ctx, int n) {
   return M25_OK;
 }
 
-// the sums that balance the block at k0 (gsum: 256 ints, zero)
+// the sums that balance the block at k0 (gsum: kOzSums ints, zero)
 static cudaError_t oz_scale(m25_ctx* ctx, const zd* A, int64_t lda, int k0, int m, int* gsum) {
   const int cl = std::min((m + 7) / 8, ctx->num_sms);
   return launch_chained(oz_scale_kernel, dim3(cl + 64), 256, 0, ctx->stream, A, lda, k0, m, gsum, cl);
 }
 
-// A22 -= L21 U12 after the block of 64 columns at k0 on the CUDA cores; work: 1 KB on the device
+// A22 -= L21 U12 after the block of 64 columns at k0 on the CUDA cores; work: 1.5 KB on the device
 int lu_oz_update_simt(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0, void* work) {
   const int m = n - k0 - 64;
   if (m <= 0) return M25_OK;
@@ -839,7 +900,7 @@ int lu_oz_update_simt(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0, void* wor
   }
   int* gsum = static_cast<int*>(work);
   StageTimer tm(ctx, ST_GEMM);
-  M25_CUDA(cudaMemsetAsync(gsum, 0, 256 * sizeof(int), ctx->stream));
+  M25_CUDA(cudaMemsetAsync(gsum, 0, kOzSums * sizeof(int), ctx->stream));
   M25_CUDA(oz_scale(ctx, A, lda, k0, m, gsum));
   oz_simt_kernel<<<dim3((m + kSimtC - 1) / kSimtC, (m + kSimtR - 1) / kSimtR), 256, kSimtSmem, ctx->stream>>>(
       A, lda, k0, m, gsum);
@@ -857,12 +918,12 @@ int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0) {
     return M25_ERR_VALUE;
   }
   char* b = ctx->Dw.as<char>();
-  int* gsum = reinterpret_cast<int*>(b + l.gsum) + 256 * (k0 / 64);
+  int* gsum = reinterpret_cast<int*>(b + l.gsum) + kOzSums * (k0 / 64);
   int* ea = reinterpret_cast<int*>(b + l.ea);
   int* eb = reinterpret_cast<int*>(b + l.eb);
-  int* xa = reinterpret_cast<int*>(b + l.xa);
-  int* xb = reinterpret_cast<int*>(b + l.xb);
-  uint8_t* mask = reinterpret_cast<uint8_t*>(b + l.mask);
+  unsigned* xa = reinterpret_cast<unsigned*>(b + l.xa);
+  unsigned* xb = reinterpret_cast<unsigned*>(b + l.xb);
+  uint16_t* mask = reinterpret_cast<uint16_t*>(b + l.mask);
   uint2* aq = reinterpret_cast<uint2*>(b + l.aq);
   uint2* bq = reinterpret_cast<uint2*>(b + l.bq);
   cudaStream_t st = ctx->stream;
@@ -878,7 +939,7 @@ int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0) {
   {
     StageTimer tm(ctx, ST_PACK);
     M25_CUDA(oz_scale(ctx, A, lda, k0, m, gsum));
-    const int ca = (m + 7) / 8, cb = (m + 31) / 32;
+    const int ca = std::min((m + 7) / 8, 2 * ctx->num_sms), cb = (m + kPackC - 1) / kPackC;
     M25_CUDA(launch_chained(oz_pack_kernel, dim3(ca + cb), 256, 0, st, A, lda, k0, m, gsum, aq, bq, ea, eb, xa, xb,
                             ca));
   }
@@ -895,7 +956,7 @@ int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0) {
   g.err = reinterpret_cast<int*>(b);
   StageTimer tm(ctx, ST_GEMM);
   M25_CUDA(launch_chained(oz_direct_kernel, dim3((m + kDirC - 1) / kDirC, (m + kDirR - 1) / kDirR), 256, 0, st, A, lda, k0,
-                          m, ea, eb, xa, xb, mask));
+                          m, ea, eb, reinterpret_cast<const uint4*>(xa), reinterpret_cast<const uint4*>(xb), mask));
   M25_CUDA(launch_chained(oz_gemm_kernel, dim3(std::min(g.ntiles, ctx->num_sms)), kOzThreads, kOzSmem, st, ma, mb, g));
   return M25_OK;
 }

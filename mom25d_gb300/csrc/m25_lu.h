@@ -38,7 +38,7 @@ int lu_strip_block(m25_ctx* ctx, cx<T>* A, int64_t lda, int n, int b0, int bw, i
 // lu_oz.cu: the complex128 trailing update of a block of 64 columns on the tensor cores
 int lu_oz_prepare(m25_ctx* ctx, int n);
 int lu_oz_update(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0);
-// the same on the CUDA cores, bit for bit (work: 1 KB on the device)
+// the same on the CUDA cores, bit for bit (work: 1.5 KB on the device)
 int lu_oz_update_simt(m25_ctx* ctx, zd* A, int64_t lda, int n, int k0, void* work);
 
 }  // namespace m25

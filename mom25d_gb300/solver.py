@@ -827,7 +827,7 @@ class Solver:
             b += b // 4                                 # the near pairs' fp64 values (Hn), a bound
         if self.precision == "fp64":
             b += 16 * N * N                             # Z, factored in place
-            b += 6500 * N + N * N // 8                  # the LU update's integer slices and marks
+            b += 6600 * N + N * N // 4                  # the LU update's integer slices, sets and marks
         else:
             b += 24 * N * (N + 1)                       # Zh, Zl, complex64 LU
             if nv or self.precision == "mixed_fill32":
